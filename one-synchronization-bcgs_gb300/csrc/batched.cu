@@ -61,7 +61,7 @@ struct Mat {
     int ldR;
     int cls;
     // workspace
-    double *G1, *G2, *Scol, *Sd, *Yd, *part, *tsqr;
+    double *G1, *G2, *Scol[2], *Sd[2], *Yd, *part, *tsqr;   // Scol, Sd: this step's and the next one's
     int* status;
 };
 
@@ -93,7 +93,7 @@ struct Blob {
     }
 };
 
-i64 small_block_doubles(int n, int s) { return 2LL * (n + s) * 2 * s + (i64)n * s + 3LL * s * s + 64; }
+i64 small_block_doubles(int n, int s) { return 2LL * (n + s) * 2 * s + 2LL * n * s + 3LL * s * s + 64; }
 
 i64 tsqr_doubles(i64 m, int s) { return tsqr_workspace_doubles(m, s); }
 
@@ -149,10 +149,11 @@ size_t layout_workspace(BatchPlan& P, char* base) {
         const int n = M.n, s = M.s;
         M.G1 = sb;
         M.G2 = sb ? M.G1 + (i64)(n + s) * 2 * s : nullptr;
-        M.Scol = sb ? M.G2 + (i64)(n + s) * 2 * s : nullptr;
-        double* S0 = sb ? M.Scol + (i64)n * s : nullptr;
-        M.Sd = sb ? S0 + (i64)s * s : nullptr;
-        M.Yd = sb ? M.Sd + (i64)s * s : nullptr;
+        M.Scol[0] = sb ? M.G2 + (i64)(n + s) * 2 * s : nullptr;
+        M.Scol[1] = sb ? M.Scol[0] + (i64)n * s : nullptr;
+        M.Sd[0] = sb ? M.Scol[1] + (i64)n * s : nullptr;
+        M.Sd[1] = sb ? M.Sd[0] + (i64)s * s : nullptr;
+        M.Yd = sb ? M.Sd[1] + (i64)s * s : nullptr;
         M.part = (double*)take((size_t)part_doubles_of(M.m, M.n, M.s) * sizeof(double));
         M.tsqr = (double*)take((size_t)tsqr_doubles(M.m, M.s) * sizeof(double));
     }
@@ -236,7 +237,7 @@ void build_schedule(BatchPlan& P, Blob& blob) {
         std::vector<int> prefix(jobs.size() + 1, 0), prefix2(jobs.size() + 1, 0);
         for (size_t j = 0; j < jobs.size(); ++j) {
             prefix[j + 1] = prefix[j] + counts[j];
-            prefix2[j + 1] = prefix2[j] + (int)ceil_div((i64)reqs[j].na * reqs[j].nb, 256);
+            prefix2[j + 1] = prefix2[j] + gram_reduce_ctas(jobs[j].na, jobs[j].nb);
         }
         S.items = prefix.back();
         S.items2 = prefix2.back();
@@ -245,7 +246,7 @@ void build_schedule(BatchPlan& P, Blob& blob) {
         S.prefix2_off = blob.put(prefix2);
         P.stages.push_back(S);
     };
-    auto add_small = [&](std::vector<SmallJob>& jobs) {
+    auto add_small = [&](std::vector<StepJob>& jobs) {
         if (jobs.empty()) return;
         std::vector<int> counts(jobs.size(), 1);
         add_prefixed(kStSmall, jobs, counts, 0);
@@ -256,25 +257,13 @@ void build_schedule(BatchPlan& P, Blob& blob) {
         for (const UpdJob& J : jobs) counts.push_back((int)ceil_div(J.m, 128));
         add_prefixed(kStUpd, jobs, counts, 0);
     };
-    auto pyth = [](const double* Om, int ldom, const double* A, int lda, int k, int nz, double* T, int step) {
-        SmallSub S{};
-        S.kind = kSmallPyth;
-        S.p0 = Om; S.ld0 = ldom; S.p1 = A; S.ld1 = lda; S.a = k; S.b = nz; S.out = T; S.ldo = nz; S.step = step;
-        return S;
-    };
-    auto scol = [](const double* G, int ldg, int mZ, int s, int nZ, const double* Yd, double* Scol) {
-        SmallSub S{};
-        S.kind = kSmallScol;
-        S.p0 = G; S.ld0 = ldg; S.a = mZ; S.b = s; S.c = nZ; S.p1 = Yd; S.ld1 = s; S.out = Scol; S.ldo = mZ + s;
-        return S;
-    };
-    auto rblock = [](int c0, int K, int ny, const double* A, int lda, const double* Bm, int ldb, const double* Sd,
-                     const double* Yd) {
-        SmallSub S{};
-        S.kind = kSmallRblock;
-        S.a = c0; S.b = K; S.c = ny; S.d = 0;
-        S.p0 = A; S.ld0 = lda; S.p1 = Bm; S.ld1 = ldb; S.p2 = Sd; S.ld2 = ny; S.p3 = Yd; S.ld3 = ny;
-        return S;
+    // T of one matrix's step (and, with nz > 0, the next block's S and Sd), without
+    // an R block.
+    auto step_job = [](const Mat& M, const double* G, int ldg, int K, int ny, double* T, int step) {
+        StepJob J;
+        J.G = G; J.ldg = ldg; J.K = K; J.ny = ny; J.T = T; J.step = step; J.status = M.status;
+        J.R = M.R; J.ldR = M.ldR;
+        return J;
     };
     auto upd = [](const Mat& M, int K, int c0, int nc, const double* S, int lds, const double* T, int ldt) {
         UpdJob J;
@@ -359,20 +348,16 @@ void build_schedule(BatchPlan& P, Blob& blob) {
             g.push_back({b, 2 * M.s, M.s, M.s, M.G2, 2 * M.s});                       // :111-114
         }
         add_gram(g);
-        std::vector<SmallJob> sj;
+        std::vector<StepJob> sj;
         for (int b = 0; b < B; ++b) {
             const Mat& M = mats[b];
-            SmallJob J{};
-            J.status = M.status; J.R = M.R; J.ldR = M.ldR;
-            J.sub[0] = pyth(M.G2 + M.s, 2 * M.s, M.G2, 2 * M.s, M.s, M.s, M.Sd, 1);     // :115-119
-            J.nsub = 1;
-            sj.push_back(J);
+            sj.push_back(step_job(M, M.G2, 2 * M.s, M.s, M.s, M.Sd[0], 1));             // :115-119
         }
         add_small(sj);
         std::vector<UpdJob> uj;
         for (int b = 0; b < B; ++b) {
             const Mat& M = mats[b];
-            uj.push_back(upd(M, M.s, M.s, M.s, M.G2, 2 * M.s, M.Sd, M.s));               // :121-124
+            uj.push_back(upd(M, M.s, M.s, M.s, M.G2, 2 * M.s, M.Sd[0], M.s));            // :121-124
         }
         add_upd(uj);
         g.clear();
@@ -388,16 +373,10 @@ void build_schedule(BatchPlan& P, Blob& blob) {
         for (int b = 0; b < B; ++b) {
             const Mat& M = mats[b];
             const int s = M.s, na = na1[b];
-            SmallJob J{};
-            J.status = M.status; J.R = M.R; J.ldR = M.ldR;
-            J.sub[0] = pyth(M.G1 + s, na, M.G1, na, s, s, M.Yd, 1);                       // :134-137
-            J.sub[1] = rblock(s, s, s, M.G2, 2 * s, M.G1, na, M.Sd, M.Yd);               // :144-147
-            J.nsub = 2;
-            if (M.p > 1) {
-                const int mScol = 2 * s;
-                J.sub[2] = scol(M.G1, na, s, s, nZ[b], M.Yd, M.Scol);                    // :155-159
-                J.sub[3] = pyth(M.G1 + mScol + (i64)s * na, na, M.Scol, mScol, mScol, nZ[b], M.Sd, 2);   // :160-171
-                J.nsub = 4;
+            StepJob J = step_job(M, M.G1, na, s, s, M.Yd, 1);                            // :134-137
+            J.mode = 0; J.c0 = s; J.A = M.G2; J.lda = 2 * s; J.Sold = M.Sd[0];           // :144-147
+            if (M.p > 1) {                                                               // :155-171
+                J.nz = nZ[b]; J.scaled = 1; J.S = M.Scol[1]; J.Sd = M.Sd[1];
             }
             sj.push_back(J);
         }
@@ -418,13 +397,13 @@ void build_schedule(BatchPlan& P, Blob& blob) {
     for (int i = 1; i < Pmax; ++i) {
         std::vector<UpdJob> uU, uQ;
         std::vector<GramReq> g;
-        std::vector<SmallJob> sj;
+        std::vector<StepJob> sj;
         std::vector<int> nY(B, 0), nZn(B, 0), na(B, 0);
         for (int b = 0; b < B; ++b) {
             const Mat& M = mats[b];
             if (i >= M.p) continue;
             const int s = M.s, n = M.n, mScol = mZ[b] + s;
-            uU.push_back(upd(M, mScol, mScol, nZ[b], M.Scol, mScol, M.Sd, nZ[b]));     // :173-176
+            uU.push_back(upd(M, mScol, mScol, nZ[b], M.Scol[i & 1], mScol, M.Sd[i & 1], nZ[b]));   // :173-176
             int nb;
             if (i < M.p - 1) {                                                           // :177-190
                 nZn[b] = n - (i + 1) * s - s < s ? n - (i + 1) * s - s : s;
@@ -445,18 +424,12 @@ void build_schedule(BatchPlan& P, Blob& blob) {
             const Mat& M = mats[b];
             if (i >= M.p) continue;
             const int s = M.s, mScol = mZ[b] + s, lg = na[b];
-            SmallJob J{};
-            J.status = M.status; J.R = M.R; J.ldR = M.ldR;
-            J.sub[0] = pyth(M.G1 + mScol, lg, M.G1, lg, mScol, nY[b], M.Yd, i + 1);    // :200-204
-            J.sub[1] = rblock(mScol, mScol, nY[b], M.Scol, mScol, M.G1, lg, M.Sd, M.Yd);  // :211-215
-            J.nsub = 2;
+            StepJob J = step_job(M, M.G1, lg, mScol, nY[b], M.Yd, i + 1);               // :200-204
+            J.mode = 0; J.c0 = mScol; J.A = M.Scol[i & 1]; J.lda = mScol; J.Sold = M.Sd[i & 1];   // :211-215
             if (i + 1 < M.p) {
-                // Start of step i+1 (:155-171): they read G, Yd and write Scol, Sd,
-                // none of which the update of Q_i below touches.
-                const int mZ2 = mScol, mScol2 = mZ2 + s;
-                J.sub[2] = scol(M.G1, lg, mZ2, s, nZn[b], M.Yd, M.Scol);
-                J.sub[3] = pyth(M.G1 + mScol2 + (i64)s * lg, lg, M.Scol, mScol2, mScol2, nZn[b], M.Sd, i + 2);
-                J.nsub = 4;
+                // Start of step i+1 (:155-171): it writes the other S and Sd, which
+                // the update of Q_i below does not touch.
+                J.nz = nZn[b]; J.scaled = 1; J.S = M.Scol[(i + 1) & 1]; J.Sd = M.Sd[(i + 1) & 1];
             }
             sj.push_back(J);
             uQ.push_back(upd(M, mScol, mScol, nY[b], M.G1, lg, M.Yd, nY[b]));           // :206-209
@@ -488,7 +461,7 @@ int enqueue_all(BatchPlan& P, cudaStream_t st) {
                 break;
             }
             case kStSmall:
-                rc = launch_small_batched((const SmallJob*)(base + S.job_off), S.njobs, st);
+                rc = launch_step_batched((const StepJob*)(base + S.job_off), S.njobs, 2 * kMaxS, st);
                 break;
             case kStUpd:
                 rc = launch_update_batched((const UpdJob*)(base + S.job_off), prefix, S.njobs, S.items, st);
@@ -548,7 +521,7 @@ int autotune(BatchPlan& P, cudaStream_t st) {
                     GramJob J = make_gram_job(P.mats[q.mat], q, tb, rows);
                     jobs.push_back(J);
                     prefix.push_back(prefix.back() + J.nchunks * J.tilesA * J.tilesB);
-                    prefix2.push_back(prefix2.back() + (int)ceil_div((i64)q.na * q.nb, 256));
+                    prefix2.push_back(prefix2.back() + gram_reduce_ctas(J.na, J.nb));
                 }
                 Blob blob;
                 const size_t jo = blob.put(jobs), po = blob.put(prefix), p2 = blob.put(prefix2);

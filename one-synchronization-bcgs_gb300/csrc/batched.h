@@ -35,25 +35,6 @@ struct UpdJob {
     int ldt;
 };
 
-// Small s x s operations of one matrix, run in order by one CTA.
-enum SmallKind { kSmallNone = 0, kSmallPyth = 1, kSmallScol = 2, kSmallRblock = 3 };
-struct SmallSub {
-    int kind;
-    int a, b, c, d, step;
-    const double *p0, *p1, *p2, *p3;
-    int ld0, ld1, ld2, ld3;
-    double* out;
-    int ldo;
-};
-constexpr int kMaxSmallSubs = 4;
-struct SmallJob {
-    SmallSub sub[kMaxSmallSubs];
-    int nsub;
-    int* status;
-    double* R;
-    int ldR;
-};
-
 // TSQR: tiles of one level (Q in place, R factors to Rst), the root sign fix, and
 // the down-sweep multiply of one level.
 struct TsqrTileJob {
@@ -89,7 +70,6 @@ int gram_batched_panel_rows(int tb);   // A-panel height for a B-panel width
 int launch_gram_partial_batched(const GramJob* jobs, const int* prefix, int njobs, int items, cudaStream_t st);
 int launch_gram_reduce_batched(const GramJob* jobs, const int* prefix, int njobs, int items, cudaStream_t st);
 int launch_update_batched(const UpdJob* jobs, const int* prefix, int njobs, int items, cudaStream_t st);
-int launch_small_batched(const SmallJob* jobs, int njobs, cudaStream_t st);
 int launch_tsqr_tile_batched(const TsqrTileJob* jobs, const int* prefix, int njobs, int items, int ncmax,
                              cudaStream_t st);
 int launch_tsqr_root_batched(const TsqrRootJob* jobs, int njobs, cudaStream_t st);

@@ -39,19 +39,41 @@ int launch_gram_fp64(const double* X, i64 ld, i64 m, int a0, int na, int b0, int
 // out (na x nb, ld ldo) = fixed-order sum of nchunks partials part[c][i + j*na].
 int launch_gram_reduce(const double* part, int nchunks, int na, int nb, double* out, int ldo,
                        cudaStream_t st);
+int gram_reduce_ctas(int na, int nb);   // CTAs of one reduction
 
 // X[:, c0:c0+nc] = (X[:, c0:c0+nc] - X[:, q0:q0+K] S) T^{-1}; T upper (nc x nc) or null.
 int launch_update_fp64(double* X, i64 ld, i64 m, int q0, int K, int c0, int nc,
                        const double* S, int lds, const double* T, int ldt, cudaStream_t st);
 
-// Small single-CTA kernels (nz, s, ny <= 64).
-int launch_pyth_chol(const double* Om, int ldom, const double* A, int lda, int k, int nz,
-                     double* T, int ldt, int* status, int step, cudaStream_t st);
-int launch_scol(const double* G, int ldg, int mZ, int s, int nZ, const double* Yd, int ldy,
-                double* Scol, int ldsc, cudaStream_t st);
+// The small work of one block step on the reduced Gram G (small_fp64.cu): with
+// Y = G[0:K, 0:ny], Z = G[0:K, ny:ny+nz],
+//   T = chol(G[K:K+ny, 0:ny] - Y^T Y)                     (ny x ny, ld ny, lower part 0)
+// and, if nz > 0, the next block's first pass
+//   S = [Z ; T^{-T} (G[K:K+ny, ny:] - Y^T Z)]             ((K + ny) x nz, ld K + ny)
+//   Sd = chol(G[K+ny:, ny:] - S^T S), if scaled           (nz x nz, ld nz)
+// and, if mode >= 0, the R column block at columns [c0, c0 + ny): A + Y Sold above
+// the diagonal block T Sold (mode 0; Sold ny x ny, ld ny), or A + Y above upper(T)
+// (mode 1). Sold and A may be an earlier step's Sd and S but not this job's.
+// Uinv (may be null), (ny+nz) x (ny+nz): the inverse of U = [T S_mid ; 0 Sd] (Sd = I
+// if not scaled). A breakdown of T is recorded in status as block step `step`, one
+// of Sd as step + 1. ny, nz <= 64.
+struct StepJob {
+    const double* G = nullptr;
+    int ldg = 0, K = 0, ny = 0, nz = 0, scaled = 0, step = 0;
+    double *T = nullptr, *S = nullptr, *Sd = nullptr, *Uinv = nullptr;
+    int* status = nullptr;
+    int mode = -1, c0 = 0, ldR = 0, lda = 0;
+    double* R = nullptr;
+    const double *A = nullptr, *Sold = nullptr;
+};
+int launch_step(const StepJob& J, cudaStream_t st);
+// One job per matrix; nmax: the largest ny + nz, at most 32.
+int launch_step_batched(const StepJob* jobs, int njobs, int nmax, cudaStream_t st);
+
+// R[0:K, c0:c0+ny] = A + B Sd and R[c0:c0+ny, c0:] = Yd Sd (mode 0; Sd, Yd ny x ny,
+// upper, ld ny), or A + B and upper(Yd) (mode 1).
 int launch_rblock(double* R, int ldR, int c0, int K, int ny, const double* A, int lda,
-                  const double* B, int ldb, const double* Sd, int ldsd, const double* Yd,
-                  int ldyd, int mode, cudaStream_t st);
+                  const double* B, int ldb, const double* Sd, const double* Yd, int mode, cudaStream_t st);
 
 // Explicit TSQR of X[:, c0:c0+nc] in place; R (nc x nc, ldR) upper with diag >= 0.
 int tsqr_tile_rows(int nc);

@@ -147,31 +147,42 @@ extern "C" int orth_gb300_bcgsi2P1s_dev_noalloc(int m, int n, int s, double* dX,
     auto update = [&](int K, int c0, int nc, const double* S, int lds, const double* T, int ldt) {
         if (!err) err = launch_update_fp64(dX, ld, M, 0, K, c0, nc, S, lds, T, ldt, st);
     };
-    auto pchol = [&](const double* Om, int ldom, const double* A, int lda, int k, int nz, double* T,
-                     int step) {
-        if (!err) err = launch_pyth_chol(Om, ldom, A, lda, k, nz, T, nz, stat, step, st);
+    auto factor = [&](const double* G, int ldg, int K, int ny, double* T, int step) {
+        StepJob J;
+        J.G = G; J.ldg = ldg; J.K = K; J.ny = ny; J.T = T; J.step = step;
+        J.R = dR; J.ldR = ldR; J.status = stat;
+        return J;
     };
+    auto run_step = [&](const StepJob& J) {
+        if (!err) err = launch_step(J, st);
+    };
+    // S and Sd of this step and the next alternate. Their second buffers lie in W's
+    // region, (n + s) x 2s doubles, past the 2s x s first-step Gram W itself.
+    double* Sb[2] = {Scol, W + 2LL * s * s};
+    double* Sdb[2] = {Sd, Sb[1] + (i64)n * s};
 
     // BCGSI+P-1S, the same schedule as the allocating entry point
     // (reference SRC/orth.c:48-222).
     const int s0 = s, p = (n - s + s - 1) / s;
     if (!err) err = launch_tsqr(dX, ld, M, 0, s0, dR, ldR, tws, st);
     gram(2 * s, s0, s, W);
-    pchol(W + s0, 2 * s, W, 2 * s, s0, s, Sd, 1);
+    run_step(factor(W, 2 * s, s0, s, Sd, 1));
     update(s0, s0, s, W, 2 * s, Sd, s);
     int nZ = n - s - s0 < s ? n - s - s0 : s;
     int na = 2 * s + nZ, nb = s + nZ;
     double* G = G1;
     gram(na, s0, nb, G);
-    pchol(G + s0, na, G, na, s0, s, Yd, 1);
+    {
+        StepJob J = factor(G, na, s0, s, Yd, 1);
+        J.mode = 0; J.c0 = s0; J.A = W; J.lda = 2 * s; J.Sold = Sd;
+        if (p > 1) { J.nz = nZ; J.scaled = 1; J.S = Sb[1]; J.Sd = Sdb[1]; }
+        run_step(J);
+    }
     update(s0, s0, s, G, na, Yd, s);
-    if (!err) err = launch_rblock(dR, ldR, s0, s0, s, W, 2 * s, G, na, Sd, s, Yd, s, 0, st);
     int ldg = na, mZ = s0;
     for (int i = 1; i < p; ++i) {
         const int mScol = mZ + s;
-        if (!err) err = launch_scol(G, ldg, mZ, s, nZ, Yd, s, Scol, mScol, st);
-        pchol(G + mScol + (i64)s * ldg, ldg, Scol, mScol, mScol, nZ, Sd, i + 1);
-        update(mScol, mScol, nZ, Scol, mScol, Sd, nZ);
+        update(mScol, mScol, nZ, Sb[i & 1], mScol, Sdb[i & 1], nZ);
         int nY, nZn;
         if (i < p - 1) {
             nZn = n - (i + 1) * s - s0 < s ? n - (i + 1) * s - s0 : s;
@@ -186,9 +197,11 @@ extern "C" int orth_gb300_bcgsi2P1s_dev_noalloc(int m, int n, int s, double* dX,
         }
         gram(na, mScol, nb, G);
         ldg = na;
-        pchol(G + mScol, ldg, G, ldg, mScol, nY, Yd, i + 1);
+        StepJob J = factor(G, ldg, mScol, nY, Yd, i + 1);
+        J.mode = 0; J.c0 = mScol; J.A = Sb[i & 1]; J.lda = mScol; J.Sold = Sdb[i & 1];
+        if (i < p - 1) { J.nz = nZn; J.scaled = 1; J.S = Sb[(i + 1) & 1]; J.Sd = Sdb[(i + 1) & 1]; }
+        run_step(J);
         update(mScol, mScol, nY, G, ldg, Yd, nY);
-        if (!err) err = launch_rblock(dR, ldR, mScol, mScol, nY, Scol, mScol, G, ldg, Sd, nY, Yd, nY, 0, st);
         mZ += s;
         nZ = nZn;
     }

@@ -205,26 +205,30 @@ i64 part_doubles(i64 m, int n, int s, int num_sms) {
 struct Small {
     double* G1;    // (n+s) x 2s reduced Gram
     double* G2;    // (n+s) x 2s second reduced Gram (two-sync variants)
-    double* Scol;  // n x s
-    double* S0;    // s x s first-step coefficients
-    double* Sd;    // s x s
-    double* Yd;    // s x s
-    double* Cq;    // 3 s x s: CholQR2's panel Gram, R1 and R2
+    double* Scol[2];  // n x s, this block step's and the next one's
+    double* S0;       // s x s first-step coefficients
+    double* Sd[2];    // s x s, likewise
+    double* Yd;       // s x s
+    double* Cq;       // 3 s x s: CholQR2's panel Gram, R1 and R2
+    double* Uinv;     // 2s x 2s: the inverse of the last step's factors (split modes)
 };
 
 i64 small_doubles(int n, int s) {
-    return 2LL * (n + s) * 2 * s + (i64)n * s + 6LL * s * s + 64;
+    return 2LL * (n + s) * 2 * s + 2LL * n * s + 11LL * s * s + 64;
 }
 
 Small carve_small(double* base, int n, int s) {
     Small w;
     w.G1 = base;
     w.G2 = w.G1 + (i64)(n + s) * 2 * s;
-    w.Scol = w.G2 + (i64)(n + s) * 2 * s;
-    w.S0 = w.Scol + (i64)n * s;
-    w.Sd = w.S0 + (i64)s * s;
-    w.Yd = w.Sd + (i64)s * s;
+    w.Scol[0] = w.G2 + (i64)(n + s) * 2 * s;
+    w.Scol[1] = w.Scol[0] + (i64)n * s;
+    w.S0 = w.Scol[1] + (i64)n * s;
+    w.Sd[0] = w.S0 + (i64)s * s;
+    w.Sd[1] = w.Sd[0] + (i64)s * s;
+    w.Yd = w.Sd[1] + (i64)s * s;
     w.Cq = w.Yd + (i64)s * s;
+    w.Uinv = w.Cq + 3LL * s * s;
     return w;
 }
 
@@ -660,8 +664,10 @@ struct Engine {
         }
         gram_fp64(0, na, b0, nb, C, na);
     }
-    // X[:, c0:c0+nc] = (X[:, c0:c0+nc] - X[:, 0:K] S) T^{-1}
-    void update(int K, int c0, int nc, const double* S, int lds, const double* T, int ldt) {
+    // X[:, c0:c0+nc] = (X[:, c0:c0+nc] - X[:, 0:K] S) T^{-1}, T nc x nc (ld nc) or null.
+    // Split modes take T^{-1} from w.Uinv, where the step that made T left it
+    // (ld ldinv).
+    void update(int K, int c0, int nc, const double* S, int lds, const double* T, int ldinv) {
         if (err || nc <= 0) return;
         host_sync(K > c0 + nc ? K : c0 + nc, c0);
         if (is_split(precision)) {
@@ -673,15 +679,14 @@ struct Engine {
                                                    : 8.0 * m * (K + 2.0 * nc);
         ProfScope ps(1, st, 2.0 * m * K * nc + (T ? (double)m * nc * nc : 0.0), 8.0 * m * (K + 2.0 * nc), traffic);
         if (is_split(precision)) {
-            err = launch_update_split(X, ld, m, K, c0, nc, S, lds, T, ldt, scr().split.as<char>(),
-                                      scr().split.bytes, g_ctx.num_sms, st);
+            err = launch_update_split(X, ld, m, K, c0, nc, S, lds, T ? w.Uinv : nullptr, ldinv, g_ctx.num_sms, st);
             return;
         }
-        err = launch_update_fp64(X, ld, m, 0, K, c0, nc, S, lds, T, ldt, st);
+        err = launch_update_fp64(X, ld, m, 0, K, c0, nc, S, lds, T, nc, st);
     }
     // Split modes: Q_k and U_{k+1} of the lagged variants in one tensor-core pass.
-    void fused_update(int K, int nz, const double* G, int ldg, const double* Ty, const double* Sp,
-                      const double* Ts) {
+    // The step that reduced G left the inverse of both factors in w.Uinv.
+    void fused_update(int K, int nz, const double* G, int ldg) {
         if (err) return;
         host_sync(K + s + nz, K);
         {
@@ -692,24 +697,35 @@ struct Engine {
         const double traffic = 2.0 * split_digits() * m * (K + s + nz) + 8.0 * m * (s + nz);
         ProfScope ps(1, st, 2.0 * m * K * (s + nz) + (double)m * (s * s + nz * nz),
                      8.0 * m * (K + s + nz) + 8.0 * m * (s + nz), traffic);
-        err = launch_fused_update_split(X, ld, m, K, s, nz, G, ldg, Ty, Sp, K + s, Ts, g_ctx.num_sms, st);
+        err = launch_fused_update_split(X, ld, m, K, s, nz, G, ldg, w.Uinv, g_ctx.num_sms, st);
     }
-    void pyth_chol(const double* Om, int ldom, const double* A, int lda, int k, int nz, double* T,
-                   int step) {
+    // T = chol(G[K:K+ny, 0:ny] - Y^T Y), Y = G[0:K, 0:ny]; callers add what else the
+    // step computes (StepJob) before step().
+    StepJob factor(const double* G, int ldg, int K, int ny, double* T, int stepno) const {
+        StepJob J;
+        J.G = G; J.ldg = ldg; J.K = K; J.ny = ny; J.T = T; J.step = stepno;
+        J.R = R; J.ldR = ldR; J.status = status;
+        if (is_split(precision)) J.Uinv = w.Uinv;
+        return J;
+    }
+    // Adds the R block at columns [c0, c0 + J.ny) to J: A above, from this step's Sold.
+    static void add_rblock(StepJob& J, int c0, const double* A, int lda, const double* Sold) {
+        J.mode = Sold ? 0 : 1; J.c0 = c0; J.A = A; J.lda = lda; J.Sold = Sold;
+    }
+    // Adds the next block's S (and Sd, unless null) to J.
+    static void add_next(StepJob& J, int nz, double* S, double* Sd) {
+        J.nz = nz; J.S = S; J.Sd = Sd; J.scaled = Sd ? 1 : 0;
+    }
+    void step(const StepJob& J) {
         if (err) return;
         ProfScope ps(2, st, 0.0, 0.0);
-        err = launch_pyth_chol(Om, ldom, A, lda, k, nz, T, nz, status, step, st);
-    }
-    void scol(const double* G, int ldg, int mZ, int nZ, const double* Yd, double* Scol) {
-        if (err) return;
-        ProfScope ps(2, st, 0.0, 0.0);
-        err = launch_scol(G, ldg, mZ, s, nZ, Yd, s, Scol, mZ + s, st);
+        err = launch_step(J, st);
     }
     void rblock(int c0, int K, int ny, const double* A, int lda, const double* B, int ldb,
                 const double* Sd, const double* Yd, int mode) {
         if (err) return;
         ProfScope ps(2, st, 0.0, 0.0);
-        err = launch_rblock(R, ldR, c0, K, ny, A, lda, B, ldb, Sd, ny, Yd, ny, mode, st);
+        err = launch_rblock(R, ldR, c0, K, ny, A, lda, B, ldb, Sd, Yd, mode, st);
     }
     // Explicit TSQR of X[:, c0:c0+nc]; R into (Rout, ldr).
     void tsqr(int c0, int nc, double* Rout, int ldr) {
@@ -741,10 +757,12 @@ struct Engine {
         for (int pass = 0; pass < 2 && !err; ++pass) {
             double* T = pass ? R2 : R1;
             gram_fp64(c0, nc, c0, nc, G, nc);
-            if (!err) err = launch_pyth_chol(G, nc, nullptr, 0, 0, nc, T, nc, status, step, st);
+            StepJob J;
+            J.G = G; J.ldg = nc; J.ny = nc; J.T = T; J.step = step; J.status = status;
+            if (!err) err = launch_step(J, st);
             if (!err) err = launch_update_fp64(X, ld, m, 0, 0, c0, nc, nullptr, 0, T, nc, st);
         }
-        if (!err) err = launch_rblock(Rout, ldr, 0, 0, nc, nullptr, 0, nullptr, 0, R1, nc, R2, nc, 0, st);
+        if (!err) err = launch_rblock(Rout, ldr, 0, 0, nc, nullptr, 0, nullptr, 0, R1, R2, 0, st);
         if (is_split(precision)) split_mark_stale(c0, nc);
     }
     // IntraOrtho of the panel X[:, c0:c0+nc] (where the reference calls TSQR).
@@ -766,23 +784,25 @@ void run_p1s(Engine& e) {
     // First step (:110-147).
     double* W = w.G2;                                                // 2s x s, ld 2s
     e.gram(2 * s, s0, s, W);                                         // :111-114
-    e.pyth_chol(W + s0, 2 * s, W, 2 * s, s0, s, w.Sd, 1);            // :115-119
-    e.update(s0, s0, s, W, 2 * s, w.Sd, s);                          // :121-124  U2
+    e.step(e.factor(W, 2 * s, s0, s, w.Sd[0], 1));                   // :115-119
+    e.update(s0, s0, s, W, 2 * s, w.Sd[0], s);                       // :121-124  U2
     int nZ = n - s - s0 < s ? n - s - s0 : s;                        // :125
     int na = 2 * s + nZ, nb = s + nZ;
     double* G = w.G1;
     e.gram(na, s0, nb, G);                                           // :127-133
-    e.pyth_chol(G + s0, na, G, na, s0, s, w.Yd, 1);                  // :134-137
+    {
+        StepJob J = e.factor(G, na, s0, s, w.Yd, 1);                 // :134-137
+        e.add_rblock(J, s0, W, 2 * s, w.Sd[0]);                      // :144-147
+        if (p > 1) e.add_next(J, nZ, w.Scol[1], w.Sd[1]);            // :155-171
+        e.step(J);
+    }
     e.update(s0, s0, s, G, na, w.Yd, s);                             // :139-142  Q2
-    e.rblock(s0, s0, s, W, 2 * s, G, na, w.Sd, w.Yd, 0);             // :144-147
     int ldg = na;
     int mZ = s0;
     for (int i = 1; i < p; ++i) {                                    // :152-218
         const int mScol = mZ + s;
-        e.scol(G, ldg, mZ, nZ, w.Yd, w.Scol);                        // :155-159
-        // Omega_k = X_k^T X_k from the last synchronization (:160-163).
-        e.pyth_chol(G + mScol + (i64)s * ldg, ldg, w.Scol, mScol, mScol, nZ, w.Sd, i + 1);  // :160-171
-        e.update(mScol, mScol, nZ, w.Scol, mScol, w.Sd, nZ);         // :173-176  U_k
+        double *Sc = w.Scol[i & 1], *Sd = w.Sd[i & 1];
+        e.update(mScol, mScol, nZ, Sc, mScol, Sd, nZ);               // :173-176  U_k
         int nY, nZn;
         if (i < p - 1) {                                             // :177-190
             nZn = n - (i + 1) * s - s0 < s ? n - (i + 1) * s - s0 : s;
@@ -797,9 +817,12 @@ void run_p1s(Engine& e) {
         }
         e.gram(na, mScol, nb, G);                                    // the one sync
         ldg = na;
-        e.pyth_chol(G + mScol, ldg, G, ldg, mScol, nY, w.Yd, i + 1); // :200-204
+        StepJob J = e.factor(G, ldg, mScol, nY, w.Yd, i + 1);        // :200-204
+        e.add_rblock(J, mScol, Sc, mScol, Sd);                       // :211-215
+        // The next step's S and Omega - S^T S (:155-171), from the same G.
+        if (i < p - 1) e.add_next(J, nZn, w.Scol[(i + 1) & 1], w.Sd[(i + 1) & 1]);
+        e.step(J);
         e.update(mScol, mScol, nY, G, ldg, w.Yd, nY);                // :206-209  Q_k
-        e.rblock(mScol, mScol, nY, w.Scol, mScol, G, ldg, w.Sd, w.Yd, 0);  // :211-215
         mZ += s;
         nZ = nZn;
     }
@@ -814,7 +837,6 @@ void run_lagged_fused(Engine& e, bool pyth) {
     const int s = e.s, n = e.n, s0 = s;
     const int p = nblocks_after_first(n, s);
     Small& w = e.w;
-    const int mode = pyth ? 0 : 1;
     e.intra(0, s0, e.R, e.ldR, 1);
     double* W = w.G2;
     int nZ = n - s - s0 < s ? n - s - s0 : s;
@@ -822,30 +844,29 @@ void run_lagged_fused(Engine& e, bool pyth) {
     double* G = w.G1;
     if (pyth) {
         e.gram(2 * s, s0, s, W);                                     // :111-114
-        e.pyth_chol(W + s0, 2 * s, W, 2 * s, s0, s, w.Sd, 1);        // :115-119
-        e.update(s0, s0, s, W, 2 * s, w.Sd, s);                      // :121-124
+        e.step(e.factor(W, 2 * s, s0, s, w.Sd[0], 1));               // :115-119
+        e.update(s0, s0, s, W, 2 * s, w.Sd[0], s);                   // :121-124
     } else {
         e.gram(s0, s0, s, w.S0);                                     // :275-278
         e.update(s0, s0, s, w.S0, s0, nullptr, 0);                   // :280-281
     }
     na = 2 * s + (pyth ? nZ : 0);
     nb = s + nZ;
-    e.gram(pyth ? na : 2 * s, s0, nb, G);                            // :127-133 / :284-287
-    int ldg = pyth ? na : 2 * s;
-    e.pyth_chol(G + s0, ldg, G, ldg, s0, s, w.Yd, 1);                // :134-137 / :288-291
-    if (pyth) e.rblock(s0, s0, s, W, 2 * s, G, ldg, w.Sd, w.Yd, 0);  // :144-147
-    else e.rblock(s0, s0, s, w.S0, s0, G, ldg, nullptr, w.Yd, 1);    // :298-302
+    e.gram(na, s0, nb, G);                                           // :127-133 / :284-287
+    int ldg = na;
+    {
+        StepJob J = e.factor(G, ldg, s0, s, w.Yd, 1);                // :134-137 / :288-291
+        if (pyth) e.add_rblock(J, s0, W, 2 * s, w.Sd[0]);            // :144-147
+        else e.add_rblock(J, s0, w.S0, s0, nullptr);                 // :298-302
+        if (p > 1) e.add_next(J, nZ, w.Scol[1], pyth ? w.Sd[1] : nullptr);   // :155-171
+        e.step(J);
+    }
     if (p <= 1) {
         e.update(s0, s0, s, G, ldg, w.Yd, s);                        // Q_2 alone
         return;
     }
+    e.fused_update(s0, nZ, G, ldg);
     int mZ = s0;
-    {
-        const int mScolN = mZ + s;
-        e.scol(G, ldg, mZ, nZ, w.Yd, w.Scol);                        // :155-159
-        if (pyth) e.pyth_chol(G + mScolN + (i64)s * ldg, ldg, w.Scol, mScolN, mScolN, nZ, w.Sd, 2);
-        e.fused_update(s0, nZ, G, ldg, w.Yd, w.Scol, pyth ? w.Sd : nullptr);
-    }
     for (int i = 1; i < p; ++i) {
         const int mScol = mZ + s;
         int nY, nZn;
@@ -862,16 +883,12 @@ void run_lagged_fused(Engine& e, bool pyth) {
         }
         e.gram(na, mScol, nb, G);                                    // the one synchronization
         ldg = na;
-        e.pyth_chol(G + mScol, ldg, G, ldg, mScol, nY, w.Yd, i + 1);
-        e.rblock(mScol, mScol, nY, w.Scol, mScol, G, ldg, pyth ? w.Sd : nullptr, w.Yd, mode);
-        if (i < p - 1) {
-            const int mZn = mZ + s, mScolN = mZn + s;
-            e.scol(G, ldg, mZn, nZn, w.Yd, w.Scol);
-            if (pyth) e.pyth_chol(G + mScolN + (i64)s * ldg, ldg, w.Scol, mScolN, mScolN, nZn, w.Sd, i + 2);
-            e.fused_update(mScol, nZn, G, ldg, w.Yd, w.Scol, pyth ? w.Sd : nullptr);
-        } else {
-            e.update(mScol, mScol, nY, G, ldg, w.Yd, nY);            // last Q_k
-        }
+        StepJob J = e.factor(G, ldg, mScol, nY, w.Yd, i + 1);
+        e.add_rblock(J, mScol, w.Scol[i & 1], mScol, pyth ? w.Sd[i & 1] : nullptr);
+        if (i < p - 1) e.add_next(J, nZn, w.Scol[(i + 1) & 1], pyth ? w.Sd[(i + 1) & 1] : nullptr);
+        e.step(J);
+        if (i < p - 1) e.fused_update(mScol, nZn, G, ldg);
+        else e.update(mScol, mScol, nY, G, ldg, w.Yd, nY);           // last Q_k
         mZ += s;
         nZ = nZn;
     }
@@ -891,14 +908,18 @@ void run_21s(Engine& e) {
     int na = 2 * s, nb = s + nZ;
     double* G = w.G1;
     e.gram(na, s0, nb, G);                                           // :284-287
-    e.pyth_chol(G + s0, na, G, na, s0, s, w.Yd, 1);                  // :288-291
+    {
+        StepJob J = e.factor(G, na, s0, s, w.Yd, 1);                 // :288-291
+        e.add_rblock(J, s0, w.S0, s0, nullptr);                      // :298-302
+        if (p > 1) e.add_next(J, nZ, w.Scol[1], nullptr);            // :310-314
+        e.step(J);
+    }
     e.update(s0, s0, s, G, na, w.Yd, s);                             // :293-296
-    e.rblock(s0, s0, s, w.S0, s0, G, na, nullptr, w.Yd, 1);          // :298-302
     int ldg = na, mZ = s0;
     for (int i = 1; i < p; ++i) {
         const int mScol = mZ + s;
-        e.scol(G, ldg, mZ, nZ, w.Yd, w.Scol);                        // :310-314
-        e.update(mScol, mScol, nZ, w.Scol, mScol, nullptr, 0);       // :323-324
+        double* Sc = w.Scol[i & 1];
+        e.update(mScol, mScol, nZ, Sc, mScol, nullptr, 0);           // :323-324
         int nY, nZn;
         if (i < p - 1) {                                             // :325-335
             nZn = n - (i + 1) * s - s0 < s ? n - (i + 1) * s - s0 : s;
@@ -913,9 +934,11 @@ void run_21s(Engine& e) {
         }
         e.gram(na, mScol, nb, G);
         ldg = na;
-        e.pyth_chol(G + mScol, ldg, G, ldg, mScol, nY, w.Yd, i + 1); // :345-349
+        StepJob J = e.factor(G, ldg, mScol, nY, w.Yd, i + 1);        // :345-349
+        e.add_rblock(J, mScol, Sc, mScol, nullptr);                  // :356-360
+        if (i < p - 1) e.add_next(J, nZn, w.Scol[(i + 1) & 1], nullptr);   // :310-314
+        e.step(J);
         e.update(mScol, mScol, nY, G, ldg, w.Yd, nY);                // :351-354
-        e.rblock(mScol, mScol, nY, w.Scol, mScol, G, ldg, nullptr, w.Yd, 1);  // :356-360
         mZ += s;
         nZ = nZn;
     }
@@ -927,18 +950,20 @@ void run_pipi(Engine& e) {
     const int s = e.s, n = e.n, s0 = s;
     const int p = nblocks_after_first(n, s);
     Small& w = e.w;
+    double* Sd = w.Sd[0];
     e.intra(0, s0, e.R, e.ldR, 1);                                   // :411-413
     int mScol = s0;
     for (int i = 0; i < p; ++i) {
         const int nZ = n - i * s - s0 < s ? n - i * s - s0 : s;       // :419
         const int na = mScol + nZ;
         e.gram(na, mScol, nZ, w.G1);                                 // :421-424
-        e.pyth_chol(w.G1 + mScol, na, w.G1, na, mScol, nZ, w.Sd, i + 1);  // :425-429
-        e.update(mScol, mScol, nZ, w.G1, na, w.Sd, nZ);              // :431-434
+        e.step(e.factor(w.G1, na, mScol, nZ, Sd, i + 1));            // :425-429
+        e.update(mScol, mScol, nZ, w.G1, na, Sd, nZ);                // :431-434
         e.gram(na, mScol, nZ, w.G2);                                 // :435-438
-        e.pyth_chol(w.G2 + mScol, na, w.G2, na, mScol, nZ, w.Yd, i + 1);  // :440-444
+        StepJob J = e.factor(w.G2, na, mScol, nZ, w.Yd, i + 1);      // :440-444
+        e.add_rblock(J, mScol, w.G1, na, Sd);                        // :451-455
+        e.step(J);
         e.update(mScol, mScol, nZ, w.G2, na, w.Yd, nZ);              // :446-449
-        e.rblock(mScol, mScol, nZ, w.G1, na, w.G2, na, w.Sd, w.Yd, 0);    // :451-455
         mScol += s;
     }
 }
@@ -955,11 +980,11 @@ void run_bcgsi2(Engine& e) {
         const int nZ = n - i * s - s0 < s ? n - i * s - s0 : s;       // :511
         e.gram(mScol, mScol, nZ, w.G1);                              // :512-515
         e.update(mScol, mScol, nZ, w.G1, mScol, nullptr, 0);         // :518-519
-        e.intra(mScol, nZ, w.Sd, nZ, i + 1);                         // :520-523
+        e.intra(mScol, nZ, w.Sd[0], nZ, i + 1);                         // :520-523
         e.gram(mScol, mScol, nZ, w.G2);                              // :524-527
         e.update(mScol, mScol, nZ, w.G2, mScol, nullptr, 0);         // :530-531
         e.intra(mScol, nZ, w.Yd, nZ, i + 1);                         // :532-535
-        e.rblock(mScol, mScol, nZ, w.G1, mScol, w.G2, mScol, w.Sd, w.Yd, 0);  // :537-541
+        e.rblock(mScol, mScol, nZ, w.G1, mScol, w.G2, mScol, w.Sd[0], w.Yd, 0);  // :537-541
         mScol += s;
     }
 }
@@ -970,23 +995,28 @@ void run_p2s(Engine& e) {
     const int s = e.s, n = e.n, s0 = s;
     const int p = nblocks_after_first(n, s);
     Small& w = e.w;
+    double* Sd = w.Sd[0];
     e.intra(0, s0, e.R, e.ldR, 1);                                   // :599-601
     e.gram(s0, s0, s, w.S0);                                         // :605-608
     e.update(s0, s0, s, w.S0, s0, nullptr, 0);                       // :610-611
-    e.intra(s0, s, w.Sd, s, 1);                                      // :612-614
+    e.intra(s0, s, Sd, s, 1);                                        // :612-614
     int nZ = n - s - s0 < s ? n - s - s0 : s;                        // :615
     int na = 2 * s, nb = s + nZ;
     double* G = w.G1;
     e.gram(na, s0, nb, G);                                           // :617-620
-    e.pyth_chol(G + s0, na, G, na, s0, s, w.Yd, 1);                  // :621-624
-    e.update(s0, s0, s, G, na, w.Yd, s);                             // :625-628
-    e.rblock(s0, s0, s, w.S0, s0, G, na, w.Sd, w.Yd, 0);             // :609,:630-633
+    {
+        StepJob J = e.factor(G, na, s0, s, w.Yd, 1);                 // :621-624
+        e.add_rblock(J, s0, w.S0, s0, Sd);                           // :609,:630-633
+        if (p > 1) e.add_next(J, nZ, w.Scol[1], nullptr);            // :641-645
+        e.step(J);
+    }
+    e.update(s0, s0, s, G, na, w.Yd, p > 1 ? s + nZ : s);            // :625-628
     int ldg = na, mZ = s0;
     for (int i = 1; i < p; ++i) {
         const int mScol = mZ + s;
-        e.scol(G, ldg, mZ, nZ, w.Yd, w.Scol);                        // :641-645
-        e.update(mScol, mScol, nZ, w.Scol, mScol, nullptr, 0);       // :647-648
-        e.intra(mScol, nZ, w.Sd, nZ, i + 1);                         // :649-652
+        double* Sc = w.Scol[i & 1];
+        e.update(mScol, mScol, nZ, Sc, mScol, nullptr, 0);           // :647-648
+        e.intra(mScol, nZ, Sd, nZ, i + 1);                           // :649-652
         int nY, nZn;
         if (i < p - 1) {                                             // :653-666
             nZn = n - (i + 1) * s - s0 < s ? n - (i + 1) * s - s0 : s;
@@ -1001,9 +1031,11 @@ void run_p2s(Engine& e) {
         }
         e.gram(na, mScol, nb, G);
         ldg = na;
-        e.pyth_chol(G + mScol, ldg, G, ldg, mScol, nY, w.Yd, i + 1); // :676-680
-        e.update(mScol, mScol, nY, G, ldg, w.Yd, nY);                // :681-684
-        e.rblock(mScol, mScol, nY, w.Scol, mScol, G, ldg, w.Sd, w.Yd, 0);  // :686-690
+        StepJob J = e.factor(G, ldg, mScol, nY, w.Yd, i + 1);        // :676-680
+        e.add_rblock(J, mScol, Sc, mScol, Sd);                       // :686-690
+        if (i < p - 1) e.add_next(J, nZn, w.Scol[(i + 1) & 1], nullptr);   // :641-645
+        e.step(J);
+        e.update(mScol, mScol, nY, G, ldg, w.Yd, nY + J.nz);         // :681-684
         mZ += s;
         nZ = nZn;
     }

@@ -1,255 +1,521 @@
-// Small FP64 block kernels of the BCGS step (one CTA each, s <= 64).
+// Small FP64 block kernels of the BCGS step (s <= 64), run between the tall passes
+// on the reduced Gram blocks.
 //
-// These run between the tall passes on the reduced Gram blocks and replace the
-// reference's small dgemm/dtrsm/dpotrf calls on s x s and K x s matrices:
-//   pyth_chol : T = chol(Om - A^T A), upper       (SRC/orth.c:160-171, 200-204, ...)
-//   scol      : S = Q_{1:k-1}^T X_k reconstructed  (SRC/orth.c:155-159, 310-314, 641-645)
-//   rblock    : R column block assembly            (SRC/orth.c:211-215, 356-360, ...)
-// Work here is O(K s^2) per step, negligible next to the tall passes, but it
-// sits on the critical path, so every step keeps it on the device: no host
-// round trip between the synchronizations.
+//   step   : everything a block step computes on the reduced Gram G in one launch:
+//            T = chol(Om_Y - Y^T Y)                        (SRC/orth.c:200-204, ...)
+//            the next block's S = [Z ; T^{-T}(G_mid - Y^T Z)]   (:155-159, :310-314)
+//            Sd = chol(Om_Z - S^T S)                       (:160-171)
+//            and the R column block of the current step    (:211-215, :356-360)
+//   rblock : the R column block alone (the variants whose factors come from TSQR)
+//
+// One elimination. With Y = G[0:K, 0:ny] and Z = G[0:K, ny:ny+nz] the three
+// factorizations above are one upper Cholesky factorization
+//     U^T U = G[K:K+N, 0:N] - [Y Z]^T [Y Z],   U = [T  S_mid ; 0  Sd],  N = ny + nz,
+// so they run as N right-looking steps on one N x N matrix in shared memory, and
+// carrying the identity along gives U^{-1}, which the tensor-core update's factor is
+// built from ([Q U X] times [-G U^{-1} ; U^{-1}]).
+//
+// What bounds it. An FP64 instruction of one warp occupies its quarter of the SM for
+// 64 clocks, however many lanes are active, and returns after as many: there is no
+// latency left to hide, only instructions to save (a square root costs 600 clocks, a
+// division 570). So the K N^2 / 2 products of [Y Z]^T [Y Z] are spread over the CTAs of
+// a cluster (kGroups row groups, summed per group and then over the groups through
+// distributed shared memory in a fixed order). The elimination, a chain of N
+// dependent steps, runs on one CTA: in step j, warp 0 finishes row j + 1 and makes it
+// the next pivot row (five dependent instructions) while the other warps update the
+// rows below, eight lanes a row because the rows are short.
+// The arithmetic does not depend on the number of CTAs per job, so the batched
+// launches (one CTA per matrix when there are many) give the single launch's bits.
 #include "batched.h"
 #include "common.cuh"
 #include "kernels.h"
 
+#include <cooperative_groups.h>
+
 namespace bcgs {
 
+namespace cg = cooperative_groups;
+
 namespace {
-constexpr int SM_THREADS = 256;
+constexpr int ST_THREADS = 256;
+constexpr int ST_WARPS = ST_THREADS / 32;
 constexpr int SMAX = 64;
+constexpr int kGroups = 8;      // row groups of [Y Z]^T [Y Z]
+constexpr int kTileRows = 32;   // rows of [Y Z] staged at a time
+
+// Entry e of the upper trapezoid (rows r < nr, columns r <= c < n), column by column.
+__device__ __forceinline__ void trap_rc(int e, int nr, int& r, int& c) {
+    const int tri = nr * (nr + 1) / 2;
+    if (e < tri) {
+        c = (int)((sqrtf(8.0f * (float)e + 1.0f) - 1.0f) * 0.5f);
+        while ((c + 1) * (c + 2) / 2 <= e) ++c;
+        while (c * (c + 1) / 2 > e) --c;
+        r = e - c * (c + 1) / 2;
+    } else {
+        const int f = e - tri;
+        c = nr + f / nr;
+        r = f - (c - nr) * nr;
+    }
+}
+__host__ __device__ inline int trap_size(int nr, int n) { return nr * (nr + 1) / 2 + (n - nr) * nr; }
+
+// 1 / x for a normal x: the hardware's approximate reciprocal (rcp.approx.ftz.f64, 20
+// bits or more) corrected by r (1 + e + e^2), e = 1 - x r, which leaves a relative
+// error of e^3 and the roundings: three dependent operations on the elimination's
+// critical path. Only ever used as a multiplier of an elimination step.
+__device__ __forceinline__ double recip(double x) {
+    double r;
+    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(x));
+    const double e = fma(-x, r, 1.0);
+    return fma(r, fma(e, e, e), r);
+}
 }  // namespace
 
-// Cholesky of the upper triangle of the nz x nz matrix in shared memory `a`
-// (column-major, ld SMAX), the unblocked row-oriented algorithm of LAPACK's
-// dpotf2 ('U'): for j = 0..nz-1,
-//   ajj = a_jj - sum_{i<j} a_ij^2; if ajj <= 0 stop with info = j+1 and a_jj = ajj;
-//   a_jj = sqrt(ajj); a_jc = (a_jc - sum_{i<j} a_ij a_ic) / a_jj for c > j.
-// On breakdown the partial factor is left in place, as dpotrf leaves it.
-__device__ int chol_upper_shared(double* a, int nz) {
-    __shared__ int s_info;
-    __shared__ double s_ajj;
-    if (threadIdx.x == 0) s_info = 0;
-    __syncthreads();
-    for (int j = 0; j < nz; ++j) {
-        if (threadIdx.x == 0) {
-            double ajj = a[j + j * SMAX];
-            for (int i = 0; i < j; ++i) ajj -= a[i + j * SMAX] * a[i + j * SMAX];
-            if (ajj <= 0.0) {
-                a[j + j * SMAX] = ajj;
-                s_info = j + 1;
-            } else {
-                ajj = sqrt(ajj);
-                a[j + j * SMAX] = ajj;
-            }
-            s_ajj = ajj;
-        }
-        __syncthreads();
-        if (s_info != 0) break;
-        const double rajj = 1.0 / s_ajj;
-        for (int c = j + 1 + (int)threadIdx.x; c < nz; c += blockDim.x) {
-            double v = a[j + c * SMAX];
-            for (int i = 0; i < j; ++i) v -= a[i + j * SMAX] * a[i + c * SMAX];
-            a[j + c * SMAX] = v * rajj;
-        }
-        __syncthreads();
-    }
-    __syncthreads();
-    return s_info;
+// Shared memory of one CTA (doubles): the N x N matrix (also the staging tile of the
+// products and Sd of the R block), the sums of this CTA's row groups (later Sold),
+// and the pivots.
+__host__ __device__ inline int step_matrix_doubles(int n) { return (n > kTileRows ? n : kTileRows) * (n + 1); }
+__host__ __device__ inline int step_sums_doubles(int n, int ny, int ctas) {
+    const int sums = (kGroups / ctas) * trap_size(n, n);
+    return sums > ny * ny ? sums : ny * ny;   // Sold moves in when the sums have been used
+}
+static size_t step_smem_bytes(int n, int ny, int ctas) {
+    return (size_t)(step_matrix_doubles(n) + step_sums_doubles(n, ny, ctas) + 4 * n + 2) * sizeof(double);
 }
 
-// T(nz x nz, ld ldt) = chol_upper(Om(nz x nz, ld ldom) - A(k x nz, ld lda)^T A).
-// Only the upper triangle of Om is read; T's strictly lower part is zeroed
-// (dlaset 'L' + dlacpy 'U' + dpotrf 'U'). A may be null when k == 0.
-// Body shared by the single and batched kernels; `a` is SMAX*SMAX doubles of shared
-// memory. Starts and ends with a CTA barrier, so the caller may reuse `a`.
-__device__ void pyth_chol_body(const double* __restrict__ Om, int ldom, const double* __restrict__ A, int lda,
-                               int k, int nz, double* __restrict__ T, int ldt, int* __restrict__ status, int step,
-                               double* __restrict__ a) {
-    __syncthreads();
-    for (int e = threadIdx.x; e < nz * nz; e += blockDim.x) {
-        int i = e % nz, j = e / nz;
-        double v = 0.0;
-        if (i <= j) {
-            v = Om[i + (i64)j * ldom];
-            for (int l = 0; l < k; ++l) v -= A[l + (i64)i * lda] * A[l + (i64)j * lda];
-        }
-        a[i + j * SMAX] = v;
-    }
-    __syncthreads();
-    int info = chol_upper_shared(a, nz);
-    for (int e = threadIdx.x; e < nz * nz; e += blockDim.x) {
-        int i = e % nz, j = e / nz;
-        T[i + (i64)j * ldt] = (i <= j) ? a[i + j * SMAX] : 0.0;
-    }
-    if (threadIdx.x == 0 && info != 0 && status != nullptr && status[0] == 0) {
-        status[0] = step;
-        status[1] = info;
-    }
-    __syncthreads();
-}
-
-__global__ void __launch_bounds__(SM_THREADS)
-pyth_chol_kernel(const double* __restrict__ Om, int ldom, const double* __restrict__ A, int lda,
-                 int k, int nz, double* __restrict__ T, int ldt, int* __restrict__ status, int step) {
-    __shared__ double a[SMAX * SMAX];
-    pyth_chol_body(Om, ldom, A, lda, k, nz, T, ldt, status, step, a);
-}
-
-// Scol(mScol x nZ, ld ldsc), mScol = mZ + s, from the last reduced Gram G (ld ldg):
-//   Scol = G[0:mScol, s:s+nZ]
-//   Scol[mZ:mScol] -= G[0:mZ, 0:s]^T G[0:mZ, s:s+nZ]
-//   Scol[mZ:mScol]  = Ydiag^{-T} Scol[mZ:mScol]       (dtrsm 'L','U','T','N')
-// Body shared by the single and batched kernels; dsm is SMAX*(nZ+s) doubles.
-__device__ void scol_body(const double* __restrict__ G, int ldg, int mZ, int s, int nZ,
-                          const double* __restrict__ Yd, int ldy, double* __restrict__ Scol, int ldsc,
-                          double* __restrict__ dsm) {
-    __syncthreads();
-    double* b = dsm;               // s x nZ, ld SMAX (only s rows used)
-    double* y = dsm + SMAX * nZ;   // s x s, ld SMAX
-    for (int e = threadIdx.x; e < mZ * nZ; e += blockDim.x) {
-        int i = e % mZ, j = e / mZ;
-        Scol[i + (i64)j * ldsc] = G[i + (i64)(s + j) * ldg];
-    }
-    for (int e = threadIdx.x; e < s * nZ; e += blockDim.x) {
-        int i = e % s, j = e / s;
-        double v = G[(mZ + i) + (i64)(s + j) * ldg];
-        for (int l = 0; l < mZ; ++l) v -= G[l + (i64)i * ldg] * G[l + (i64)(s + j) * ldg];
-        b[i + j * SMAX] = v;
-    }
-    for (int e = threadIdx.x; e < s * s; e += blockDim.x) {
-        int i = e % s, j = e / s;
-        y[i + j * SMAX] = Yd[i + (i64)j * ldy];
-    }
-    __syncthreads();
-    // Forward substitution with Yd^T (lower): z_i = (b_i - sum_{l<i} Yd_li z_l) / Yd_ii,
-    // one right-hand side column per thread.
-    for (int j = threadIdx.x; j < nZ; j += blockDim.x) {
-        for (int i = 0; i < s; ++i) {
-            double v = b[i + j * SMAX];
-            for (int l = 0; l < i; ++l) v -= y[l + i * SMAX] * b[l + j * SMAX];
-            b[i + j * SMAX] = v / y[i + i * SMAX];
-        }
-    }
-    __syncthreads();
-    for (int e = threadIdx.x; e < s * nZ; e += blockDim.x) {
-        int i = e % s, j = e / s;
-        Scol[(mZ + i) + (i64)j * ldsc] = b[i + j * SMAX];
-    }
-    __syncthreads();
-}
-
-__global__ void __launch_bounds__(SM_THREADS)
-scol_kernel(const double* __restrict__ G, int ldg, int mZ, int s, int nZ,
-            const double* __restrict__ Yd, int ldy, double* __restrict__ Scol, int ldsc) {
-    extern __shared__ double dsm[];
-    scol_body(G, ldg, mZ, s, nZ, Yd, ldy, Scol, ldsc, dsm);
-}
-
-// R column block at columns [c0, c0+ny):
-//   mode 0: R[0:K, c0:] = A + B Sd ;  R[c0:c0+ny, c0:] = Yd Sd      (P1s, PIPI, BCGSI+, P2s)
-//   mode 1: R[0:K, c0:] = A + B    ;  upper(R[c0:c0+ny, c0:]) = upper(Yd)   (bcgsi21s)
-// A, B are K x ny (ld lda, ldb); Sd, Yd upper ny x ny.
-// Body shared by the single and batched kernels; sd is SMAX*SMAX doubles.
-__device__ void rblock_body(double* __restrict__ R, int ldR, int c0, int K, int ny,
-                            const double* __restrict__ A, int lda, const double* __restrict__ B, int ldb,
-                            const double* __restrict__ Sd, int ldsd, const double* __restrict__ Yd, int ldyd,
-                            int mode, double* __restrict__ sd) {
-    __syncthreads();
-    if (mode == 0) {
-        for (int e = threadIdx.x; e < ny * ny; e += blockDim.x) {
-            int i = e % ny, j = e / ny;
-            sd[i + j * SMAX] = (i <= j) ? Sd[i + (i64)j * ldsd] : 0.0;
-        }
-    }
-    __syncthreads();
-    for (int e = threadIdx.x; e < K * ny; e += blockDim.x) {
-        int i = e % K, j = e / K;
-        double v = A[i + (i64)j * lda];
+// R[0:K, c0:c0+ny] = A + Y Sd_old (mode 0) or A + Y (mode 1), rows [r0, r1), as
+// thread t0 of nt. sd: ny x ny, ld ny, upper (mode 0).
+__device__ __forceinline__ void r_rows(double* R, int ldR, int c0, int ny, const double* A, int lda, const double* B,
+                                       int ldb, const double* sd, int mode, int r0, int r1, int t0, int nt) {
+    const int rows = r1 - r0;
+    for (int e = t0; e < rows * ny; e += nt) {
+        const int i = r0 + e % rows, j = e / rows;
+        double v = __ldg(A + i + (i64)j * lda);
         if (mode == 0) {
             double t = 0.0;
-            for (int l = 0; l <= j; ++l) t += B[i + (i64)l * ldb] * sd[l + j * SMAX];
+            for (int l = 0; l <= j; ++l) t = fma(__ldg(B + i + (i64)l * ldb), sd[l + j * ny], t);
             v += t;
         } else {
-            v += B[i + (i64)j * ldb];
+            v += __ldg(B + i + (i64)j * ldb);
         }
         R[i + (i64)(c0 + j) * ldR] = v;
     }
+}
+
+// R[c0:c0+ny, c0:c0+ny] = Yd Sd (mode 0) or upper(Yd) on the upper part (mode 1),
+// Yd(i, l) = yd[i * yi + l * yl].
+__device__ __forceinline__ void r_diag(double* R, int ldR, int c0, int ny, const double* yd, int yi, int yl,
+                                       const double* sd, int mode) {
     for (int e = threadIdx.x; e < ny * ny; e += blockDim.x) {
-        int i = e % ny, j = e / ny;
+        const int i = e % ny, j = e / ny;
         double* dst = R + (c0 + i) + (i64)(c0 + j) * ldR;
         if (mode == 0) {
             double t = 0.0;
             if (i <= j)
-                for (int l = i; l <= j; ++l) t += Yd[i + (i64)l * ldyd] * sd[l + j * SMAX];
+                for (int l = i; l <= j; ++l) t = fma(yd[i * yi + l * yl], sd[l + j * ny], t);
             *dst = t;
         } else if (i <= j) {
-            *dst = Yd[i + (i64)j * ldyd];
+            *dst = yd[i * yi + j * yl];
         }
     }
+}
+
+// Entry e of the right-hand side: G[K + r, c] minus the groups' sums, group by group
+// in a fixed tree.
+template <int C>
+__device__ __forceinline__ double step_entry(const StepJob& J, int r, int c, int e, int E, double* gs) {
+    double g[kGroups];
+#pragma unroll
+    for (int k = 0; k < kGroups; ++k) {
+        constexpr int PER = kGroups / C;
+        double* base = gs;
+        if constexpr (C > 1) base = cg::this_cluster().map_shared_rank(gs, k / PER);
+        g[k] = base[(k % PER) * E + e];
+    }
+    return __ldg(J.G + (J.K + r) + (i64)c * J.ldg) -
+           (((g[0] + g[1]) + (g[2] + g[3])) + ((g[4] + g[5]) + (g[6] + g[7])));
+}
+
+// One job by a cluster of C CTAs (rank = this CTA's), C | kGroups.
+template <int C>
+__device__ void step_body(const StepJob& J, int rank, double* sm) {
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int ny = J.ny, nz = J.nz, n = ny + nz;
+    const int nr = (nz > 0 && !J.scaled) ? ny : n;   // pivots
+    const int ld = n + 1;
+    const int E = trap_size(nr, n);
+    double* a = sm;
+    double* gs = sm + step_matrix_doubles(n);
+    double* s_u = gs + step_sums_doubles(n, ny, C);   // pivots of U and their reciprocals
+    double* s_t = s_u + 2 * n;                        // the pivot row over the pivot, two slots
+    int* s_stop = reinterpret_cast<int*>(s_t + 2 * n);   // and whether it cannot be used
+
+    // ---- products: one sum per row group and entry, rows in order. The rows of this
+    // CTA's groups are staged in tiles that may span groups; a sum goes on from
+    // where the previous tile left it, so it does not depend on the tiling. ----
+    constexpr int PER = kGroups / C;
+    const int L = (((J.K + kGroups - 1) / kGroups) + 3) & ~3;
+    const int k0 = min(J.K, rank * PER * L), k1 = min(J.K, (rank + 1) * PER * L);
+    for (int e = tid; e < PER * E; e += ST_THREADS) gs[e] = 0.0;
+#pragma unroll 1
+    for (int t0 = k0; t0 < k1; t0 += kTileRows) {
+        const int t1 = min(k1, t0 + kTileRows);
+        for (int e = tid; e < kTileRows * n; e += ST_THREADS) {
+            const int rr = e % kTileRows, c = e / kTileRows;
+            if (t0 + rr < t1) a[rr * ld + c] = J.G[t0 + rr + (i64)c * J.ldg];
+        }
+        __syncthreads();
+        const int q0 = (t0 - k0) / L, q1 = (t1 - 1 - k0) / L;   // groups with rows in this tile
+        for (int w = tid; w < (q1 - q0 + 1) * E; w += ST_THREADS) {
+            const int q = q0 + w / E, e = w % E;
+            int r, c;
+            trap_rc(e, nr, r, c);
+            const int i0 = max(0, k0 + q * L - t0), i1 = min(t1, k0 + (q + 1) * L) - t0;
+            double acc = gs[q * E + e];
+            const double* x = a + r;
+            const double* y = a + c;
+#pragma unroll 4
+            for (int i = i0; i < i1; ++i) acc = fma(x[i * ld], y[i * ld], acc);
+            gs[q * E + e] = acc;
+        }
+        __syncthreads();
+    }
     __syncthreads();
+    if constexpr (C > 1) cg::this_cluster().sync();
+
+    // ---- S_top = Z, and the R block's rows of Q, by the CTAs that do not eliminate ----
+    if (C == 1 || rank > 0) {
+        const int nt = (C == 1 ? 1 : C - 1) * ST_THREADS;
+        const int t = (C == 1 ? 0 : rank - 1) * ST_THREADS + tid;
+        if (J.S != nullptr)
+            for (int e = t; e < J.K * nz; e += nt) {
+                const int i = e % J.K, j = e / J.K;
+                J.S[i + (i64)j * (J.K + ny)] = __ldg(J.G + i + (i64)(ny + j) * J.ldg);
+            }
+        if (J.mode >= 0) {
+            if (J.mode == 0)
+                for (int e = tid; e < ny * ny; e += ST_THREADS) {
+                    const int i = e % ny, j = e / ny;
+                    a[i + j * ny] = i <= j ? __ldg(J.Sold + i + (i64)j * ny) : 0.0;
+                }
+            __syncthreads();
+            r_rows(J.R, J.ldR, J.c0, ny, J.A, J.lda, J.G, J.ldg, a, J.mode, 0, J.K, t, nt);
+            __syncthreads();
+        }
+    }
+    if constexpr (C > 1) {
+        if (rank > 0) {
+            // This CTA's sums stay readable until rank 0 has fetched them.
+            cg::this_cluster().sync();
+            return;
+        }
+    }
+
+    // This CTA's part of Sold, for the diagonal block at the end.
+    double sold[SMAX * SMAX / ST_THREADS];
+#pragma unroll
+    for (int k = 0; k < SMAX * SMAX / ST_THREADS; ++k) {
+        const int e = tid + k * ST_THREADS;
+        sold[k] = J.mode == 0 && e < ny * ny && e % ny <= e / ny ? J.Sold[e] : 0.0;
+    }
+
+    // ---- elimination: main part in the upper triangle (diagonal included), the
+    // carried identity's strictly lower part below it (its unit diagonal implied) ----
+    for (int e = tid; e < E; e += ST_THREADS) {
+        int r, c;
+        trap_rc(e, nr, r, c);
+        a[r * ld + c] = step_entry<C>(J, r, c, e, E, gs);
+    }
+    for (int e = tid; e < n * n; e += ST_THREADS) {
+        const int r = e / n, c = e % n;
+        if (c < r) a[r * ld + c] = 0.0;
+        if (r >= nr && c >= r) a[r * ld + c] = c == r ? 1.0 : 0.0;   // rows that are not eliminated
+    }
+    __syncthreads();
+    // Warp 0: row r becomes the pivot row. Its pivot's reciprocal and the row over the
+    // pivot go to slot r & 1 (the carried identity has 1 at c = r). A pivot that is
+    // not a positive number of ordinary size ends the fast path (an integer test: a
+    // comparison would be one more FP64 instruction).
+    const bool carry = J.Uinv != nullptr;
+    // (Loops over the columns are kept rolled: an FP64 instruction that is only
+    // predicated off still takes its 64 clocks.)
+    auto publish = [&](int r, double d, double x0) {
+        const double inv = recip(d);
+        const unsigned hi = (unsigned)__double2hiint(d);
+        if (lane == 0) s_stop[r & 1] = !(hi >= 0x05D00000u && hi < 0x7A100000u);   // 2^-930 .. 2^930
+        double* t = s_t + (r & 1) * n;
+        if (n <= 32) {
+            const double y = x0 * inv;
+            if (lane < n) t[lane] = lane == r ? inv : y;
+            return;
+        }
+#pragma unroll 1
+        for (int c = carry ? lane : (r & ~31) + lane; c < n; c += 32) {
+            const double y = a[r * ld + c] * inv;
+            t[c] = c == r ? inv : y;
+        }
+    };
+    if (warp == 0) publish(0, a[0], lane < n ? a[lane] : 0.0);
+    __syncthreads();
+    // Workers: eight lanes a row, four rows a warp, the warps of warp 0's quarter last.
+    const int slot = warp == 0 ? -1 : (warp == 4 ? 6 : (warp > 4 ? warp - 2 : warp - 1)) * 4 + (lane >> 3);
+    const int l8 = lane & 7;
+    bool fast = s_stop[0] == 0;
+    for (int j = 0; j < nr && fast; ++j) {
+        const double* pr = a + j * ld;
+        const double* t = s_t + (j & 1) * n;
+        if (warp == 0) {
+            const int r = j + 1;
+            if (r < n) {
+                double* row = a + r * ld;
+                const double f = -pr[r];
+                if (n <= 32) {
+                    const int c = min(lane, n - 1);
+                    const double x = row[c], y = fma(f, t[c], x);
+                    const double z = (c <= j ? carry : r < nr) ? y : x;
+                    if (lane < n) row[lane] = z;
+                    if (r < nr) publish(r, __shfl_sync(0xffffffffu, z, r), z);
+                } else {
+#pragma unroll 1
+                    for (int c = carry ? lane : (r & ~31) + lane; c < n; c += 32) {
+                        const double x = row[c], y = fma(f, t[c], x);
+                        row[c] = (c <= j ? carry : r < nr) ? y : x;
+                    }
+                    __syncwarp();
+                    if (r < nr) publish(r, row[r], 0.0);
+                }
+            }
+        } else {
+            const int na = carry ? j + 1 : 0;   // carried columns of every row
+            for (int r = j + 2 + slot; r < n; r += 4 * (ST_WARPS - 1)) {
+                double* row = a + r * ld;
+                const double f = -pr[r];
+                const int len = na + (r < nr ? n - r : 0);
+                int q = l8, c = q < na ? q : r + q - na;
+                double x = q < len ? row[c] : 0.0, y = q < len ? t[c] : 0.0;
+#pragma unroll 1
+                while (q < len) {
+                    const int q1 = q + 8, c1 = q1 < na ? q1 : r + q1 - na;
+                    double x1 = 0.0, y1 = 0.0;
+                    if (q1 < len) { x1 = row[c1]; y1 = t[c1]; }
+                    row[c] = fma(f, y, x);
+                    q = q1; c = c1; x = x1; y = y1;
+                }
+            }
+        }
+        __syncthreads();
+        // Slot (j + 1) & 1 is next written after the barrier that ends step j + 1.
+        if (j + 1 < nr) fast = s_stop[(j + 1) & 1] == 0;
+    }
+
+    if (fast) {
+        // Row r of U is the eliminated row over the square root of its pivot; the
+        // carried rows scale the same way and give U^{-T}.
+        for (int r = tid; r < n; r += ST_THREADS) {
+            // v = 1 / sqrt(d), u = sqrt(d) = d v corrected once (half the cost of a
+            // square root and a division).
+            const double d = r < nr ? a[r * ld + r] : 1.0;
+            const double v = rsqrt(d), u = d * v;
+            s_u[r] = fma(fma(-u, u, d), 0.5 * v, u);
+            s_u[n + r] = v;
+        }
+        __syncthreads();
+        for (int r = warp; r < n; r += ST_WARPS) {
+            const double v = s_u[n + r];
+            for (int c = lane; c < n; c += 32) {
+                const double x = c == r ? s_u[r] : a[r * ld + c] * v;
+                a[r * ld + c] = x;
+                if (r < ny && c < ny) J.T[r + (i64)c * ny] = c >= r ? x : 0.0;
+                else if (r < ny) J.S[(J.K + r) + (i64)(c - ny) * (J.K + ny)] = x;
+                else if (c >= ny && J.scaled) J.Sd[(r - ny) + (i64)(c - ny) * nz] = c >= r ? x : 0.0;
+                if (J.Uinv != nullptr) J.Uinv[c + (i64)r * n] = c < r ? x : (c == r ? v : 0.0);
+            }
+        }
+        __syncthreads();
+    } else {
+        // A pivot out of range: the same factorization by dot products. At a
+        // breakdown (a pivot <= 0) the factor keeps the rows before it, and the rows
+        // from it on hold the matrix that was to be factored, as dpotrf leaves
+        // them; what follows goes on with that factor. Not a path for speed.
+        __syncthreads();
+        for (int e = tid; e < E; e += ST_THREADS) {
+            int r, c;
+            trap_rc(e, nr, r, c);
+            a[r * ld + c] = step_entry<C>(J, r, c, e, E, gs);
+        }
+        for (int e = tid; e < n * n; e += ST_THREADS) {
+            const int r = e / n, c = e % n;
+            if (c < r) a[r * ld + c] = 0.0;
+            if (r >= nr && c >= r) a[r * ld + c] = c == r ? 1.0 : 0.0;
+        }
+        __syncthreads();
+        // Upper Cholesky of rows and columns [o, o + k): false at a breakdown.
+        auto chol = [&](int o, int k, int step) {
+            for (int j = o; j < o + k; ++j) {
+                __syncthreads();
+                if (tid == 0) {
+                    double d = a[j * ld + j];
+                    for (int i = o; i < j; ++i) d = fma(-a[i * ld + j], a[i * ld + j], d);
+                    s_stop[0] = d <= 0.0;
+                    a[j * ld + j] = d <= 0.0 ? d : sqrt(d);
+                    if (d <= 0.0 && J.status != nullptr && J.status[0] == 0) {
+                        J.status[0] = step;
+                        J.status[1] = j - o + 1;
+                    }
+                }
+                __syncthreads();
+                if (s_stop[0] != 0) break;
+                for (int c = j + 1 + tid; c < o + k; c += ST_THREADS) {
+                    double v = a[j * ld + c];
+                    for (int i = o; i < j; ++i) v = fma(-a[i * ld + j], a[i * ld + c], v);
+                    a[j * ld + c] = v / a[j * ld + j];
+                }
+            }
+            __syncthreads();
+        };
+        chol(0, ny, J.step);
+        // S_mid = T^{-T} (G_mid - Y^T Z), one column per thread.
+        for (int c = ny + tid; c < n; c += ST_THREADS)
+            for (int i = 0; i < ny; ++i) {
+                double v = a[i * ld + c];
+                for (int l = 0; l < i; ++l) v = fma(-a[l * ld + i], a[l * ld + c], v);
+                a[i * ld + c] = v / a[i * ld + i];
+            }
+        __syncthreads();
+        if (nr > ny) {
+            for (int e = tid; e < nz * nz; e += ST_THREADS) {
+                const int r = ny + e % nz, c = ny + e / nz;
+                if (r > c) continue;
+                double v = a[r * ld + c];
+                for (int l = 0; l < ny; ++l) v = fma(-a[l * ld + r], a[l * ld + c], v);
+                a[r * ld + c] = v;
+            }
+            chol(ny, nz, J.step + 1);
+        }
+        for (int e = tid; e < n * n; e += ST_THREADS) {
+            const int r = e / n, c = e % n;
+            const double x = a[r * ld + c];
+            if (r < ny && c < ny) J.T[r + (i64)c * ny] = x;
+            else if (r < ny) J.S[(J.K + r) + (i64)(c - ny) * (J.K + ny)] = x;
+            else if (c >= ny && J.scaled) J.Sd[(r - ny) + (i64)(c - ny) * nz] = x;
+        }
+        if (J.Uinv != nullptr) {
+            // Column c of U^{-1} by back substitution, through global memory.
+            for (int c = tid; c < n; c += ST_THREADS) {
+                double* y = J.Uinv + (i64)c * n;
+                for (int i = n - 1; i >= 0; --i) {
+                    double v = i == c ? 1.0 : 0.0;
+                    for (int l = i + 1; l <= c; ++l) v = fma(-a[i * ld + l], y[l], v);
+                    y[i] = i <= c ? v / a[i * ld + i] : 0.0;
+                }
+            }
+        }
+        __syncthreads();
+    }
+    if (J.mode >= 0) {
+        // a's leading block is T (row by row) on either path; the sums are done with.
+#pragma unroll
+        for (int k = 0; k < SMAX * SMAX / ST_THREADS; ++k)
+            if (tid + k * ST_THREADS < ny * ny) gs[tid + k * ST_THREADS] = sold[k];
+        __syncthreads();
+        r_diag(J.R, J.ldR, J.c0, ny, a, ld, 1, gs, J.mode);
+    }
+    if constexpr (C > 1) cg::this_cluster().sync();
 }
 
-__global__ void __launch_bounds__(SM_THREADS)
-rblock_kernel(double* __restrict__ R, int ldR, int c0, int K, int ny,
-              const double* __restrict__ A, int lda, const double* __restrict__ B, int ldb,
-              const double* __restrict__ Sd, int ldsd, const double* __restrict__ Yd, int ldyd,
-              int mode) {
+template <int C>
+__global__ void __launch_bounds__(ST_THREADS) step_kernel(const __grid_constant__ StepJob job) {
+    extern __shared__ double sm[];
+    step_body<C>(job, C == 1 ? 0 : (int)blockIdx.x, sm);
+}
+
+// Batched form: CTAs [b C, (b + 1) C) run job b.
+template <int C>
+__global__ void __launch_bounds__(ST_THREADS) step_batched(const StepJob* __restrict__ jobs) {
+    extern __shared__ double sm[];
+    const StepJob J = jobs[blockIdx.x / C];
+    step_body<C>(J, (int)(blockIdx.x % C), sm);
+}
+
+// The R column block alone: K x ny rows of Q by 32-row CTAs, the diagonal block by
+// the last CTA.
+__global__ void __launch_bounds__(ST_THREADS)
+rblock_kernel(double* R, int ldR, int c0, int K, int ny, const double* A, int lda, const double* B, int ldb,
+              const double* Sd, const double* Yd, int mode) {
     __shared__ double sd[SMAX * SMAX];
-    rblock_body(R, ldR, c0, K, ny, A, lda, B, ldb, Sd, ldsd, Yd, ldyd, mode, sd);
+    if ((int)blockIdx.x == (int)gridDim.x - 1) {
+        r_diag(R, ldR, c0, ny, Yd, 1, ny, Sd, mode);
+        return;
+    }
+    if (mode == 0)
+        for (int e = threadIdx.x; e < ny * ny; e += blockDim.x) {
+            const int i = e % ny, j = e / ny;
+            sd[i + j * ny] = (i <= j) ? Sd[i + (i64)j * ny] : 0.0;
+        }
+    __syncthreads();
+    const int r0 = (int)blockIdx.x * 32;
+    r_rows(R, ldR, c0, ny, A, lda, B, ldb, sd, mode, r0, min(K, r0 + 32), threadIdx.x, blockDim.x);
 }
 
-int launch_pyth_chol(const double* Om, int ldom, const double* A, int lda, int k, int nz,
-                     double* T, int ldt, int* status, int step, cudaStream_t st) {
-    if (nz <= 0) return 0;
-    if (nz > SMAX) return (int)cudaErrorInvalidValue;
-    pyth_chol_kernel<<<1, SM_THREADS, 0, st>>>(Om, ldom, A, lda, k, nz, T, ldt, status, step);
+namespace {
+
+template <class K>
+int launch_clustered(K kernel, unsigned grid, int ctas, size_t smem, cudaStream_t st, void** args) {
+    const int rc = smem > 48 * 1024 ? smem_attr((const void*)kernel, (int)smem) : 0;
+    if (rc) return rc;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(grid);
+    cfg.blockDim = dim3(ST_THREADS);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = (unsigned)ctas;
+    at[0].val.clusterDim.y = 1;
+    at[0].val.clusterDim.z = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = ctas > 1 ? 1 : 0;
+    const cudaError_t ce = cudaLaunchKernelExC(&cfg, (const void*)kernel, args);
     g_launch_count += 1;
-    return (int)cudaGetLastError();
+    return (int)(ce != cudaSuccess ? ce : cudaGetLastError());
 }
 
-int launch_scol(const double* G, int ldg, int mZ, int s, int nZ, const double* Yd, int ldy,
-                double* Scol, int ldsc, cudaStream_t st) {
-    if (nZ <= 0) return 0;
-    if (s > SMAX || nZ > SMAX) return (int)cudaErrorInvalidValue;
-    const size_t smem = (size_t)SMAX * (nZ + s) * sizeof(double);
-    const int attr_rc = smem_attr((const void*)scol_kernel, (int)(SMAX * 2 * SMAX * sizeof(double)));
-    if (attr_rc) return attr_rc;
-    scol_kernel<<<1, SM_THREADS, smem, st>>>(G, ldg, mZ, s, nZ, Yd, ldy, Scol, ldsc);
-    g_launch_count += 1;
-    return (int)cudaGetLastError();
+bool step_valid(const StepJob& J) {
+    return J.ny >= 1 && J.ny <= SMAX && J.nz >= 0 && J.nz <= SMAX && J.K >= 0 && J.G != nullptr && J.T != nullptr &&
+           (J.nz == 0 || J.S != nullptr) && (!J.scaled || J.nz == 0 || J.Sd != nullptr);
 }
 
-int launch_rblock(double* R, int ldR, int c0, int K, int ny, const double* A, int lda,
-                  const double* B, int ldb, const double* Sd, int ldsd, const double* Yd,
-                  int ldyd, int mode, cudaStream_t st) {
+}  // namespace
+
+// CTAs per job: a cluster of 8 once the products take longer on one CTA (two
+// multiply-adds per clock, the rows in one tile) than the cluster's barriers and
+// remote reads, about 2 us.
+int launch_step(const StepJob& J, cudaStream_t st) {
+    if (!step_valid(J)) return (int)cudaErrorInvalidValue;
+    const int n = J.ny + J.nz;
+    void* args[1] = {const_cast<StepJob*>(&J)};
+    if (J.K <= kTileRows && (i64)trap_size(n, n) * J.K <= 8192)
+        return launch_clustered(step_kernel<1>, 1, 1, step_smem_bytes(n, J.ny, 1), st, args);
+    return launch_clustered(step_kernel<8>, 8, 8, step_smem_bytes(n, J.ny, 8), st, args);
+}
+
+// Batched: nmax = the largest ny + nz (<= 32). Enough CTAs per job to spread a small
+// batch over the SMs; one each once the jobs alone fill them.
+int launch_step_batched(const StepJob* jobs, int njobs, int nmax, cudaStream_t st) {
+    if (njobs <= 0) return 0;
+    if (nmax < 1 || nmax > 32) return (int)cudaErrorInvalidValue;
+    void* args[1] = {(void*)&jobs};
+    if (njobs <= 64) return launch_clustered(step_batched<8>, (unsigned)njobs * 8, 8, step_smem_bytes(nmax, nmax / 2, 8), st, args);
+    if (njobs <= 512) return launch_clustered(step_batched<2>, (unsigned)njobs * 2, 2, step_smem_bytes(nmax, nmax / 2, 2), st, args);
+    return launch_clustered(step_batched<1>, (unsigned)njobs, 1, step_smem_bytes(nmax, nmax / 2, 1), st, args);
+}
+
+int launch_rblock(double* R, int ldR, int c0, int K, int ny, const double* A, int lda, const double* B, int ldb,
+                  const double* Sd, const double* Yd, int mode, cudaStream_t st) {
     if (ny <= 0) return 0;
     if (ny > SMAX) return (int)cudaErrorInvalidValue;
-    rblock_kernel<<<1, SM_THREADS, 0, st>>>(R, ldR, c0, K, ny, A, lda, B, ldb, Sd, ldsd, Yd,
-                                            ldyd, mode);
-    g_launch_count += 1;
-    return (int)cudaGetLastError();
-}
-
-// Batched form: one CTA per matrix runs that matrix's small operations of one stage
-// in order (each with the single-matrix body, so the arithmetic is the same).
-__global__ void __launch_bounds__(SM_THREADS)
-small_batched(const SmallJob* __restrict__ jobs) {
-    __shared__ double sm[SMAX * SMAX];
-    const SmallJob& J = jobs[blockIdx.x];
-    for (int q = 0; q < J.nsub; ++q) {
-        const SmallSub& S = J.sub[q];
-        if (S.kind == kSmallPyth)
-            pyth_chol_body(S.p0, S.ld0, S.p1, S.ld1, S.a, S.b, S.out, S.ldo, J.status, S.step, sm);
-        else if (S.kind == kSmallScol)
-            scol_body(S.p0, S.ld0, S.a, S.b, S.c, S.p1, S.ld1, S.out, S.ldo, sm);
-        else if (S.kind == kSmallRblock)
-            rblock_body(J.R, J.ldR, S.a, S.b, S.c, S.p0, S.ld0, S.p1, S.ld1, S.p2, S.ld2, S.p3, S.ld3, S.d, sm);
-    }
-}
-
-int launch_small_batched(const SmallJob* jobs, int njobs, cudaStream_t st) {
-    if (njobs <= 0) return 0;
-    small_batched<<<(unsigned)njobs, SM_THREADS, 0, st>>>(jobs);
+    rblock_kernel<<<(unsigned)((K + 31) / 32 + 1), ST_THREADS, 0, st>>>(R, ldR, c0, K, ny, A, lda, B, ldb, Sd, Yd,
+                                                                        mode);
     g_launch_count += 1;
     return (int)cudaGetLastError();
 }

@@ -44,16 +44,15 @@ int split_last_error();
 // c0 == K and nc <= 64; output columns are written in groups of 32).
 int launch_gram_split(const double* X, i64 ld, i64 m, int na, int b0, int nb, double* out, int ldo,
                       char* ws, size_t ws_bytes, int num_sms, cudaStream_t st);
+// Tinv: T^{-1}, upper (ld ldt), or null for the identity.
 int launch_update_split(double* X, i64 ld, i64 m, int K, int c0, int nc, const double* S, int lds,
-                        const double* T, int ldt, char* ws, size_t ws_bytes, int num_sms,
-                        cudaStream_t st);
+                        const double* Tinv, int ldt, int num_sms, cudaStream_t st);
 
 // Fused update of the lagged one-sync variants (s, nz <= 64), in one product over
-// X[:, 0:K+s+nz]: X[:, K:K+s] = (U_k - Q Y) Ty^{-1} (Y = G[0:K, 0:s]) and
-// X[:, K+s:K+s+nz] = (X_{k+1} - [Q Q_k] S') Ts^{-1} (S' = Sp, K+s rows; Ts may be null).
+// X[:, 0:K+s+nz]: [Q_k U_{k+1}] = (X[:, K:K+s+nz] - X[:, 0:K] G[0:K, 0:s+nz]) Uinv, Uinv the
+// (s+nz) x (s+nz) inverse of the step's joint factor (StepJob).
 int launch_fused_update_split(double* X, i64 ld, i64 m, int K, int s, int nz, const double* G, int ldg,
-                              const double* Ty, const double* Sp, int ldsp, const double* Ts, int num_sms,
-                              cudaStream_t st);
+                              const double* Uinv, int num_sms, cudaStream_t st);
 
 // Staged split-precision batches (BCGSI+P-1S, s <= 16): one launch per stage for
 // all matrices of a wave, each wave one captured graph (split_bf16.cu).

@@ -291,190 +291,124 @@ slice_kernel(const double* __restrict__ X, i64 ld, i64 m, int n, int c0, int nc,
 }
 
 
-// Right-hand factor of the update, scaled: Bp[c + j*ldb] for c < K + nc, j < nc:
-//   c <  K : -(S T^{-1})[c, j] * 2^{cexp[c]}      (or -S[c, j] * 2^{cexp[c]} if T is null)
-//   c >= K :  T^{-1}[c-K, j]   * 2^{cexp[c]}      (or the identity)
-// and the per-column max |Bp| into bmax (bit patterns).
-__device__ __forceinline__ void bbuild_body(const double* __restrict__ S, int lds, const double* __restrict__ T,
-                                            int ldt, int K, int nc, const int* __restrict__ cexp,
+// Right-hand factor of an update, scaled. With A = G[0:K, 0:n] and the n x n upper
+// triangular inverse Ui (ld ldu; null for the identity), row c of
+//   [ -A Ui ]  c <  K
+//   [   Ui  ]  K <= c < K + n
+// times 2^cexp[c] goes to Bp[c + j*ldb], j < n, and the per-column max |Bp| to bmax
+// (bit patterns). This is the factor of one update (X_c - Q S) T^{-1} (A = S,
+// Ui = T^{-1}) and of the fused one of the lagged variants: with U the joint
+// Cholesky factor of the step (StepJob), [Q_k U_{k+1}] = ([U_k X_{k+1}] - Q G) U^{-1}.
+// K n^2 / 2 multiply-adds, spread over CTAs of BB_ROWS rows; a warp holds BB_ROWS
+// rows of two columns, so each Ui entry is one broadcast load.
+constexpr int BB_ROWS = 16;
+constexpr int BB_THREADS = 256;
+
+__device__ __forceinline__ void bbuild_body(const double* __restrict__ G, int ldg, const double* __restrict__ Ui,
+                                            int ldu, int K, int n, const int* __restrict__ cexp,
                                             double* __restrict__ Bp, int ldb, unsigned long long* __restrict__ bmax,
                                             int bx) {
-    __shared__ double ti[64][65];
+    __shared__ double g[BB_ROWS][2 * 64 + 1];
     const int tid = threadIdx.x;
-    // T^{-1} (upper, nc x nc, nc <= 64): column j solves T y = e_j by back substitution.
-    if (T != nullptr) {
-        if (tid < nc) {
-            const int j = tid;
-            for (int i = nc - 1; i >= 0; --i) {
-                double v = (i == j) ? 1.0 : 0.0;
-                for (int l = i + 1; l <= j; ++l) v -= T[i + (i64)l * ldt] * ti[l][j];
-                ti[i][j] = (i <= j) ? v / T[i + (i64)i * ldt] : 0.0;
-            }
-        }
-    } else {
-        for (int e = tid; e < 64 * 64; e += blockDim.x) ti[e / 64][e % 64] = (e / 64 == e % 64) ? 1.0 : 0.0;
+    const int c0 = bx * BB_ROWS;
+    for (int e = tid; e < BB_ROWS * n; e += BB_THREADS) {
+        const int rr = e % BB_ROWS, q = e / BB_ROWS;
+        g[rr][q] = c0 + rr < K ? G[c0 + rr + (i64)q * ldg] : 0.0;
     }
     __syncthreads();
-    const int c = bx * 64 + (tid & 63);
-    for (int j = tid >> 6; j < nc; j += 4) {
+    const int rr = tid % BB_ROWS, c = c0 + rr;
+    const int kin = K + n;
+    const int e2 = c < kin ? cexp[c] : 0;
+    for (int j0 = 0; j0 < n; j0 += BB_THREADS / BB_ROWS) {
+        const int j = j0 + tid / BB_ROWS;
         double v = 0.0;
-        if (c < K) {
-            if (T != nullptr) {
-                for (int l = 0; l <= j; ++l) v -= S[c + (i64)l * lds] * ti[l][j];
+        if (j < n && c < K) {
+            if (Ui != nullptr) {
+                const double* u = Ui + (i64)j * ldu;
+#pragma unroll 4
+                for (int q = 0; q <= j; ++q) v = fma(-g[rr][q], u[q], v);
             } else {
-                v = -S[c + (i64)j * lds];
+                v = -g[rr][j];
             }
-        } else if (c < K + nc) {
-            v = ti[c - K][j];
+        } else if (j < n && c < kin) {
+            if (Ui != nullptr) v = c - K <= j ? Ui[(c - K) + (i64)j * ldu] : 0.0;
+            else v = c - K == j ? 1.0 : 0.0;
         }
-        if (c < K + nc) {
-            v = ldexp(v, cexp[c]);
+        unsigned long long b = 0;
+        if (j < n && c < kin) {
+            v = ldexp(v, e2);
             Bp[c + (i64)j * ldb] = v;
-            unsigned long long b = (unsigned long long)__double_as_longlong(v) & 0x7FFFFFFFFFFFFFFFULL;
+            b = (unsigned long long)__double_as_longlong(v) & 0x7FFFFFFFFFFFFFFFULL;
             if ((b >> 52) == 0x7FF) b = 0;
-            atomicMax(bmax + j, b);
         }
+#pragma unroll
+        for (int o = BB_ROWS / 2; o > 0; o >>= 1) {
+            const unsigned long long w = __shfl_xor_sync(0xffffffffu, b, o);
+            b = b > w ? b : w;
+        }
+        if (rr == 0 && j < n && b) atomicMax(bmax + j, b);
     }
 }
 
-__global__ void __launch_bounds__(256)
-bbuild_kernel(const double* __restrict__ S, int lds, const double* __restrict__ T, int ldt, int K, int nc,
-              const int* __restrict__ cexp, double* __restrict__ Bp, int ldb,
-              unsigned long long* __restrict__ bmax) {
-    bbuild_body(S, lds, T, ldt, K, nc, cexp, Bp, ldb, bmax, (int)blockIdx.x);
+__global__ void __launch_bounds__(BB_THREADS)
+bbuild_kernel(const double* __restrict__ G, int ldg, const double* __restrict__ Ui, int ldu, int K, int n,
+              const int* __restrict__ cexp, double* __restrict__ Bp, int ldb, unsigned long long* __restrict__ bmax) {
+    bbuild_body(G, ldg, Ui, ldu, K, n, cexp, Bp, ldb, bmax, (int)blockIdx.x);
 }
 
-// Right-hand factor of the fused update of the lagged one-sync variants. With
-// Q = X[:, 0:K], U_k = X[:, K:K+s], X_{k+1} = X[:, K+s:K+s+nz] it produces, in one
-// product over those K + s + nz columns,
-//   Q_k     = (U_k - Q Y) Ty^{-1}                      (columns j < s)
-//   U_{k+1} = (X_{k+1} - [Q Q_k] S') Ts^{-1}           (columns s + l, l < nz)
-// by substituting Q_k into the second line: with M = Ty^{-1} S'_mid and W = Ts^{-1},
-//   rows of Q:        [-Y Ty^{-1}        | (-S'_top + Y M) W]
-//   rows of U_k:      [ Ty^{-1}          | -M W             ]
-//   rows of X_{k+1}:  [ 0                |  W               ]
-// (Y = G[0:K, 0:s], S' = [S'_top; S'_mid] of K + s rows; W = I when Ts is null, the
-// unscaled first pass of bcgsi21s). Rows are scaled by 2^cexp[c]; bmax collects
-// the column maxima.
-__device__ __forceinline__ void bbuild_fused_body(const double* __restrict__ G, int ldg, int K, int s,
-                                                  const double* __restrict__ Ty, int ldty,
-                                                  const double* __restrict__ Sp, int ldsp,
-                                                  const double* __restrict__ Ts, int ldts, int nz,
-                                                  const int* __restrict__ cexp, double* __restrict__ Bp, int ldb,
-                                                  unsigned long long* __restrict__ bmax, int bx, double* fsm) {
-    // Ty^{-1} (s x s), Ts^{-1} (nz x nz) and M (s x nz) in shared memory (fsm),
-    // row stride FW = 65 (s, nz <= 64).
-    constexpr int FW = 65;
-    double* w1 = fsm;
-    double* w2 = fsm + 64 * FW;
-    double* mm = fsm + 2 * 64 * FW;
-#define W1(i, j) w1[(i) * FW + (j)]
-#define W2(i, j) w2[(i) * FW + (j)]
-#define MM(i, j) mm[(i) * FW + (j)]
-    const int tid = threadIdx.x;
-    // Ty^{-1} and Ts^{-1} (upper), one column per thread (threads 0..63 and 64..127).
-    if (tid < s) {
-        const int j = tid;
-        for (int i = s - 1; i >= 0; --i) {
-            double v = (i == j) ? 1.0 : 0.0;
-            for (int l = i + 1; l <= j; ++l) v -= Ty[i + (i64)l * ldty] * W1(l, j);
-            W1(i, j) = (i <= j) ? v / Ty[i + (i64)i * ldty] : 0.0;
-        }
-    } else if (tid >= 64 && tid < 64 + nz) {
-        const int j = tid - 64;
-        for (int i = nz - 1; i >= 0; --i) {
-            double v = (i == j) ? 1.0 : 0.0;
-            if (Ts != nullptr) {
-                for (int l = i + 1; l <= j; ++l) v -= Ts[i + (i64)l * ldts] * W2(l, j);
-                W2(i, j) = (i <= j) ? v / Ts[i + (i64)i * ldts] : 0.0;
-            } else {
-                W2(i, j) = v;
-            }
-        }
-    }
-    __syncthreads();
-    // M = Ty^{-1} S'_mid  (s x nz)
-    for (int e = tid; e < s * nz; e += blockDim.x) {
-        const int a = e % s, l = e / s;
-        double v = 0.0;
-        for (int b = a; b < s; ++b) v += W1(a, b) * Sp[(K + b) + (i64)l * ldsp];
-        MM(a, l) = v;
-    }
-    __syncthreads();
-    const int kin = K + s + nz, nout = s + nz;
-    const int c = bx * 64 + (tid & 63);
-    if (c >= kin) return;
-    for (int j = tid >> 6; j < nout; j += 4) {
-        double v = 0.0;
-        if (j < s) {
-            if (c < K) {
-                for (int l = 0; l <= j; ++l) v -= G[c + (i64)l * ldg] * W1(l, j);
-            } else if (c < K + s) {
-                v = W1(c - K, j);
-            }
-        } else {
-            const int l = j - s;
-            if (c < K) {
-                for (int q = 0; q <= l; ++q) {
-                    double tq = -Sp[c + (i64)q * ldsp];
-                    for (int a = 0; a < s; ++a) tq += G[c + (i64)a * ldg] * MM(a, q);
-                    v += tq * W2(q, l);
-                }
-            } else if (c < K + s) {
-                for (int q = 0; q <= l; ++q) v -= MM(c - K, q) * W2(q, l);
-            } else {
-                v = W2(c - K - s, l);
-            }
-        }
-        v = ldexp(v, cexp[c]);
-        Bp[c + (i64)j * ldb] = v;
-        unsigned long long b = (unsigned long long)__double_as_longlong(v) & 0x7FFFFFFFFFFFFFFFULL;
-        if ((b >> 52) == 0x7FF) b = 0;
-        atomicMax(bmax + j, b);
-    }
-}
+// Output columns of an update go in groups of at most 32; group gi holds columns
+// [32 gi, 32 gi + width) in NB = 16 or 32 columns of the tensor-core product.
+__host__ __device__ inline int upd_group_width(int nout, int gi) { return nout - 32 * gi < 32 ? nout - 32 * gi : 32; }
+__host__ __device__ inline int upd_group_nb(int nout, int gi) { return upd_group_width(nout, gi) <= 16 ? 16 : 32; }
 
-__global__ void __launch_bounds__(256)
-bbuild_fused_kernel(const double* __restrict__ G, int ldg, int K, int s, const double* __restrict__ Ty,
-                    int ldty, const double* __restrict__ Sp, int ldsp, const double* __restrict__ Ts,
-                    int ldts, int nz, const int* __restrict__ cexp, double* __restrict__ Bp, int ldb,
-                    unsigned long long* __restrict__ bmax) {
-    extern __shared__ double fsm[];
-    bbuild_fused_body(G, ldg, K, s, Ty, ldty, Sp, ldsp, Ts, ldts, nz, cexp, Bp, ldb, bmax, (int)blockIdx.x, fsm);
-}
+// Digits of the right-hand factor (kin x nout): group gi's at
+// bdig[gi][plane][j][c] (K-major, NB columns, zero padded to (NB, Kpad); group
+// stride KD_MAX * 32 * Kpad), and fexp[32 gi + j] = its column scale exponents. One
+// element per thread, in CTAs of BD_C inner x BD_J output columns, so that the few
+// thousand elements fill the chip. The first CTA also clears what the update that
+// follows accumulates into: the output columns' maxima cmax and tile_ctr, a counter
+// per group.
+constexpr int BD_C = 64, BD_J = 4;
 
-#undef W1
-#undef W2
-#undef MM
-
-// Digits of the right-hand factor: bdig[plane][j][c] (K-major), zero padded to
-// (NB rows, Kpad columns); fexp[j] = its column scale exponent.
 template <int KD>
-__device__ __forceinline__ void bdigit_body(const double* __restrict__ Bp, int ldb, int K, int nc, int NB, int Kpad,
+__device__ __forceinline__ void bdigit_body(const double* __restrict__ Bp, int ldb, int kin, int nout, int Kpad,
                                             const unsigned long long* __restrict__ bmax, int* __restrict__ fexp,
-                                            unsigned short* __restrict__ bdig, int bx) {
-    const int c = bx * blockDim.x + threadIdx.x;
-    if (bx == 0 && threadIdx.x < NB) fexp[threadIdx.x] = threadIdx.x < nc ? scale_exp(bmax[threadIdx.x]) : 0;
-    if (c >= Kpad) return;
-    for (int j = 0; j < NB; ++j) {
-        int d[KD];
-        if (c < K + nc && j < nc) {
-            split_digits<KD>(Bp[c + (i64)j * ldb], scale_exp(bmax[j]), d);
-        } else {
-#pragma unroll
-            for (int i = 0; i < KD; ++i) d[i] = 0;
-        }
-#pragma unroll
-        for (int i = 0; i < KD; ++i) bdig[((i64)i * NB + j) * Kpad + c] = bf16_bits_of_int(d[i]);
+                                            unsigned short* __restrict__ bdig, unsigned long long* __restrict__ cmax,
+                                            int* __restrict__ tile_ctr, int bx) {
+    const int t = threadIdx.x;
+    if (bx == 0) {
+        if (t < 128) fexp[t] = t < nout ? scale_exp(bmax[t]) : 0;
+        if (t < nout) cmax[t] = 0ULL;
+        if (tile_ctr != nullptr && t < 4) tile_ctr[t] = 0;
     }
+    const int ncb = Kpad / BD_C;
+    const int c = (bx % ncb) * BD_C + t % BD_C;
+    const int jg = (bx / ncb) * BD_J + t / BD_C;   // column, groups counted in 32s
+    const int gi = jg / 32, j = jg % 32;
+    const int NB = upd_group_nb(nout, gi);
+    if (j >= NB) return;
+    int d[KD];
+    if (c < kin && jg < nout) {
+        split_digits<KD>(Bp[c + (i64)jg * ldb], scale_exp(bmax[jg]), d);
+    } else {
+#pragma unroll
+        for (int i = 0; i < KD; ++i) d[i] = 0;
+    }
+    unsigned short* out = bdig + (i64)gi * KD_MAX * 32 * Kpad;
+#pragma unroll
+    for (int i = 0; i < KD; ++i) out[((i64)i * NB + j) * Kpad + c] = bf16_bits_of_int(d[i]);
+}
+__host__ __device__ inline int bdigit_ctas(int nout, int Kpad) {
+    const int groups = (nout + 31) / 32;
+    return (Kpad / BD_C) * (32 * (groups - 1) + upd_group_nb(nout, groups - 1)) / BD_J;
 }
 
 template <int KD>
-__global__ void __launch_bounds__(256)
-bdigit_kernel(const double* __restrict__ Bp, int ldb, int K, int nc, int NB, int Kpad,
+__global__ void __launch_bounds__(BD_C * BD_J)
+bdigit_kernel(const double* __restrict__ Bp, int ldb, int kin, int nout, int Kpad,
               const unsigned long long* __restrict__ bmax, int* __restrict__ fexp,
-              unsigned short* __restrict__ bdig) {
-    bdigit_body<KD>(Bp, ldb, K, nc, NB, Kpad, bmax, fexp, bdig, (int)blockIdx.x);
+              unsigned short* __restrict__ bdig, unsigned long long* __restrict__ cmax, int* __restrict__ tile_ctr) {
+    bdigit_body<KD>(Bp, ldb, kin, nout, Kpad, bmax, fexp, bdig, cmax, tile_ctr, (int)blockIdx.x);
 }
 
 // ---------------------------------------------------------------------------
@@ -905,6 +839,7 @@ struct UpdateParams {
     unsigned long long* cmax;   // column max |X[:, c0 + j]| of the written block (bit patterns; the
                                 // high word only, which holds the exponent the digit scale uses)
     int* err;
+    unsigned long long* bmax;   // the factor's column maxima (128 words), cleared for the next factor
     int* tile_ctr;              // zeroed before the launch; CTAs take row tiles from it
     int kr_last;                // columns the last K chunk's A box holds: kin - 64 (chunks - 1) rounded up to 16
 };
@@ -1113,6 +1048,7 @@ update_tc_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant
                 if (lane == 0) tc::mbar_arrive(&bars->t_empty[buf]);   // one arrival per warp
             }
             if (__any_sync(0xffffffffu, !ok || abort_flag)) break;
+            if (BATCH && lt == 0 && threadIdx.x < 64 + 128) q->bmax[threadIdx.x - 64] = 0ULL;
             const i64 r = (i64)lt * TILE_M + rloc;
             double* xr = q->X + r + (i64)q->c0 * q->ld;
 #pragma unroll
@@ -1144,6 +1080,7 @@ update_tc_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant
         }
     }
     __syncthreads();
+    if (!BATCH && blockIdx.x == 0 && threadIdx.x < 128) p0.bmax[threadIdx.x] = 0ULL;
     if (!BATCH && threadIdx.x < p0.nc && s_cmax[threadIdx.x])
         atomicMax(p0.cmax + p0.c0 + threadIdx.x, s_cmax[threadIdx.x]);
     if (warp == 1) {
@@ -1212,12 +1149,14 @@ struct Plan {
     double *bfull = nullptr, *part = nullptr;
     i64 part_doubles = 0;
     // maps
-    CUtensorMap map_col_a, map_col_b, map_col_b16, map_col_u, map_bdig16, map_bdig32;
+    CUtensorMap map_col_a, map_col_b, map_col_b16, map_col_u;
+    CUtensorMap map_bdig16[4], map_bdig32[4];   // the factor's digits, per group of 32 output columns
     CUtensorMap map_col_a_part[7];   // Gram A boxes of 16, 32, ..., 112 columns (a partial last M-block)
     CUtensorMap map_col_u_part[3];   // update A boxes of 16, 32, 48 columns x two 64-row chunks
     int kd = 7;
     std::vector<char> fresh;
     std::vector<char> cmax_valid;   // cmax[c] already holds max |X[:, c]| (set by the update)
+    std::vector<char> cmax_zero;    // cmax[c] is zero
     const void* zeroed_base = nullptr;   // stores zeroed for this base and shape
     i64 zeroed_m = -1;
     int zeroed_n = -1;
@@ -1254,17 +1193,23 @@ i64 gram_part_doubles(i64 m, int n, int s, int num_sms) {
     return best + 1024;
 }
 
+constexpr int kClearHead = 8 + 128;   // words before cmax in the region cleared at the start of a run
+
 size_t layout_bytes(i64 m, int n, int s, int num_sms, Plan* out, char* base) {
     Carve cv{base};
     const i64 nrc = ceil_div(m, 64), kpad = round_up(n, 64);
     unsigned short* col = cv.take<unsigned short>((i64)KD_MAX * nrc * n * 64);
-    unsigned short* bd = cv.take<unsigned short>((i64)KD_MAX * 32 * kpad);
+    const int groups = (2 * s + 31) / 32;
+    unsigned short* bd = cv.take<unsigned short>((i64)groups * KD_MAX * 32 * kpad);
     int* cexp = cv.take<int>(n + 64);
-    int* fexp = cv.take<int>(64);
-    int* err = cv.take<int>(16);
+    int* fexp = cv.take<int>(128);
+    // Cleared together when a run begins: the error word, the factor's column
+    // maxima and the columns' maxima.
+    unsigned long long* clr = cv.take<unsigned long long>(kClearHead + n + 64);
+    int* err = reinterpret_cast<int*>(clr);
+    unsigned long long* bmax = clr + 8;
+    unsigned long long* cmax = clr + kClearHead;
     int* tctr = cv.take<int>(16);
-    unsigned long long* cmax = cv.take<unsigned long long>(n + 64);
-    unsigned long long* bmax = cv.take<unsigned long long>(128);
     double* bfull = cv.take<double>(kpad * 128);
     const i64 pd = gram_part_doubles(m, n, s, num_sms);
     double* part = cv.take<double>(pd);
@@ -1283,31 +1228,48 @@ int set_smem(K kernel, int bytes) {
     return smem_attr((const void*)kernel, bytes);
 }
 
+// Brings the digits of columns [c_begin, c_end) up to date: first the maxima of the
+// stale columns that have none (32 columns a launch), then the slicing of every run
+// of stale columns, whichever way their maxima came.
 int ensure_fresh(int c_begin, int c_end, cudaStream_t st) {
     Plan& P = cur_plan();
-    int c = c_begin;
-    while (c < c_end) {
+    for (int c = c_begin; c < c_end;) {
+        if (P.fresh[c] || P.cmax_valid[c]) { ++c; continue; }
+        int e = c;
+        while (e < c_end && !P.fresh[e] && !P.cmax_valid[e] && e - c < 32 && P.cmax_zero[e] == P.cmax_zero[c]) ++e;
+        if (!P.cmax_zero[c]) {
+            cudaError_t ce = (cudaError_t)zero_async(P.cmax + c, (size_t)(e - c) * sizeof(unsigned long long), st);
+            if (ce != cudaSuccess) return (int)ce;
+        }
+        colmax_kernel<<<dim3((unsigned)ceil_div(P.m, 4096), (unsigned)(e - c)), 256, 0, st>>>(P.X, P.ld, P.m, c, P.cmax);
+        g_launch_count += 1;
+        for (; c < e; ++c) { P.cmax_valid[c] = 1; P.cmax_zero[c] = 0; }
+    }
+    for (int c = c_begin; c < c_end;) {
         if (P.fresh[c]) { ++c; continue; }
         int e = c;
-        while (e < c_end && !P.fresh[e] && e - c < 32 && P.cmax_valid[e] == P.cmax_valid[c]) ++e;
+        while (e < c_end && !P.fresh[e]) ++e;
         const int nc = e - c;
-        if (!P.cmax_valid[c]) {
-            cudaError_t ce = (cudaError_t)zero_async(P.cmax + c, (size_t)nc * sizeof(unsigned long long), st);
-            if (ce != cudaSuccess) return (int)ce;
-            dim3 g1((unsigned)ceil_div(P.m, 4096), (unsigned)nc);
-            colmax_kernel<<<g1, 256, 0, st>>>(P.X, P.ld, P.m, c, P.cmax);
-            g_launch_count += 1;
-        }
         const dim3 sgrid((unsigned)ceil_div(P.m, 128), (unsigned)ceil_div(nc, 16));
         if (P.kd == 6)
             slice_kernel<6><<<sgrid, 128, 0, st>>>(P.X, P.ld, P.m, P.n, c, nc, P.cmax, P.cexp, P.colstore, P.nrc);
         else
             slice_kernel<7><<<sgrid, 128, 0, st>>>(P.X, P.ld, P.m, P.n, c, nc, P.cmax, P.cexp, P.colstore, P.nrc);
         g_launch_count += 1;
-        for (int k = c; k < e; ++k) { P.fresh[k] = 1; P.cmax_valid[k] = 0; }
-        c = e;
+        for (; c < e; ++c) { P.fresh[c] = 1; P.cmax_valid[c] = 0; }
     }
     return (int)cudaGetLastError();
+}
+
+// Maps of the factor's digits, one per group of 32 output columns.
+int make_bdig_maps(Plan& P, int groups) {
+    int rc = 0;
+    for (int gi = 0; gi < groups && !rc; ++gi) {
+        unsigned short* base = P.bdig + (i64)gi * KD_MAX * 32 * P.kpad;
+        rc = make_map3(&P.map_bdig16[gi], base, P.kpad, 16, KD_MAX, P.kpad, 16 * P.kpad, 16);
+        if (!rc) rc = make_map3(&P.map_bdig32[gi], base, P.kpad, 32, KD_MAX, P.kpad, 32 * P.kpad, 32);
+    }
+    return rc;
 }
 
 }  // namespace
@@ -1328,6 +1290,7 @@ int split_begin(double* X, i64 ld, i64 m, int n, int s, int kd, char* ws, size_t
     P.X = X; P.ld = ld; P.m = m; P.n = n; P.num_sms = num_sms;
     P.fresh.assign((size_t)n, 0);
     P.cmax_valid.assign((size_t)n, 0);
+    P.cmax_zero.assign((size_t)n, 1);
     // The store is zeroed whenever the workspace or the shape changes. The chunk
     // padding the slicing never writes (rows past m in the last 64-row chunk) lies
     // inside the TMA boxes and must read as zero. The rest must hold digits or
@@ -1343,7 +1306,7 @@ int split_begin(double* X, i64 ld, i64 m, int n, int s, int kd, char* ws, size_t
         P.zeroed_m = m;
         P.zeroed_n = n;
     }
-    cudaError_t ce = (cudaError_t)zero_async(P.err, sizeof(int), st);
+    cudaError_t ce = (cudaError_t)zero_async(P.err, (size_t)(kClearHead + n) * sizeof(unsigned long long), st);
     if (ce != cudaSuccess) return (int)ce;
     // Chunked stores as 3-D tensors {64, columns or rows, plane x chunk}.
     int rc = make_map3(&P.map_col_a, P.colstore, 64, n, KD_MAX * P.nrc, 64, (i64)n * 64, TILE_M);
@@ -1357,8 +1320,7 @@ int split_begin(double* X, i64 ld, i64 m, int n, int s, int kd, char* ws, size_t
         rc = make_map3(&P.map_col_a_part[q], P.colstore, 64, n, KD_MAX * P.nrc, 64, (i64)n * 64, 16 * (q + 1));
     for (int q = 0; q < 3 && !rc; ++q)
         rc = make_map3(&P.map_col_u_part[q], P.colstore, 64, n, KD_MAX * P.nrc, 64, (i64)n * 64, 16 * (q + 1), 2);
-    if (!rc) rc = make_map3(&P.map_bdig16, P.bdig, P.kpad, 16, KD_MAX, P.kpad, 16 * P.kpad, 16);
-    if (!rc) rc = make_map3(&P.map_bdig32, P.bdig, P.kpad, 32, KD_MAX, P.kpad, 32 * P.kpad, 32);
+    if (!rc) rc = make_bdig_maps(P, (2 * s + 31) / 32);
     if (rc) return rc;
     // Shared-memory limits of the tensor-core kernels on this device.
     rc = set_smem(gram_tc_kernel<32, 6, 6, false>, SmemLayout<32, 6>::BYTES);
@@ -1474,85 +1436,64 @@ int launch_gram_split(const double* X, i64 ld, i64 m, int na, int b0, int nb, do
     return launch_gram_reduce(P.part, gp.rc, na, nb, out, ldo, st);
 }
 
-// bdigit + the tensor-core product X[:, c0:c0+nc] = digits[:, 0:kin] * Bp, after the
-// caller has filled Bp/bmax.
-// Output columns go in groups of at most 32 (one tensor-core pass each). Every
-// group reads the same digit planes of X[:, 0:kin], which were sliced before the
-// first group wrote anything, and its own 32 columns of the factor in Bp.
-static int finish_update(double* X, i64 ld, i64 m, int kin, int c0, int nc, int num_sms, cudaStream_t st) {
+// The factor [-A Ui ; Ui] (bbuild_body; A = G[0:K, 0:nout]), its digits, and the
+// tensor-core product X[:, K:K+nout] = digits[:, 0:K+nout] * factor, in groups of at
+// most 32 output columns (one pass each). Every group reads the same digit planes of
+// X[:, 0:K+nout], which were sliced before the first group writes anything. bmax is
+// zero on entry and again after the product.
+static int run_update(double* X, i64 ld, i64 m, int K, int nout, const double* G, int ldg, const double* Ui, int ldu,
+                      int num_sms, cudaStream_t st) {
     Plan& P = cur_plan();
-    for (int j0 = 0; j0 < nc; j0 += 32) {
-        const int ng = nc - j0 < 32 ? nc - j0 : 32;
-        const int NB = ng <= 16 ? 16 : 32;
-        const double* Bg = P.bfull + (i64)j0 * P.kpad;
-        if (P.kd == 6)
-            bdigit_kernel<6><<<(unsigned)ceil_div(P.kpad, 256), 256, 0, st>>>(Bg, (int)P.kpad, kin - ng, ng, NB,
-                                                                               (int)P.kpad, P.bmax + j0, P.fexp,
-                                                                               P.bdig);
-        else
-            bdigit_kernel<7><<<(unsigned)ceil_div(P.kpad, 256), 256, 0, st>>>(Bg, (int)P.kpad, kin - ng, ng, NB,
-                                                                               (int)P.kpad, P.bmax + j0, P.fexp,
-                                                                               P.bdig);
-        cudaError_t ce = (cudaError_t)zero_async(P.cmax + c0 + j0, (size_t)ng * sizeof(unsigned long long), st);
-        if (ce != cudaSuccess) return (int)ce;
+    const int kin = K + nout;
+    bbuild_kernel<<<(unsigned)ceil_div(kin, BB_ROWS), BB_THREADS, 0, st>>>(G, ldg, Ui, ldu, K, nout, P.cexp, P.bfull,
+                                                                           (int)P.kpad, P.bmax);
+    const unsigned bd = (unsigned)bdigit_ctas(nout, (int)P.kpad);
+    if (P.kd == 6)
+        bdigit_kernel<6><<<bd, BD_C * BD_J, 0, st>>>(P.bfull, (int)P.kpad, kin, nout, (int)P.kpad, P.bmax, P.fexp, P.bdig,
+                                                     P.cmax + K, P.tile_ctr);
+    else
+        bdigit_kernel<7><<<bd, BD_C * BD_J, 0, st>>>(P.bfull, (int)P.kpad, kin, nout, (int)P.kpad, P.bmax, P.fexp, P.bdig,
+                                                     P.cmax + K, P.tile_ctr);
+    g_launch_count += 2;
+    for (int gi = 0; 32 * gi < nout; ++gi) {
+        const int NB = upd_group_nb(nout, gi);
         UpdateParams up;
         up.nrc = (int)P.nrc;
-        up.m = m; up.kin = kin; up.nc = ng; up.c0 = c0 + j0; up.ld = ld; up.X = X; up.fexp = P.fexp;
-        up.cmax = P.cmax; up.err = P.err; up.tile_ctr = P.tile_ctr;
+        up.m = m; up.kin = kin; up.nc = upd_group_width(nout, gi); up.c0 = K + 32 * gi; up.ld = ld; up.X = X;
+        up.fexp = P.fexp + 32 * gi;
+        up.cmax = P.cmax; up.err = P.err; up.bmax = P.bmax; up.tile_ctr = P.tile_ctr + gi;
         up.kr_last = (int)round_up(kin - (i64)(ceil_div(kin, KCH) - 1) * KCH, 16);
         const CUtensorMap& ulast_map = up.kr_last < KCH ? P.map_col_u_part[up.kr_last / 16 - 1] : P.map_col_u;
-        ce = (cudaError_t)zero_async(P.tile_ctr, sizeof(int), st);
-        if (ce != cudaSuccess) return (int)ce;
         const int ntiles = (int)ceil_div(m, TILE_M);
         const int grid = ntiles < num_sms ? ntiles : num_sms;
 #define BCGS_UPD(NBT, KDT) \
         update_tc_kernel<NBT, KDT, false><<<grid, UTHREADS, SmemLayout<NBT, KDT>::BYTES, st>>>(                 \
-            P.map_col_u, ulast_map, P.map_bdig##NBT, up, nullptr, nullptr, 0)
+            P.map_col_u, ulast_map, P.map_bdig##NBT[gi], up, nullptr, nullptr, 0)
         if (NB == 16) {
             if (P.kd == 6) BCGS_UPD(16, 6); else BCGS_UPD(16, 7);
         } else {
             if (P.kd == 6) BCGS_UPD(32, 6); else BCGS_UPD(32, 7);
         }
 #undef BCGS_UPD
-        g_launch_count += 2;
+        g_launch_count += 1;
     }
-    for (int c = c0; c < c0 + nc; ++c) { P.fresh[c] = 0; P.cmax_valid[c] = 1; }
+    for (int c = K; c < K + nout; ++c) { P.fresh[c] = 0; P.cmax_valid[c] = 1; P.cmax_zero[c] = 0; }
     return (int)cudaGetLastError();
 }
 
 int launch_update_split(double* X, i64 ld, i64 m, int K, int c0, int nc, const double* S, int lds,
-                        const double* T, int ldt, char* ws, size_t ws_bytes, int num_sms, cudaStream_t st) {
-    (void)ws; (void)ws_bytes;
-    Plan& P = cur_plan();
+                        const double* Tinv, int ldt, int num_sms, cudaStream_t st) {
     if (nc <= 0) return 0;
-    if (c0 != K || nc > 64 || X != P.X) return (int)cudaErrorInvalidValue;
-    int rc = ensure_fresh(0, K + nc, st);
-    if (rc) return rc;
-    cudaError_t ce = (cudaError_t)zero_async(P.bmax, 64 * sizeof(unsigned long long), st);
-    if (ce != cudaSuccess) return (int)ce;
-    const int kin = K + nc;
-    bbuild_kernel<<<(unsigned)ceil_div(kin, 64), 256, 0, st>>>(S, lds, T, ldt, K, nc, P.cexp, P.bfull,
-                                                                  (int)P.kpad, P.bmax);
-    g_launch_count += 1;
-    return finish_update(X, ld, m, kin, c0, nc, num_sms, st);
+    if (c0 != K || nc > 64 || X != cur_plan().X) return (int)cudaErrorInvalidValue;
+    const int rc = ensure_fresh(0, K + nc, st);
+    return rc ? rc : run_update(X, ld, m, K, nc, S, lds, Tinv, ldt, num_sms, st);
 }
 
 int launch_fused_update_split(double* X, i64 ld, i64 m, int K, int s, int nz, const double* G, int ldg,
-                              const double* Ty, const double* Sp, int ldsp, const double* Ts, int num_sms,
-                              cudaStream_t st) {
-    Plan& P = cur_plan();
-    const int kin = K + s + nz, nout = s + nz;
-    if (s > 64 || nz > 64 || X != P.X) return (int)cudaErrorInvalidValue;
-    int rc = ensure_fresh(0, kin, st);
-    if (rc) return rc;
-    cudaError_t ce = (cudaError_t)zero_async(P.bmax, 128 * sizeof(unsigned long long), st);
-    if (ce != cudaSuccess) return (int)ce;
-    const int fattr_rc = set_smem(bbuild_fused_kernel, (int)(3 * 64 * 65 * sizeof(double)));
-    if (fattr_rc) return fattr_rc;
-    bbuild_fused_kernel<<<(unsigned)ceil_div(kin, 64), 256, 3 * 64 * 65 * sizeof(double), st>>>(G, ldg, K, s, Ty, s, Sp, ldsp, Ts, nz, nz,
-                                                                        P.cexp, P.bfull, (int)P.kpad, P.bmax);
-    g_launch_count += 1;
-    return finish_update(X, ld, m, kin, K, nout, num_sms, st);
+                              const double* Uinv, int num_sms, cudaStream_t st) {
+    if (s > 64 || nz > 64 || X != cur_plan().X) return (int)cudaErrorInvalidValue;
+    const int rc = ensure_fresh(0, K + s + nz, st);
+    return rc ? rc : run_update(X, ld, m, K, s + nz, G, ldg, Uinv, s + nz, num_sms, st);
 }
 
 // ===========================================================================
@@ -1588,9 +1529,8 @@ struct SliceJob {
     unsigned short* colstore;
 };
 struct BbuildJob {
-    int fused;
-    const double *S, *T, *G, *Ty, *Sp, *Ts;
-    int lds, ldt, ldg, ldsp, K, nc, s, nz;
+    const double *G, *Ui;
+    int ldg, ldu, K, n;
     const int* cexp;
     double* Bp;
     int ldb;
@@ -1598,10 +1538,11 @@ struct BbuildJob {
 };
 struct BdigitJob {
     const double* Bp;
-    int ldb, K, nc, NB, Kpad;
+    int ldb, kin, nout, Kpad;
     const unsigned long long* bmax;
     int* fexp;
     unsigned short* bdig;
+    unsigned long long* cmax;
 };
 struct ZeroJob {
     void* p;
@@ -1625,25 +1566,22 @@ slice_batched(const SliceJob* __restrict__ jobs, const int* __restrict__ prefix,
     slice_body<KD>(J.X, J.ld, J.m, J.n, J.c0, J.nc, J.cmax, J.cexp, J.colstore, J.nrc, it % J.ntile, it / J.ntile);
 }
 
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(BB_THREADS)
 bbuild_batched(const BbuildJob* __restrict__ jobs, const int* __restrict__ prefix, int njobs) {
-    extern __shared__ double fsm[];
     const int j = batched_job_of(prefix, njobs, blockIdx.x);
     const BbuildJob& J = jobs[j];
-    const int it = blockIdx.x - prefix[j];
-    if (J.fused)
-        bbuild_fused_body(J.G, J.ldg, J.K, J.s, J.Ty, J.s, J.Sp, J.ldsp, J.Ts, J.nz, J.nz, J.cexp, J.Bp, J.ldb,
-                          J.bmax, it, fsm);
-    else
-        bbuild_body(J.S, J.lds, J.T, J.ldt, J.K, J.nc, J.cexp, J.Bp, J.ldb, J.bmax, it);
+    bbuild_body(J.G, J.ldg, J.Ui, J.ldu, J.K, J.n, J.cexp, J.Bp, J.ldb, J.bmax, blockIdx.x - prefix[j]);
 }
 
+// tile_ctr: the launch's counters of the two updates that follow.
 template <int KD>
-__global__ void __launch_bounds__(256)
-bdigit_batched(const BdigitJob* __restrict__ jobs, const int* __restrict__ prefix, int njobs) {
+__global__ void __launch_bounds__(BD_C * BD_J)
+bdigit_batched(const BdigitJob* __restrict__ jobs, const int* __restrict__ prefix, int njobs, int* tile_ctr) {
+    if (blockIdx.x == 0 && threadIdx.x < 2) tile_ctr[threadIdx.x] = 0;
     const int j = batched_job_of(prefix, njobs, blockIdx.x);
     const BdigitJob& J = jobs[j];
-    bdigit_body<KD>(J.Bp, J.ldb, J.K, J.nc, J.NB, J.Kpad, J.bmax, J.fexp, J.bdig, blockIdx.x - prefix[j]);
+    bdigit_body<KD>(J.Bp, J.ldb, J.kin, J.nout, J.Kpad, J.bmax, J.fexp, J.bdig, J.cmax, nullptr,
+                    blockIdx.x - prefix[j]);
 }
 
 __global__ void __launch_bounds__(256) zero_list(const ZeroJob* __restrict__ jobs) {
@@ -1657,8 +1595,6 @@ __global__ void spread_error(const int* __restrict__ err, int* __restrict__ dsta
     const int b = blockIdx.x * blockDim.x + threadIdx.x;
     if (b < count) dstatus[8 * (i64)b + 4] = *err;
 }
-
-constexpr size_t kBbuildSmem = 3 * 64 * 65 * sizeof(double);
 
 enum SKind {
     kSZero, kSColmax, kSSlice, kSGram, kSGram16, kSReduce, kSSmall, kSBbuild, kSBdigit, kSUpdate, kSUpdate16, kSTile, kSRoot,
@@ -1694,10 +1630,10 @@ struct SMat {
     int* status;
     size_t off = 0, bytes = 0;   // its region of the wave buffer
     Plan P;                      // digit store, maps and freshness (as a single run's)
-    double *G1 = nullptr, *G2 = nullptr, *Scol = nullptr, *Sd = nullptr, *Yd = nullptr, *tsqr = nullptr;
+    double *G1 = nullptr, *G2 = nullptr, *Scol[2] = {}, *Sd[2] = {}, *Yd = nullptr, *Uinv = nullptr, *tsqr = nullptr;
 };
 
-i64 smat_small_doubles(int n, int s) { return 2LL * (n + s) * 2 * s + (i64)n * s + 3LL * s * s + 64; }
+i64 smat_small_doubles(int n, int s) { return 2LL * (n + s) * 2 * s + 2LL * n * s + 7LL * s * s + 64; }
 
 // Bytes of one matrix's region of the wave buffer (digit store, factor, Gram
 // partials, FP64 small blocks, TSQR stack); with base != nullptr also carves it.
@@ -1713,10 +1649,12 @@ size_t smat_layout(SMat& M, int num_sms, char* base) {
         const int n = M.n, s = M.s;
         M.G1 = sb;
         M.G2 = M.G1 + (i64)(n + s) * 2 * s;
-        M.Scol = M.G2 + (i64)(n + s) * 2 * s;
-        double* S0 = M.Scol + (i64)n * s;
-        M.Sd = S0 + (i64)s * s;
-        M.Yd = M.Sd + (i64)s * s;
+        M.Scol[0] = M.G2 + (i64)(n + s) * 2 * s;
+        M.Scol[1] = M.Scol[0] + (i64)n * s;
+        M.Sd[0] = M.Scol[1] + (i64)n * s;
+        M.Sd[1] = M.Sd[0] + (i64)s * s;
+        M.Yd = M.Sd[1] + (i64)s * s;
+        M.Uinv = M.Yd + (i64)s * s;
         M.tsqr = tw;
     }
     return off + 1024;
@@ -1768,6 +1706,7 @@ int plan_wave(SplitStaged& S, SWave& W) {
         P.X = M.X; P.ld = M.ld; P.m = M.m; P.n = M.n; P.num_sms = S.num_sms;
         P.fresh.assign((size_t)M.n, 0);
         P.cmax_valid.assign((size_t)M.n, 0);
+        P.cmax_zero.assign((size_t)M.n, 1);
         if (S.device) {
             const int n = M.n;
             int rc = make_map3(&P.map_col_a, P.colstore, 64, n, KD_MAX * P.nrc, 64, (i64)n * 64, TILE_M);
@@ -1779,8 +1718,7 @@ int plan_wave(SplitStaged& S, SWave& W) {
             for (int q = 0; q < 3 && !rc; ++q)
                 rc = make_map3(&P.map_col_u_part[q], P.colstore, 64, n, KD_MAX * P.nrc, 64, (i64)n * 64, 16 * (q + 1),
                                2);
-            if (!rc) rc = make_map3(&P.map_bdig16, P.bdig, P.kpad, 16, KD_MAX, P.kpad, 16 * P.kpad, 16);
-            if (!rc) rc = make_map3(&P.map_bdig32, P.bdig, P.kpad, 32, KD_MAX, P.kpad, 32 * P.kpad, 32);
+            if (!rc) rc = make_bdig_maps(P, 1);
             if (rc) return rc;
         }
     }
@@ -1819,23 +1757,24 @@ int plan_wave(SplitStaged& S, SWave& W) {
     // ensure_fresh of one matrix, as jobs.
     auto prepare = [&](SMat& M, int c_end) {
         Plan& P = M.P;
-        int c = 0;
-        while (c < c_end) {
+        for (int c = 0; c < c_end;) {
+            if (P.fresh[c] || P.cmax_valid[c]) { ++c; continue; }
+            int e = c;
+            while (e < c_end && !P.fresh[e] && !P.cmax_valid[e] && e - c < 32 && P.cmax_zero[e] == P.cmax_zero[c]) ++e;
+            if (!P.cmax_zero[c]) zj.push_back({P.cmax + c, (int)((e - c) * sizeof(unsigned long long))});
+            const int nrb = (int)ceil_div(P.m, 4096);
+            cj.push_back({P.X, P.ld, P.m, c, nrb, P.cmax});
+            cc.push_back(nrb * (e - c));
+            for (; c < e; ++c) { P.cmax_valid[c] = 1; P.cmax_zero[c] = 0; }
+        }
+        for (int c = 0; c < c_end;) {
             if (P.fresh[c]) { ++c; continue; }
             int e = c;
-            while (e < c_end && !P.fresh[e] && e - c < 32 && P.cmax_valid[e] == P.cmax_valid[c]) ++e;
-            const int nc = e - c;
-            if (!P.cmax_valid[c]) {
-                zj.push_back({P.cmax + c, (int)(nc * sizeof(unsigned long long))});
-                const int nrb = (int)ceil_div(P.m, 4096);
-                cj.push_back({P.X, P.ld, P.m, c, nrb, P.cmax});
-                cc.push_back(nrb * nc);
-            }
+            while (e < c_end && !P.fresh[e]) ++e;
             const int ntile = (int)ceil_div(P.m, 128);
-            sj.push_back({P.X, P.ld, P.m, P.nrc, P.n, c, nc, ntile, P.cmax, P.cexp, P.colstore});
-            sc.push_back(ntile * (int)ceil_div(nc, 16));
-            for (int k = c; k < e; ++k) { P.fresh[k] = 1; P.cmax_valid[k] = 0; }
-            c = e;
+            sj.push_back({P.X, P.ld, P.m, P.nrc, P.n, c, e - c, ntile, P.cmax, P.cexp, P.colstore});
+            sc.push_back(ntile * (int)ceil_div(e - c, 16));
+            for (; c < e; ++c) { P.fresh[c] = 1; P.cmax_valid[c] = 0; }
         }
     };
 
@@ -1875,7 +1814,7 @@ int plan_wave(SplitStaged& S, SWave& W) {
         GramJob R{};
         R.na = na; R.nb = nb; R.nchunks = gp.rc; R.part = P.part; R.C = C; R.ldc = ldc;
         rj.push_back(R);
-        rc2.push_back((int)ceil_div((i64)na * nb, 256));
+        rc2.push_back(gram_reduce_ctas(na, nb));
     };
     auto flush_gram = [&]() {
         flush_prepare();
@@ -1885,101 +1824,62 @@ int plan_wave(SplitStaged& S, SWave& W) {
         gj.clear(); gc.clear(); gj16.clear(); gc16.clear(); rj.clear(); rc2.clear();
     };
 
-    std::vector<SmallJob> smj;
+    std::vector<StepJob> smj;
     auto flush_small = [&]() {
         if (smj.empty()) return;
         std::vector<int> ones(smj.size(), 1);
         push(kSSmall, smj, ones);
         smj.clear();
     };
-    auto pyth = [](const double* Om, int ldom, const double* A, int lda, int k, int nz, double* T, int step) {
-        SmallSub X{};
-        X.kind = kSmallPyth;
-        X.p0 = Om; X.ld0 = ldom; X.p1 = A; X.ld1 = lda; X.a = k; X.b = nz; X.out = T; X.ldo = nz; X.step = step;
-        return X;
-    };
-    auto scol = [](const double* G, int ldg, int mZ, int s, int nZ, const double* Yd, double* Scol) {
-        SmallSub X{};
-        X.kind = kSmallScol;
-        X.p0 = G; X.ld0 = ldg; X.a = mZ; X.b = s; X.c = nZ; X.p1 = Yd; X.ld1 = s; X.out = Scol; X.ldo = mZ + s;
-        return X;
-    };
-    auto rblock = [](int c0, int K, int ny, const double* A, int lda, const double* Bm, int ldb, const double* Sd,
-                     const double* Yd) {
-        SmallSub X{};
-        X.kind = kSmallRblock;
-        X.a = c0; X.b = K; X.c = ny; X.d = 0;
-        X.p0 = A; X.ld0 = lda; X.p1 = Bm; X.ld1 = ldb; X.p2 = Sd; X.ld2 = ny; X.p3 = Yd; X.ld3 = ny;
-        return X;
+    // Engine::factor.
+    auto factor = [](const SMat& M, const double* G, int ldg, int K, int ny, double* T, int step) {
+        StepJob J;
+        J.G = G; J.ldg = ldg; J.K = K; J.ny = ny; J.T = T; J.step = step;
+        J.R = M.R; J.ldR = M.ldR; J.status = M.status; J.Uinv = M.Uinv;
+        return J;
     };
 
-    std::vector<ZeroJob> uz;
     std::vector<BbuildJob> bj;
     std::vector<int> bc;
     std::vector<BdigitJob> dj;
     std::vector<int> dc;
     std::vector<SplitUpdJob> uj, uj16;
     std::vector<int> ut, ut16;
-    // finish_update for one matrix: kin digit columns in, nout (<= 32) columns out at
-    // c0; as finish_update, 16-column tiles when nout <= 16 (blocks of s <= 8), each
-    // width one batched launch.
-    auto finish = [&](SMat& M, int kin, int c0, int nout) {
+    // launch_update_split and launch_fused_update_split for one matrix (run_update):
+    // X[:, K:K+nout] = [Q X] [-G Ui ; Ui], nout <= 32; as there, 16-column tiles when
+    // nout <= 16 (blocks of s <= 8), each width one batched launch.
+    auto update = [&](SMat& M, int K, int nout, const double* G, int ldg, const double* Ui, int ldu) {
+        const int kin = K + nout;
+        prepare(M, kin);
         Plan& P = M.P;
-        const int NB = nout <= 16 ? 16 : 32;
-        dj.push_back({P.bfull, (int)P.kpad, kin - nout, nout, NB, (int)P.kpad, P.bmax, P.fexp, P.bdig});
-        dc.push_back((int)ceil_div(P.kpad, 256));
-        uz.push_back({P.cmax + c0, (int)(nout * sizeof(unsigned long long))});
+        bj.push_back({G, Ui, ldg, ldu, K, nout, P.cexp, P.bfull, (int)P.kpad, P.bmax});
+        bc.push_back((int)ceil_div(kin, BB_ROWS));
+        const int NB = upd_group_nb(nout, 0);
+        dj.push_back({P.bfull, (int)P.kpad, kin, nout, (int)P.kpad, P.bmax, P.fexp, P.bdig, P.cmax + K});
+        dc.push_back(bdigit_ctas(nout, (int)P.kpad));
         UpdateParams up{};
         up.nrc = (int)P.nrc;
-        up.m = P.m; up.kin = kin; up.nc = nout; up.c0 = c0; up.ld = P.ld; up.X = P.X; up.fexp = P.fexp;
-        up.cmax = P.cmax; up.err = nullptr; up.tile_ctr = nullptr;
+        up.m = P.m; up.kin = kin; up.nc = nout; up.c0 = K; up.ld = P.ld; up.X = P.X; up.fexp = P.fexp;
+        up.cmax = P.cmax; up.err = nullptr; up.bmax = P.bmax; up.tile_ctr = nullptr;
         up.kr_last = (int)round_up(kin - (i64)(ceil_div(kin, KCH) - 1) * KCH, 16);
         SplitUpdJob J;
         std::memset(&J, 0, sizeof(J));
         J.mapA = P.map_col_u;
         J.mapAlast = up.kr_last < KCH ? P.map_col_u_part[up.kr_last / 16 - 1] : P.map_col_u;
-        J.mapB = NB == 16 ? P.map_bdig16 : P.map_bdig32;
+        J.mapB = NB == 16 ? P.map_bdig16[0] : P.map_bdig32[0];
         J.p = up;
         (NB == 16 ? uj16 : uj).push_back(J);
         (NB == 16 ? ut16 : ut).push_back((int)ceil_div(P.m, TILE_M));
-        for (int c = c0; c < c0 + nout; ++c) { P.fresh[c] = 0; P.cmax_valid[c] = 1; }
-    };
-    // Engine::update (launch_update_split): X[:, c0:c0+nc] = (X_c - X[:, 0:K] S) T^{-1}, c0 == K.
-    auto update = [&](SMat& M, int K, int c0, int nc, const double* Sm, int lds, const double* T, int ldt) {
-        prepare(M, K + nc);
-        Plan& P = M.P;
-        uz.push_back({P.bmax, (int)(64 * sizeof(unsigned long long))});
-        BbuildJob B{};
-        B.fused = 0; B.S = Sm; B.lds = lds; B.T = T; B.ldt = ldt; B.K = K; B.nc = nc;
-        B.cexp = P.cexp; B.Bp = P.bfull; B.ldb = (int)P.kpad; B.bmax = P.bmax;
-        bj.push_back(B);
-        bc.push_back((int)ceil_div(K + nc, 64));
-        finish(M, K + nc, c0, nc);
-    };
-    // Engine::fused_update (launch_fused_update_split).
-    auto fused = [&](SMat& M, int K, int nz, const double* G, int ldg, const double* Ty, const double* Sp,
-                     const double* Ts) {
-        const int s = M.s;
-        prepare(M, K + s + nz);
-        Plan& P = M.P;
-        uz.push_back({P.bmax, (int)(128 * sizeof(unsigned long long))});
-        BbuildJob B{};
-        B.fused = 1; B.G = G; B.ldg = ldg; B.K = K; B.s = s; B.Ty = Ty; B.Sp = Sp; B.ldsp = K + s; B.Ts = Ts;
-        B.nz = nz; B.cexp = P.cexp; B.Bp = P.bfull; B.ldb = (int)P.kpad; B.bmax = P.bmax;
-        bj.push_back(B);
-        bc.push_back((int)ceil_div(K + s + nz, 64));
-        finish(M, K + s + nz, K, s + nz);
+        for (int c = K; c < K + nout; ++c) { P.fresh[c] = 0; P.cmax_valid[c] = 1; P.cmax_zero[c] = 0; }
     };
     auto flush_update = [&]() {
         flush_prepare();
         if (uj.empty() && uj16.empty()) return;
-        if (S.device) uz.push_back({S.dtile, (int)(2 * sizeof(int))});   // both launches' tile counters
-        push_zero(uz);
         push(kSBbuild, bj, bc);
         push(kSBdigit, dj, dc);
         if (!uj.empty()) push(kSUpdate, uj, ut);
         if (!uj16.empty()) push(kSUpdate16, uj16, ut16);
-        uz.clear(); bj.clear(); bc.clear(); dj.clear(); dc.clear(); uj.clear(); ut.clear(); uj16.clear(); ut16.clear();
+        bj.clear(); bc.clear(); dj.clear(); dc.clear(); uj.clear(); ut.clear(); uj16.clear(); ut16.clear();
     };
 
     // ---- TSQR of block 1 (the single-panel tree of launch_tsqr, per matrix) ----
@@ -2075,16 +1975,12 @@ int plan_wave(SplitStaged& S, SWave& W) {
     flush_gram();
     for (int k = 0; k < B; ++k) {
         SMat& M = S.mats[W.mats[k]];
-        SmallJob J{};
-        J.status = M.status; J.R = M.R; J.ldR = M.ldR;
-        J.sub[0] = pyth(M.G2 + M.s, 2 * M.s, M.G2, 2 * M.s, M.s, M.s, M.Sd, 1);
-        J.nsub = 1;
-        smj.push_back(J);
+        smj.push_back(factor(M, M.G2, 2 * M.s, M.s, M.s, M.Sd[0], 1));
     }
     flush_small();
     for (int k = 0; k < B; ++k) {
         SMat& M = S.mats[W.mats[k]];
-        update(M, M.s, M.s, M.s, M.G2, 2 * M.s, M.Sd, M.s);
+        update(M, M.s, M.s, M.G2, 2 * M.s, M.Uinv, M.s);
     }
     flush_update();
     // Phase 1: the first synchronization of Q_2 (:127-147), then Q_2 and U_3.
@@ -2101,25 +1997,17 @@ int plan_wave(SplitStaged& S, SWave& W) {
     for (int k = 0; k < B; ++k) {
         SMat& M = S.mats[W.mats[k]];
         const int s = M.s;
-        SmallJob J{};
-        J.status = M.status; J.R = M.R; J.ldR = M.ldR;
-        J.sub[0] = pyth(M.G1 + s, ldg[k], M.G1, ldg[k], s, s, M.Yd, 1);
-        J.sub[1] = rblock(s, s, s, M.G2, 2 * s, M.G1, ldg[k], M.Sd, M.Yd);
-        J.nsub = 2;
-        if (M.p > 1) {
-            const int mScolN = mZ[k] + s;
-            J.sub[2] = scol(M.G1, ldg[k], mZ[k], s, nZ[k], M.Yd, M.Scol);
-            J.sub[3] = pyth(M.G1 + mScolN + (i64)s * ldg[k], ldg[k], M.Scol, mScolN, mScolN, nZ[k], M.Sd, 2);
-            J.nsub = 4;
-        }
+        StepJob J = factor(M, M.G1, ldg[k], s, s, M.Yd, 1);
+        J.mode = 0; J.c0 = s; J.A = M.G2; J.lda = 2 * s; J.Sold = M.Sd[0];
+        if (M.p > 1) { J.nz = nZ[k]; J.scaled = 1; J.S = M.Scol[1]; J.Sd = M.Sd[1]; }
         smj.push_back(J);
     }
     flush_small();
     for (int k = 0; k < B; ++k) {
         SMat& M = S.mats[W.mats[k]];
         const int s = M.s;
-        if (M.p <= 1) update(M, s, s, s, M.G1, ldg[k], M.Yd, s);
-        else fused(M, s, nZ[k], M.G1, ldg[k], M.Yd, M.Scol, M.Sd);
+        const int nout = M.p <= 1 ? s : s + nZ[k];
+        update(M, s, nout, M.G1, ldg[k], M.Uinv, nout);
     }
     flush_update();
     // Phases 2 .. pmax: block step i = phase - 1 (:152-218).
@@ -2150,16 +2038,10 @@ int plan_wave(SplitStaged& S, SWave& W) {
             SMat& M = S.mats[W.mats[k]];
             if (i > M.p - 1) continue;
             const int s = M.s, mScol = mZ[k] + s;
-            SmallJob J{};
-            J.status = M.status; J.R = M.R; J.ldR = M.ldR;
-            J.sub[0] = pyth(M.G1 + mScol, ldg[k], M.G1, ldg[k], mScol, nY[k], M.Yd, i + 1);
-            J.sub[1] = rblock(mScol, mScol, nY[k], M.Scol, mScol, M.G1, ldg[k], M.Sd, M.Yd);
-            J.nsub = 2;
+            StepJob J = factor(M, M.G1, ldg[k], mScol, nY[k], M.Yd, i + 1);
+            J.mode = 0; J.c0 = mScol; J.A = M.Scol[i & 1]; J.lda = mScol; J.Sold = M.Sd[i & 1];
             if (i < M.p - 1) {
-                const int mZn = mZ[k] + s, mScolN = mZn + s;
-                J.sub[2] = scol(M.G1, ldg[k], mZn, s, nZn[k], M.Yd, M.Scol);
-                J.sub[3] = pyth(M.G1 + mScolN + (i64)s * ldg[k], ldg[k], M.Scol, mScolN, mScolN, nZn[k], M.Sd, i + 2);
-                J.nsub = 4;
+                J.nz = nZn[k]; J.scaled = 1; J.S = M.Scol[(i + 1) & 1]; J.Sd = M.Sd[(i + 1) & 1];
             }
             smj.push_back(J);
         }
@@ -2168,8 +2050,8 @@ int plan_wave(SplitStaged& S, SWave& W) {
             SMat& M = S.mats[W.mats[k]];
             if (i > M.p - 1) continue;
             const int s = M.s, mScol = mZ[k] + s;
-            if (i < M.p - 1) fused(M, mScol, nZn[k], M.G1, ldg[k], M.Yd, M.Scol, M.Sd);
-            else update(M, mScol, mScol, nY[k], M.G1, ldg[k], M.Yd, nY[k]);
+            const int nout = i < M.p - 1 ? s + nZn[k] : nY[k];
+            update(M, mScol, nout, M.G1, ldg[k], M.Uinv, nout);
             mZ[k] += s;
             nZ[k] = nZn[k];
         }
@@ -2233,20 +2115,19 @@ int enqueue_wave(SplitStaged& S, SWave& W, cudaStream_t st) {
                                                 L.items, st);
                 break;
             case kSSmall:
-                rc = launch_small_batched(reinterpret_cast<const SmallJob*>(jb + L.job_off), L.njobs, st);
+                rc = launch_step_batched(reinterpret_cast<const StepJob*>(jb + L.job_off), L.njobs, 32, st);
                 break;
             case kSBbuild:
-                bbuild_batched<<<items, 256, kBbuildSmem, st>>>(reinterpret_cast<const BbuildJob*>(jb + L.job_off), pre,
-                                                               L.njobs);
+                bbuild_batched<<<items, BB_THREADS, 0, st>>>(reinterpret_cast<const BbuildJob*>(jb + L.job_off), pre, L.njobs);
                 ++g_launch_count;
                 break;
             case kSBdigit:
                 if (KD == 6)
-                    bdigit_batched<6><<<items, 256, 0, st>>>(reinterpret_cast<const BdigitJob*>(jb + L.job_off), pre,
-                                                             L.njobs);
+                    bdigit_batched<6><<<items, BD_C * BD_J, 0, st>>>(reinterpret_cast<const BdigitJob*>(jb + L.job_off), pre,
+                                                                     L.njobs, S.dtile);
                 else
-                    bdigit_batched<7><<<items, 256, 0, st>>>(reinterpret_cast<const BdigitJob*>(jb + L.job_off), pre,
-                                                             L.njobs);
+                    bdigit_batched<7><<<items, BD_C * BD_J, 0, st>>>(reinterpret_cast<const BdigitJob*>(jb + L.job_off), pre,
+                                                                     L.njobs, S.dtile);
                 ++g_launch_count;
                 break;
             case kSUpdate: {
@@ -2381,7 +2262,6 @@ int split_staged_create(int count, const int* m, const int* n, const int* s, dou
     if (!rc) rc = set_smem(update_tc_kernel<32, 7, true>, SmemLayout<32, 7>::BYTES);
     if (!rc) rc = set_smem(update_tc_kernel<16, 6, true>, SmemLayout<16, 6>::BYTES);
     if (!rc) rc = set_smem(update_tc_kernel<16, 7, true>, SmemLayout<16, 7>::BYTES);
-    if (!rc) rc = set_smem(bbuild_batched, (int)kBbuildSmem);
     if (!rc) rc = tsqr_tile_batched_prepare();
     if (rc) { free_staged(S); return 3; }
     if (budget < 0) {
