@@ -24,6 +24,10 @@
 // dependent steps, runs on one CTA: in step j, warp 0 finishes row j + 1 and makes it
 // the next pivot row (five dependent instructions) while the other warps update the
 // rows below, eight lanes a row because the rows are short.
+// One launch replaces four per block step. Measured per step, K = 240: 65 us before
+// (two Choleskys, S, R block) and 18.5 us now at N = 20; 145 and 31 us at N = 32; 1850
+// and 430 us at N = 128, where the elimination fills its SM (N^3 / 3 multiply-adds,
+// 270 us of it).
 // The arithmetic does not depend on the number of CTAs per job, so the batched
 // launches (one CTA per matrix when there are many) give the single launch's bits.
 #include "batched.h"

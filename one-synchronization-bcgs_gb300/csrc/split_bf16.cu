@@ -301,6 +301,9 @@ slice_kernel(const double* __restrict__ X, i64 ld, i64 m, int n, int c0, int nc,
 // Cholesky factor of the step (StepJob), [Q_k U_{k+1}] = ([U_k X_{k+1}] - Q G) U^{-1}.
 // K n^2 / 2 multiply-adds, spread over CTAs of BB_ROWS rows; a warp holds BB_ROWS
 // rows of two columns, so each Ui entry is one broadcast load.
+// Measured per step: 7.5 us at n = 32, K = 256 and 46 us at n = 128 (72 and 2970 us when
+// every 64-row CTA inverted both triangles itself and formed the products term by
+// term).
 constexpr int BB_ROWS = 16;
 constexpr int BB_THREADS = 256;
 
@@ -365,7 +368,7 @@ __host__ __device__ inline int upd_group_nb(int nout, int gi) { return upd_group
 // bdig[gi][plane][j][c] (K-major, NB columns, zero padded to (NB, Kpad); group
 // stride KD_MAX * 32 * Kpad), and fexp[32 gi + j] = its column scale exponents. One
 // element per thread, in CTAs of BD_C inner x BD_J output columns, so that the few
-// thousand elements fill the chip. The first CTA also clears what the update that
+// thousand elements fill the chip (2.6 us; 13 us with a thread per inner column). The first CTA also clears what the update that
 // follows accumulates into: the output columns' maxima cmax and tile_ctr, a counter
 // per group.
 constexpr int BD_C = 64, BD_J = 4;

@@ -163,8 +163,8 @@ gram_fp64_partial_seg(const double* __restrict__ X, i64 ld, i64 m, int a0, int n
 // run to run for a given (m, na, nb). The chain of additions is short next to the
 // latency of the loads that feed it, so RD_AHEAD loads are issued ahead of the
 // additions, and the CTAs are small so that a few thousand entries reach most SMs.
-// m = 10^5, na x nb = 200 x 20, about 190 chunks: 33 us with the loads issued four at
-// a time from 256-thread CTAs.
+// m = 10^5, na x nb = 200 x 20, about 190 chunks: 25 us (33 us with the loads issued
+// four at a time from 256-thread CTAs).
 constexpr int RD_THREADS = 64;
 constexpr int RD_AHEAD = 16;
 
