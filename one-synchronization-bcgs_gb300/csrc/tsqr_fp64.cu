@@ -4,11 +4,10 @@
 // call sites :107,:271,:413,:505,:522,:534,:601,:613,:651). Trilinos is not part of
 // the reference, so the algorithm here is the published TSQR reduction tree:
 //
-//   level 0: the panel is cut into tiles of TR rows; one CTA of 1-4 warps per
-//            tile computes a Householder QR of its tile in shared memory (warp
-//            butterfly sums; the warps share out the columns each reflector is
-//            applied to), writes the explicit tile Q in place and its nc x nc R
-//            into the next level's stack.
+//   level 0: the panel is cut into tiles of TR rows; one CTA of W warps per tile
+//            computes a Householder QR of its tile in shared memory (warp butterfly
+//            sums; the warps share out the columns), writes the explicit tile Q in
+//            place and its nc x nc R into the next level's stack.
 //   level l: the stacked R factors (a (tiles * nc) x nc matrix) are cut into tiles
 //            of TR rows again and factored the same way, until one tile remains.
 //   root   : R is sign-normalized (diag(R) >= 0, the column signs moved into Q).
@@ -23,108 +22,81 @@
 
 namespace bcgs {
 
-// Tile rows and warps per tile of the single-panel tile kernel by template width.
-// All tiles hold 256 rows (BCGS_TSQR_TR64 for nc > 32). A level of the tree
-// divides the row count by TR / nc, so taller tiles mean fewer levels and fewer
-// flops, at the price of fewer tiles resident per SM. The reflector application
-// is split over W warps by groups of columns. Measured on GB300 at m = 2^23,
-// n = 512 (TSQR of block 1 per BCGSI+P-1S QR), 256-row tiles (one per SM at
-// nc = 64): nc = 64 with 4 warps 431 ms, 8 warps 353 ms, 16 warps 346 ms; nc = 32
-// with 2 warps 69.6 ms, 4 warps 64.2 ms, 8 warps 71.4 ms; nc = 16 with one warp
-// 16.4 ms. (With the earlier per-warp reflectors and per-column butterflies,
-// 128-row tiles were slower at every warp count: 632 ms with 4 warps at nc = 64.)
-#ifndef BCGS_TSQR_TR64
-#define BCGS_TSQR_TR64 256
-#endif
-#ifndef BCGS_TSQR_W64
-#define BCGS_TSQR_W64 16
-#endif
-#ifndef BCGS_TSQR_W32
-#define BCGS_TSQR_W32 4
-#endif
+// Tile rows and warps per tile by template width. All tiles hold 256 rows: a level of
+// the tree divides the row count by TR / nc, so taller tiles mean fewer levels and
+// fewer flops, at the price of fewer tiles resident per SM. One FP64 instruction of a
+// warp occupies its quarter of the SM for 64 clocks whatever the other warps do, so
+// what counts is the number of FP64 instructions and that all four quarters have
+// some: four columns per warp (their four lane sums cost 6 additions together, one
+// column's alone 5) and no fewer than four warps from 16 columns on.
+constexpr int TSQR_TR = 256;
 template <int NC>
-constexpr int tsqr_tr() { return NC <= 32 ? 256 : BCGS_TSQR_TR64; }
-template <int NC>
-constexpr int tsqr_tile_warps() { return NC > 32 ? BCGS_TSQR_W64 : (NC > 16 ? BCGS_TSQR_W32 : 1); }
+constexpr int tsqr_tile_warps() { return NC > 32 ? 16 : (NC > 16 ? 8 : (NC > 8 ? 4 : 2)); }
 
-int tsqr_tile_rows(int nc) { return nc <= 32 ? 256 : BCGS_TSQR_TR64; }
+int tsqr_tile_rows(int nc) { (void)nc; return TSQR_TR; }
 
-// Shared memory of one tile: the TR x NC tile, column-major (ld TR), its NC
-// Householder scalars, and two TR-row slots for tau * v of the reflector being
-// applied and the next one.
-static size_t tsqr_tile_smem_bytes(int TR, int NC) { return (size_t)(TR * NC + NC + 2 * TR) * sizeof(double); }
+// Shared memory of one tile: the TR x NC tile, column-major (ld TR), the reflectors'
+// scalars and R's diagonal.
+static size_t tsqr_tile_smem_bytes(int NC) { return (size_t)(TSQR_TR * NC + 2 * NC) * sizeof(double); }
 
 // Sum of one value over the warp by an xor butterfly. Lane pairs add the same two
 // operands (a + b == b + a), so every lane ends with the same bits.
 __device__ __forceinline__ double warp_sum1(double w) {
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) w += __shfl_xor_sync(0xffffffffu, w, o);
+    for (int o = 1; o < 32; o <<= 1) w += __shfl_xor_sync(0xffffffffu, w, o);
     return w;
 }
 
-// One reflector H = I - t v v^T applied to column c: w = sum_r v[r] a[r][c] (lane
-// `lane` owns rows lane + 32 i, i < RPL), then a[r][c] -= w (t v[r]) with tv = t v.
-// v is zero above the reflector's pivot row, so those rows keep their values.
-template <int RPL>
-__device__ __forceinline__ void apply1(double* a, int TR, int c, const double* v, const double* tv, int lane) {
-    double w = 0.0;
+// One reflector H = I - t v v^T applied to the K columns c, c + W, ... (lane `lane` owns
+// rows lane + 32 i, i < RPL): w_g = sum_r v[r] a[r][c_g], then a[r][c_g] -= t w_g v[r]. v is
+// zero above the reflector's pivot row, so those rows keep their values. The K sums are
+// reduced together: lane bit 0 splits the columns into pairs and bit 1 into singles
+// (each lane adds the partner's half it keeps), then the remaining bits finish by a
+// butterfly. Every column is summed in warp_sum1's order, so the result does not depend
+// on which columns are taken together.
+template <int RPL, int K>
+__device__ __forceinline__ void apply_cols(double* a, int c, int W, const double* v, double t, int lane) {
+    double x[K][RPL], w[4] = {0.0, 0.0, 0.0, 0.0};
 #pragma unroll
-    for (int i = 0; i < RPL; ++i) w = fma(v[i], a[c * TR + lane + 32 * i], w);
-    w = warp_sum1(w);
+    for (int g = 0; g < K; ++g)
 #pragma unroll
-    for (int i = 0; i < RPL; ++i) {
-        double* e = &a[c * TR + lane + 32 * i];
-        *e = fma(-w, tv[i], *e);
-    }
-}
-
-// The same for the four columns c0 .. c0+3. The four sums are reduced together:
-// lane bit 4 splits the columns into pairs and bit 3 into singles (each lane adds
-// the partner's half it keeps), then bits 2-0 finish one column per group of 8
-// lanes by a butterfly; lanes 8g .. 8g+7 end with column g's sum, which is then
-// broadcast. Six FP64 additions per lane for four columns instead of twenty, in a
-// fixed order.
-template <int RPL>
-__device__ __forceinline__ void apply4(double* a, int TR, int c0, const double* v, const double* tv, int lane) {
-    double w[4];
-#pragma unroll
-    for (int g = 0; g < 4; ++g) {
-        w[g] = 0.0;
-#pragma unroll
-        for (int i = 0; i < RPL; ++i) w[g] = fma(v[i], a[(c0 + g) * TR + lane + 32 * i], w[g]);
-    }
-    const bool b4 = (lane & 16) != 0, b3 = (lane & 8) != 0;
-    double k0 = b4 ? w[2] : w[0], k1 = b4 ? w[3] : w[1];
-    const double s0 = b4 ? w[0] : w[2], s1 = b4 ? w[1] : w[3];
-    k0 += __shfl_xor_sync(0xffffffffu, s0, 16);
-    k1 += __shfl_xor_sync(0xffffffffu, s1, 16);
-    double k = b3 ? k1 : k0;
-    k += __shfl_xor_sync(0xffffffffu, b3 ? k0 : k1, 8);
-    k += __shfl_xor_sync(0xffffffffu, k, 4);
-    k += __shfl_xor_sync(0xffffffffu, k, 2);
-    k += __shfl_xor_sync(0xffffffffu, k, 1);
-#pragma unroll
-    for (int g = 0; g < 4; ++g) {
-        const double wg = __shfl_sync(0xffffffffu, k, 8 * g);
-#pragma unroll
-        for (int i = 0; i < RPL; ++i) {
-            double* e = &a[(c0 + g) * TR + lane + 32 * i];
-            *e = fma(-wg, tv[i], *e);
+        for (int i = RPL - 1; i >= 0; --i) {
+            x[g][i] = a[(c + g * W) * (32 * RPL) + lane + 32 * i];
+            w[g] = fma(v[i], x[g][i], w[g]);
         }
+    double k;
+    const bool b0 = (lane & 1) != 0, b1 = (lane & 2) != 0;
+    if constexpr (K >= 3) {
+        double k0 = b0 ? w[2] : w[0], k1 = b0 ? w[3] : w[1];
+        k0 += __shfl_xor_sync(0xffffffffu, b0 ? w[0] : w[2], 1);
+        k1 += __shfl_xor_sync(0xffffffffu, b0 ? w[1] : w[3], 1);
+        k = b1 ? k1 : k0;
+        k += __shfl_xor_sync(0xffffffffu, b1 ? k0 : k1, 2);
+    } else {
+        k = w[0];
+        if constexpr (K == 2) k = b0 ? w[1] : w[0];
+        k += __shfl_xor_sync(0xffffffffu, K == 2 ? (b0 ? w[0] : w[1]) : w[0], 1);
+        k += __shfl_xor_sync(0xffffffffu, k, 2);
+    }
+    k += __shfl_xor_sync(0xffffffffu, k, 4);
+    k += __shfl_xor_sync(0xffffffffu, k, 8);
+    k += __shfl_xor_sync(0xffffffffu, k, 16);
+    k *= -t;
+#pragma unroll
+    for (int g = 0; g < K; ++g) {
+        const double wg = K == 1 ? k : __shfl_sync(0xffffffffu, k, K == 2 ? g : (g >> 1) + 2 * (g & 1));
+#pragma unroll
+        for (int i = 0; i < RPL; ++i) a[(c + g * W) * (32 * RPL) + lane + 32 * i] = fma(wg, v[i], x[g][i]);
     }
 }
 
-// Applies (v, tv) to the columns of group q (columns [4q, 4q + 4)) that lie in
-// [c_lo, nc): four at once when the whole group does.
-template <int RPL>
-__device__ __forceinline__ void apply_group(double* a, int TR, int q, int c_lo, int nc, const double* v,
-                                            const double* tv, int lane) {
-    const int g0 = 4 * q;
-    if (g0 >= c_lo && g0 + 4 <= nc) {
-        apply4<RPL>(a, TR, g0, v, tv, lane);
-        return;
-    }
-    for (int c = g0 > c_lo ? g0 : c_lo; c < g0 + 4 && c < nc; ++c) apply1<RPL>(a, TR, c, v, tv, lane);
+// H applied to the columns c, c + W, ... below nc.
+template <int RPL, int W>
+__device__ __forceinline__ void apply_own(double* a, int c, int nc, const double* v, double t, int lane) {
+    for (; c + 3 * W < nc; c += 4 * W) apply_cols<RPL, 4>(a, c, W, v, t, lane);
+    if (c + 2 * W < nc) apply_cols<RPL, 3>(a, c, W, v, t, lane);
+    else if (c + W < nc) apply_cols<RPL, 2>(a, c, W, v, t, lane);
+    else if (c < nc) apply_cols<RPL, 1>(a, c, W, v, t, lane);
 }
 
 template <int W>
@@ -132,98 +104,124 @@ __device__ __forceinline__ void tile_sync() {
     if (W == 1) __syncwarp(); else __syncthreads();
 }
 
-// Householder reflector of column c by the conventions of LAPACK's dlarfg
-// (beta = -sign(alpha) sqrt(alpha^2 + ||x||^2), tau = (beta - alpha)/beta,
-// v = x / (alpha - beta)), computed by one warp from the column in shared memory
-// and stored back in place: v below the diagonal, beta on it, tau in tau[c].
-template <int RPL>
-__device__ __forceinline__ void make_reflector(double* a, double* tau, double* tvb, int TR, int c, int lane) {
-    __syncwarp();   // the column's rows were just written by this warp's lanes
-    double x[RPL];
-    double p = 0.0;
-#pragma unroll
-    for (int i = 0; i < RPL; ++i) {
-        const int r = lane + 32 * i;
-        x[i] = a[c * TR + r];
-        if (r > c) p = fma(x[i], x[i], p);
-    }
-    p = warp_sum1(p);
-    const double alpha = a[c * TR + c];
-    double t = 0.0, beta = alpha, scal = 0.0;
-    if (p > 0.0) {
-        beta = -copysign(sqrt(alpha * alpha + p), alpha);
-        t = (beta - alpha) / beta;
-        scal = 1.0 / (alpha - beta);
-    }
-    __syncwarp();
-    double* tv = tvb + (c & 1) * TR;
-#pragma unroll
-    for (int i = 0; i < RPL; ++i) {
-        const int r = lane + 32 * i;
-        const double vr = x[i] * scal;
-        if (r > c) a[c * TR + r] = vr;
-        else if (r == c) a[c * TR + r] = beta;
-        tv[r] = r > c ? t * vr : (r == c ? t : 0.0);
-    }
-    if (lane == 0) tau[c] = t;
+// Whether d is a positive number of ordinary size, 2^-900 .. 2^900 (an integer test: a
+// comparison would be one more FP64 instruction).
+__device__ __forceinline__ bool ordinary(double d) {
+    const unsigned hi = (unsigned)__double2hiint(d);
+    return hi >= 0x07B00000u && hi < 0x78300000u;
 }
 
-// tau_c * v_c of the reflector stored in column c, into slot c & 1 (one warp).
+// Householder reflector of column c (held in x, lane's rows lane + 32 i): H = I - t v v^T
+// with v = x below row c and alpha - beta at it, beta = -sign(alpha) ||x[c:]||,
+// t = 2 / v^T v: LAPACK's dlarfg without scaling v to a unit
+// pivot, which saves a multiply per row and a division. A column whose squares leave
+// the ordinary range is scaled first (v may have any scale). Written back in place: v
+// from row c down, R's entries above; t to tau[c], beta to rdiag[c].
 template <int RPL>
-__device__ __forceinline__ void publish_tv(const double* a, const double* tau, double* tvb, int TR, int c,
-                                           int lane) {
-    const double t = tau[c];
-    double* tv = tvb + (c & 1) * TR;
+__device__ __forceinline__ void make_reflector(double* a, double* tau, double* rdiag, int c, int lane, double* x) {
+    auto below = [&]() {
+        double p = 0.0;
+#pragma unroll
+        for (int i = 0; i < RPL; ++i) {
+            const double y = lane + 32 * i > c ? x[i] : 0.0;
+            p = fma(y, y, p);
+        }
+        return warp_sum1(p);
+    };
+    double p = below();
+    double alpha = __shfl_sync(0xffffffffu, c < 32 ? x[0] : x[1], c & 31);
+    double t = 0.0, beta = alpha, vc = 0.0;
+    bool live = __double_as_longlong(p) != 0LL;
+    if (!live) {   // squares that all underflowed are not a zero column
+        unsigned long long any = 0;
+#pragma unroll
+        for (int i = 0; i < RPL; ++i)
+            if (lane + 32 * i > c) any |= (unsigned long long)__double_as_longlong(x[i]) << 1;
+        live = __any_sync(0xffffffffu, any != 0) != 0;
+    }
+    if (live) {
+        double q = fma(alpha, alpha, p), back = 1.0;
+        if (!ordinary(q)) {
+            const bool small = (unsigned)__double2hiint(q) < 0x3FF00000u;
+            const double sc = __longlong_as_double(small ? 0x7830000000000000LL : 0x1FF0000000000000LL);   // 2^900, 2^-512
+            back = __longlong_as_double(small ? 0x07B0000000000000LL : 0x5FF0000000000000LL);
+#pragma unroll
+            for (int i = 0; i < RPL; ++i)
+                if (lane + 32 * i >= c) x[i] *= sc;
+            alpha *= sc;
+            p = below();
+            q = fma(alpha, alpha, p);
+        }
+        // 1 / sqrt(q), and sqrt(q) = q / sqrt(q) corrected once.
+        const double rs = rsqrt(q);
+        double nrm = q * rs;
+        nrm = fma(fma(-nrm, nrm, q), 0.5 * rs, nrm);
+        beta = -copysign(nrm, alpha);
+        vc = alpha - beta;
+        const double e = 0.5 * fma(vc, vc, p);   // t v^T v = 2 for the v that is stored
+        if (ordinary(e)) {
+            // 1 / e: the hardware's approximate reciprocal r (20 bits or more) times
+            // 1 + d + d^2, d = 1 - e r.
+            double r;
+            asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(e));
+            const double d = fma(-e, r, 1.0);
+            t = fma(r, fma(d, d, d), r);
+        } else {
+            t = 1.0 / e;
+        }
+        if (__double_as_longlong(back) != __double_as_longlong(1.0)) beta *= back;
+    }
 #pragma unroll
     for (int i = 0; i < RPL; ++i) {
         const int r = lane + 32 * i;
-        tv[r] = r > c ? t * a[c * TR + r] : (r == c ? t : 0.0);
+        a[c * (32 * RPL) + r] = r == c ? vc : x[i];
+    }
+    if (lane == 0) {
+        tau[c] = t;
+        rdiag[c] = beta;
     }
 }
 
-// Reflector j (stored in column j) into registers: v (1 on the diagonal, zero
-// above) and tv = tau_j v from its published slot.
+// Reflector j (stored in column j) into registers, zero above its pivot row.
 template <int RPL>
-__device__ __forceinline__ double load_reflector(const double* a, const double* tau, const double* tvb, int TR,
-                                                 int j, int lane, double* v, double* tv) {
-    const double t = tau[j];
-    const double* tj = tvb + (j & 1) * TR;
+__device__ __forceinline__ double load_reflector(const double* a, const double* tau, int j, int lane, double* v) {
 #pragma unroll
     for (int i = 0; i < RPL; ++i) {
         const int r = lane + 32 * i;
-        v[i] = r > j ? a[j * TR + r] : (r == j ? 1.0 : 0.0);
-        tv[i] = tj[r];
+        v[i] = r >= j ? a[j * (32 * RPL) + r] : 0.0;
     }
-    return t;
+    return tau[j];
 }
 
 // W warps per tile, the tile in shared memory (lane L owns rows L, L+32, ...).
 // A: rows x nc (lda); tile `tile` covers rows [tile*TR, min(rows, (tile+1)*TR)).
-// Householder QR by the conventions of LAPACK's dgeqr2/dlarfg, then the tile's R
-// (upper, lower part zero) to Rst rows [tile*nc, (tile+1)*nc) (ld ldr), then the
-// explicit tile Q formed in place in dorg2r's order (backward over the reflectors)
-// and written to Q (ldq; may alias A). Tiles shorter than nc rows are padded with
-// zero rows; padded rows of Q are not written. smem holds
-// tsqr_tile_smem_bytes(TR, NC).
+// Householder QR (dgeqr2's order), then the tile's R (upper, lower part zero) to Rst
+// rows [tile*nc, (tile+1)*nc) (ld ldr), then the explicit tile Q formed in place in
+// dorg2r's order (backward over the reflectors) and written to Q (ldq; may alias A).
+// Tiles shorter than nc rows are padded with zero rows; padded rows of Q are not
+// written. smem holds tsqr_tile_smem_bytes(NC).
 //
-// The columns are dealt out in groups of four, group q to warp q mod W, and every
-// column is only ever updated by its group's warp. Each reflector is formed once,
-// by the warp owning its column, and published in shared memory: while applying
-// reflector j, the owner of column j+1 updates that column first and forms
-// reflector j+1 from it before its other columns (look-ahead), so one barrier per
-// reflector separates the steps. Every sum has a fixed order, so the result is
-// bit-identical run to run (for a given W).
+// Column c belongs to warp c mod W, so the warps' shares stay even as columns are
+// finished. Each reflector is formed once, by its column's warp: while reflector j is
+// applied, the owner of column j + 1 updates that column first, alone, and forms
+// reflector j + 1 from it before its other columns (look-ahead), so one barrier per
+// reflector separates the steps. Every sum has a fixed order that depends on
+// neither W nor the grouping, so results are bit-identical for every W.
+// Measured (before: one, four or 16 warps a tile with fixed groups of four columns,
+// unit-pivot reflectors with a division each, tau v published beside v): a level of one
+// tile of 256 x 10, whose chain of reflectors nothing hides, 124 -> 53 us; the leaves of
+// 10^5 x 10 133 -> 76 us, of 2^21 x 16 2.81 -> 2.70 ms, of 2^19 x 64 11.9 -> 11.3 ms, where
+// the FP64 pipe is active 86 %, 84 % and 76 % of the time at 16, 32 and 64 columns.
 template <int NC, int W>
 __device__ void tsqr_tile_body(const double* A, i64 lda, i64 rows, int nc, double* Q, i64 ldq,
                                double* __restrict__ Rst, i64 ldr, i64 tile, double* smem) {
-    constexpr int TR = tsqr_tr<NC>();
+    constexpr int TR = TSQR_TR;
     constexpr int RPL = TR / 32;
     double* a = smem;              // a[c * TR + r]
     double* tau = smem + TR * NC;
-    double* tvb = tau + NC;        // tau * v of reflectors j and j + 1 (slots j & 1)
+    double* rdiag = tau + NC;
     const int lane = threadIdx.x & 31;
     const int warp = W == 1 ? 0 : (int)(threadIdx.x >> 5);
-    const int ngroups = (nc + 3) / 4;
     const i64 row0 = tile * TR;
     const i64 h = min((i64)TR, rows - row0);
     tile_sync<W>();
@@ -233,64 +231,68 @@ __device__ void tsqr_tile_body(const double* A, i64 lda, i64 rows, int nc, doubl
             const int r = lane + 32 * i;
             a[c * TR + r] = (r < h) ? A[row0 + r + (i64)c * lda] : 0.0;
         }
-    tile_sync<W>();
-    if (warp == 0) make_reflector<RPL>(a, tau, tvb, TR, 0, lane);   // group 0 belongs to warp 0
+    // (each warp has only written columns of its own so far)
+    double v[RPL];
+    if (warp == 0) {
+        double x[RPL];
+#pragma unroll
+        for (int i = 0; i < RPL; ++i) x[i] = a[lane + 32 * i];
+        make_reflector<RPL>(a, tau, rdiag, 0, lane, x);
+    }
     tile_sync<W>();
 
-    double v[RPL], tv[RPL];
-    for (int j = 0; j < nc; ++j) {
-        const double t = load_reflector<RPL>(a, tau, tvb, TR, j, lane, v, tv);
-        const int jn = j + 1;
-        if (jn < nc) {
-            const int qn = jn >> 2;                 // group of column j + 1
-            int q0 = qn + ((warp - qn) % W + W) % W; // this warp's first group at or after qn
-            if (q0 == qn) {
-                if (t != 0.0) apply_group<RPL>(a, TR, qn, jn, nc, v, tv, lane);
-                make_reflector<RPL>(a, tau, tvb, TR, jn, lane);
-                q0 += W;
+    for (int j = 0; j + 1 < nc; ++j) {
+        const double t = load_reflector<RPL>(a, tau, j, lane, v);
+        const bool live = __double_as_longlong(t) != 0LL;
+        int c = j + 1 + ((warp - (j + 1)) % W + W) % W;   // this warp's first column after j
+        if (c == j + 1) {
+            double x[RPL], w = 0.0;
+#pragma unroll
+            for (int i = 0; i < RPL; ++i) x[i] = a[c * TR + lane + 32 * i];
+            if (live) {
+#pragma unroll
+                for (int i = RPL - 1; i >= 0; --i) w = fma(v[i], x[i], w);
+                w = warp_sum1(w) * -t;
+#pragma unroll
+                for (int i = 0; i < RPL; ++i) x[i] = fma(w, v[i], x[i]);
             }
-            if (t != 0.0)
-                for (int q = q0; q < ngroups; q += W) apply_group<RPL>(a, TR, q, jn, nc, v, tv, lane);
+            make_reflector<RPL>(a, tau, rdiag, c, lane, x);
+            c += W;
         }
+        if (live) apply_own<RPL, W>(a, c, nc, v, t, lane);
         tile_sync<W>();
     }
     // R to the stack (upper, lower zero).
     for (int e = threadIdx.x; e < nc * nc; e += 32 * W) {
         const int i = e % nc, c = e / nc;
-        Rst[tile * nc + i + (i64)c * ldr] = (i <= c) ? a[c * TR + i] : 0.0;
+        Rst[tile * nc + i + (i64)c * ldr] = i < c ? a[c * TR + i] : (i == c ? rdiag[c] : 0.0);
     }
     tile_sync<W>();
-    // Explicit Q in place (dorg2r): for j = nc-1 .. 0, apply H_j to columns j+1..
-    // and set column j to (I - tau v v^T) e_j (its owner, after the barrier that
-    // ends every warp's reading of reflector j). tau * v of reflector j - 1 is
-    // published during step j by the owner of column j - 1.
-    if (((nc - 1) >> 2) % W == warp) publish_tv<RPL>(a, tau, tvb, TR, nc - 1, lane);
-    tile_sync<W>();
+    // Explicit Q in place (dorg2r): for j = nc-1 .. 0, apply H_j to columns j+1.. and set
+    // column j to (I - t v v^T) e_j (its owner, after the barrier that ends every
+    // warp's reading of reflector j).
     for (int j = nc - 1; j >= 0; --j) {
-        const double t = load_reflector<RPL>(a, tau, tvb, TR, j, lane, v, tv);
-        if (j >= 1 && ((j - 1) >> 2) % W == warp) publish_tv<RPL>(a, tau, tvb, TR, j - 1, lane);
-        if (t != 0.0 && j + 1 < nc) {
-            const int qn = (j + 1) >> 2;
-            for (int q = qn + ((warp - qn) % W + W) % W; q < ngroups; q += W)
-                apply_group<RPL>(a, TR, q, j + 1, nc, v, tv, lane);
-        }
+        const double t = load_reflector<RPL>(a, tau, j, lane, v);
+        if (__double_as_longlong(t) != 0LL)
+            apply_own<RPL, W>(a, j + 1 + ((warp - (j + 1)) % W + W) % W, nc, v, t, lane);
         tile_sync<W>();
-        if ((j >> 2) % W == warp) {
+        if (j % W == warp) {
+            const double s = -t * __shfl_sync(0xffffffffu, j < 32 ? v[0] : v[1], j & 31);
 #pragma unroll
             for (int i = 0; i < RPL; ++i) {
                 const int r = lane + 32 * i;
-                a[j * TR + r] = (r > j) ? -tv[i] : (r == j ? 1.0 - t : 0.0);
+                const double y = s * v[i];
+                a[j * TR + r] = r == j ? 1.0 + y : y;
             }
         }
     }
-    tile_sync<W>();
+    // (column c's owner is the only one that has written it since the last barrier)
     for (int c = warp; c < nc; c += W)
 #pragma unroll
         for (int i = 0; i < RPL; ++i) {
             const int r = lane + 32 * i;
             if (r < h) Q[row0 + r + (i64)c * ldq] = a[c * TR + r];
         }
-    tile_sync<W>();
 }
 
 template <int NC>
@@ -328,17 +330,19 @@ __global__ void tsqr_root_fix(double* Q, i64 ldq, int hq, int nc, const double* 
 
 // Down-sweep: for each tile t of TR rows of Q (rows x nc, ldq):
 //   Q[tile t] = Q[tile t] * P[t*nc:(t+1)*nc, 0:nc]   (P: ld ldp)
-// Body shared by the single and batched kernels: rows [blk*blockDim, ...) of Q.
+// Body shared by the single and batched kernels: rows [blk*AP_THREADS, ...) of Q, one per
+// thread. NC is nc rounded up to the next width there is code for: the FP64 pipe runs every term, so
+// padding 10 columns to 16 would cost 60 %.
+constexpr int AP_THREADS = 128;
+
 template <int NC>
 __device__ void tsqr_apply_body(double* Q, i64 ldq, i64 rows, int nc, int TR, const double* __restrict__ P,
-                                i64 ldp, i64 blk) {
-    __shared__ double p[NC * NC];
-    __syncthreads();
-    const i64 r = blk * blockDim.x + threadIdx.x;
-    const i64 t = (blk * blockDim.x) / TR;   // blockDim.x divides TR
+                                i64 ldp, i64 blk, double* p) {
+    const i64 r = blk * AP_THREADS + threadIdx.x;
+    const i64 t = (blk * AP_THREADS) / TR;   // AP_THREADS divides TR
     // The whole NC x NC tile: the product below runs over NC terms, and entries
     // past nc must be zeros, not whatever an earlier CTA left in shared memory.
-    for (int e = threadIdx.x; e < NC * NC; e += blockDim.x) {
+    for (int e = threadIdx.x; e < NC * NC; e += AP_THREADS) {
         const int i = e % NC, c = e / NC;
         p[e] = (i < nc && c < nc) ? P[t * nc + i + (i64)c * ldp] : 0.0;
     }
@@ -347,9 +351,8 @@ __device__ void tsqr_apply_body(double* Q, i64 ldq, i64 rows, int nc, int TR, co
     double x[NC];
 #pragma unroll
     for (int c = 0; c < NC; ++c) x[c] = (c < nc) ? Q[r + (i64)c * ldq] : 0.0;
-#pragma unroll
-    for (int c = 0; c < NC; ++c) {
-        if (c >= nc) break;
+#pragma unroll 2
+    for (int c = 0; c < nc; ++c) {
         double y = 0.0;
 #pragma unroll
         for (int i = 0; i < NC; ++i) y = fma(x[i], p[i + c * NC], y);
@@ -358,9 +361,25 @@ __device__ void tsqr_apply_body(double* Q, i64 ldq, i64 rows, int nc, int TR, co
 }
 
 template <int NC>
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(AP_THREADS)
 tsqr_apply_kernel(double* Q, i64 ldq, i64 rows, int nc, int TR, const double* __restrict__ P, i64 ldp) {
-    tsqr_apply_body<NC>(Q, ldq, rows, nc, TR, P, ldp, blockIdx.x);
+    __shared__ double p[NC * NC];
+    tsqr_apply_body<NC>(Q, ldq, rows, nc, TR, P, ldp, blockIdx.x, p);
+}
+
+static int launch_apply(double* Q, i64 ldq, i64 rows, int nc, int TR, const double* P, i64 ldp, cudaStream_t st) {
+    const unsigned blocks = (unsigned)ceil_div(rows, AP_THREADS);
+#define BCGS_APPLY(N) \
+    if (nc <= N) { tsqr_apply_kernel<N><<<blocks, AP_THREADS, 0, st>>>(Q, ldq, rows, nc, TR, P, ldp); break; }
+    do {
+        BCGS_APPLY(2) BCGS_APPLY(4) BCGS_APPLY(5) BCGS_APPLY(6) BCGS_APPLY(8) BCGS_APPLY(10) BCGS_APPLY(12)
+        BCGS_APPLY(14) BCGS_APPLY(16) BCGS_APPLY(20) BCGS_APPLY(24) BCGS_APPLY(28) BCGS_APPLY(32) BCGS_APPLY(40)
+        BCGS_APPLY(48) BCGS_APPLY(56) BCGS_APPLY(64)
+        return (int)cudaErrorInvalidValue;
+    } while (0);
+#undef BCGS_APPLY
+    g_launch_count += 1;
+    return (int)cudaGetLastError();
 }
 
 i64 tsqr_workspace_doubles(i64 m, int nc) {
@@ -381,7 +400,7 @@ i64 tsqr_workspace_doubles(i64 m, int nc) {
 template <int NC>
 static int tsqr_levels(double* A0, i64 ld0, i64 rows0, int nc, double* R, int ldR, double* ws, cudaStream_t st) {
     const int TR = tsqr_tile_rows(nc);
-    const size_t smem = tsqr_tile_smem_bytes(TR, NC);
+    const size_t smem = tsqr_tile_smem_bytes(NC);
     const int attr_rc = smem_attr((const void*)tsqr_tile_kernel<NC>, (int)smem);
     if (attr_rc) return attr_rc;
     constexpr int kMaxLevels = 48;   // each level divides the rows by TR / nc >= 2: 2^k rows need at most k levels
@@ -413,10 +432,8 @@ static int tsqr_levels(double* A0, i64 ld0, i64 rows0, int nc, double* R, int ld
     g_launch_count += 2;
     // Down-sweep.
     for (int l = L - 1; l >= 0; --l) {
-        const unsigned blocks = (unsigned)ceil_div(lvl_rows[l], 128);
-        tsqr_apply_kernel<NC><<<blocks, 128, 0, st>>>(lvl_ptr[l], lvl_ld[l], lvl_rows[l], nc, TR,
-                                                      lvl_ptr[l + 1], lvl_ld[l + 1]);
-        g_launch_count += 1;
+        const int rc = launch_apply(lvl_ptr[l], lvl_ld[l], lvl_rows[l], nc, TR, lvl_ptr[l + 1], lvl_ld[l + 1], st);
+        if (rc) return rc;
     }
     return (int)cudaGetLastError();
 }
@@ -439,7 +456,7 @@ template <int NC>
 static int tsqr_sharded_run(double* X, i64 ld, i64 m_local, int c0, int nc, double* R, int ldR, double* ws,
                             const TsqrShard& sh, cudaStream_t st) {
     const int TR = tsqr_tile_rows(nc);
-    const size_t smem = tsqr_tile_smem_bytes(TR, NC);
+    const size_t smem = tsqr_tile_smem_bytes(NC);
     const int attr_rc = smem_attr((const void*)tsqr_tile_kernel<NC>, (int)smem);
     if (attr_rc) return attr_rc;
     if (sh.T <= 1) return tsqr_run<NC>(X, ld, m_local, c0, nc, R, ldR, ws, st);   // one tile: one rank holds it
@@ -467,9 +484,8 @@ static int tsqr_sharded_run(double* X, i64 ld, i64 m_local, int c0, int nc, doub
     rc = tsqr_levels<NC>(lvl1, ld1, ld1, nc, R, ldR, ws + ld1 * nc, st);
     if (rc) return rc;
     if (nt > 0) {
-        tsqr_apply_kernel<NC><<<(unsigned)ceil_div(m_local, 128), 128, 0, st>>>(panel, ld, m_local, nc, TR,
-                                                                                 lvl1 + sh.t0[sh.rank] * nc, ld1);
-        g_launch_count += 1;
+        rc = launch_apply(panel, ld, m_local, nc, TR, lvl1 + sh.t0[sh.rank] * nc, ld1, st);
+        if (rc) return rc;
     }
     return (int)cudaGetLastError();
 }
@@ -499,16 +515,15 @@ int launch_tsqr(double* X, i64 ld, i64 m, int c0, int nc, double* R, int ldR, do
 // down-sweep level over many panels (nc <= 16, TR = 256), with the single-panel
 // bodies.
 // ---------------------------------------------------------------------------
-__global__ void __launch_bounds__(32)
+constexpr int kTileBatchWarps = tsqr_tile_warps<16>();
+
+__global__ void __launch_bounds__(32 * kTileBatchWarps)
 tsqr_tile_batched(const TsqrTileJob* __restrict__ jobs, const int* __restrict__ prefix, int njobs) {
     extern __shared__ double smem[];
     const int j = batched_job_of(prefix, njobs, blockIdx.x);
-    const TsqrTileJob& J = jobs[j];
-    const i64 tile = blockIdx.x - prefix[j];
-    if (J.nc <= 8)
-        tsqr_tile_body<8, 1>(J.A, J.lda, J.rows, J.nc, J.A, J.lda, J.Rst, J.ldr, tile, smem);
-    else
-        tsqr_tile_body<16, 1>(J.A, J.lda, J.rows, J.nc, J.A, J.lda, J.Rst, J.ldr, tile, smem);
+    const TsqrTileJob J = jobs[j];
+    tsqr_tile_body<16, kTileBatchWarps>(J.A, J.lda, J.rows, J.nc, J.A, J.lda, J.Rst, J.ldr, blockIdx.x - prefix[j],
+                                        smem);
 }
 
 __global__ void tsqr_root_batched(const TsqrRootJob* __restrict__ jobs) {
@@ -516,29 +531,30 @@ __global__ void tsqr_root_batched(const TsqrRootJob* __restrict__ jobs) {
     tsqr_root_fix_body(J.Q, J.ldq, J.hq, J.nc, J.R, J.ldr, J.Rout, J.ldro);
 }
 
-__global__ void __launch_bounds__(128)
+__global__ void __launch_bounds__(AP_THREADS)
 tsqr_apply_batched(const TsqrApplyJob* __restrict__ jobs, const int* __restrict__ prefix, int njobs) {
+    __shared__ double p[16 * 16];
     const int j = batched_job_of(prefix, njobs, blockIdx.x);
-    const TsqrApplyJob& J = jobs[j];
+    const TsqrApplyJob J = jobs[j];
     const i64 blk = blockIdx.x - prefix[j];
-    if (J.nc <= 8)
-        tsqr_apply_body<8>(J.Q, J.ldq, J.rows, J.nc, J.TR, J.P, J.ldp, blk);
-    else
-        tsqr_apply_body<16>(J.Q, J.ldq, J.rows, J.nc, J.TR, J.P, J.ldp, blk);
+    if (J.nc <= 4) tsqr_apply_body<4>(J.Q, J.ldq, J.rows, J.nc, J.TR, J.P, J.ldp, blk, p);
+    else if (J.nc <= 8) tsqr_apply_body<8>(J.Q, J.ldq, J.rows, J.nc, J.TR, J.P, J.ldp, blk, p);
+    else if (J.nc <= 12) tsqr_apply_body<12>(J.Q, J.ldq, J.rows, J.nc, J.TR, J.P, J.ldp, blk, p);
+    else tsqr_apply_body<16>(J.Q, J.ldq, J.rows, J.nc, J.TR, J.P, J.ldp, blk, p);
 }
 
 // Sets the batched tile kernel's shared-memory limit (outside any stream capture).
 int tsqr_tile_batched_prepare() {
     return (int)cudaFuncSetAttribute(tsqr_tile_batched, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     (int)tsqr_tile_smem_bytes(256, 16));
+                                     (int)tsqr_tile_smem_bytes(16));
 }
 
 int launch_tsqr_tile_batched(const TsqrTileJob* jobs, const int* prefix, int njobs, int items, int ncmax,
                              cudaStream_t st) {
     if (items <= 0) return 0;
     if (ncmax > 16) return (int)cudaErrorInvalidValue;
-    const size_t smem = tsqr_tile_smem_bytes(256, 16);
-    tsqr_tile_batched<<<(unsigned)items, 32, smem, st>>>(jobs, prefix, njobs);
+    const size_t smem = tsqr_tile_smem_bytes(16);
+    tsqr_tile_batched<<<(unsigned)items, 32 * kTileBatchWarps, smem, st>>>(jobs, prefix, njobs);
     g_launch_count += 1;
     return (int)cudaGetLastError();
 }
@@ -554,7 +570,7 @@ int launch_tsqr_apply_batched(const TsqrApplyJob* jobs, const int* prefix, int n
                               cudaStream_t st) {
     if (items <= 0) return 0;
     if (ncmax > 16) return (int)cudaErrorInvalidValue;
-    tsqr_apply_batched<<<(unsigned)items, 128, 0, st>>>(jobs, prefix, njobs);
+    tsqr_apply_batched<<<(unsigned)items, AP_THREADS, 0, st>>>(jobs, prefix, njobs);
     g_launch_count += 1;
     return (int)cudaGetLastError();
 }
