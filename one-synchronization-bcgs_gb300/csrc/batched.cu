@@ -18,10 +18,9 @@
 // summation orders of the single-matrix driver: with the same Gram chunking
 // (orth_gb300_set_gram_chunk_rows) the results are bit-identical.
 //
-// Tuning: per block size s, the Gram's B-panel width (8, 16 or 32 columns; the
-// A-panel holds 512 / width columns, 64 threads per CTA) and the rows per Gram
-// chunk (4096 ... 32768) are picked by timing each candidate on a representative
-// Gram stage of that class's matrices.
+// Tuning: per block size s, the rows per Gram chunk are picked by timing each candidate
+// on a representative Gram stage of that class's matrices: 4096 ... 32768 rows, or
+// smaller chunks where the batch is too small to fill the GPU with those.
 #include <algorithm>
 #include <cmath>
 #include <cstdio>
@@ -47,9 +46,9 @@ namespace {
 constexpr int kTR = 256;                // TSQR tile rows for nc <= 32
 constexpr int kMaxS = 16;
 constexpr int kClasses = 3;             // s <= 4, s <= 8, s <= 16
-constexpr int kRowsMin = 4096;          // smallest Gram chunk candidate
-constexpr int kTbCand[3] = {8, 16, 32};
-constexpr int kRowsCand[4] = {4096, 8192, 16384, 32768};
+constexpr int kRowsMin = 4096;          // smallest Gram chunk candidate of a batch that fills the GPU,
+constexpr int kRowsLeast = 256;         // and of any batch
+constexpr int kRowsCands = 4;           // candidates, each twice the one before
 
 int class_of(int s) { return s <= 4 ? 0 : (s <= 8 ? 1 : 2); }
 
@@ -74,7 +73,7 @@ struct Stage {
 };
 
 // A Gram request of one matrix in one stage (filled into a GramJob once the
-// matrix class's panel and chunk rows are known).
+// matrix class's chunk rows are known).
 struct GramReq {
     int mat;
     int na, b0, nb;
@@ -97,8 +96,8 @@ i64 small_block_doubles(int n, int s) { return 2LL * (n + s) * 2 * s + 2LL * n *
 
 i64 tsqr_doubles(i64 m, int s) { return tsqr_workspace_doubles(m, s); }
 
-i64 part_doubles_of(i64 m, int n, int s) {
-    return ceil_div(m, kRowsMin) * (i64)(n + s) * (2 * s) + 64;
+i64 part_doubles_of(i64 m, int n, int s, int rows_min) {
+    return ceil_div(m, rows_min) * (i64)(n + s) * (2 * s) + 64;
 }
 
 }  // namespace
@@ -106,8 +105,9 @@ i64 part_doubles_of(i64 m, int n, int s) {
 struct BatchPlan {
     int count = 0;
     std::vector<Mat> mats;
-    int tb[kClasses] = {16, 16, 32};
+    int tb[kClasses] = {16, 16, 32};   // C columns of a Gram tile, for the report
     int rows[kClasses] = {8192, 8192, 8192};
+    int rows_min = kRowsMin;
     bool tuned = false;
     // device memory: workspace (per-matrix blocks + status) and the job blob
     void* ws = nullptr;
@@ -154,7 +154,7 @@ size_t layout_workspace(BatchPlan& P, char* base) {
         M.Sd[0] = sb ? M.Scol[1] + (i64)n * s : nullptr;
         M.Sd[1] = sb ? M.Sd[0] + (i64)s * s : nullptr;
         M.Yd = sb ? M.Sd[1] + (i64)s * s : nullptr;
-        M.part = (double*)take((size_t)part_doubles_of(M.m, M.n, M.s) * sizeof(double));
+        M.part = (double*)take((size_t)part_doubles_of(M.m, M.n, M.s, P.rows_min) * sizeof(double));
         M.tsqr = (double*)take((size_t)tsqr_doubles(M.m, M.s) * sizeof(double));
     }
     int* st = (int*)take((size_t)P.count * kStatusWords * sizeof(int));
@@ -181,7 +181,7 @@ void step_gram_shape(const Mat& M, int i, int& na, int& b0, int& nb) {
     }
 }
 
-GramJob make_gram_job(const Mat& M, const GramReq& q, int tb, int rows) {
+GramJob make_gram_job(const Mat& M, const GramReq& q, int rows) {
     GramJob J;
     J.X = M.X; J.ld = M.ld; J.m = M.m;
     J.na = q.na; J.b0 = q.b0; J.nb = q.nb;
@@ -192,9 +192,7 @@ GramJob make_gram_job(const Mat& M, const GramReq& q, int tb, int rows) {
     J.rows_per_chunk = ceil_div(rpc, 32) * 32;   // the single-matrix driver's rule
     J.part = M.part;
     J.C = q.C; J.ldc = q.ldc;
-    J.tb = tb;
-    J.tilesA = (int)ceil_div(q.na, gram_batched_panel_rows(tb));
-    J.tilesB = (int)ceil_div(q.nb, tb);
+    J.tiles = gram_batched_tile(q.na, q.b0, q.nb, &J.ta, &J.r);
     return J;
 }
 
@@ -225,9 +223,9 @@ void build_schedule(BatchPlan& P, Blob& blob) {
         std::vector<int> counts;
         for (const GramReq& q : reqs) {
             const Mat& M = mats[q.mat];
-            GramJob J = make_gram_job(M, q, P.tb[M.cls], P.rows[M.cls]);
+            GramJob J = make_gram_job(M, q, P.rows[M.cls]);
             jobs.push_back(J);
-            counts.push_back(J.nchunks * J.tilesA * J.tilesB);
+            counts.push_back(J.nchunks * J.tiles);
         }
         P.gram_stage_idx.push_back((int)P.stages.size());
         P.gram_reqs.push_back(reqs);
@@ -254,7 +252,11 @@ void build_schedule(BatchPlan& P, Blob& blob) {
     auto add_upd = [&](std::vector<UpdJob>& jobs) {
         if (jobs.empty()) return;
         std::vector<int> counts;
-        for (const UpdJob& J : jobs) counts.push_back((int)ceil_div(J.m, 128));
+        for (UpdJob& J : jobs) {
+            int ctas = 0;
+            update_batched_ctas(J.m, J.K, &J.split, &ctas);
+            counts.push_back(ctas);
+        }
         add_prefixed(kStUpd, jobs, counts, 0);
     };
     // T of one matrix's step (and, with nz > 0, the next block's S and Sd), without
@@ -496,7 +498,7 @@ int upload_schedule(BatchPlan& P) {
 }
 
 // Times the Gram of each class's matrices at their middle block step for every
-// (panel width, chunk rows) candidate and keeps the fastest.
+// candidate of the chunk rows and keeps the fastest.
 int autotune(BatchPlan& P, cudaStream_t st) {
     cudaEvent_t e0, e1;
     BCGS_CUDA_TRY(cudaEventCreate(&e0));
@@ -513,38 +515,37 @@ int autotune(BatchPlan& P, cudaStream_t st) {
         }
         if (reqs.empty()) continue;
         float best = 1e30f;
-        for (int tb : kTbCand) {
-            for (int rows : kRowsCand) {
-                std::vector<GramJob> jobs;
-                std::vector<int> prefix(1, 0), prefix2(1, 0);
-                for (const GramReq& q : reqs) {
-                    GramJob J = make_gram_job(P.mats[q.mat], q, tb, rows);
-                    jobs.push_back(J);
-                    prefix.push_back(prefix.back() + J.nchunks * J.tilesA * J.tilesB);
-                    prefix2.push_back(prefix2.back() + gram_reduce_ctas(J.na, J.nb));
-                }
-                Blob blob;
-                const size_t jo = blob.put(jobs), po = blob.put(prefix), p2 = blob.put(prefix2);
-                void* d = nullptr;
-                if ((rc = (int)cudaMalloc(&d, blob.bytes.size()))) break;
-                rc = (int)cudaMemcpy(d, blob.bytes.data(), blob.bytes.size(), cudaMemcpyHostToDevice);
-                float ms = 0.f;
-                for (int rep = 0; rep < 2 && !rc; ++rep) {
-                    cudaEventRecord(e0, st);
-                    rc = launch_gram_partial_batched((const GramJob*)((char*)d + jo), (const int*)((char*)d + po),
-                                                     (int)jobs.size(), prefix.back(), st);
-                    if (!rc)
-                        rc = launch_gram_reduce_batched((const GramJob*)((char*)d + jo), (const int*)((char*)d + p2),
-                                                        (int)jobs.size(), prefix2.back(), st);
-                    cudaEventRecord(e1, st);
-                    if (!rc) rc = (int)cudaEventSynchronize(e1);
-                    if (!rc) rc = (int)cudaEventElapsedTime(&ms, e0, e1);
-                }
-                cudaFree(d);
-                if (rc) break;
-                if (ms < best) { best = ms; P.tb[c] = tb; P.rows[c] = rows; }
+        for (int k = 0; k < kRowsCands; ++k) {
+            const int rows = P.rows_min << k;
+            std::vector<GramJob> jobs;
+            std::vector<int> prefix(1, 0), prefix2(1, 0);
+            for (const GramReq& q : reqs) {
+                GramJob J = make_gram_job(P.mats[q.mat], q, rows);
+                P.tb[c] = J.r * (128 / J.ta);
+                jobs.push_back(J);
+                prefix.push_back(prefix.back() + J.nchunks * J.tiles);
+                prefix2.push_back(prefix2.back() + gram_reduce_ctas(J.na, J.nb));
             }
+            Blob blob;
+            const size_t jo = blob.put(jobs), po = blob.put(prefix), p2 = blob.put(prefix2);
+            void* d = nullptr;
+            if ((rc = (int)cudaMalloc(&d, blob.bytes.size()))) break;
+            rc = (int)cudaMemcpy(d, blob.bytes.data(), blob.bytes.size(), cudaMemcpyHostToDevice);
+            float ms = 0.f;
+            for (int rep = 0; rep < 2 && !rc; ++rep) {
+                cudaEventRecord(e0, st);
+                rc = launch_gram_partial_batched((const GramJob*)((char*)d + jo), (const int*)((char*)d + po),
+                                                 (int)jobs.size(), prefix.back(), st);
+                if (!rc)
+                    rc = launch_gram_reduce_batched((const GramJob*)((char*)d + jo), (const int*)((char*)d + p2),
+                                                    (int)jobs.size(), prefix2.back(), st);
+                cudaEventRecord(e1, st);
+                if (!rc) rc = (int)cudaEventSynchronize(e1);
+                if (!rc) rc = (int)cudaEventElapsedTime(&ms, e0, e1);
+            }
+            cudaFree(d);
             if (rc) break;
+            if (ms < best) { best = ms; P.rows[c] = rows; }
         }
     }
     cudaEventDestroy(e0);
@@ -577,6 +578,17 @@ int fill_mats(BatchPlan& P, int count, const int* m, const int* n, const int* s,
         if (M.s < 1 || M.s > kMaxS || M.n < 2 * M.s || M.m < M.n || M.ld < M.m || M.ldR < M.n) return 2;
         M.p = (M.n - M.s + M.s - 1) / M.s;
         M.cls = class_of(M.s);
+    }
+    // Chunks of 4096 rows and more unless their Gram tiles would leave SMs idle (fewer
+    // than 16 CTAs per SM at the matrices' middle block steps).
+    for (P.rows_min = kRowsMin; P.rows_min > kRowsLeast; P.rows_min /= 2) {
+        i64 ctas = 0;
+        for (const Mat& M : P.mats) {
+            int na, b0, nb, ta, r;
+            step_gram_shape(M, M.p > 1 ? std::max(1, (M.p - 1) / 2) : 0, na, b0, nb);
+            ctas += ceil_div(M.m, P.rows_min) * gram_batched_tile(na, b0, nb, &ta, &r);
+        }
+        if (ctas >= 16LL * kNumSMsDefault) break;
     }
     return 0;
 }

@@ -20,8 +20,8 @@ struct GramJob {
     double* part;   // nchunks * na * nb doubles
     double* C;
     int ldc;
-    int tb;         // B-panel width: 8, 16 or 32 (A-panel height 512 / tb)
-    int tilesA, tilesB;
+    int ta, r;      // tile: ta columns of A, r 128 / ta of B
+    int tiles;
 };
 
 // X[:, c0:c0+nc] = (X[:, c0:c0+nc] - X[:, q0:q0+K] S) T^{-1}, nc <= 16.
@@ -33,6 +33,7 @@ struct UpdJob {
     int lds;
     const double* T;
     int ldt;
+    int split;      // update_batched_ctas
 };
 
 // TSQR: tiles of one level (Q in place, R factors to Rst), the root sign fix, and
@@ -66,7 +67,10 @@ struct TsqrApplyJob {
 int tsqr_tile_batched_prepare();
 
 // Launchers (items = prefix[njobs] CTAs).
-int gram_batched_panel_rows(int tb);   // A-panel height for a B-panel width
+// The Gram's tile for the entries of X[:, 0:na]^T X[:, b0:b0+nb] on or above the diagonal
+// of X^T X, and a job's CTAs in an update.
+int gram_batched_tile(int na, int b0, int nb, int* ta, int* r);   // returns the number of tiles
+void update_batched_ctas(i64 m, int K, int* split, int* ctas);
 int launch_gram_partial_batched(const GramJob* jobs, const int* prefix, int njobs, int items, cudaStream_t st);
 int launch_gram_reduce_batched(const GramJob* jobs, const int* prefix, int njobs, int items, cudaStream_t st);
 int launch_update_batched(const UpdJob* jobs, const int* prefix, int njobs, int items, cudaStream_t st);

@@ -29,12 +29,13 @@ extern std::atomic<long long> g_aux_launch_count;
 int smem_attr(const void* fn, int bytes);
 
 // C (na x nb, ld ldo) = X[:, a0:a0+na]^T X[:, b0:b0+nb] over m rows, FP64, with a
-// fixed-order two-stage reduction through `part` (nchunks * na * nb doubles).
-int gram_chunks_fp64(i64 m, int na, int nb, int num_sms);
+// fixed-order two-stage reduction through `part` (gram_part_doubles_fp64 doubles).
+// upper_only: only the entries on or above the diagonal of X^T X are defined.
+i64 gram_part_doubles_fp64(i64 m, int na_max, int nb_max);   // for any na, nb up to these
 // Rows per chunk forced by orth_gb300_set_gram_chunk_rows (0: default policy).
 extern long long g_gram_chunk_rows;
 int launch_gram_fp64(const double* X, i64 ld, i64 m, int a0, int na, int b0, int nb,
-                     double* out, int ldo, double* part, int nchunks, cudaStream_t st);
+                     double* out, int ldo, double* part, bool upper_only, int num_sms, cudaStream_t st);
 
 // out (na x nb, ld ldo) = fixed-order sum of nchunks partials part[c][i + j*na].
 int launch_gram_reduce(const double* part, int nchunks, int na, int nb, double* out, int ldo,
@@ -42,8 +43,10 @@ int launch_gram_reduce(const double* part, int nchunks, int na, int nb, double* 
 int gram_reduce_ctas(int na, int nb);   // CTAs of one reduction
 
 // X[:, c0:c0+nc] = (X[:, c0:c0+nc] - X[:, q0:q0+K] S) T^{-1}; T upper (nc x nc) or null.
+// any_split: K may be summed in quarters, by a rule on m; without it each row's result
+// does not depend on how many rows there are (the row-sharded path).
 int launch_update_fp64(double* X, i64 ld, i64 m, int q0, int K, int c0, int nc,
-                       const double* S, int lds, const double* T, int ldt, cudaStream_t st);
+                       const double* S, int lds, const double* T, int ldt, bool any_split, cudaStream_t st);
 
 // The small work of one block step on the reduced Gram G (small_fp64.cu): with
 // Y = G[0:K, 0:ny], Z = G[0:K, ny:ny+nz],

@@ -77,13 +77,7 @@ struct Layout {
 
 i64 round32(i64 v) { return (v + 31) / 32 * 32; }
 
-Layout layout_for(i64 m, int n, int s, int num_sms) {
-    i64 part = 0;
-    for (int na = 1; na <= n + s; ++na)
-        for (int nb = 1; nb <= 2 * s; ++nb) {
-            i64 v = gram_chunks_fp64(m, na, nb, num_sms) * (i64)na * nb;
-            if (v > part) part = v;
-        }
+Layout layout_for(i64 m, int n, int s) {
     Layout L;
     i64 off = 0;
     L.status = off; off += 32;                                   // 4 int32 status words
@@ -92,7 +86,7 @@ Layout layout_for(i64 m, int n, int s, int num_sms) {
     L.Scol = off;   off += round32((i64)n * s);
     L.Sd = off;     off += round32((i64)s * s);
     L.Yd = off;     off += round32((i64)s * s);
-    L.part = off;   off += round32(part);
+    L.part = off;   off += round32(gram_part_doubles_fp64(m, n + s, 2 * s));
     L.tsqr = off;   off += round32(tsqr_workspace_doubles(m, s));
     L.total = off;
     return L;
@@ -115,7 +109,7 @@ extern "C" int orth_gb300_bcgsi2P1s_dev_noalloc(int m, int n, int s, double* dX,
         if (status) status->cuda_error = rc;
         return 3;
     }
-    const Layout L = layout_for(m, n, s, d->num_sms);
+    const Layout L = layout_for(m, n, s);
     if ((size_t)L.total > kNoAllocDoubles) {
         fprintf(stderr,
                 "orth_gb300_bcgsi2P1s_dev_noalloc: m=%d n=%d s=%d needs %lld bytes of scratch; "
@@ -141,11 +135,10 @@ extern "C" int orth_gb300_bcgsi2P1s_dev_noalloc(int m, int n, int s, double* dX,
     int err = zero_async(stat, kStatusWords * sizeof(int), st);
     auto gram = [&](int na, int b0, int nb, double* C) {
         if (err) return;
-        err = launch_gram_fp64(dX, ld, M, 0, na, b0, nb, C, na, part,
-                               gram_chunks_fp64(M, na, nb, d->num_sms), st);
+        err = launch_gram_fp64(dX, ld, M, 0, na, b0, nb, C, na, part, true, d->num_sms, st);
     };
     auto update = [&](int K, int c0, int nc, const double* S, int lds, const double* T, int ldt) {
-        if (!err) err = launch_update_fp64(dX, ld, M, 0, K, c0, nc, S, lds, T, ldt, st);
+        if (!err) err = launch_update_fp64(dX, ld, M, 0, K, c0, nc, S, lds, T, ldt, true, st);
     };
     auto factor = [&](const double* G, int ldg, int K, int ny, double* T, int step) {
         StepJob J;

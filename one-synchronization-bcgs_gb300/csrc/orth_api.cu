@@ -189,17 +189,7 @@ int init_ctx() {
 }
 
 // Largest Gram-partial buffer any step needs (doubles).
-i64 part_doubles(i64 m, int n, int s, int num_sms) {
-    i64 best = 0;
-    const int na_max = n + s, nb_max = 2 * s;
-    for (int na = 1; na <= na_max; ++na) {
-        for (int nb = 1; nb <= nb_max; ++nb) {
-            i64 v = gram_chunks_fp64(m, na, nb, num_sms) * (i64)na * nb;
-            if (v > best) best = v;
-        }
-    }
-    return best + 1024;
-}
+i64 part_doubles(i64 m, int n, int s) { return gram_part_doubles_fp64(m, n + s, 2 * s); }
 
 // Small buffers carved from one allocation (doubles).
 struct Small {
@@ -235,7 +225,7 @@ Small carve_small(double* base, int n, int s) {
 int reserve(i64 m, int n, int s, int precision) {
     int rc = init_ctx();
     if (rc) return rc;
-    rc = scr().part.ensure((size_t)part_doubles(m, n, s, g_ctx.num_sms) * sizeof(double));
+    rc = scr().part.ensure((size_t)part_doubles(m, n, s) * sizeof(double));
     if (rc) return rc;
     rc = scr().small.ensure((size_t)small_doubles(n, s) * sizeof(double));
     if (rc) return rc;
@@ -620,12 +610,12 @@ struct Engine {
     Shard* shard = nullptr;     // row-sharded runs only (FP64)
 
     // C (na x nb, ldc) = X[:, a0:a0+na]^T X[:, b0:b0+nb] in FP64: one deterministic
-    // reduction, over all ranks in a row-sharded run.
+    // reduction, over all ranks in a row-sharded run. Entries below the diagonal of
+    // X^T X may be undefined (no caller reads them).
     void gram_fp64(int a0, int na, int b0, int nb, double* C, int ldc) {
         if (err) return;
         if (!shard) {
-            const int chunks = gram_chunks_fp64(m, na, nb, g_ctx.num_sms);
-            err = launch_gram_fp64(X, ld, m, a0, na, b0, nb, C, ldc, scr().part.as<double>(), chunks, st);
+            err = launch_gram_fp64(X, ld, m, a0, na, b0, nb, C, ldc, scr().part.as<double>(), true, g_ctx.num_sms, st);
             return;
         }
         Shard& sh = *shard;
@@ -682,7 +672,7 @@ struct Engine {
             err = launch_update_split(X, ld, m, K, c0, nc, S, lds, T ? w.Uinv : nullptr, ldinv, g_ctx.num_sms, st);
             return;
         }
-        err = launch_update_fp64(X, ld, m, 0, K, c0, nc, S, lds, T, nc, st);
+        err = launch_update_fp64(X, ld, m, 0, K, c0, nc, S, lds, T, nc, shard == nullptr, st);
     }
     // Split modes: Q_k and U_{k+1} of the lagged variants in one tensor-core pass.
     // The step that reduced G left the inverse of both factors in w.Uinv.
@@ -760,7 +750,7 @@ struct Engine {
             StepJob J;
             J.G = G; J.ldg = nc; J.ny = nc; J.T = T; J.step = step; J.status = status;
             if (!err) err = launch_step(J, st);
-            if (!err) err = launch_update_fp64(X, ld, m, 0, 0, c0, nc, nullptr, 0, T, nc, st);
+            if (!err) err = launch_update_fp64(X, ld, m, 0, 0, c0, nc, nullptr, 0, T, nc, shard == nullptr, st);
         }
         if (!err) err = launch_rblock(Rout, ldr, 0, 0, nc, nullptr, 0, nullptr, 0, R1, R2, 0, st);
         if (is_split(precision)) split_mark_stale(c0, nc);
@@ -1369,7 +1359,7 @@ int split_batch_plan(int count, const int* m, const int* n, const int* s, int nu
         std::vector<double> wsz(count);
         for (int b = 0; b < count; ++b)
             wsz[b] = (double)split_workspace_bytes(m[b], n[b], s[b], num_sms) +
-                     8.0 * ((double)part_doubles(m[b], n[b], s[b], num_sms) + (double)tsqr_workspace_doubles(m[b], s[b]));
+                     8.0 * ((double)part_doubles(m[b], n[b], s[b]) + (double)tsqr_workspace_doubles(m[b], s[b]));
         std::sort(wsz.begin(), wsz.end(), [](double a, double b) { return a > b; });
         double acc = 0.0;
         int fit = 0;
@@ -1542,9 +1532,8 @@ int orth_gb300_gram_dev(int m, int na, int b0, int nb, const double* dX, long lo
     int rc = init_ctx();
     if (rc) return 3;
     if (precision == ORTH_GB300_FP64) {
-        if (scr().part.ensure((size_t)part_doubles(m, n, s, g_ctx.num_sms) * sizeof(double))) return 3;
-        const int chunks = gram_chunks_fp64(m, na, nb, g_ctx.num_sms);
-        rc = launch_gram_fp64(dX, ldX, m, 0, na, b0, nb, dC, ldc, scr().part.as<double>(), chunks, st);
+        if (scr().part.ensure((size_t)gram_part_doubles_fp64(m, na, nb) * sizeof(double))) return 3;
+        rc = launch_gram_fp64(dX, ldX, m, 0, na, b0, nb, dC, ldc, scr().part.as<double>(), false, g_ctx.num_sms, st);
     } else {
         if (scr().split.ensure((size_t)split_workspace_bytes(m, n, s, g_ctx.num_sms))) return 3;
         rc = split_begin(const_cast<double*>(dX), ldX, m, n, s, split_digits_of(precision), scr().split.as<char>(), scr().split.bytes,
@@ -1613,13 +1602,7 @@ int orth_gb300_accuracy_dev(int m, int n, const double* dX, long long ldX, const
     double* dout = part + pd;
     int rc = 0;
     if (gram_precision == ORTH_GB300_FP64) {
-        i64 need = 0;
-        for (int na = GW; na < n + GW; na += GW) {
-            const int a = na < n ? na : n;
-            const i64 v = (i64)gram_chunks_fp64(m, a, GW, g_ctx.num_sms) * a * GW;
-            if (v > need) need = v;
-        }
-        if (scr().part.ensure((size_t)(need + 1024) * sizeof(double))) return 3;
+        if (scr().part.ensure((size_t)gram_part_doubles_fp64(m, n, GW) * sizeof(double))) return 3;
     } else {
         if (scr().split.ensure((size_t)split_workspace_bytes(m, n, 16, g_ctx.num_sms))) return 3;
         rc = split_begin(const_cast<double*>(dQ), ldQ, m, n, 16, 7, scr().split.as<char>(), scr().split.bytes,
@@ -1631,8 +1614,8 @@ int orth_gb300_accuracy_dev(int m, int n, const double* dX, long long ldX, const
         const int nb = n - c0 < GW ? n - c0 : GW;
         const int na = c0 + nb;
         if (gram_precision == ORTH_GB300_FP64) {
-            const int chunks = gram_chunks_fp64(m, na, nb, g_ctx.num_sms);
-            rc = launch_gram_fp64(dQ, ldQ, m, 0, na, c0, nb, G + (i64)c0 * n, n, scr().part.as<double>(), chunks, st);
+            rc = launch_gram_fp64(dQ, ldQ, m, 0, na, c0, nb, G + (i64)c0 * n, n, scr().part.as<double>(), true,
+                                  g_ctx.num_sms, st);
         } else {
             rc = launch_gram_split(dQ, ldQ, m, na, c0, nb, G + (i64)c0 * n, n, scr().split.as<char>(),
                                    scr().split.bytes, g_ctx.num_sms, st);

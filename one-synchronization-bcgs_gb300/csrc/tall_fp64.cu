@@ -1,161 +1,205 @@
-// Plain-FP64 tall kernels of the BCGS hot path.
+// Plain-FP64 tall Gram of the BCGS hot path (the update: update_fp64.cu).
 //
 // On GB300 the FP64 pipe delivers about 1.2 TFLOP/s (two DFMA per SM per clock),
-// while the tall products carry about 16 FLOP per byte of HBM traffic, so every
-// kernel in this file is bound by the FP64 pipe, not by HBM. The kernels are
-// therefore shaped to keep the DFMA pipe fed with few other instructions per
-// DFMA, and to reduce deterministically.
+// while the tall products carry about 16 FLOP per byte of HBM traffic, so the
+// product is bound by the FP64 pipe, not by HBM. The kernels are therefore shaped
+// for few FP64 instructions, and to reduce deterministically.
 //
 //   gram_fp64_partial  + gram_reduce : C = X[:, a0:a0+na]^T X[:, b0:b0+nb]
 //       replaces the reference's dgemm('T','N') + MPI_Allreduce pair
 //       (e.g. SRC/orth.c:182-188). One "synchronization" = one partial pass plus
 //       one fixed-order reduction.
-//   update_fp64 : Xc = (Xc - X[:, 0:K] S) T^{-1}, T upper triangular
-//       replaces dgemm('N','N') + dtrsm('R','U','N','N') (SRC/orth.c:173-176).
 #include "batched.h"
 #include "common.cuh"
 #include "kernels.h"
 
 namespace bcgs {
 
+// ---------------------------------------------------------------------------
+// Gram partials. A CTA of 128 threads owns TA columns of A x W = R 128 / TA columns of B
+// and walks a contiguous row range of X in stages of GR rows, copied to shared memory
+// asynchronously GST stages deep. Thread (ta, tb) keeps R sums: its column of A against
+// columns tb, tb + 128 / TA, ... of the W. Partial sums go to part[chunk][i + j * na]
+// (column-major na x nb per chunk). Every entry is a sequential FMA chain over the rows of
+// the chunk in order, so the result depends on the chunking only, not on TA or R.
+//
+// One FP64 instruction of a warp occupies its quarter of the SM for 64 clocks, so the
+// time is the number of instructions, 4 R per row and CTA, and every column the tile
+// has beyond na or nb is paid in full; loads, at most (1 + R) / R per product, are not.
+// The tile is therefore chosen per Gram for the least padding (gram_tile below): 32 x 20
+// for the 20 columns of blocks of 10, 32 x 4 for blocks of 4, instead of 16 x 32 for all.
+// Measured (16 x 32 tiles staged without copies in flight -> now): m = 3001, 64 x 4 97 ->
+// 6 us; m = 10^5, 200 x 20 1130 -> 700 us; m = 3 10^5, 272 x 32 4100 -> 3900 us, 1.23 TFLOP/s,
+// of which 3 % is the tile below the diagonal.
+// ---------------------------------------------------------------------------
 namespace {
-// Single-matrix Gram: one CTA per 16-column strip of A x 32 columns of B x row
-// chunk, so na (a multiple of s) wastes no work on zero padding.
-constexpr int GS_A = 16;            // C rows per CTA
-constexpr int GS_B = 32;            // C columns per CTA
-constexpr int GS_R = 16;            // X rows per shared-memory sub-tile
-constexpr int GS_CTAS_PER_SM = 16;  // resident strip CTAs per SM (64 registers, 7 KB)
+constexpr int GR = 16;              // X rows per stage
+constexpr int GST = 3;              // stages in flight
 constexpr int GT_R = 32;            // chunk row ranges are multiples of this
+constexpr int GTHREADS = 128;
+constexpr int GR_MAX = 8;           // columns of B per thread
+
+__host__ __device__ inline int gram_width(int ta, int r) { return r * (GTHREADS / ta); }
+__host__ __device__ inline int gram_stage_doubles(int ta, int r) { return GR * ((ta + gram_width(ta, r)) | 1); }
+
+__device__ __forceinline__ void cp_async8(double* dst, const double* src, bool valid) {
+    const uint32_t d = (uint32_t)__cvta_generic_to_shared(dst);
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(d), "l"(src), "r"(valid ? 8 : 0) : "memory");
+}
+__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int N>
+__device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
 }  // namespace
 
-// ---------------------------------------------------------------------------
-// Gram partials. CTA tile: GA rows of C (columns of A) x TB columns of C (columns
-// of B); (GA/4) x (TB/2) threads, each owning a 4 x 2 register tile. The CTA walks
-// a contiguous row range of X in sub-tiles of GR rows staged in shared memory.
-// Partial sums go to part[chunk][i + j * na] (column-major na x nb per chunk).
-// Every entry is a sequential FMA chain over the rows of the chunk in order, so
-// the result depends on the chunking only, not on GA, TB or GR.
-// ---------------------------------------------------------------------------
-template <int GA_, int TB_, int GR_>
-struct GramTile {
-    static constexpr int GA = GA_, TB = TB_, GR = GR_;
-    static constexpr int NT = (GA / 4) * (TB / 2);                // threads
-    static constexpr int SMEM = GR * (GA + 1) + GR * (TB + 1);    // doubles
-};
-// Batched form: 64 threads, GA = 512 / TB, TB in {8, 16, 32} (B panels of 2s
-// columns for s = 4, 8, 16 against A strips of 64, 32 or 16 columns).
-template <int TB>
-using GramPanel = GramTile<512 / TB, TB, 16>;
-using GramStrip = GramTile<GS_A, GS_B, GS_R>;
-static_assert(GramStrip::NT == 64 && GramPanel<8>::NT == 64 && GramPanel<16>::NT == 64 && GramPanel<32>::NT == 64,
-              "strip CTAs are two warps");
-constexpr int kGramSmemMax = GramPanel<32>::SMEM > GramPanel<8>::SMEM
-                                 ? (GramPanel<32>::SMEM > GramPanel<16>::SMEM ? GramPanel<32>::SMEM
-                                                                              : GramPanel<16>::SMEM)
-                                 : (GramPanel<8>::SMEM > GramPanel<16>::SMEM ? GramPanel<8>::SMEM
-                                                                             : GramPanel<16>::SMEM);
-
 // The tile at C rows ia0.., C columns jb0.., rows [r_begin, r_end) of X, written to
-// `out` (na x nb, ld na). Tile::NT threads; sm holds Tile::SMEM doubles.
+// `out` (na x nb, ld na). sm holds GST stages of gram_stage_doubles(ta, R).
 // SEGR > 0: every SEGR rows the running sums are added to a total and restarted,
 // so no FMA chain is longer than SEGR rows however long the row range is
 // (SEGR = 0: one chain over the range).
-template <class Tile, int SEGR = 0>
+template <int R, int SEGR = 0>
 __device__ __forceinline__ void gram_partial_body(const double* __restrict__ X, i64 ld, int a0, int na, int b0,
-                                                  int nb, i64 r_begin, i64 r_end, int ia0, int jb0,
+                                                  int nb, int ta, i64 r_begin, i64 r_end, int ia0, int jb0,
                                                   double* __restrict__ out, double* __restrict__ sm) {
-    constexpr int GA = Tile::GA, TB = Tile::TB, GR = Tile::GR, NT = Tile::NT;
-    constexpr int SEG = SEGR / GR;  // sub-tiles per segment
-    static_assert(SEGR % GR == 0, "segments are whole sub-tiles");
-    constexpr int TI = GA / 4;      // threads along C rows -> 4 rows each
-    double (*sA)[GA + 1] = reinterpret_cast<double (*)[GA + 1]>(sm);
-    double (*sB)[TB + 1] = reinterpret_cast<double (*)[TB + 1]>(sm + GR * (GA + 1));
+    constexpr int SEG = SEGR / GR;  // stages per segment
+    static_assert(SEGR % GR == 0, "segments are whole stages");
+    const int tbn = GTHREADS / ta, w = R * tbn;
+    const int ldr = (ta + w) | 1;
     const int tid = threadIdx.x;
-    const int ti = tid % TI;
-    const int tj = tid / TI;        // TB/2 threads along C cols -> 2 cols each
+    const int ca = tid & (ta - 1), tb = tid / ta;
+    const int nst = r_end > r_begin ? (int)((r_end - r_begin + GR - 1) / GR) : 0;
 
-    double acc[4][2], tot[4][2];
+    // Stage s into its buffer: consecutive threads copy consecutive rows of a column;
+    // rows past r_end and columns past na or nb become zeros.
+    const int rr = tid % GR, cc0 = tid / GR;
+    auto fill = [&](int s) {
+        const i64 r = r_begin + (i64)s * GR + rr;
+        double* dst = sm + (s % GST) * (GR * ldr) + rr * ldr;
+        const bool row = r < r_end;
+        for (int cc = cc0; cc < ta + w; cc += GTHREADS / GR) {
+            const bool isa = cc < ta;
+            const int c = isa ? ia0 + cc : jb0 + cc - ta;
+            const bool ok = row && c < (isa ? na : nb);
+            cp_async8(dst + cc, ok ? X + r + (i64)((isa ? a0 : b0) + c) * ld : X, ok);
+        }
+    };
+    double acc[R], tot[R];
 #pragma unroll
-    for (int a = 0; a < 4; ++a) { acc[a][0] = 0.0; acc[a][1] = 0.0; tot[a][0] = 0.0; tot[a][1] = 0.0; }
-
+    for (int k = 0; k < R; ++k) { acc[k] = 0.0; tot[k] = 0.0; }
+#pragma unroll
+    for (int s = 0; s < GST - 1; ++s) {
+        if (s < nst) fill(s);
+        cp_async_commit();
+    }
     int sub = 0;
-    for (i64 r0 = r_begin; r0 < r_end; r0 += GR) {
+    for (int s = 0; s < nst; ++s) {
         if (SEG > 0 && sub == SEG) {
 #pragma unroll
-            for (int a = 0; a < 4; ++a) {
-                tot[a][0] += acc[a][0]; tot[a][1] += acc[a][1];
-                acc[a][0] = 0.0; acc[a][1] = 0.0;
-            }
+            for (int k = 0; k < R; ++k) { tot[k] += acc[k]; acc[k] = 0.0; }
             sub = 0;
         }
         ++sub;
-        // Stage A[r0:r0+GR, ia0:ia0+GA] and B[r0:r0+GR, jb0:jb0+TB]. Consecutive
-        // threads read consecutive rows of one column.
-        for (int e = tid; e < GR * GA; e += NT) {
-            int rr = e % GR, cc = e / GR;
-            i64 r = r0 + rr;
-            int c = ia0 + cc;
-            sA[rr][cc] = (r < r_end && c < na) ? X[r + (i64)(a0 + c) * ld] : 0.0;
-        }
-        for (int e = tid; e < GR * TB; e += NT) {
-            int rr = e % GR, cc = e / GR;
-            i64 r = r0 + rr;
-            int c = jb0 + cc;
-            sB[rr][cc] = (r < r_end && c < nb) ? X[r + (i64)(b0 + c) * ld] : 0.0;
-        }
-        __syncthreads();
+        cp_async_wait<GST - 2>();
+        __syncthreads();   // stage s is here, and every thread is done with stage s - 1
+        if (s + GST - 1 < nst) fill(s + GST - 1);
+        cp_async_commit();
+        const double* pa = sm + (s % GST) * (GR * ldr) + ca;
+        const double* pb = pa - ca + ta + tb;
 #pragma unroll 4
-        for (int rr = 0; rr < GR; ++rr) {
-            double av[4], bv[2];
+        for (int q = 0; q < GR; ++q) {
+            const double av = pa[q * ldr];
 #pragma unroll
-            for (int a = 0; a < 4; ++a) av[a] = sA[rr][ti + TI * a];
-            bv[0] = sB[rr][tj];
-            bv[1] = sB[rr][tj + TB / 2];
-#pragma unroll
-            for (int a = 0; a < 4; ++a) {
-                acc[a][0] = fma(av[a], bv[0], acc[a][0]);
-                acc[a][1] = fma(av[a], bv[1], acc[a][1]);
-            }
+            for (int k = 0; k < R; ++k) acc[k] = fma(av, pb[q * ldr + k * tbn], acc[k]);
         }
-        __syncthreads();
     }
     if (SEG > 0) {
 #pragma unroll
-        for (int a = 0; a < 4; ++a) { acc[a][0] += tot[a][0]; acc[a][1] += tot[a][1]; }
+        for (int k = 0; k < R; ++k) acc[k] += tot[k];
     }
+    const int i = ia0 + ca;
 #pragma unroll
-    for (int a = 0; a < 4; ++a) {
-        int i = ia0 + ti + TI * a;
-#pragma unroll
-        for (int b = 0; b < 2; ++b) {
-            int j = jb0 + tj + (TB / 2) * b;
-            if (i < na && j < nb) out[i + (i64)j * na] = acc[a][b];
+    for (int k = 0; k < R; ++k) {
+        const int j = jb0 + tb + k * tbn;
+        if (i < na && j < nb) out[i + (i64)j * na] = acc[k];
+    }
+}
+
+// Tile (ta, r) of a Gram and the number of its tiles that are not skipped. With
+// `upper` (>= 0: b0 - a0) only entries on or above the diagonal of X^T X are needed, and
+// tiles wholly below it are left out (their part is not written).
+struct GramTile {
+    int ta = 32, r = 1, tilesA = 1, tilesB = 1;
+    i64 live = 1;
+};
+// Strips of A a tile column (columns [jb w, (jb + 1) w) of the nb) has above the diagonal.
+__host__ __device__ inline int gram_live_strips(int upper, int jb, int w, int nb, int ta, int tilesA) {
+    if (upper < 0) return tilesA;
+    const int end = upper + (jb * w + w < nb ? jb * w + w : nb);
+    const int hi = (end + ta - 1) / ta;
+    return hi < tilesA ? hi : tilesA;
+}
+// Live tile t: its strip and column, counted column by column.
+__device__ __forceinline__ void gram_tile_of(int t, int upper, int w, int nb, int ta, int tilesA, int& ia0, int& jb0) {
+    int jb = 0;
+    for (;; ++jb) {
+        const int hi = gram_live_strips(upper, jb, w, nb, ta, tilesA);
+        if (t < hi) break;
+        t -= hi;
+    }
+    ia0 = t * ta;
+    jb0 = jb * w;
+}
+static GramTile gram_tile(int na, int nb, int upper) {
+    GramTile best;
+    i64 best_cost = -1, best_loads = 0;
+    for (int ta = 16; ta <= 64; ta *= 2)
+        for (int r = 1; r <= GR_MAX; ++r) {
+            const int w = gram_width(ta, r);
+            if (r > 1 && gram_width(ta, r - 1) >= nb) break;
+            GramTile t;
+            t.ta = ta; t.r = r;
+            t.tilesA = (int)ceil_div(na, ta); t.tilesB = (int)ceil_div(nb, w);
+            t.live = 0;
+            for (int jb = 0; jb < t.tilesB; ++jb) t.live += gram_live_strips(upper, jb, w, nb, ta, t.tilesA);
+            const i64 cost = t.live * r, loads = t.live * (ta + w);
+            if (best_cost < 0 || cost < best_cost || (cost == best_cost && loads < best_loads)) {
+                best_cost = cost; best_loads = loads;
+                best = t;
+            }
         }
-    }
+    return best;
 }
 
-__global__ void __launch_bounds__(GramStrip::NT, GS_CTAS_PER_SM)
-gram_fp64_partial(const double* __restrict__ X, i64 ld, i64 m, int a0, int na, int b0, int nb,
+// blockIdx: chunk, live tile (no CTA for a skipped one: an SM that got one would be left
+// with less than its share while others take one more).
+template <int R, int SEGR>
+__global__ void __launch_bounds__(GTHREADS)
+gram_fp64_partial(const double* __restrict__ X, i64 ld, i64 m, int a0, int na, int b0, int nb, int ta, int upper,
                   i64 rows_per_chunk, double* __restrict__ part) {
-    __shared__ double sm[GramStrip::SMEM];
+    extern __shared__ double sm[];
     const int chunk = blockIdx.x;
+    int ia0, jb0;
+    gram_tile_of((int)blockIdx.y, upper, gram_width(ta, R), nb, ta, (na + ta - 1) / ta, ia0, jb0);
     const i64 r_begin = (i64)chunk * rows_per_chunk;
     const i64 r_end = min(m, r_begin + rows_per_chunk);
-    gram_partial_body<GramStrip>(X, ld, a0, na, b0, nb, r_begin, r_end, blockIdx.y * GS_A, blockIdx.z * GS_B,
-                                 part + (i64)chunk * na * nb, sm);
+    gram_partial_body<R, SEGR>(X, ld, a0, na, b0, nb, ta, r_begin, r_end, ia0, jb0, part + (i64)chunk * na * nb, sm);
 }
 
-// The same over chunks of rows_per_chunk rows, each summed in segments of
-// 256 rows (the row-sharded path's long chunks).
-__global__ void __launch_bounds__(GramStrip::NT, GS_CTAS_PER_SM)
-gram_fp64_partial_seg(const double* __restrict__ X, i64 ld, i64 m, int a0, int na, int b0, int nb,
-                      i64 rows_per_chunk, double* __restrict__ part) {
-    __shared__ double sm[GramStrip::SMEM];
-    const int chunk = blockIdx.x;
-    const i64 r_begin = (i64)chunk * rows_per_chunk;
-    const i64 r_end = min(m, r_begin + rows_per_chunk);
-    gram_partial_body<GramStrip, 256>(X, ld, a0, na, b0, nb, r_begin, r_end, blockIdx.y * GS_A,
-                                      blockIdx.z * GS_B, part + (i64)chunk * na * nb, sm);
+template <int SEGR>
+static int launch_partial(const GramTile& t, int nchunks, const double* X, i64 ld, i64 m, int a0, int na, int b0,
+                          int nb, int upper, i64 rows, double* part, cudaStream_t st) {
+    const dim3 grid((unsigned)nchunks, (unsigned)t.live);
+    const size_t smem = (size_t)GST * gram_stage_doubles(t.ta, t.r) * sizeof(double);
+    switch (t.r) {
+#define BCGS_GP(RR)                                                                                              \
+    case RR:                                                                                                     \
+        gram_fp64_partial<RR, SEGR><<<grid, GTHREADS, smem, st>>>(X, ld, m, a0, na, b0, nb, t.ta, upper, rows, part); \
+        break;
+        BCGS_GP(1) BCGS_GP(2) BCGS_GP(3) BCGS_GP(4) BCGS_GP(5) BCGS_GP(6) BCGS_GP(7) BCGS_GP(8)
+#undef BCGS_GP
+        default: return (int)cudaErrorInvalidValue;
+    }
+    g_launch_count += 1;
+    return (int)cudaGetLastError();
 }
 
 // Fixed-order sum over chunks: out[i + j*ldo] = sum_{c=0}^{nchunks-1} part[c][i + j*na].
@@ -174,17 +218,33 @@ __device__ __forceinline__ void gram_reduce_body(const double* __restrict__ part
     const i64 e = blk * RD_THREADS + threadIdx.x;
     if (e >= total) return;
     const double* p = part + e;
-    double s = 0.0;
+    double s = 0.0, v[RD_AHEAD], n[RD_AHEAD];
     int c = 0;
-    for (; c + RD_AHEAD <= nchunks; c += RD_AHEAD) {
-        double v[RD_AHEAD];
+    if (nchunks >= RD_AHEAD) {
 #pragma unroll
-        for (int k = 0; k < RD_AHEAD; ++k) v[k] = p[(i64)(c + k) * total];
+        for (int k = 0; k < RD_AHEAD; ++k) v[k] = p[(i64)k * total];
+        for (; c + 2 * RD_AHEAD <= nchunks; c += RD_AHEAD) {
+#pragma unroll
+            for (int k = 0; k < RD_AHEAD; ++k) n[k] = p[(i64)(c + RD_AHEAD + k) * total];
+#pragma unroll
+            for (int k = 0; k < RD_AHEAD; ++k) s += v[k];
+#pragma unroll
+            for (int k = 0; k < RD_AHEAD; ++k) v[k] = n[k];
+        }
 #pragma unroll
         for (int k = 0; k < RD_AHEAD; ++k) s += v[k];
+        c += RD_AHEAD;
     }
-#pragma unroll 4
-    for (; c < nchunks; ++c) s += p[(i64)c * total];
+#pragma unroll
+    for (int k = 0; k < RD_AHEAD; ++k) v[k] = c + k < nchunks ? p[(i64)(c + k) * total] : 0.0;
+#pragma unroll 1
+    for (int k = 0; c < nchunks; ++c, ++k) {
+        double x = v[0];
+#pragma unroll
+        for (int q = 1; q < RD_AHEAD; ++q)
+            if (q == k) x = v[q];
+        s += x;
+    }
     out[e % na + (e / na) * ldo] = s;
 }
 
@@ -199,33 +259,62 @@ int gram_reduce_ctas(int na, int nb) { return (int)ceil_div((i64)na * nb, RD_THR
 // policy below).
 long long g_gram_chunk_rows = 0;
 
-int gram_chunks_fp64(i64 m, int na, int nb, int num_sms) {
+// Doubles of partials a Gram may take: at most what a full SM's worth of 16 x 32 tiles
+// per SM would (for narrower B in proportion), and chunks of no fewer than GC_MIN rows.
+constexpr int GC_MIN = 64;
+static i64 gram_part_cap(int nb) { return 16LL * kNumSMsDefault * 16 * (nb < 32 ? nb : 32); }
+
+i64 gram_part_doubles_fp64(i64 m, int na_max, int nb_max) {
+    const i64 one = (i64)na_max * nb_max;
+    if (g_gram_chunk_rows > 0) return ceil_div(m, g_gram_chunk_rows) * one + 1024;
+    const i64 cap = gram_part_cap(nb_max), all = ceil_div(m, GC_MIN) * one;
+    const i64 most = cap < all ? cap : all;
+    return (most > one ? most : one) + 1024;
+}
+
+// Chunks: the CTAs (live tiles x chunks, equal work each) are laid on the SMs in w
+// rounds, w = 1 .. 16, as many as fit; a round of L rows takes 64 R L clocks on each
+// SM quarter, and every chunk adds about 130 clocks to the reduction's chain. More
+// rounds mean fewer SMs idle in the last one and shorter chains, fewer mean fewer
+// partials. One CTA of four warps keeps the FP64 pipe 63 % busy (its barriers and loads
+// have nothing beside them), two 91 %, three 97 % (ncu, m = 10^5, na x nb = 100 x 10 to
+// 200 x 8).
+static int gram_chunks(i64 m, int na, int nb, const GramTile& t, int num_sms) {
     if (g_gram_chunk_rows > 0) {
         const i64 c = ceil_div(m, g_gram_chunk_rows);
         return (int)(c < 1 ? 1 : c);
     }
-    // One wave: the most chunks whose strip CTAs all fit on the SMs at once, so
-    // every SM gets the same number of equal CTAs (within one), each with at
-    // least 256 rows. The FP64 pipe is saturated by two resident CTAs per SM;
-    // what costs time is an SM holding more CTAs than the others.
-    const i64 ctas_per_chunk = ceil_div(na, GS_A) * ceil_div(nb, GS_B);
-    i64 want = (i64)GS_CTAS_PER_SM * num_sms / ctas_per_chunk;
-    i64 max_by_rows = ceil_div(m, 256);
-    i64 c = want < max_by_rows ? want : max_by_rows;
-    if (c < 1) c = 1;
-    if (c > 4096) c = 4096;
-    return (int)c;
+    const i64 one = (i64)na * nb;
+    i64 cmax = gram_part_cap(nb) / one;
+    const i64 crows = ceil_div(m, GC_MIN);
+    if (cmax > crows) cmax = crows;
+    if (cmax > 4096) cmax = 4096;
+    if (cmax < 1) cmax = 1;
+    i64 best = 1;
+    double best_cost = 0.0;
+    for (int w = 1; w <= 16; ++w) {
+        i64 c = (i64)w * num_sms / t.live;
+        if (c < 1) c = 1;
+        if (c > cmax) c = cmax;
+        const i64 rows = ceil_div(ceil_div(m, c), GT_R) * GT_R;
+        c = ceil_div(m, rows);
+        const double rounds = (double)ceil_div(c * t.live, num_sms);
+        const double busy = rounds < 1.5 ? 0.63 : (rounds < 2.5 ? 0.91 : 0.97);
+        const double cost = rounds * (64.0 * t.r * (double)rows / busy + 1000.0) + 130.0 * (double)c;
+        if (w == 1 || cost < best_cost) { best = c; best_cost = cost; }
+    }
+    return (int)best;
 }
 
-int launch_gram_fp64(const double* X, i64 ld, i64 m, int a0, int na, int b0, int nb,
-                     double* out, int ldo, double* part, int nchunks, cudaStream_t st) {
+int launch_gram_fp64(const double* X, i64 ld, i64 m, int a0, int na, int b0, int nb, double* out, int ldo,
+                     double* part, bool upper_only, int num_sms, cudaStream_t st) {
     if (na <= 0 || nb <= 0) return 0;
+    const int upper = upper_only ? b0 - a0 : -1;
+    const GramTile t = gram_tile(na, nb, upper);
+    const int nchunks = gram_chunks(m, na, nb, t, num_sms);
     i64 rows_per_chunk = ceil_div(m, nchunks);
     rows_per_chunk = ceil_div(rows_per_chunk, GT_R) * GT_R;
-    dim3 grid((unsigned)nchunks, (unsigned)ceil_div(na, GS_A), (unsigned)ceil_div(nb, GS_B));
-    gram_fp64_partial<<<grid, GramStrip::NT, 0, st>>>(X, ld, m, a0, na, b0, nb, rows_per_chunk, part);
-    g_launch_count += 1;
-    const int rc = (int)cudaGetLastError();
+    const int rc = launch_partial<0>(t, nchunks, X, ld, m, a0, na, b0, nb, upper, rows_per_chunk, part, st);
     return rc ? rc : launch_gram_reduce(part, nchunks, na, nb, out, ldo, st);
 }
 
@@ -233,11 +322,8 @@ int launch_gram_partials_fp64(const double* X, i64 ld, i64 m, int a0, int na, in
                               i64 rows, cudaStream_t st) {
     if (na <= 0 || nb <= 0 || m <= 0) return 0;
     if (rows <= 0 || rows % GT_R != 0) return (int)cudaErrorInvalidValue;
-    const i64 nchunks = ceil_div(m, rows);
-    dim3 grid((unsigned)nchunks, (unsigned)ceil_div(na, GS_A), (unsigned)ceil_div(nb, GS_B));
-    gram_fp64_partial_seg<<<grid, GramStrip::NT, 0, st>>>(X, ld, m, a0, na, b0, nb, rows, part);
-    g_launch_count += 1;
-    return (int)cudaGetLastError();
+    return launch_partial<256>(gram_tile(na, nb, -1), (int)ceil_div(m, rows), X, ld, m, a0, na, b0, nb, -1, rows, part,
+                               st);
 }
 
 int launch_gram_reduce(const double* part, int nchunks, int na, int nb, double* out, int ldo,
@@ -249,143 +335,34 @@ int launch_gram_reduce(const double* part, int nchunks, int na, int nb, double* 
 }
 
 // ---------------------------------------------------------------------------
-// Update: Xc[r, 0:nc] = (Xc[r, :] - sum_c Q[r, c] S[c, :]) * T^{-1}.
-// One thread per row with NC register accumulators; S is staged through shared
-// memory in chunks of 64 rows (broadcast reads). T is upper triangular (nc x nc,
-// ld ldt); its diagonal is inverted once per CTA. If T is null the scaling is
-// skipped (bcgsi21s's unscaled first pass, SRC/orth.c:323-324).
-// ---------------------------------------------------------------------------
-namespace {
-constexpr int UP_THREADS = 128;
-}  // namespace
-
-// Rows of S staged per shared-memory chunk; keeps static shared memory < 48 KB.
-template <int NC>
-struct UpChunk { static constexpr int value = NC <= 16 ? 64 : (NC <= 32 ? 32 : 16); };
-
-// Shared-memory doubles update_body<NC> needs: S chunk, T, T's reciprocal diagonal.
-template <int NC>
-struct UpSmem { static constexpr int value = UpChunk<NC>::value * NC + NC * NC + NC; };
-
-// Rows [r0, r0 + 128) of the update, one row per thread (128 threads). sm holds
-// UpSmem<NC>::value doubles. Every output is an FMA chain over k in order, then the
-// forward substitution in column order, so the result does not depend on NC >= nc.
-template <int NC>
-__device__ __forceinline__ void update_body(double* __restrict__ X, i64 ld, i64 m, int q0, int K, int c0, int nc,
-                                            const double* __restrict__ S, int lds, const double* __restrict__ T,
-                                            int ldt, i64 r0, double* __restrict__ sm) {
-    constexpr int KCH = UpChunk<NC>::value;
-    double (*sS)[NC] = reinterpret_cast<double (*)[NC]>(sm);
-    double (*sT)[NC] = reinterpret_cast<double (*)[NC]>(sm + KCH * NC);
-    double* sRd = sm + KCH * NC + NC * NC;
-    const int tid = threadIdx.x;
-    const i64 r = r0 + tid;
-    if (T != nullptr) {
-        for (int e = tid; e < NC * NC; e += UP_THREADS) {
-            int i = e % NC, j = e / NC;
-            sT[i][j] = (i < nc && j < nc && i <= j) ? T[i + (i64)j * ldt] : 0.0;
-        }
-    }
-    __syncthreads();
-    if (T != nullptr && tid < NC) sRd[tid] = (tid < nc) ? 1.0 / sT[tid][tid] : 0.0;
-
-    double acc[NC];
-#pragma unroll
-    for (int j = 0; j < NC; ++j) acc[j] = 0.0;
-    const bool live = r < m;
-    for (int k0 = 0; k0 < K; k0 += KCH) {
-        const int kc = min(KCH, K - k0);
-        __syncthreads();
-        for (int e = tid; e < KCH * NC; e += UP_THREADS) {
-            int kk = e / NC, j = e % NC;
-            sS[kk][j] = (kk < kc && j < nc) ? S[(k0 + kk) + (i64)j * lds] : 0.0;
-        }
-        __syncthreads();
-        if (live) {
-            const double* qrow = X + r + (i64)(q0 + k0) * ld;
-#pragma unroll 4
-            for (int kk = 0; kk < kc; ++kk) {
-                const double q = qrow[(i64)kk * ld];
-#pragma unroll
-                for (int j = 0; j < NC; ++j) acc[j] = fma(q, sS[kk][j], acc[j]);
-            }
-        }
-    }
-    __syncthreads();
-    if (live) {
-        double* xr = X + r + (i64)c0 * ld;
-        // acc becomes w = x - Q S in place.
-#pragma unroll
-        for (int j = 0; j < NC; ++j) acc[j] = (j < nc) ? xr[(i64)j * ld] - acc[j] : 0.0;
-        if (T != nullptr) {
-            // Forward substitution u T = w (dtrsm 'R','U','N','N'), column by column.
-#pragma unroll
-            for (int j = 0; j < NC; ++j) {
-                double v = acc[j];
-#pragma unroll
-                for (int i = 0; i < j; ++i) v = fma(-acc[i], sT[i][j], v);
-                acc[j] = v * sRd[j];
-            }
-        }
-#pragma unroll
-        for (int j = 0; j < NC; ++j)
-            if (j < nc) xr[(i64)j * ld] = acc[j];
-    }
-    __syncthreads();   // sm is reused by the caller's next tile
-}
-
-template <int NC>
-__global__ void __launch_bounds__(UP_THREADS)
-update_fp64(double* __restrict__ X, i64 ld, i64 m, int q0, int K, int c0, int nc,
-            const double* __restrict__ S, int lds, const double* __restrict__ T, int ldt) {
-    __shared__ double sm[UpSmem<NC>::value];
-    update_body<NC>(X, ld, m, q0, K, c0, nc, S, lds, T, ldt, blockIdx.x * (i64)UP_THREADS, sm);
-}
-
-int launch_update_fp64(double* X, i64 ld, i64 m, int q0, int K, int c0, int nc,
-                       const double* S, int lds, const double* T, int ldt, cudaStream_t st) {
-    if (nc <= 0 || m <= 0) return 0;
-    dim3 grid((unsigned)ceil_div(m, UP_THREADS));
-    if (nc <= 4)
-        update_fp64<4><<<grid, UP_THREADS, 0, st>>>(X, ld, m, q0, K, c0, nc, S, lds, T, ldt);
-    else if (nc <= 8)
-        update_fp64<8><<<grid, UP_THREADS, 0, st>>>(X, ld, m, q0, K, c0, nc, S, lds, T, ldt);
-    else if (nc <= 16)
-        update_fp64<16><<<grid, UP_THREADS, 0, st>>>(X, ld, m, q0, K, c0, nc, S, lds, T, ldt);
-    else if (nc <= 32)
-        update_fp64<32><<<grid, UP_THREADS, 0, st>>>(X, ld, m, q0, K, c0, nc, S, lds, T, ldt);
-    else if (nc <= 64)
-        update_fp64<64><<<grid, UP_THREADS, 0, st>>>(X, ld, m, q0, K, c0, nc, S, lds, T, ldt);
-    else
-        return (int)cudaErrorInvalidValue;
-    g_launch_count += 1;
-    return (int)cudaGetLastError();
-}
-
-// ---------------------------------------------------------------------------
 // Batched forms: one launch over many matrices' jobs (batched.h).
 // ---------------------------------------------------------------------------
-int gram_batched_panel_rows(int tb) { return 512 / tb; }
+int gram_batched_tile(int na, int b0, int nb, int* ta, int* r) {
+    const GramTile t = gram_tile(na, nb, b0);
+    *ta = t.ta; *r = t.r;
+    return (int)t.live;
+}
 
-__global__ void __launch_bounds__(64, GS_CTAS_PER_SM)
+// Job j's CTAs: chunk fastest, then live tile.
+__global__ void __launch_bounds__(GTHREADS)
 gram_partial_batched(const GramJob* __restrict__ jobs, const int* __restrict__ prefix, int njobs) {
-    __shared__ double sm[kGramSmemMax];
+    extern __shared__ double sm[];
     const int j = batched_job_of(prefix, njobs, blockIdx.x);
-    const GramJob& J = jobs[j];
+    const GramJob J = jobs[j];
     const int local = blockIdx.x - prefix[j];
     const int chunk = local % J.nchunks;
     const int t = local / J.nchunks;
-    const int ia = t % J.tilesA, jb = t / J.tilesA;
+    int ia0, jb0;
+    gram_tile_of(t, J.b0, gram_width(J.ta, J.r), J.nb, J.ta, (J.na + J.ta - 1) / J.ta, ia0, jb0);
     const i64 r_begin = (i64)chunk * J.rows_per_chunk;
     const i64 r_end = min(J.m, r_begin + J.rows_per_chunk);
     double* out = J.part + (i64)chunk * J.na * J.nb;
-    const int ia0 = ia * (512 / J.tb);
-    if (J.tb == 8)
-        gram_partial_body<GramPanel<8>>(J.X, J.ld, 0, J.na, J.b0, J.nb, r_begin, r_end, ia0, jb * 8, out, sm);
-    else if (J.tb == 16)
-        gram_partial_body<GramPanel<16>>(J.X, J.ld, 0, J.na, J.b0, J.nb, r_begin, r_end, ia0, jb * 16, out, sm);
-    else
-        gram_partial_body<GramPanel<32>>(J.X, J.ld, 0, J.na, J.b0, J.nb, r_begin, r_end, ia0, jb * 32, out, sm);
+    switch (J.r) {
+#define BCGS_GB(RR) \
+    case RR: gram_partial_body<RR>(J.X, J.ld, 0, J.na, J.b0, J.nb, J.ta, r_begin, r_end, ia0, jb0, out, sm); break;
+        BCGS_GB(1) BCGS_GB(2) BCGS_GB(3) BCGS_GB(4) BCGS_GB(5) BCGS_GB(6) BCGS_GB(7) BCGS_GB(8)
+#undef BCGS_GB
+    }
 }
 
 // Each job's sum in the single launch's order (items: gram_reduce_ctas per job).
@@ -396,23 +373,11 @@ gram_reduce_batched(const GramJob* __restrict__ jobs, const int* __restrict__ pr
     gram_reduce_body(J.part, J.nchunks, J.na, J.nb, J.C, J.ldc, blockIdx.x - prefix[j]);
 }
 
-__global__ void __launch_bounds__(UP_THREADS)
-update_batched(const UpdJob* __restrict__ jobs, const int* __restrict__ prefix, int njobs) {
-    __shared__ double sm[UpSmem<16>::value];
-    const int j = batched_job_of(prefix, njobs, blockIdx.x);
-    const UpdJob& J = jobs[j];
-    const i64 r0 = (i64)(blockIdx.x - prefix[j]) * UP_THREADS;
-    if (J.nc <= 4)
-        update_body<4>(J.X, J.ld, J.m, J.q0, J.K, J.c0, J.nc, J.S, J.lds, J.T, J.ldt, r0, sm);
-    else if (J.nc <= 8)
-        update_body<8>(J.X, J.ld, J.m, J.q0, J.K, J.c0, J.nc, J.S, J.lds, J.T, J.ldt, r0, sm);
-    else
-        update_body<16>(J.X, J.ld, J.m, J.q0, J.K, J.c0, J.nc, J.S, J.lds, J.T, J.ldt, r0, sm);
-}
-
 int launch_gram_partial_batched(const GramJob* jobs, const int* prefix, int njobs, int items, cudaStream_t st) {
     if (items <= 0) return 0;
-    gram_partial_batched<<<(unsigned)items, 64, 0, st>>>(jobs, prefix, njobs);
+    // Stages for the widest tile a batch's blocks (s <= 16) can take.
+    constexpr size_t smem = (size_t)GST * GR * ((64 + 2 * GR_MAX) | 1) * sizeof(double);
+    gram_partial_batched<<<(unsigned)items, GTHREADS, smem, st>>>(jobs, prefix, njobs);
     g_launch_count += 1;
     return (int)cudaGetLastError();
 }
@@ -420,13 +385,6 @@ int launch_gram_partial_batched(const GramJob* jobs, const int* prefix, int njob
 int launch_gram_reduce_batched(const GramJob* jobs, const int* prefix, int njobs, int items, cudaStream_t st) {
     if (items <= 0) return 0;
     gram_reduce_batched<<<(unsigned)items, RD_THREADS, 0, st>>>(jobs, prefix, njobs);
-    g_launch_count += 1;
-    return (int)cudaGetLastError();
-}
-
-int launch_update_batched(const UpdJob* jobs, const int* prefix, int njobs, int items, cudaStream_t st) {
-    if (items <= 0) return 0;
-    update_batched<<<(unsigned)items, UP_THREADS, 0, st>>>(jobs, prefix, njobs);
     g_launch_count += 1;
     return (int)cudaGetLastError();
 }

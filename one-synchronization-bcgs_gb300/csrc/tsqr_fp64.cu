@@ -122,7 +122,7 @@ __device__ __forceinline__ void make_reflector(double* a, double* tau, double* r
     auto below = [&]() {
         double p = 0.0;
 #pragma unroll
-        for (int i = 0; i < RPL; ++i) {
+        for (int i = RPL - 1; i >= 0; --i) {
             const double y = lane + 32 * i > c ? x[i] : 0.0;
             p = fma(y, y, p);
         }
