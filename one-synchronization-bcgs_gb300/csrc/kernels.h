@@ -30,12 +30,15 @@ int smem_attr(const void* fn, int bytes);
 
 // C (na x nb, ld ldo) = X[:, a0:a0+na]^T X[:, b0:b0+nb] over m rows, FP64, with a
 // fixed-order two-stage reduction through `part` (gram_part_doubles_fp64 doubles).
-// upper_only: only the entries on or above the diagonal of X^T X are defined.
+// upper_only: only the entries on or above the diagonal of X^T X are defined. gate: if
+// not null and *gate is 0, the product is left out (out is then undefined). counted:
+// whether this is one of the algorithm's synchronizations (g_reduce_count).
 i64 gram_part_doubles_fp64(i64 m, int na_max, int nb_max);   // for any na, nb up to these
 // Rows per chunk forced by orth_gb300_set_gram_chunk_rows (0: default policy).
 extern long long g_gram_chunk_rows;
 int launch_gram_fp64(const double* X, i64 ld, i64 m, int a0, int na, int b0, int nb,
-                     double* out, int ldo, double* part, bool upper_only, int num_sms, cudaStream_t st);
+                     double* out, int ldo, double* part, bool upper_only, int num_sms, cudaStream_t st,
+                     const int* gate = nullptr, bool counted = true);
 
 // out (na x nb, ld ldo) = fixed-order sum of nchunks partials part[c][i + j*na].
 int launch_gram_reduce(const double* part, int nchunks, int na, int nb, double* out, int ldo,
@@ -44,9 +47,11 @@ int gram_reduce_ctas(int na, int nb);   // CTAs of one reduction
 
 // X[:, c0:c0+nc] = (X[:, c0:c0+nc] - X[:, q0:q0+K] S) T^{-1}; T upper (nc x nc) or null.
 // any_split: K may be summed in quarters, by a rule on m; without it each row's result
-// does not depend on how many rows there are (the row-sharded path).
+// does not depend on how many rows there are (the row-sharded path). gate: if not null
+// and *gate is 0, X is left as it is.
 int launch_update_fp64(double* X, i64 ld, i64 m, int q0, int K, int c0, int nc,
-                       const double* S, int lds, const double* T, int ldt, bool any_split, cudaStream_t st);
+                       const double* S, int lds, const double* T, int ldt, bool any_split, cudaStream_t st,
+                       const int* gate = nullptr);
 
 // The small work of one block step on the reduced Gram G (small_fp64.cu): with
 // Y = G[0:K, 0:ny], Z = G[0:K, ny:ny+nz],
@@ -68,6 +73,10 @@ struct StepJob {
     int mode = -1, c0 = 0, ldR = 0, lda = 0;
     double* R = nullptr;
     const double *A = nullptr, *Sold = nullptr;
+    // If not null (K = 0): *ok = every pivot of T is at least ok_ratio times its diagonal
+    // entry of G, i.e. no column is closer than sqrt(ok_ratio) to those before it.
+    int* ok = nullptr;
+    double ok_ratio = 0.0;
 };
 int launch_step(const StepJob& J, cudaStream_t st);
 // One job per matrix; nmax: the largest ny + nz, at most 32.
@@ -81,7 +90,8 @@ int launch_rblock(double* R, int ldR, int c0, int K, int ny, const double* A, in
 // Explicit TSQR of X[:, c0:c0+nc] in place; R (nc x nc, ldR) upper with diag >= 0.
 int tsqr_tile_rows(int nc);
 i64 tsqr_workspace_doubles(i64 m, int nc);
-int launch_tsqr(double* X, i64 ld, i64 m, int c0, int nc, double* R, int ldR, double* ws,
+// part: gram_part_doubles_fp64(m, nc, nc) doubles.
+int launch_tsqr(double* X, i64 ld, i64 m, int c0, int nc, double* R, int ldR, double* ws, double* part, int num_sms,
                 cudaStream_t st);
 
 // Exchange of the row-sharded path: gathers `count` doubles from every rank into

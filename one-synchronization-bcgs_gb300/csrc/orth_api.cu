@@ -731,7 +731,7 @@ struct Engine {
             err = launch_tsqr_sharded(X, ld, m, c0, nc, Rout, ldr, scr().tsqr.as<double>(), ts, st);
             return;
         }
-        err = launch_tsqr(X, ld, m, c0, nc, Rout, ldr, scr().tsqr.as<double>(), st);
+        err = launch_tsqr(X, ld, m, c0, nc, Rout, ldr, scr().tsqr.as<double>(), scr().part.as<double>(), g_ctx.num_sms, st);
         if (is_split(precision)) split_mark_stale(c0, nc);
     }
     // CholQR2 of X[:, c0:c0+nc] (FP64 in every precision): twice G = V^T V (one

@@ -315,6 +315,7 @@ __device__ void step_body(const StepJob& J, int rank, double* sm) {
     if (fast) {
         // Row r of U is the eliminated row over the square root of its pivot; the
         // carried rows scale the same way and give U^{-T}.
+        bool close = false;
         for (int r = tid; r < n; r += ST_THREADS) {
             // v = 1 / sqrt(d), u = sqrt(d) = d v corrected once (half the cost of a
             // square root and a division).
@@ -322,6 +323,11 @@ __device__ void step_body(const StepJob& J, int rank, double* sm) {
             const double v = rsqrt(d), u = d * v;
             s_u[r] = fma(fma(-u, u, d), 0.5 * v, u);
             s_u[n + r] = v;
+            if (J.ok != nullptr) close |= !(d >= J.ok_ratio * __ldg(J.G + r + (i64)r * J.ldg));
+        }
+        if (J.ok != nullptr) {
+            const int any = __syncthreads_or(close);
+            if (tid == 0) *J.ok = !any;
         }
         __syncthreads();
         for (int r = warp; r < n; r += ST_WARPS) {
@@ -341,6 +347,7 @@ __device__ void step_body(const StepJob& J, int rank, double* sm) {
         // breakdown (a pivot <= 0) the factor keeps the rows before it, and the rows
         // from it on hold the matrix that was to be factored, as dpotrf leaves
         // them; what follows goes on with that factor. Not a path for speed.
+        if (tid == 0 && J.ok != nullptr) *J.ok = 0;
         __syncthreads();
         for (int e = tid; e < E; e += ST_THREADS) {
             int r, c;

@@ -174,8 +174,9 @@ static GramTile gram_tile(int na, int nb, int upper) {
 template <int R, int SEGR>
 __global__ void __launch_bounds__(GTHREADS)
 gram_fp64_partial(const double* __restrict__ X, i64 ld, i64 m, int a0, int na, int b0, int nb, int ta, int upper,
-                  i64 rows_per_chunk, double* __restrict__ part) {
+                  i64 rows_per_chunk, double* __restrict__ part, const int* __restrict__ gate) {
     extern __shared__ double sm[];
+    if (gate != nullptr && *gate == 0) return;
     const int chunk = blockIdx.x;
     int ia0, jb0;
     gram_tile_of((int)blockIdx.y, upper, gram_width(ta, R), nb, ta, (na + ta - 1) / ta, ia0, jb0);
@@ -186,13 +187,14 @@ gram_fp64_partial(const double* __restrict__ X, i64 ld, i64 m, int a0, int na, i
 
 template <int SEGR>
 static int launch_partial(const GramTile& t, int nchunks, const double* X, i64 ld, i64 m, int a0, int na, int b0,
-                          int nb, int upper, i64 rows, double* part, cudaStream_t st) {
+                          int nb, int upper, i64 rows, double* part, const int* gate, cudaStream_t st) {
     const dim3 grid((unsigned)nchunks, (unsigned)t.live);
     const size_t smem = (size_t)GST * gram_stage_doubles(t.ta, t.r) * sizeof(double);
     switch (t.r) {
 #define BCGS_GP(RR)                                                                                              \
     case RR:                                                                                                     \
-        gram_fp64_partial<RR, SEGR><<<grid, GTHREADS, smem, st>>>(X, ld, m, a0, na, b0, nb, t.ta, upper, rows, part); \
+        gram_fp64_partial<RR, SEGR><<<grid, GTHREADS, smem, st>>>(X, ld, m, a0, na, b0, nb, t.ta, upper, rows, part,  \
+                                                            gate);                                            \
         break;
         BCGS_GP(1) BCGS_GP(2) BCGS_GP(3) BCGS_GP(4) BCGS_GP(5) BCGS_GP(6) BCGS_GP(7) BCGS_GP(8)
 #undef BCGS_GP
@@ -307,15 +309,18 @@ static int gram_chunks(i64 m, int na, int nb, const GramTile& t, int num_sms) {
 }
 
 int launch_gram_fp64(const double* X, i64 ld, i64 m, int a0, int na, int b0, int nb, double* out, int ldo,
-                     double* part, bool upper_only, int num_sms, cudaStream_t st) {
+                     double* part, bool upper_only, int num_sms, cudaStream_t st, const int* gate, bool counted) {
     if (na <= 0 || nb <= 0) return 0;
     const int upper = upper_only ? b0 - a0 : -1;
     const GramTile t = gram_tile(na, nb, upper);
     const int nchunks = gram_chunks(m, na, nb, t, num_sms);
     i64 rows_per_chunk = ceil_div(m, nchunks);
     rows_per_chunk = ceil_div(rows_per_chunk, GT_R) * GT_R;
-    const int rc = launch_partial<0>(t, nchunks, X, ld, m, a0, na, b0, nb, upper, rows_per_chunk, part, st);
-    return rc ? rc : launch_gram_reduce(part, nchunks, na, nb, out, ldo, st);
+    const int rc = launch_partial<0>(t, nchunks, X, ld, m, a0, na, b0, nb, upper, rows_per_chunk, part, gate,
+                                   st);
+    if (rc) return rc;
+    if (!counted) g_reduce_count -= 1;   // launch_gram_reduce counts it
+    return launch_gram_reduce(part, nchunks, na, nb, out, ldo, st);
 }
 
 int launch_gram_partials_fp64(const double* X, i64 ld, i64 m, int a0, int na, int b0, int nb, double* part,
@@ -323,7 +328,7 @@ int launch_gram_partials_fp64(const double* X, i64 ld, i64 m, int a0, int na, in
     if (na <= 0 || nb <= 0 || m <= 0) return 0;
     if (rows <= 0 || rows % GT_R != 0) return (int)cudaErrorInvalidValue;
     return launch_partial<256>(gram_tile(na, nb, -1), (int)ceil_div(m, rows), X, ld, m, a0, na, b0, nb, -1, rows, part,
-                               st);
+                               nullptr, st);
 }
 
 int launch_gram_reduce(const double* part, int nchunks, int na, int nb, double* out, int ldo,

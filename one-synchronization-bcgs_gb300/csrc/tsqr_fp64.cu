@@ -27,11 +27,19 @@ namespace bcgs {
 // fewer flops, at the price of fewer tiles resident per SM. One FP64 instruction of a
 // warp occupies its quarter of the SM for 64 clocks whatever the other warps do, so
 // what counts is the number of FP64 instructions and that all four quarters have
-// some: four columns per warp (their four lane sums cost 6 additions together, one
-// column's alone 5) and no fewer than four warps from 16 columns on.
+// some: four or eight columns per warp (four columns' lane sums cost 6 additions
+// together, one column's alone 5).
 constexpr int TSQR_TR = 256;
 template <int NC>
-constexpr int tsqr_tile_warps() { return NC > 32 ? 16 : (NC > 16 ? 8 : (NC > 8 ? 4 : 2)); }
+constexpr int tsqr_tile_warps() { return NC > 16 ? 8 : (NC > 8 ? 4 : 2); }
+// Levels with tiles for several CTAs on every SM have the quarters busy with half as
+// many warps per tile, twice the columns each: fewer lane sums. us, half against full:
+// 2^21 x 16 2395 / 2697, 10^5 x 16 (391 tiles) 165 / 157; 391 tiles x 32 529 / 628, 49 tiles 316 / 250;
+// a tile of 64 columns is best with 8 warps everywhere (789 / 803 alone).
+template <int NC>
+constexpr int tsqr_many_tiles() { return (NC <= 16 ? 4 : 2) * kNumSMsDefault; }
+template <int NC>
+constexpr int tsqr_many_warps() { return NC > 32 ? 8 : (NC > 8 ? tsqr_tile_warps<NC>() / 2 : tsqr_tile_warps<NC>()); }
 
 int tsqr_tile_rows(int nc) { (void)nc; return TSQR_TR; }
 
@@ -211,7 +219,8 @@ __device__ __forceinline__ double load_reflector(const double* a, const double* 
 // unit-pivot reflectors with a division each, tau v published beside v): a level of one
 // tile of 256 x 10, whose chain of reflectors nothing hides, 124 -> 53 us; the leaves of
 // 10^5 x 10 133 -> 76 us, of 2^21 x 16 2.81 -> 2.70 ms, of 2^19 x 64 11.9 -> 11.3 ms, where
-// the FP64 pipe is active 86 %, 84 % and 76 % of the time at 16, 32 and 64 columns.
+// the FP64 pipe is active 86 %, 84 % and 76 % of the time at 16, 32 and 64 columns (4, 8 and
+// 16 warps); with half the warps 2.40 ms at 2^21 x 16.
 template <int NC, int W>
 __device__ void tsqr_tile_body(const double* A, i64 lda, i64 rows, int nc, double* Q, i64 ldq,
                                double* __restrict__ Rst, i64 ldr, i64 tile, double* smem) {
@@ -295,12 +304,30 @@ __device__ void tsqr_tile_body(const double* A, i64 lda, i64 rows, int nc, doubl
         }
 }
 
-template <int NC>
-__global__ void __launch_bounds__(32 * tsqr_tile_warps<NC>())
+template <int NC, int W>
+__global__ void __launch_bounds__(32 * W)
 tsqr_tile_kernel(const double* A, i64 lda, i64 rows, int nc, double* Q, i64 ldq,
-                 double* __restrict__ Rst, i64 ldr) {
+                 double* __restrict__ Rst, i64 ldr, const int* __restrict__ done) {
     extern __shared__ double smem[];
-    tsqr_tile_body<NC, tsqr_tile_warps<NC>()>(A, lda, rows, nc, Q, ldq, Rst, ldr, blockIdx.x, smem);
+    if (done != nullptr && *done) return;
+    tsqr_tile_body<NC, W>(A, lda, rows, nc, Q, ldq, Rst, ldr, blockIdx.x, smem);
+}
+
+template <int NC, int W>
+static int launch_tiles_w(double* A, i64 lda, i64 rows, int nc, double* Rst, i64 ldr, const int* done, cudaStream_t st) {
+    const size_t smem = tsqr_tile_smem_bytes(NC);
+    const int rc = smem_attr((const void*)tsqr_tile_kernel<NC, W>, (int)smem);
+    if (rc) return rc;
+    tsqr_tile_kernel<NC, W><<<(unsigned)ceil_div(rows, TSQR_TR), 32 * W, smem, st>>>(A, lda, rows, nc, A, lda, Rst, ldr,
+                                                                                    done);
+    g_launch_count += 1;
+    return (int)cudaGetLastError();
+}
+template <int NC>
+static int launch_tiles(double* A, i64 lda, i64 rows, int nc, double* Rst, i64 ldr, const int* done, cudaStream_t st) {
+    if (ceil_div(rows, TSQR_TR) >= tsqr_many_tiles<NC>())
+        return launch_tiles_w<NC, tsqr_many_warps<NC>()>(A, lda, rows, nc, Rst, ldr, done, st);
+    return launch_tiles_w<NC, tsqr_tile_warps<NC>()>(A, lda, rows, nc, Rst, ldr, done, st);
 }
 
 // Root fix-up: make diag(R) >= 0. R (nc x nc, ld ldr) rows with a negative
@@ -324,7 +351,8 @@ __device__ void tsqr_root_fix_body(double* Q, i64 ldq, int hq, int nc, const dou
 }
 
 __global__ void tsqr_root_fix(double* Q, i64 ldq, int hq, int nc, const double* R, i64 ldr,
-                              double* Rout, int ldro) {
+                              double* Rout, int ldro, const int* __restrict__ done) {
+    if (done != nullptr && *done) return;
     tsqr_root_fix_body(Q, ldq, hq, nc, R, ldr, Rout, ldro);
 }
 
@@ -362,15 +390,18 @@ __device__ void tsqr_apply_body(double* Q, i64 ldq, i64 rows, int nc, int TR, co
 
 template <int NC>
 __global__ void __launch_bounds__(AP_THREADS)
-tsqr_apply_kernel(double* Q, i64 ldq, i64 rows, int nc, int TR, const double* __restrict__ P, i64 ldp) {
+tsqr_apply_kernel(double* Q, i64 ldq, i64 rows, int nc, int TR, const double* __restrict__ P, i64 ldp,
+                  const int* __restrict__ done) {
     __shared__ double p[NC * NC];
+    if (done != nullptr && *done) return;
     tsqr_apply_body<NC>(Q, ldq, rows, nc, TR, P, ldp, blockIdx.x, p);
 }
 
-static int launch_apply(double* Q, i64 ldq, i64 rows, int nc, int TR, const double* P, i64 ldp, cudaStream_t st) {
+static int launch_apply(double* Q, i64 ldq, i64 rows, int nc, int TR, const double* P, i64 ldp, const int* done,
+                        cudaStream_t st) {
     const unsigned blocks = (unsigned)ceil_div(rows, AP_THREADS);
 #define BCGS_APPLY(N) \
-    if (nc <= N) { tsqr_apply_kernel<N><<<blocks, AP_THREADS, 0, st>>>(Q, ldq, rows, nc, TR, P, ldp); break; }
+    if (nc <= N) { tsqr_apply_kernel<N><<<blocks, AP_THREADS, 0, st>>>(Q, ldq, rows, nc, TR, P, ldp, done); break; }
     do {
         BCGS_APPLY(2) BCGS_APPLY(4) BCGS_APPLY(5) BCGS_APPLY(6) BCGS_APPLY(8) BCGS_APPLY(10) BCGS_APPLY(12)
         BCGS_APPLY(14) BCGS_APPLY(16) BCGS_APPLY(20) BCGS_APPLY(24) BCGS_APPLY(28) BCGS_APPLY(32) BCGS_APPLY(40)
@@ -390,7 +421,9 @@ i64 tsqr_workspace_doubles(i64 m, int nc) {
         total += tiles * nc * nc;
         h = tiles * nc;
     }
-    return total + 64 * 64;  // + the root tile's R
+    total += 64 * 64;                                  // + the root tile's R
+    const i64 chol = nc > 16 ? 3LL * nc * nc : 0;      // or the checked Cholesky's three blocks
+    return 32 + (total > chol ? total : chol);         // + its flag
 }
 
 // The tree from a given level on: level 0 here is (A0, rows0, ld0), factored in
@@ -398,11 +431,9 @@ i64 tsqr_workspace_doubles(i64 m, int nc) {
 // until one tile remains (the root). Then the root's signs are fixed, R is
 // written to (R, ldR), and the down-sweep brings the explicit Q back to level 0.
 template <int NC>
-static int tsqr_levels(double* A0, i64 ld0, i64 rows0, int nc, double* R, int ldR, double* ws, cudaStream_t st) {
+static int tsqr_levels(double* A0, i64 ld0, i64 rows0, int nc, double* R, int ldR, double* ws, const int* done,
+                       cudaStream_t st) {
     const int TR = tsqr_tile_rows(nc);
-    const size_t smem = tsqr_tile_smem_bytes(NC);
-    const int attr_rc = smem_attr((const void*)tsqr_tile_kernel<NC>, (int)smem);
-    if (attr_rc) return attr_rc;
     constexpr int kMaxLevels = 48;   // each level divides the rows by TR / nc >= 2: 2^k rows need at most k levels
     double* lvl_ptr[kMaxLevels];
     i64 lvl_rows[kMaxLevels], lvl_ld[kMaxLevels];
@@ -416,9 +447,8 @@ static int tsqr_levels(double* A0, i64 ld0, i64 rows0, int nc, double* R, int ld
         const i64 tiles = ceil_div(lvl_rows[L], TR);
         double* next = cursor;
         cursor += tiles * nc * nc;
-        tsqr_tile_kernel<NC><<<(unsigned)tiles, 32 * tsqr_tile_warps<NC>(), smem, st>>>(
-            lvl_ptr[L], lvl_ld[L], lvl_rows[L], nc, lvl_ptr[L], lvl_ld[L], next, tiles * nc);
-        g_launch_count += 1;
+        const int rc = launch_tiles<NC>(lvl_ptr[L], lvl_ld[L], lvl_rows[L], nc, next, tiles * nc, done, st);
+        if (rc) return rc;
         ++L;
         lvl_ptr[L] = next;
         lvl_rows[L] = tiles * nc;
@@ -426,13 +456,13 @@ static int tsqr_levels(double* A0, i64 ld0, i64 rows0, int nc, double* R, int ld
     }
     // Root: one tile; its R goes to a small slot after the stacks.
     double* rroot = cursor;
-    tsqr_tile_kernel<NC><<<1, 32 * tsqr_tile_warps<NC>(), smem, st>>>(lvl_ptr[L], lvl_ld[L], lvl_rows[L], nc, lvl_ptr[L],
-                                              lvl_ld[L], rroot, nc);
-    tsqr_root_fix<<<1, 256, 0, st>>>(lvl_ptr[L], lvl_ld[L], (int)lvl_rows[L], nc, rroot, nc, R, ldR);
-    g_launch_count += 2;
+    int root_rc = launch_tiles<NC>(lvl_ptr[L], lvl_ld[L], lvl_rows[L], nc, rroot, nc, done, st);
+    if (root_rc) return root_rc;
+    tsqr_root_fix<<<1, 256, 0, st>>>(lvl_ptr[L], lvl_ld[L], (int)lvl_rows[L], nc, rroot, nc, R, ldR, done);
+    g_launch_count += 1;
     // Down-sweep.
     for (int l = L - 1; l >= 0; --l) {
-        const int rc = launch_apply(lvl_ptr[l], lvl_ld[l], lvl_rows[l], nc, TR, lvl_ptr[l + 1], lvl_ld[l + 1], st);
+        const int rc = launch_apply(lvl_ptr[l], lvl_ld[l], lvl_rows[l], nc, TR, lvl_ptr[l + 1], lvl_ld[l + 1], done, st);
         if (rc) return rc;
     }
     return (int)cudaGetLastError();
@@ -440,8 +470,8 @@ static int tsqr_levels(double* A0, i64 ld0, i64 rows0, int nc, double* R, int ld
 
 template <int NC>
 static int tsqr_run(double* X, i64 ld, i64 m, int c0, int nc, double* R, int ldR, double* ws,
-                    cudaStream_t st) {
-    return tsqr_levels<NC>(X + (i64)c0 * ld, ld, m, nc, R, ldR, ws, st);
+                    const int* done, cudaStream_t st) {
+    return tsqr_levels<NC>(X + (i64)c0 * ld, ld, m, nc, R, ldR, ws, done, st);
 }
 
 // Row-sharded TSQR: this rank's rows are the TR-row tiles [t0, t0 + nt) of a
@@ -456,21 +486,15 @@ template <int NC>
 static int tsqr_sharded_run(double* X, i64 ld, i64 m_local, int c0, int nc, double* R, int ldR, double* ws,
                             const TsqrShard& sh, cudaStream_t st) {
     const int TR = tsqr_tile_rows(nc);
-    const size_t smem = tsqr_tile_smem_bytes(NC);
-    const int attr_rc = smem_attr((const void*)tsqr_tile_kernel<NC>, (int)smem);
-    if (attr_rc) return attr_rc;
-    if (sh.T <= 1) return tsqr_run<NC>(X, ld, m_local, c0, nc, R, ldR, ws, st);   // one tile: one rank holds it
+    if (sh.T <= 1) return tsqr_run<NC>(X, ld, m_local, c0, nc, R, ldR, ws, nullptr, st);   // one tile: one rank holds it
     double* panel = X + (i64)c0 * ld;
     const i64 nt = ceil_div(m_local, TR);
     const i64 ldm = sh.maxt * nc;
     if (nt > 0) {
-        tsqr_tile_kernel<NC><<<(unsigned)nt, 32 * tsqr_tile_warps<NC>(), smem, st>>>(panel, ld, m_local, nc, panel, ld,
-                                                                                   sh.mine, ldm);
-        g_launch_count += 1;
+        const int trc = launch_tiles<NC>(panel, ld, m_local, nc, sh.mine, ldm, nullptr, st);
+        if (trc) return trc;
     }
-    int rc = (int)cudaGetLastError();
-    if (rc) return rc;
-    rc = sh.gather(sh.ctx, sh.mine, sh.all, ldm * nc, st);
+    int rc = sh.gather(sh.ctx, sh.mine, sh.all, ldm * nc, st);
     if (rc) return rc;
     double* lvl1 = ws;
     const i64 ld1 = sh.T * nc;
@@ -481,10 +505,10 @@ static int tsqr_sharded_run(double* X, i64 ld, i64 m_local, int c0, int nc, doub
                                     cudaMemcpyDeviceToDevice, st);
         if (rc) return rc;
     }
-    rc = tsqr_levels<NC>(lvl1, ld1, ld1, nc, R, ldR, ws + ld1 * nc, st);
+    rc = tsqr_levels<NC>(lvl1, ld1, ld1, nc, R, ldR, ws + ld1 * nc, nullptr, st);
     if (rc) return rc;
     if (nt > 0) {
-        rc = launch_apply(panel, ld, m_local, nc, TR, lvl1 + sh.t0[sh.rank] * nc, ld1, st);
+        rc = launch_apply(panel, ld, m_local, nc, TR, lvl1 + sh.t0[sh.rank] * nc, ld1, nullptr, st);
         if (rc) return rc;
     }
     return (int)cudaGetLastError();
@@ -500,13 +524,53 @@ int launch_tsqr_sharded(double* X, i64 ld, i64 m_local, int c0, int nc, double* 
     return (int)cudaErrorInvalidValue;
 }
 
-int launch_tsqr(double* X, i64 ld, i64 m, int c0, int nc, double* R, int ldR, double* ws,
+// Panels wider than kCheckedCols columns: Cholesky QR twice first (Fukaya, Nakatsukasa,
+// Yanagisawa, Yamamoto 2014), if the panel allows it. G = V^T V, R1 = chol(G); if every
+// pivot of R1 is at least kPivotRatio of its diagonal entry, V R1^{-1} departs from
+// orthonormal by at most about the Gram's rounding over that ratio (10^-5), and a second
+// round brings it to roundoff, as the tree does. If not (or a pivot is not a positive
+// number) nothing has been written yet, and the tree factors the panel; its kernels
+// read the flag and end at once otherwise. Twice m nc^2 / 2 products for the upper Gram
+// and as many for the substitution, against some 3.5 m nc^2 issued by the tree, a chain
+// of nc reflectors at every level. Measured at 4 10^5 x 32: 4.24 ms by the tree, 1.9 ms this
+// way; at 2^19 x 64: 23.7 and 8.5 ms. A panel that fails the test has cost the first Gram
+// (0.5 ms at 4 10^5 x 32). For 16 columns and fewer the Gram's tiles are padded and the two
+// take the same time, so those panels go straight to the tree.
+constexpr int kCheckedCols = 16;
+constexpr double kPivotRatio = 1e-9;
+
+static int tsqr_checked(double* X, i64 ld, i64 m, int c0, int nc, double* R, int ldR, double* ws, double* part,
+                        int num_sms, int* done, cudaStream_t st) {
+    const i64 nn = (i64)nc * nc;
+    double *G = ws, *R1 = ws + nn, *R2 = ws + 2 * nn;
+    for (int pass = 0; pass < 2; ++pass) {
+        const int* gate = pass ? done : nullptr;
+        int rc = launch_gram_fp64(X, ld, m, c0, nc, c0, nc, G, nc, part, true, num_sms, st, gate, false);
+        StepJob J;
+        J.G = G; J.ldg = nc; J.ny = nc; J.T = pass ? R2 : R1;
+        if (!pass) { J.ok = done; J.ok_ratio = kPivotRatio; }
+        if (!rc) rc = launch_step(J, st);
+        if (!rc) rc = launch_update_fp64(X, ld, m, 0, 0, c0, nc, nullptr, 0, J.T, nc, true, st, done);
+        if (rc) return rc;
+    }
+    // R = R2 R1 (overwritten by the tree if the flag is not set).
+    return launch_rblock(R, ldR, 0, 0, nc, nullptr, 0, nullptr, 0, R1, R2, 0, st);
+}
+
+int launch_tsqr(double* X, i64 ld, i64 m, int c0, int nc, double* R, int ldR, double* ws, double* part, int num_sms,
                 cudaStream_t st) {
     if (nc <= 0) return 0;
-    if (nc <= 8) return tsqr_run<8>(X, ld, m, c0, nc, R, ldR, ws, st);
-    if (nc <= 16) return tsqr_run<16>(X, ld, m, c0, nc, R, ldR, ws, st);
-    if (nc <= 32) return tsqr_run<32>(X, ld, m, c0, nc, R, ldR, ws, st);
-    if (nc <= 64) return tsqr_run<64>(X, ld, m, c0, nc, R, ldR, ws, st);
+    int* done = nullptr;
+    if (nc > kCheckedCols) {
+        done = reinterpret_cast<int*>(ws);
+        ws += 32;
+        const int rc = tsqr_checked(X, ld, m, c0, nc, R, ldR, ws, part, num_sms, done, st);
+        if (rc) return rc;
+    }
+    if (nc <= 8) return tsqr_run<8>(X, ld, m, c0, nc, R, ldR, ws, done, st);
+    if (nc <= 16) return tsqr_run<16>(X, ld, m, c0, nc, R, ldR, ws, done, st);
+    if (nc <= 32) return tsqr_run<32>(X, ld, m, c0, nc, R, ldR, ws, done, st);
+    if (nc <= 64) return tsqr_run<64>(X, ld, m, c0, nc, R, ldR, ws, done, st);
     return (int)cudaErrorInvalidValue;
 }
 
@@ -515,15 +579,13 @@ int launch_tsqr(double* X, i64 ld, i64 m, int c0, int nc, double* R, int ldR, do
 // down-sweep level over many panels (nc <= 16, TR = 256), with the single-panel
 // bodies.
 // ---------------------------------------------------------------------------
-constexpr int kTileBatchWarps = tsqr_tile_warps<16>();
-
-__global__ void __launch_bounds__(32 * kTileBatchWarps)
+template <int W>
+__global__ void __launch_bounds__(32 * W)
 tsqr_tile_batched(const TsqrTileJob* __restrict__ jobs, const int* __restrict__ prefix, int njobs) {
     extern __shared__ double smem[];
     const int j = batched_job_of(prefix, njobs, blockIdx.x);
     const TsqrTileJob J = jobs[j];
-    tsqr_tile_body<16, kTileBatchWarps>(J.A, J.lda, J.rows, J.nc, J.A, J.lda, J.Rst, J.ldr, blockIdx.x - prefix[j],
-                                        smem);
+    tsqr_tile_body<16, W>(J.A, J.lda, J.rows, J.nc, J.A, J.lda, J.Rst, J.ldr, blockIdx.x - prefix[j], smem);
 }
 
 __global__ void tsqr_root_batched(const TsqrRootJob* __restrict__ jobs) {
@@ -545,8 +607,11 @@ tsqr_apply_batched(const TsqrApplyJob* __restrict__ jobs, const int* __restrict_
 
 // Sets the batched tile kernel's shared-memory limit (outside any stream capture).
 int tsqr_tile_batched_prepare() {
-    return (int)cudaFuncSetAttribute(tsqr_tile_batched, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     (int)tsqr_tile_smem_bytes(16));
+    const int bytes = (int)tsqr_tile_smem_bytes(16);
+    const int rc = (int)cudaFuncSetAttribute(tsqr_tile_batched<tsqr_many_warps<16>()>,
+                                             cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+    return rc ? rc : (int)cudaFuncSetAttribute(tsqr_tile_batched<tsqr_tile_warps<16>()>,
+                                               cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
 }
 
 int launch_tsqr_tile_batched(const TsqrTileJob* jobs, const int* prefix, int njobs, int items, int ncmax,
@@ -554,7 +619,11 @@ int launch_tsqr_tile_batched(const TsqrTileJob* jobs, const int* prefix, int njo
     if (items <= 0) return 0;
     if (ncmax > 16) return (int)cudaErrorInvalidValue;
     const size_t smem = tsqr_tile_smem_bytes(16);
-    tsqr_tile_batched<<<(unsigned)items, 32 * kTileBatchWarps, smem, st>>>(jobs, prefix, njobs);
+    constexpr int W = tsqr_tile_warps<16>(), WM = tsqr_many_warps<16>();
+    if (items >= tsqr_many_tiles<16>())
+        tsqr_tile_batched<WM><<<(unsigned)items, 32 * WM, smem, st>>>(jobs, prefix, njobs);
+    else
+        tsqr_tile_batched<W><<<(unsigned)items, 32 * W, smem, st>>>(jobs, prefix, njobs);
     g_launch_count += 1;
     return (int)cudaGetLastError();
 }

@@ -150,19 +150,21 @@ __device__ __forceinline__ void update_body(double* __restrict__ X, i64 ld, i64 
 template <int NC, bool SPLIT>
 __global__ void __launch_bounds__(UP_THREADS)
 update_fp64(double* __restrict__ X, i64 ld, i64 m, int q0, int K, int c0, int nc,
-            const double* __restrict__ S, int lds, const double* __restrict__ T, int ldt) {
+            const double* __restrict__ S, int lds, const double* __restrict__ T, int ldt,
+            const int* __restrict__ gate) {
     __shared__ double sm[up_smem<NC, SPLIT>()];
+    if (gate != nullptr && *gate == 0) return;
     update_body<NC, SPLIT>(X, ld, m, q0, K, c0, nc, S, lds, T, ldt, blockIdx.x, sm);
 }
 
 // The kernel for width nc (64 or less; 32 or less if SPLIT), launched over m rows.
 template <bool SPLIT>
 int launch_update_width(double* X, i64 ld, i64 m, int q0, int K, int c0, int nc, const double* S, int lds,
-                        const double* T, int ldt, cudaStream_t st) {
+                        const double* T, int ldt, const int* gate, cudaStream_t st) {
     const unsigned grid = (unsigned)ceil_div(m, SPLIT ? 32 : UP_THREADS);
 #define BCGS_UPD(N)                                                                                        \
     if (nc <= N) {                                                                                         \
-        update_fp64<N, SPLIT><<<grid, UP_THREADS, 0, st>>>(X, ld, m, q0, K, c0, nc, S, lds, T, ldt);          \
+        update_fp64<N, SPLIT><<<grid, UP_THREADS, 0, st>>>(X, ld, m, q0, K, c0, nc, S, lds, T, ldt, gate);    \
         break;                                                                                             \
     }
     do {
@@ -177,6 +179,6 @@ int launch_update_width(double* X, i64 ld, i64 m, int q0, int K, int c0, int nc,
     return (int)cudaGetLastError();
 }
 int launch_update_split_k(double* X, i64 ld, i64 m, int q0, int K, int c0, int nc, const double* S, int lds,
-                          const double* T, int ldt, cudaStream_t st);
+                          const double* T, int ldt, const int* gate, cudaStream_t st);
 
 }  // namespace bcgs

@@ -4,8 +4,8 @@
 namespace bcgs {
 
 int launch_update_split_k(double* X, i64 ld, i64 m, int q0, int K, int c0, int nc, const double* S, int lds,
-                          const double* T, int ldt, cudaStream_t st) {
-    return launch_update_width<true>(X, ld, m, q0, K, c0, nc, S, lds, T, ldt, st);
+                          const double* T, int ldt, const int* gate, cudaStream_t st) {
+    return launch_update_width<true>(X, ld, m, q0, K, c0, nc, S, lds, T, ldt, gate, st);
 }
 
 // ---------------------------------------------------------------------------

@@ -62,3 +62,14 @@ def test_tsqr_rank_deficient(lib, s):
     P[:, 3] = P[:, 0]
     P[600:, 2] = 0.0
     _check(P)
+
+
+@pytest.mark.parametrize("s", [17, 20, 33, 64])
+@pytest.mark.parametrize("kappa", [1e2, 1e4, 3e4, 1e5, 1e8, 1e13])
+def test_tsqr_conditions(lib, s, kappa):
+    """Panels wider than 16 columns take Cholesky QR where no column is too close to
+    those before it and the tree otherwise; the contract is the same on both sides."""
+    rng = np.random.default_rng(s)
+    V, _ = np.linalg.qr(rng.standard_normal((3000, s)))
+    W, _ = np.linalg.qr(rng.standard_normal((s, s)))
+    _check((V * np.logspace(0, -np.log10(kappa), s)) @ W)
