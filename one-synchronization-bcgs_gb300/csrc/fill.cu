@@ -21,6 +21,7 @@ namespace {
 // Bytes [0, head) and [head + 16 n16, head + 16 n16 + tail) one at a time; the
 // 16-byte-aligned body with 128-bit stores, grid-strided.
 __global__ void __launch_bounds__(256) zero_kernel(unsigned char* __restrict__ p, int head, uint64_t n16, int tail) {
+    chain_enter();
     const uint64_t tid = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
     const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
     if (tid < (uint64_t)head) p[tid] = 0;
@@ -43,7 +44,7 @@ int zero_async(void* p, size_t bytes, cudaStream_t st) {
     const uint64_t want = (n16 + 255) / 256;
     const uint64_t cap = (uint64_t)kNumSMsDefault * 8;
     const unsigned grid = (unsigned)(want < 1 ? 1 : (want > cap ? cap : want));
-    zero_kernel<<<grid, 256, 0, st>>>(b, (int)head, n16, tail);
+    launch_chained(zero_kernel, grid, 256, 0, st, b, (int)head, n16, tail);
     ++g_launch_count;
     ++g_aux_launch_count;
     return (int)cudaGetLastError();

@@ -437,6 +437,7 @@ __device__ void step_body(const StepJob& J, int rank, double* sm) {
 template <int C>
 __global__ void __launch_bounds__(ST_THREADS) step_kernel(const __grid_constant__ StepJob job) {
     extern __shared__ double sm[];
+    chain_enter();
     step_body<C>(job, C == 1 ? 0 : (int)blockIdx.x, sm);
 }
 
@@ -454,6 +455,7 @@ __global__ void __launch_bounds__(ST_THREADS)
 rblock_kernel(double* R, int ldR, int c0, int K, int ny, const double* A, int lda, const double* B, int ldb,
               const double* Sd, const double* Yd, int mode) {
     __shared__ double sd[SMAX * SMAX];
+    chain_enter();
     if ((int)blockIdx.x == (int)gridDim.x - 1) {
         r_diag(R, ldR, c0, ny, Yd, 1, ny, Sd, mode);
         return;
@@ -471,7 +473,7 @@ rblock_kernel(double* R, int ldR, int c0, int K, int ny, const double* A, int ld
 namespace {
 
 template <class K>
-int launch_clustered(K kernel, unsigned grid, int ctas, size_t smem, cudaStream_t st, void** args) {
+int launch_clustered(K kernel, unsigned grid, int ctas, size_t smem, bool chained, cudaStream_t st, void** args) {
     const int rc = smem > 48 * 1024 ? smem_attr((const void*)kernel, (int)smem) : 0;
     if (rc) return rc;
     cudaLaunchConfig_t cfg = {};
@@ -479,13 +481,20 @@ int launch_clustered(K kernel, unsigned grid, int ctas, size_t smem, cudaStream_
     cfg.blockDim = dim3(ST_THREADS);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = st;
-    cudaLaunchAttribute at[1];
-    at[0].id = cudaLaunchAttributeClusterDimension;
-    at[0].val.clusterDim.x = (unsigned)ctas;
-    at[0].val.clusterDim.y = 1;
-    at[0].val.clusterDim.z = 1;
+    cudaLaunchAttribute at[2];
+    int na = 0;
+    if (chained) {   // as launch_chained
+        at[na].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        at[na++].val.programmaticStreamSerializationAllowed = 1;
+    }
+    if (ctas > 1) {
+        at[na].id = cudaLaunchAttributeClusterDimension;
+        at[na].val.clusterDim.x = (unsigned)ctas;
+        at[na].val.clusterDim.y = 1;
+        at[na++].val.clusterDim.z = 1;
+    }
     cfg.attrs = at;
-    cfg.numAttrs = ctas > 1 ? 1 : 0;
+    cfg.numAttrs = na;
     const cudaError_t ce = cudaLaunchKernelExC(&cfg, (const void*)kernel, args);
     g_launch_count += 1;
     return (int)(ce != cudaSuccess ? ce : cudaGetLastError());
@@ -506,8 +515,8 @@ int launch_step(const StepJob& J, cudaStream_t st) {
     const int n = J.ny + J.nz;
     void* args[1] = {const_cast<StepJob*>(&J)};
     if (J.K <= kTileRows && (i64)trap_size(n, n) * J.K <= 8192)
-        return launch_clustered(step_kernel<1>, 1, 1, step_smem_bytes(n, J.ny, 1), st, args);
-    return launch_clustered(step_kernel<8>, 8, 8, step_smem_bytes(n, J.ny, 8), st, args);
+        return launch_clustered(step_kernel<1>, 1, 1, step_smem_bytes(n, J.ny, 1), true, st, args);
+    return launch_clustered(step_kernel<8>, 8, 8, step_smem_bytes(n, J.ny, 8), true, st, args);
 }
 
 // Batched: nmax = the largest ny + nz (<= 32). Enough CTAs per job to spread a small
@@ -516,16 +525,16 @@ int launch_step_batched(const StepJob* jobs, int njobs, int nmax, cudaStream_t s
     if (njobs <= 0) return 0;
     if (nmax < 1 || nmax > 32) return (int)cudaErrorInvalidValue;
     void* args[1] = {(void*)&jobs};
-    if (njobs <= 64) return launch_clustered(step_batched<8>, (unsigned)njobs * 8, 8, step_smem_bytes(nmax, nmax / 2, 8), st, args);
-    if (njobs <= 512) return launch_clustered(step_batched<2>, (unsigned)njobs * 2, 2, step_smem_bytes(nmax, nmax / 2, 2), st, args);
-    return launch_clustered(step_batched<1>, (unsigned)njobs, 1, step_smem_bytes(nmax, nmax / 2, 1), st, args);
+    if (njobs <= 64) return launch_clustered(step_batched<8>, (unsigned)njobs * 8, 8, step_smem_bytes(nmax, nmax / 2, 8), false, st, args);
+    if (njobs <= 512) return launch_clustered(step_batched<2>, (unsigned)njobs * 2, 2, step_smem_bytes(nmax, nmax / 2, 2), false, st, args);
+    return launch_clustered(step_batched<1>, (unsigned)njobs, 1, step_smem_bytes(nmax, nmax / 2, 1), false, st, args);
 }
 
 int launch_rblock(double* R, int ldR, int c0, int K, int ny, const double* A, int lda, const double* B, int ldb,
                   const double* Sd, const double* Yd, int mode, cudaStream_t st) {
     if (ny <= 0) return 0;
     if (ny > SMAX) return (int)cudaErrorInvalidValue;
-    rblock_kernel<<<(unsigned)((K + 31) / 32 + 1), ST_THREADS, 0, st>>>(R, ldR, c0, K, ny, A, lda, B, ldb, Sd, Yd,
+    launch_chained(rblock_kernel, (unsigned)((K + 31) / 32 + 1), ST_THREADS, 0, st, R, ldR, c0, K, ny, A, lda, B, ldb, Sd, Yd,
                                                                         mode);
     g_launch_count += 1;
     return (int)cudaGetLastError();

@@ -170,6 +170,7 @@ __device__ __forceinline__ void colmax_body(const double* __restrict__ X, i64 ld
 
 __global__ void colmax_kernel(const double* __restrict__ X, i64 ld, i64 m, int c0,
                               unsigned long long* __restrict__ cmax) {
+    chain_enter();
     colmax_body(X, ld, m, c0 + (int)blockIdx.y, (int)blockIdx.x, cmax);
 }
 
@@ -287,6 +288,7 @@ __global__ void __launch_bounds__(128, 7)
 slice_kernel(const double* __restrict__ X, i64 ld, i64 m, int n, int c0, int nc,
              const unsigned long long* __restrict__ cmax, int* __restrict__ cexp,
              unsigned short* __restrict__ colstore, i64 nrc) {
+    chain_enter();
     slice_body<KD>(X, ld, m, n, c0, nc, cmax, cexp, colstore, nrc, (int)blockIdx.x, (int)blockIdx.y);
 }
 
@@ -356,6 +358,7 @@ __device__ __forceinline__ void bbuild_body(const double* __restrict__ G, int ld
 __global__ void __launch_bounds__(BB_THREADS)
 bbuild_kernel(const double* __restrict__ G, int ldg, const double* __restrict__ Ui, int ldu, int K, int n,
               const int* __restrict__ cexp, double* __restrict__ Bp, int ldb, unsigned long long* __restrict__ bmax) {
+    chain_enter();
     bbuild_body(G, ldg, Ui, ldu, K, n, cexp, Bp, ldb, bmax, (int)blockIdx.x);
 }
 
@@ -411,6 +414,7 @@ __global__ void __launch_bounds__(BD_C * BD_J)
 bdigit_kernel(const double* __restrict__ Bp, int ldb, int kin, int nout, int Kpad,
               const unsigned long long* __restrict__ bmax, int* __restrict__ fexp,
               unsigned short* __restrict__ bdig, unsigned long long* __restrict__ cmax, int* __restrict__ tile_ctr) {
+    chain_enter();
     bdigit_body<KD>(Bp, ldb, kin, nout, Kpad, bmax, fexp, bdig, cmax, tile_ctr, (int)blockIdx.x);
 }
 
@@ -707,6 +711,7 @@ gram_tc_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__
     uint8_t *sA, *sB;
     if (threadIdx.x == 0) abort_flag = 0;
     Bars* bars = setup_cta<NB, KD>(smem_raw, sA, sB, &tmem_slot);
+    chain_enter();   // barriers and TMEM are set up while the kernel before finishes
     const uint32_t tmem = tmem_slot;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
 
@@ -872,6 +877,7 @@ update_tc_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant
     uint8_t *sA, *sB;
     if (threadIdx.x == 0) abort_flag = 0;
     Bars* bars = setup_cta<NB, KD>(smem_raw, sA, sB, &tmem_slot, UNEPI);
+    chain_enter();   // barriers and TMEM are set up while the kernel before finishes
     const uint32_t tmem = tmem_slot;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
 
@@ -1244,7 +1250,7 @@ int ensure_fresh(int c_begin, int c_end, cudaStream_t st) {
             cudaError_t ce = (cudaError_t)zero_async(P.cmax + c, (size_t)(e - c) * sizeof(unsigned long long), st);
             if (ce != cudaSuccess) return (int)ce;
         }
-        colmax_kernel<<<dim3((unsigned)ceil_div(P.m, 4096), (unsigned)(e - c)), 256, 0, st>>>(P.X, P.ld, P.m, c, P.cmax);
+        launch_chained(colmax_kernel, dim3((unsigned)ceil_div(P.m, 4096), (unsigned)(e - c)), 256, 0, st, P.X, P.ld, P.m, c, P.cmax);
         g_launch_count += 1;
         for (; c < e; ++c) { P.cmax_valid[c] = 1; P.cmax_zero[c] = 0; }
     }
@@ -1255,9 +1261,9 @@ int ensure_fresh(int c_begin, int c_end, cudaStream_t st) {
         const int nc = e - c;
         const dim3 sgrid((unsigned)ceil_div(P.m, 128), (unsigned)ceil_div(nc, 16));
         if (P.kd == 6)
-            slice_kernel<6><<<sgrid, 128, 0, st>>>(P.X, P.ld, P.m, P.n, c, nc, P.cmax, P.cexp, P.colstore, P.nrc);
+            launch_chained(slice_kernel<6>, sgrid, 128, 0, st, P.X, P.ld, P.m, P.n, c, nc, P.cmax, P.cexp, P.colstore, P.nrc);
         else
-            slice_kernel<7><<<sgrid, 128, 0, st>>>(P.X, P.ld, P.m, P.n, c, nc, P.cmax, P.cexp, P.colstore, P.nrc);
+            launch_chained(slice_kernel<7>, sgrid, 128, 0, st, P.X, P.ld, P.m, P.n, c, nc, P.cmax, P.cexp, P.colstore, P.nrc);
         g_launch_count += 1;
         for (; c < e; ++c) { P.fresh[c] = 1; P.cmax_valid[c] = 0; }
     }
@@ -1382,12 +1388,12 @@ int split_slice_columns(const double* X, i64 ld, i64 m, int n, int kd, unsigned 
     int rc = zero_async(digits, (size_t)kd * nrc * 64 * n * sizeof(unsigned short), st);
     if (!rc) rc = zero_async(cmax, (size_t)n * sizeof(unsigned long long), st);
     if (rc) return rc;
-    colmax_kernel<<<dim3((unsigned)ceil_div(m, 4096), (unsigned)n), 256, 0, st>>>(X, ld, m, 0, cmax);
+    launch_chained(colmax_kernel, dim3((unsigned)ceil_div(m, 4096), (unsigned)n), 256, 0, st, X, ld, m, 0, cmax);
     const dim3 sgrid((unsigned)ceil_div(m, 128), (unsigned)ceil_div(n, 16));
     if (kd == 6)
-        slice_kernel<6><<<sgrid, 128, 0, st>>>(X, ld, m, n, 0, n, cmax, cexp, digits, nrc);
+        launch_chained(slice_kernel<6>, sgrid, 128, 0, st, X, ld, m, n, 0, n, cmax, cexp, digits, nrc);
     else
-        slice_kernel<7><<<sgrid, 128, 0, st>>>(X, ld, m, n, 0, n, cmax, cexp, digits, nrc);
+        launch_chained(slice_kernel<7>, sgrid, 128, 0, st, X, ld, m, n, 0, n, cmax, cexp, digits, nrc);
     g_launch_count += 2;
     return (int)cudaGetLastError();
 }
@@ -1425,7 +1431,7 @@ int launch_gram_split(const double* X, i64 ld, i64 m, int na, int b0, int nb, do
     const CUtensorMap& bmap = NB == 16 ? P.map_col_b16 : P.map_col_b;
     const int ka = gram_a_planes(P.kd);
 #define BCGS_GRAM(NBT, KDT, KAT)                                                                                  \
-    gram_tc_kernel<NBT, KDT, KAT, false><<<grid, NTHREADS, SmemLayout<NBT, KDT>::BYTES, st>>>(                \
+    launch_chained(gram_tc_kernel<NBT, KDT, KAT, false>, grid, NTHREADS, SmemLayout<NBT, KDT>::BYTES, st,        \
         P.map_col_a, alast_map, bmap, gp, nullptr, nullptr, 0)
     if (NB == 16) {
         if (P.kd == 6) BCGS_GRAM(16, 6, 6); else if (ka == 6) BCGS_GRAM(16, 7, 6); else BCGS_GRAM(16, 7, 7);
@@ -1448,14 +1454,14 @@ static int run_update(double* X, i64 ld, i64 m, int K, int nout, const double* G
                       int num_sms, cudaStream_t st) {
     Plan& P = cur_plan();
     const int kin = K + nout;
-    bbuild_kernel<<<(unsigned)ceil_div(kin, BB_ROWS), BB_THREADS, 0, st>>>(G, ldg, Ui, ldu, K, nout, P.cexp, P.bfull,
+    launch_chained(bbuild_kernel, (unsigned)ceil_div(kin, BB_ROWS), BB_THREADS, 0, st, G, ldg, Ui, ldu, K, nout, P.cexp, P.bfull,
                                                                            (int)P.kpad, P.bmax);
     const unsigned bd = (unsigned)bdigit_ctas(nout, (int)P.kpad);
     if (P.kd == 6)
-        bdigit_kernel<6><<<bd, BD_C * BD_J, 0, st>>>(P.bfull, (int)P.kpad, kin, nout, (int)P.kpad, P.bmax, P.fexp, P.bdig,
+        launch_chained(bdigit_kernel<6>, bd, BD_C * BD_J, 0, st, P.bfull, (int)P.kpad, kin, nout, (int)P.kpad, P.bmax, P.fexp, P.bdig,
                                                      P.cmax + K, P.tile_ctr);
     else
-        bdigit_kernel<7><<<bd, BD_C * BD_J, 0, st>>>(P.bfull, (int)P.kpad, kin, nout, (int)P.kpad, P.bmax, P.fexp, P.bdig,
+        launch_chained(bdigit_kernel<7>, bd, BD_C * BD_J, 0, st, P.bfull, (int)P.kpad, kin, nout, (int)P.kpad, P.bmax, P.fexp, P.bdig,
                                                      P.cmax + K, P.tile_ctr);
     g_launch_count += 2;
     for (int gi = 0; 32 * gi < nout; ++gi) {
@@ -1470,7 +1476,7 @@ static int run_update(double* X, i64 ld, i64 m, int K, int nout, const double* G
         const int ntiles = (int)ceil_div(m, TILE_M);
         const int grid = ntiles < num_sms ? ntiles : num_sms;
 #define BCGS_UPD(NBT, KDT) \
-        update_tc_kernel<NBT, KDT, false><<<grid, UTHREADS, SmemLayout<NBT, KDT>::BYTES, st>>>(                 \
+        launch_chained(update_tc_kernel<NBT, KDT, false>, grid, UTHREADS, SmemLayout<NBT, KDT>::BYTES, st,          \
             P.map_col_u, ulast_map, P.map_bdig##NBT[gi], up, nullptr, nullptr, 0)
         if (NB == 16) {
             if (P.kd == 6) BCGS_UPD(16, 6); else BCGS_UPD(16, 7);

@@ -176,6 +176,7 @@ __global__ void __launch_bounds__(GTHREADS)
 gram_fp64_partial(const double* __restrict__ X, i64 ld, i64 m, int a0, int na, int b0, int nb, int ta, int upper,
                   i64 rows_per_chunk, double* __restrict__ part, const int* __restrict__ gate) {
     extern __shared__ double sm[];
+    chain_enter();
     if (gate != nullptr && *gate == 0) return;
     const int chunk = blockIdx.x;
     int ia0, jb0;
@@ -193,7 +194,7 @@ static int launch_partial(const GramTile& t, int nchunks, const double* X, i64 l
     switch (t.r) {
 #define BCGS_GP(RR)                                                                                              \
     case RR:                                                                                                     \
-        gram_fp64_partial<RR, SEGR><<<grid, GTHREADS, smem, st>>>(X, ld, m, a0, na, b0, nb, t.ta, upper, rows, part,  \
+        launch_spread(gram_fp64_partial<RR, SEGR>, grid, GTHREADS, smem, st, X, ld, m, a0, na, b0, nb, t.ta, upper, rows, part,  \
                                                             gate);                                            \
         break;
         BCGS_GP(1) BCGS_GP(2) BCGS_GP(3) BCGS_GP(4) BCGS_GP(5) BCGS_GP(6) BCGS_GP(7) BCGS_GP(8)
@@ -252,6 +253,7 @@ __device__ __forceinline__ void gram_reduce_body(const double* __restrict__ part
 
 __global__ void __launch_bounds__(RD_THREADS)
 gram_reduce(const double* __restrict__ part, int nchunks, int na, int nb, double* __restrict__ out, int ldo) {
+    chain_enter();
     gram_reduce_body(part, nchunks, na, nb, out, ldo, blockIdx.x);
 }
 
@@ -333,7 +335,7 @@ int launch_gram_partials_fp64(const double* X, i64 ld, i64 m, int a0, int na, in
 
 int launch_gram_reduce(const double* part, int nchunks, int na, int nb, double* out, int ldo,
                        cudaStream_t st) {
-    gram_reduce<<<(unsigned)gram_reduce_ctas(na, nb), RD_THREADS, 0, st>>>(part, nchunks, na, nb, out, ldo);
+    launch_chained(gram_reduce, (unsigned)gram_reduce_ctas(na, nb), RD_THREADS, 0, st, part, nchunks, na, nb, out, ldo);
     g_launch_count += 1;
     g_reduce_count += 1;
     return (int)cudaGetLastError();

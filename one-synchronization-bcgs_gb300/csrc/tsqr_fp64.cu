@@ -309,6 +309,7 @@ __global__ void __launch_bounds__(32 * W)
 tsqr_tile_kernel(const double* A, i64 lda, i64 rows, int nc, double* Q, i64 ldq,
                  double* __restrict__ Rst, i64 ldr, const int* __restrict__ done) {
     extern __shared__ double smem[];
+    chain_enter();
     if (done != nullptr && *done) return;
     tsqr_tile_body<NC, W>(A, lda, rows, nc, Q, ldq, Rst, ldr, blockIdx.x, smem);
 }
@@ -318,7 +319,7 @@ static int launch_tiles_w(double* A, i64 lda, i64 rows, int nc, double* Rst, i64
     const size_t smem = tsqr_tile_smem_bytes(NC);
     const int rc = smem_attr((const void*)tsqr_tile_kernel<NC, W>, (int)smem);
     if (rc) return rc;
-    tsqr_tile_kernel<NC, W><<<(unsigned)ceil_div(rows, TSQR_TR), 32 * W, smem, st>>>(A, lda, rows, nc, A, lda, Rst, ldr,
+    launch_spread(tsqr_tile_kernel<NC, W>, (unsigned)ceil_div(rows, TSQR_TR), 32 * W, smem, st, A, lda, rows, nc, A, lda, Rst, ldr,
                                                                                     done);
     g_launch_count += 1;
     return (int)cudaGetLastError();
@@ -352,6 +353,7 @@ __device__ void tsqr_root_fix_body(double* Q, i64 ldq, int hq, int nc, const dou
 
 __global__ void tsqr_root_fix(double* Q, i64 ldq, int hq, int nc, const double* R, i64 ldr,
                               double* Rout, int ldro, const int* __restrict__ done) {
+    chain_enter();
     if (done != nullptr && *done) return;
     tsqr_root_fix_body(Q, ldq, hq, nc, R, ldr, Rout, ldro);
 }
@@ -393,6 +395,7 @@ __global__ void __launch_bounds__(AP_THREADS)
 tsqr_apply_kernel(double* Q, i64 ldq, i64 rows, int nc, int TR, const double* __restrict__ P, i64 ldp,
                   const int* __restrict__ done) {
     __shared__ double p[NC * NC];
+    chain_enter();
     if (done != nullptr && *done) return;
     tsqr_apply_body<NC>(Q, ldq, rows, nc, TR, P, ldp, blockIdx.x, p);
 }
@@ -401,7 +404,7 @@ static int launch_apply(double* Q, i64 ldq, i64 rows, int nc, int TR, const doub
                         cudaStream_t st) {
     const unsigned blocks = (unsigned)ceil_div(rows, AP_THREADS);
 #define BCGS_APPLY(N) \
-    if (nc <= N) { tsqr_apply_kernel<N><<<blocks, AP_THREADS, 0, st>>>(Q, ldq, rows, nc, TR, P, ldp, done); break; }
+    if (nc <= N) { launch_spread(tsqr_apply_kernel<N>, blocks, AP_THREADS, 0, st, Q, ldq, rows, nc, TR, P, ldp, done); break; }
     do {
         BCGS_APPLY(2) BCGS_APPLY(4) BCGS_APPLY(5) BCGS_APPLY(6) BCGS_APPLY(8) BCGS_APPLY(10) BCGS_APPLY(12)
         BCGS_APPLY(14) BCGS_APPLY(16) BCGS_APPLY(20) BCGS_APPLY(24) BCGS_APPLY(28) BCGS_APPLY(32) BCGS_APPLY(40)
@@ -458,7 +461,7 @@ static int tsqr_levels(double* A0, i64 ld0, i64 rows0, int nc, double* R, int ld
     double* rroot = cursor;
     int root_rc = launch_tiles<NC>(lvl_ptr[L], lvl_ld[L], lvl_rows[L], nc, rroot, nc, done, st);
     if (root_rc) return root_rc;
-    tsqr_root_fix<<<1, 256, 0, st>>>(lvl_ptr[L], lvl_ld[L], (int)lvl_rows[L], nc, rroot, nc, R, ldR, done);
+    launch_chained(tsqr_root_fix, 1, 256, 0, st, lvl_ptr[L], lvl_ld[L], (int)lvl_rows[L], nc, rroot, nc, R, ldR, done);
     g_launch_count += 1;
     // Down-sweep.
     for (int l = L - 1; l >= 0; --l) {

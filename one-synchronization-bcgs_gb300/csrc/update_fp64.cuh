@@ -153,6 +153,7 @@ update_fp64(double* __restrict__ X, i64 ld, i64 m, int q0, int K, int c0, int nc
             const double* __restrict__ S, int lds, const double* __restrict__ T, int ldt,
             const int* __restrict__ gate) {
     __shared__ double sm[up_smem<NC, SPLIT>()];
+    chain_enter();
     if (gate != nullptr && *gate == 0) return;
     update_body<NC, SPLIT>(X, ld, m, q0, K, c0, nc, S, lds, T, ldt, blockIdx.x, sm);
 }
@@ -164,7 +165,7 @@ int launch_update_width(double* X, i64 ld, i64 m, int q0, int K, int c0, int nc,
     const unsigned grid = (unsigned)ceil_div(m, SPLIT ? 32 : UP_THREADS);
 #define BCGS_UPD(N)                                                                                        \
     if (nc <= N) {                                                                                         \
-        update_fp64<N, SPLIT><<<grid, UP_THREADS, 0, st>>>(X, ld, m, q0, K, c0, nc, S, lds, T, ldt, gate);    \
+        launch_spread(update_fp64<N, SPLIT>, grid, UP_THREADS, 0, st, X, ld, m, q0, K, c0, nc, S, lds, T, ldt, gate);    \
         break;                                                                                             \
     }
     do {
