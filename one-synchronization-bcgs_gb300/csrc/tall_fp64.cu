@@ -20,7 +20,7 @@ namespace bcgs {
 // and walks a contiguous row range of X in stages of GR rows, copied to shared memory
 // asynchronously GST stages deep. Thread (ta, tb) keeps R sums: its column of A against
 // columns tb, tb + 128 / TA, ... of the W. Partial sums go to part[chunk][i + j * na]
-// (column-major na x nb per chunk). Every entry is a sequential FMA chain over the rows of
+// (column-major na x nb per chunk). Every entry is a sum of FMA chains over the rows of
 // the chunk in order, so the result depends on the chunking only, not on TA or R.
 //
 // One FP64 instruction of a warp occupies its quarter of the SM for 64 clocks, so the
@@ -38,6 +38,8 @@ constexpr int GST = 3;              // stages in flight
 constexpr int GT_R = 32;            // chunk row ranges are multiples of this
 constexpr int GTHREADS = 128;
 constexpr int GR_MAX = 8;           // columns of B per thread
+constexpr int GSEG = 2048;          // rows of one FMA chain: the chunks of a large m are long, and one
+                                    // chain over them would lose digits (one addition per 2048 products)
 
 __host__ __device__ inline int gram_width(int ta, int r) { return r * (GTHREADS / ta); }
 __host__ __device__ inline int gram_stage_doubles(int ta, int r) { return GR * ((ta + gram_width(ta, r)) | 1); }
@@ -53,15 +55,14 @@ __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_gr
 
 // The tile at C rows ia0.., C columns jb0.., rows [r_begin, r_end) of X, written to
 // `out` (na x nb, ld na). sm holds GST stages of gram_stage_doubles(ta, R).
-// SEGR > 0: every SEGR rows the running sums are added to a total and restarted,
-// so no FMA chain is longer than SEGR rows however long the row range is
-// (SEGR = 0: one chain over the range).
-template <int R, int SEGR = 0>
+// Every SEGR rows the running sums are added to a total and restarted, so no FMA
+// chain is longer than SEGR rows however long the row range is.
+template <int R, int SEGR = GSEG>
 __device__ __forceinline__ void gram_partial_body(const double* __restrict__ X, i64 ld, int a0, int na, int b0,
                                                   int nb, int ta, i64 r_begin, i64 r_end, int ia0, int jb0,
                                                   double* __restrict__ out, double* __restrict__ sm) {
     constexpr int SEG = SEGR / GR;  // stages per segment
-    static_assert(SEGR % GR == 0, "segments are whole stages");
+    static_assert(SEGR > 0 && SEGR % GR == 0, "segments are whole stages");
     const int tbn = GTHREADS / ta, w = R * tbn;
     const int ldr = (ta + w) | 1;
     const int tid = threadIdx.x;
@@ -90,36 +91,33 @@ __device__ __forceinline__ void gram_partial_body(const double* __restrict__ X, 
         if (s < nst) fill(s);
         cp_async_commit();
     }
-    int sub = 0;
-    for (int s = 0; s < nst; ++s) {
-        if (SEG > 0 && sub == SEG) {
-#pragma unroll
-            for (int k = 0; k < R; ++k) { tot[k] += acc[k]; acc[k] = 0.0; }
-            sub = 0;
-        }
-        ++sub;
-        cp_async_wait<GST - 2>();
-        __syncthreads();   // stage s is here, and every thread is done with stage s - 1
-        if (s + GST - 1 < nst) fill(s + GST - 1);
-        cp_async_commit();
-        const double* pa = sm + (s % GST) * (GR * ldr) + ca;
-        const double* pb = pa - ca + ta + tb;
+    // (Segments are an outer loop: additions behind a condition in the stage loop would
+    // be predicated off, and still take their 64 clocks, at every stage.)
+    for (int s0 = 0; s0 < nst; s0 += SEG) {
+        const int s1 = min(nst, s0 + SEG);
+#pragma unroll 1
+        for (int s = s0; s < s1; ++s) {
+            cp_async_wait<GST - 2>();
+            __syncthreads();   // stage s is here, and every thread is done with stage s - 1
+            if (s + GST - 1 < nst) fill(s + GST - 1);
+            cp_async_commit();
+            const double* pa = sm + (s % GST) * (GR * ldr) + ca;
+            const double* pb = pa - ca + ta + tb;
 #pragma unroll 4
-        for (int q = 0; q < GR; ++q) {
-            const double av = pa[q * ldr];
+            for (int q = 0; q < GR; ++q) {
+                const double av = pa[q * ldr];
 #pragma unroll
-            for (int k = 0; k < R; ++k) acc[k] = fma(av, pb[q * ldr + k * tbn], acc[k]);
+                for (int k = 0; k < R; ++k) acc[k] = fma(av, pb[q * ldr + k * tbn], acc[k]);
+            }
         }
-    }
-    if (SEG > 0) {
 #pragma unroll
-        for (int k = 0; k < R; ++k) acc[k] += tot[k];
+        for (int k = 0; k < R; ++k) { tot[k] += acc[k]; acc[k] = 0.0; }
     }
     const int i = ia0 + ca;
 #pragma unroll
     for (int k = 0; k < R; ++k) {
         const int j = jb0 + tb + k * tbn;
-        if (i < na && j < nb) out[i + (i64)j * na] = acc[k];
+        if (i < na && j < nb) out[i + (i64)j * na] = tot[k];
     }
 }
 
@@ -318,7 +316,7 @@ int launch_gram_fp64(const double* X, i64 ld, i64 m, int a0, int na, int b0, int
     const int nchunks = gram_chunks(m, na, nb, t, num_sms);
     i64 rows_per_chunk = ceil_div(m, nchunks);
     rows_per_chunk = ceil_div(rows_per_chunk, GT_R) * GT_R;
-    const int rc = launch_partial<0>(t, nchunks, X, ld, m, a0, na, b0, nb, upper, rows_per_chunk, part, gate,
+    const int rc = launch_partial<GSEG>(t, nchunks, X, ld, m, a0, na, b0, nb, upper, rows_per_chunk, part, gate,
                                    st);
     if (rc) return rc;
     if (!counted) g_reduce_count -= 1;   // launch_gram_reduce counts it
