@@ -73,6 +73,7 @@ int gram_batched_tile(int na, int b0, int nb, int* ta, int* r);   // returns the
 void update_batched_ctas(i64 m, int K, int* split, int* ctas);
 int launch_gram_partial_batched(const GramJob* jobs, const int* prefix, int njobs, int items, cudaStream_t st);
 int launch_gram_reduce_batched(const GramJob* jobs, const int* prefix, int njobs, int items, cudaStream_t st);
+int launch_gram_reduce_sliced_batched(const GramJob* jobs, const int* prefix, int njobs, int items, cudaStream_t st);
 int launch_update_batched(const UpdJob* jobs, const int* prefix, int njobs, int items, cudaStream_t st);
 int launch_tsqr_tile_batched(const TsqrTileJob* jobs, const int* prefix, int njobs, int items, int ncmax,
                              cudaStream_t st);

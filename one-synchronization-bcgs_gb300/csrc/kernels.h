@@ -44,6 +44,10 @@ int launch_gram_fp64(const double* X, i64 ld, i64 m, int a0, int na, int b0, int
 int launch_gram_reduce(const double* part, int nchunks, int na, int nb, double* out, int ldo,
                        cudaStream_t st);
 int gram_reduce_ctas(int na, int nb);   // CTAs of one reduction
+// The same sum in another fixed order, with a shorter chain. counted: as launch_gram_fp64.
+int launch_gram_reduce_sliced(const double* part, int nchunks, int na, int nb, double* out, int ldo, bool counted,
+                              cudaStream_t st);
+int gram_reduce_sliced_ctas(int na, int nb);
 
 // X[:, c0:c0+nc] = (X[:, c0:c0+nc] - X[:, q0:q0+K] S) T^{-1}; T upper (nc x nc) or null.
 // any_split: K may be summed in quarters, by a rule on m; without it each row's result
@@ -87,12 +91,19 @@ int launch_step_batched(const StepJob* jobs, int njobs, int nmax, cudaStream_t s
 int launch_rblock(double* R, int ldR, int c0, int K, int ny, const double* A, int lda,
                   const double* B, int ldb, const double* Sd, const double* Yd, int mode, cudaStream_t st);
 
+// Upper Gram (nc x nc, ld nc) of X[:, c0:c0+nc], nc <= 16, through part (panel_gram_part_doubles);
+// gate as launch_gram_fp64.
+i64 panel_gram_part_doubles(int nc);
+int launch_panel_gram(const double* X, i64 ld, i64 m, int c0, int nc, double* G, double* part, int num_sms,
+                      const int* gate, cudaStream_t st);
+
 // Explicit TSQR of X[:, c0:c0+nc] in place; R (nc x nc, ldR) upper with diag >= 0.
 int tsqr_tile_rows(int nc);
 i64 tsqr_workspace_doubles(i64 m, int nc);
-// part: gram_part_doubles_fp64(m, nc, nc) doubles.
+// part: gram_part_doubles_fp64(m, nc, nc) doubles. checked: panels of up to 16 columns may take
+// Cholesky QR too (not in BCGSI+P-1S, whose batched plans use the tree).
 int launch_tsqr(double* X, i64 ld, i64 m, int c0, int nc, double* R, int ldR, double* ws, double* part, int num_sms,
-                cudaStream_t st);
+                bool checked, cudaStream_t st);
 
 // Exchange of the row-sharded path: gathers `count` doubles from every rank into
 // `all` (size * count doubles, rank order), ordered on stream st. 0 on success.

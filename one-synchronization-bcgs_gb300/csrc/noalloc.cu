@@ -157,7 +157,7 @@ extern "C" int orth_gb300_bcgsi2P1s_dev_noalloc(int m, int n, int s, double* dX,
     // BCGSI+P-1S, the same schedule as the allocating entry point
     // (reference SRC/orth.c:48-222).
     const int s0 = s, p = (n - s + s - 1) / s;
-    if (!err) err = launch_tsqr(dX, ld, M, 0, s0, dR, ldR, tws, part, d->num_sms, st);
+    if (!err) err = launch_tsqr(dX, ld, M, 0, s0, dR, ldR, tws, part, d->num_sms, false, st);
     gram(2 * s, s0, s, W);
     run_step(factor(W, 2 * s, s0, s, Sd, 1));
     update(s0, s0, s, W, 2 * s, Sd, s);

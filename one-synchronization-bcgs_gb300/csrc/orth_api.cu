@@ -188,8 +188,10 @@ int init_ctx() {
     return 0;
 }
 
-// Largest Gram-partial buffer any step needs (doubles).
-i64 part_doubles(i64 m, int n, int s) { return gram_part_doubles_fp64(m, n + s, 2 * s); }
+// Largest Gram-partial buffer any step or panel needs (doubles).
+i64 part_doubles(i64 m, int n, int s) {
+    return std::max(gram_part_doubles_fp64(m, n + s, 2 * s), panel_gram_part_doubles(s < 16 ? s : 16));
+}
 
 // Small buffers carved from one allocation (doubles).
 struct Small {
@@ -608,6 +610,7 @@ struct Engine {
     int err = 0;
     HostLink* link = nullptr;   // host-buffer runs only
     Shard* shard = nullptr;     // row-sharded runs only (FP64)
+    bool checked = false;       // launch_tsqr's
 
     // C (na x nb, ldc) = X[:, a0:a0+na]^T X[:, b0:b0+nb] in FP64: one deterministic
     // reduction, over all ranks in a row-sharded run. Entries below the diagonal of
@@ -731,7 +734,7 @@ struct Engine {
             err = launch_tsqr_sharded(X, ld, m, c0, nc, Rout, ldr, scr().tsqr.as<double>(), ts, st);
             return;
         }
-        err = launch_tsqr(X, ld, m, c0, nc, Rout, ldr, scr().tsqr.as<double>(), scr().part.as<double>(), g_ctx.num_sms, st);
+        err = launch_tsqr(X, ld, m, c0, nc, Rout, ldr, scr().tsqr.as<double>(), scr().part.as<double>(), g_ctx.num_sms, checked, st);
         if (is_split(precision)) split_mark_stale(c0, nc);
     }
     // CholQR2 of X[:, c0:c0+nc] (FP64 in every precision): twice G = V^T V (one
@@ -1051,6 +1054,7 @@ int run_device(int variant, int m, int n, int s, double* dX, i64 ldX, double* dR
     Engine e{dX, (i64)ldX, (i64)m, n, s, dR, ldR, precision, st,
              carve_small(scr().small.as<double>(), n, s), scr().status.as<int>()};
     e.link = link;
+    e.checked = variant != ORTH_GB300_BCGSI2P1S;
     cudaError_t ce = (cudaError_t)zero_async(e.status, kStatusWords * sizeof(int), st);
     if (ce != cudaSuccess) e.err = (int)ce;
     if (!e.err && is_split(precision))

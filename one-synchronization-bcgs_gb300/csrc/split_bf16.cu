@@ -64,7 +64,8 @@ constexpr int KD_MAX = 7;      // digit planes held by the stores
 constexpr int TILE_M = 128;    // MMA M (rows of D = TMEM lanes)
 constexpr int KCH = 64;        // K elements per chunk (one 128-byte swizzle row)
 constexpr int WIN = 2;         // chunks per accumulation window (128 summation steps)
-constexpr int ROW_ALIGN = 256; // Gram row ranges: multiples of 256 rows (whole windows)
+constexpr int ROW_ALIGN = 256; // Gram row ranges: multiples of 256 rows (whole windows); 64 rows gain nothing
+                               // at m = 10^5 and cost a batch of small matrices 14 %
 constexpr int RA = 8;          // A ring depth (16 KB slots)
 constexpr int RB = 2;          // B ring depth
 constexpr int A_SLOT = TILE_M * KCH * 2;   // 16 KB
@@ -1442,7 +1443,7 @@ int launch_gram_split(const double* X, i64 ld, i64 m, int na, int b0, int nb, do
     g_launch_count += 1;
     rc = (int)cudaGetLastError();
     if (rc) return rc;
-    return launch_gram_reduce(P.part, gp.rc, na, nb, out, ldo, st);
+    return launch_gram_reduce_sliced(P.part, gp.rc, na, nb, out, ldo, true, st);
 }
 
 // The factor [-A Ui ; Ui] (bbuild_body; A = G[0:K, 0:nout]), its digits, and the
@@ -1823,7 +1824,7 @@ int plan_wave(SplitStaged& S, SWave& W) {
         GramJob R{};
         R.na = na; R.nb = nb; R.nchunks = gp.rc; R.part = P.part; R.C = C; R.ldc = ldc;
         rj.push_back(R);
-        rc2.push_back(gram_reduce_ctas(na, nb));
+        rc2.push_back(gram_reduce_sliced_ctas(na, nb));
     };
     auto flush_gram = [&]() {
         flush_prepare();
@@ -2120,8 +2121,8 @@ int enqueue_wave(SplitStaged& S, SWave& W, cudaStream_t st) {
                 break;
             }
             case kSReduce:
-                rc = launch_gram_reduce_batched(reinterpret_cast<const GramJob*>(jb + L.job_off), pre, L.njobs,
-                                                L.items, st);
+                rc = launch_gram_reduce_sliced_batched(reinterpret_cast<const GramJob*>(jb + L.job_off), pre, L.njobs,
+                                                       L.items, st);
                 break;
             case kSSmall:
                 rc = launch_step_batched(reinterpret_cast<const StepJob*>(jb + L.job_off), L.njobs, 32, st);

@@ -425,7 +425,7 @@ i64 tsqr_workspace_doubles(i64 m, int nc) {
         h = tiles * nc;
     }
     total += 64 * 64;                                  // + the root tile's R
-    const i64 chol = nc > 16 ? 3LL * nc * nc : 0;      // or the checked Cholesky's three blocks
+    const i64 chol = 3LL * nc * nc;                    // or the checked Cholesky's three blocks
     return 32 + (total > chol ? total : chol);         // + its flag
 }
 
@@ -527,19 +527,20 @@ int launch_tsqr_sharded(double* X, i64 ld, i64 m_local, int c0, int nc, double* 
     return (int)cudaErrorInvalidValue;
 }
 
-// Panels wider than kCheckedCols columns: Cholesky QR twice first (Fukaya, Nakatsukasa,
-// Yanagisawa, Yamamoto 2014), if the panel allows it. G = V^T V, R1 = chol(G); if every
-// pivot of R1 is at least kPivotRatio of its diagonal entry, V R1^{-1} departs from
-// orthonormal by at most about the Gram's rounding over that ratio (10^-5), and a second
-// round brings it to roundoff, as the tree does. If not (or a pivot is not a positive
-// number) nothing has been written yet, and the tree factors the panel; its kernels
-// read the flag and end at once otherwise. Twice m nc^2 / 2 products for the upper Gram
-// and as many for the substitution, against some 3.5 m nc^2 issued by the tree, a chain
-// of nc reflectors at every level. Measured at 4 10^5 x 32: 4.24 ms by the tree, 1.9 ms this
-// way; at 2^19 x 64: 23.7 and 8.5 ms. A panel that fails the test has cost the first Gram
-// (0.5 ms at 4 10^5 x 32). For 16 columns and fewer the Gram's tiles are padded and the two
-// take the same time, so those panels go straight to the tree.
-constexpr int kCheckedCols = 16;
+// Cholesky QR twice (Fukaya, Nakatsukasa, Yanagisawa, Yamamoto 2014), if the panel allows
+// it: G = V^T V, R1 = chol(G); if every pivot of R1 is at least kPivotRatio of its diagonal
+// entry, V R1^{-1} departs from orthonormal by at most about the Gram's rounding over
+// that ratio (10^-5), and a second round brings it to roundoff, as the tree does. If not
+// (or a pivot is not a positive number) nothing has been written yet, and the tree
+// factors the panel; its kernels read the flag and end at once otherwise. Twice
+// m nc^2 / 2 products for the upper Gram and as many for the substitution, against some
+// 3.5 m nc^2 issued by the tree, a chain of nc reflectors at every level. Measured at
+// 4 10^5 x 32: 4.24 ms by the tree, 1.9 ms this way; at 2^19 x 64: 23.7 and 8.5 ms; at 10^5 x 10:
+// 213 and 115 us. A panel that fails the test has cost the first Gram (0.5 ms at
+// 4 10^5 x 32).
+// All panels of more than 16 columns take this; of 8 and more where the caller allows it
+// and the tree has at least two levels (below 8 columns its levels are short: 19 us at 4).
+constexpr int kCheckedCols = 8;
 constexpr double kPivotRatio = 1e-9;
 
 static int tsqr_checked(double* X, i64 ld, i64 m, int c0, int nc, double* R, int ldR, double* ws, double* part,
@@ -548,7 +549,8 @@ static int tsqr_checked(double* X, i64 ld, i64 m, int c0, int nc, double* R, int
     double *G = ws, *R1 = ws + nn, *R2 = ws + 2 * nn;
     for (int pass = 0; pass < 2; ++pass) {
         const int* gate = pass ? done : nullptr;
-        int rc = launch_gram_fp64(X, ld, m, c0, nc, c0, nc, G, nc, part, true, num_sms, st, gate, false);
+        int rc = nc <= 16 ? launch_panel_gram(X, ld, m, c0, nc, G, part, num_sms, gate, st)
+                          : launch_gram_fp64(X, ld, m, c0, nc, c0, nc, G, nc, part, true, num_sms, st, gate, false);
         StepJob J;
         J.G = G; J.ldg = nc; J.ny = nc; J.T = pass ? R2 : R1;
         if (!pass) { J.ok = done; J.ok_ratio = kPivotRatio; }
@@ -561,10 +563,10 @@ static int tsqr_checked(double* X, i64 ld, i64 m, int c0, int nc, double* R, int
 }
 
 int launch_tsqr(double* X, i64 ld, i64 m, int c0, int nc, double* R, int ldR, double* ws, double* part, int num_sms,
-                cudaStream_t st) {
+                bool checked, cudaStream_t st) {
     if (nc <= 0) return 0;
     int* done = nullptr;
-    if (nc > kCheckedCols) {
+    if (nc > 16 || (checked && nc >= kCheckedCols && m > TSQR_TR)) {
         done = reinterpret_cast<int*>(ws);
         ws += 32;
         const int rc = tsqr_checked(X, ld, m, c0, nc, R, ldR, ws, part, num_sms, done, st);

@@ -64,10 +64,10 @@ def test_tsqr_rank_deficient(lib, s):
     _check(P)
 
 
-@pytest.mark.parametrize("s", [17, 20, 33, 64])
+@pytest.mark.parametrize("s", [8, 9, 11, 12, 14, 16, 17, 20, 33, 64])
 @pytest.mark.parametrize("kappa", [1e2, 1e4, 3e4, 1e5, 1e8, 1e13])
 def test_tsqr_conditions(lib, s, kappa):
-    """Panels wider than 16 columns take Cholesky QR where no column is too close to
+    """Panels of 8 columns and more (in bcgsi2) take Cholesky QR where no column is too close to
     those before it and the tree otherwise; the contract is the same on both sides."""
     rng = np.random.default_rng(s)
     V, _ = np.linalg.qr(rng.standard_normal((3000, s)))
