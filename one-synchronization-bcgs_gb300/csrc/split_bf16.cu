@@ -697,9 +697,13 @@ struct SplitGramJob {   // the CUtensorMap members keep the struct 64-byte align
     GramParams p;
 };
 
-// BATCH: the CTAs of many Grams in one launch; CTA b runs item b - prefix[j] of
-// job j (prefix[j] <= b < prefix[j + 1]) with job j's maps and parameters, and
-// exactly the arithmetic of a single launch of that Gram. p0.err is the launch's.
+// BATCH: many Grams in one persistent launch. Item b (prefix[j] <= b < prefix[j + 1]) is item
+// b - prefix[j] of job j, with job j's maps and parameters and exactly the arithmetic of
+// a single launch of that Gram; CTA c takes items c, c + gridDim.x, ... . The items are
+// small (256 rows of a matrix of a few thousand), so a CTA of its own for each spent
+// most of its time on barriers, TMEM and a pipeline that fills and drains; here the
+// loads of an item run while the one before is multiplied and drained. p0.err is the
+// launch's.
 template <int NB, int KD, int KA, bool BATCH>
 __global__ void __launch_bounds__(NTHREADS, 1)
 gram_tc_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ CUtensorMap mapAlast,
@@ -716,53 +720,69 @@ gram_tc_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__
     const uint32_t tmem = tmem_slot;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
 
-    int item = blockIdx.x;
-    GramParams p = p0;
-    const CUtensorMap *mA = &mapA, *mAl = &mapAlast, *mB = &mapB;
-    if constexpr (BATCH) {
-        const int j = batched_job_of(prefix, njobs, item);
-        item -= prefix[j];
-        p = jobs[j].p;
-        p.err = p0.err;
-        mA = &jobs[j].mapA; mAl = &jobs[j].mapAlast; mB = &jobs[j].mapB;
-        if (threadIdx.x == 0) {   // the producer: maps written by the host before the launch
-            tc::fence_tensormap(mA);
-            tc::fence_tensormap(mAl);
-            tc::fence_tensormap(mB);
+    const int nitems = BATCH ? prefix[njobs] : (int)gridDim.x;   // (not BATCH: one item per CTA)
+    // Item -> its job's parameters, maps and place.
+    struct Item {
+        const GramParams* p;
+        const CUtensorMap *mA, *mAl, *mB;
+        int job, mb, ng, rcI, nchunks;
+        i64 r0;
+    };
+    auto resolve = [&](int item) -> Item {
+        Item I;
+        I.p = &p0;
+        I.mA = &mapA; I.mAl = &mapAlast; I.mB = &mapB;
+        I.job = 0;
+        if constexpr (BATCH) {
+            I.job = batched_job_of(prefix, njobs, item);
+            item -= prefix[I.job];
+            I.p = &jobs[I.job].p;
+            I.mA = &jobs[I.job].mapA; I.mAl = &jobs[I.job].mapAlast; I.mB = &jobs[I.job].mapB;
         }
-    }
-    const int mb = item % p.numMB;
-    const int ng = (item / p.numMB) % p.numNG;
-    const int rcI = item / (p.numMB * p.numNG);
-    const i64 r0 = (i64)rcI * p.rows_per;
-    const i64 r1 = min(p.m, r0 + p.rows_per);
-    const int nchunks = r1 > r0 ? (int)ceil_div(r1 - r0, KCH) : 0;
-    const int nwin = (nchunks + WIN - 1) / WIN;
-
-    // The last M-block, when na is not a multiple of 128, loads only its
-    // p.alast columns (mapAlast's box); the tile's other rows keep stale data
-    // and give D rows that are not written.
-    const bool last_part = mb == p.numMB - 1 && p.alast < TILE_M;
-    auto coords = [&](int, int ch, int& ax, int& ay, int& az, int& azs, int& bx, int& by, int& bz, int& bzs,
-                      const CUtensorMap*& amap, uint32_t& abytes) {
-        const int rc = (int)((r0 + (i64)ch * KCH) / KCH);   // 64-row chunk of the column store
-        ax = 0; ay = mb * TILE_M; az = rc; azs = p.nrc;
-        bx = 0; by = p.b0 + ng * NB; bz = rc; bzs = p.nrc;
-        amap = last_part ? mAl : mA;
-        abytes = last_part ? (uint32_t)(p.alast * KCH * 2) : (uint32_t)A_SLOT;
+        I.mb = item % I.p->numMB;
+        I.ng = (item / I.p->numMB) % I.p->numNG;
+        I.rcI = item / (I.p->numMB * I.p->numNG);
+        I.r0 = (i64)I.rcI * I.p->rows_per;
+        const i64 r1 = min(I.p->m, I.r0 + I.p->rows_per);
+        I.nchunks = r1 > I.r0 ? (int)ceil_div(r1 - I.r0, KCH) : 0;
+        return I;
     };
 
     if (warp == 0) {
         if (lane == 0) {
-            // The numMB CTAs of one (row range, N-group) read the same B tiles at
-            // about the same time: B stays in L2 (evict_last) for the others.
-            const uint64_t polA = p.a_once ? tc::policy_evict_first() : tc::policy_evict_normal();
+            const uint64_t pol_first = tc::policy_evict_first(), pol_normal = tc::policy_evict_normal();
             const uint64_t polB = tc::policy_evict_last();
             Ring ra, rb;
-            for (int ch = 0; ch < nchunks; ++ch)
-                if (!produce_chunk<NB, KD, KA>(mB, sA, sB, bars, ra, rb, coords, 0, ch, &abort_flag, p.err, polA,
-                                               polB))
-                    break;
+            bool ok = true;
+            int fenced = -1;
+            for (int item = blockIdx.x; item < nitems && ok; item += gridDim.x) {
+                const Item I = resolve(item);
+                if (BATCH && I.job != fenced) {   // maps written by the host before the launch
+                    tc::fence_tensormap(I.mA);
+                    tc::fence_tensormap(I.mAl);
+                    tc::fence_tensormap(I.mB);
+                    fenced = I.job;
+                }
+                // The last M-block, when na is not a multiple of 128, loads only its
+                // p.alast columns (mapAlast's box); the tile's other rows keep stale data
+                // and give D rows that are not written.
+                const bool last_part = I.mb == I.p->numMB - 1 && I.p->alast < TILE_M;
+                auto coords = [&](int, int ch, int& ax, int& ay, int& az, int& azs, int& bx, int& by, int& bz, int& bzs,
+                                  const CUtensorMap*& amap, uint32_t& abytes) {
+                    const int rc = (int)((I.r0 + (i64)ch * KCH) / KCH);   // 64-row chunk of the column store
+                    ax = 0; ay = I.mb * TILE_M; az = rc; azs = I.p->nrc;
+                    bx = 0; by = I.p->b0 + I.ng * NB; bz = rc; bzs = I.p->nrc;
+                    amap = last_part ? I.mAl : I.mA;
+                    abytes = last_part ? (uint32_t)(I.p->alast * KCH * 2) : (uint32_t)A_SLOT;
+                };
+                // The numMB items of one (row range, N-group) read the same B tiles at
+                // about the same time: B stays in L2 (evict_last) for the others.
+                const uint64_t polA = I.p->a_once ? pol_first : pol_normal;
+                for (int ch = 0; ch < I.nchunks && ok; ++ch)
+                    ok = produce_chunk<NB, KD, KA>(I.mB, sA, sB, bars, ra, rb, coords, 0, ch, &abort_flag, p0.err, polA,
+                                                   polB);
+                if constexpr (!BATCH) break;
+            }
             if (abort_flag) {
                 drain_ring(bars->a_full, RA, ra);
                 drain_ring(bars->b_full, RB, rb);
@@ -772,16 +792,22 @@ gram_tc_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__
         if (lane == 0) {
             Ring ra, rb;
             bool ok = true;
-            for (int w = 0; w < nwin && ok; ++w) {
-                const int buf = w & 1;
-                const uint32_t tph = (uint32_t)((w >> 1) & 1);
-                if (!tc::mbar_wait(&bars->t_empty[buf], tph ^ 1u, &abort_flag, p.err, 31)) break;
-                tc::tc_fence_after();
-                const int c_end = min(nchunks, (w + 1) * WIN);
-                for (int ch = w * WIN; ch < c_end && ok; ++ch)
-                    ok = mma_chunk<NB, KD, false, KA>(tmem, (uint32_t)(buf * L::TMEM_COLS_PER_BUF), sA, sB, bars, ra,
-                                                      rb, ch == w * WIN, &abort_flag, p.err);
-                if (ok) tc::mma_commit(&bars->t_full[buf]);
+            int wc = 0;   // window counter across items
+            for (int item = blockIdx.x; item < nitems && ok; item += gridDim.x) {
+                const int nchunks = resolve(item).nchunks;
+                const int nwin = (nchunks + WIN - 1) / WIN;
+                for (int w = 0; w < nwin && ok; ++w, ++wc) {
+                    const int buf = wc & 1;
+                    const uint32_t tph = (uint32_t)((wc >> 1) & 1);
+                    if (!tc::mbar_wait(&bars->t_empty[buf], tph ^ 1u, &abort_flag, p0.err, 31)) { ok = false; break; }
+                    tc::tc_fence_after();
+                    const int c_end = min(nchunks, (w + 1) * WIN);
+                    for (int ch = w * WIN; ch < c_end && ok; ++ch)
+                        ok = mma_chunk<NB, KD, false, KA>(tmem, (uint32_t)(buf * L::TMEM_COLS_PER_BUF), sA, sB, bars,
+                                                          ra, rb, ch == w * WIN, &abort_flag, p0.err);
+                    if (ok) tc::mma_commit(&bars->t_full[buf]);
+                }
+                if constexpr (!BATCH) break;
             }
             tc::mma_commit(&bars->drain);
         }
@@ -792,41 +818,48 @@ gram_tc_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__
         const int quarter = warp & 3;
         const int half = (warp - 2) >> 2;
         const int row = quarter * 32 + lane;
-        long long hi[NH], mid[NH];
-        float lo[NH];
-#pragma unroll
-        for (int j = 0; j < NH; ++j) { hi[j] = 0; mid[j] = 0; lo[j] = 0.f; }
         bool ok = true;
-        for (int w = 0; w < nwin; ++w) {
-            const int buf = w & 1;
-            const uint32_t tph = (uint32_t)((w >> 1) & 1);
-            // Warp-uniform: the TMEM loads below are .sync.aligned.
-            const bool got = tc::mbar_wait(&bars->t_full[buf], tph, &abort_flag, p.err, 41);
-            if (!__all_sync(0xffffffffu, got)) { ok = false; break; }
-            tc::tc_fence_after();
-            const uint32_t taddr = tmem + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(buf * L::TMEM_COLS_PER_BUF);
-            accumulate_window<NB, KD>(taddr, half * NH, hi, mid, lo);
-            tc::tc_fence_before();
-            __syncwarp();
-            if (lane == 0) tc::mbar_arrive(&bars->t_empty[buf]);   // one arrival per warp
-        }
-        if (ok && !abort_flag) {
-            const int c = mb * TILE_M + row;
-            if (c < p.na) {
-                const int ec = p.cexp[c];
-                double* out = p.part + (i64)rcI * p.na * p.nb;
+        int wc = 0;
+        for (int item = blockIdx.x; item < nitems; item += gridDim.x) {
+            const Item I = resolve(item);
+            const int nwin = (I.nchunks + WIN - 1) / WIN;
+            long long hi[NH], mid[NH];
+            float lo[NH];
+#pragma unroll
+            for (int j = 0; j < NH; ++j) { hi[j] = 0; mid[j] = 0; lo[j] = 0.f; }
+            for (int w = 0; w < nwin; ++w, ++wc) {
+                const int buf = wc & 1;
+                const uint32_t tph = (uint32_t)((wc >> 1) & 1);
+                // Warp-uniform: the TMEM loads below are .sync.aligned.
+                const bool got = tc::mbar_wait(&bars->t_full[buf], tph, &abort_flag, p0.err, 41);
+                if (!__all_sync(0xffffffffu, got)) { ok = false; break; }
+                tc::tc_fence_after();
+                const uint32_t taddr =
+                    tmem + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(buf * L::TMEM_COLS_PER_BUF);
+                accumulate_window<NB, KD>(taddr, half * NH, hi, mid, lo);
+                tc::tc_fence_before();
+                __syncwarp();
+                if (lane == 0) tc::mbar_arrive(&bars->t_empty[buf]);   // one arrival per warp
+            }
+            if (__any_sync(0xffffffffu, !ok || abort_flag)) break;
+            const int c = I.mb * TILE_M + row;
+            if (c < I.p->na) {
+                const int ec = I.p->cexp[c];
+                double* out = I.p->part + (i64)I.rcI * I.p->na * I.p->nb;
 #pragma unroll
                 for (int jj = 0; jj < NH; ++jj) {
-                    const int j = ng * NB + half * NH + jj;
-                    if (j < p.nb) out[c + (i64)j * p.na] = assemble(hi[jj], mid[jj], lo[jj], ec + p.cexp[p.b0 + j] - 78);
+                    const int j = I.ng * NB + half * NH + jj;
+                    if (j < I.p->nb)
+                        out[c + (i64)j * I.p->na] = assemble(hi[jj], mid[jj], lo[jj], ec + I.p->cexp[I.p->b0 + j] - 78);
                 }
             }
+            if constexpr (!BATCH) break;
         }
     }
     __syncthreads();
     if (warp == 1) {
         // All MMAs issued by this CTA have completed once `drain` fires.
-        if (lane == 0) tc::mbar_wait(&bars->drain, 0, &abort_flag, p.err, 51);
+        if (lane == 0) tc::mbar_wait(&bars->drain, 0, &abort_flag, p0.err, 51);
         __syncwarp();
         tc::tc_fence_after();
         tc::tmem_dealloc(tmem, (uint32_t)L::TMEM_ALLOC);
@@ -2108,8 +2141,9 @@ int enqueue_wave(SplitStaged& S, SWave& W, cudaStream_t st) {
             case kSGram16: {
                 const auto* J = reinterpret_cast<const SplitGramJob*>(jb + L.job_off);
                 const int ka = gram_a_planes(KD);
+                const unsigned ggrid = items < (unsigned)S.num_sms ? items : (unsigned)S.num_sms;
 #define BCGS_GRAMB(NBT, KDT, KAT)                                                                              \
-    gram_tc_kernel<NBT, KDT, KAT, true><<<items, NTHREADS, SmemLayout<NBT, KDT>::BYTES, st>>>(none, none, none, \
+    gram_tc_kernel<NBT, KDT, KAT, true><<<ggrid, NTHREADS, SmemLayout<NBT, KDT>::BYTES, st>>>(none, none, none, \
                                                                                             g0, J, pre, L.njobs)
                 if (L.kind == kSGram16) {
                     if (KD == 6) BCGS_GRAMB(16, 6, 6); else if (ka == 6) BCGS_GRAMB(16, 7, 6); else BCGS_GRAMB(16, 7, 7);
