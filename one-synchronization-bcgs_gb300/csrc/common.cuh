@@ -69,6 +69,15 @@ inline cudaError_t launch_spread(void (*kernel)(Params...), dim3 grid, dim3 bloc
     kernel<<<grid, block, smem, st>>>(static_cast<Params>(args)...);
     return cudaPeekAtLastError();
 }
+// Asynchronous copy of one double into shared memory; zero if not valid (src then only has to be
+// readable).
+__device__ __forceinline__ void cp_async8(double* dst, const double* src, bool valid) {
+    const uint32_t d = (uint32_t)__cvta_generic_to_shared(dst);
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(d), "l"(src), "r"(valid ? 8 : 0) : "memory");
+}
+__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int N>
+__device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
 #endif
 
 }  // namespace bcgs

@@ -91,9 +91,9 @@ int launch_step_batched(const StepJob* jobs, int njobs, int nmax, cudaStream_t s
 int launch_rblock(double* R, int ldR, int c0, int K, int ny, const double* A, int lda,
                   const double* B, int ldb, const double* Sd, const double* Yd, int mode, cudaStream_t st);
 
-// Upper Gram (nc x nc, ld nc) of X[:, c0:c0+nc], nc <= 16, through part (panel_gram_part_doubles);
-// gate as launch_gram_fp64.
-i64 panel_gram_part_doubles(int nc);
+// Upper Gram (nc x nc, ld nc) of X[:, c0:c0+nc], nc <= 32, through part (panel_gram_part_doubles
+// of the widest panel); gate as launch_gram_fp64.
+i64 panel_gram_part_doubles(int s);
 int launch_panel_gram(const double* X, i64 ld, i64 m, int c0, int nc, double* G, double* part, int num_sms,
                       const int* gate, cudaStream_t st);
 

@@ -1,10 +1,16 @@
-// Upper Gram of a narrow panel (nc <= 16 columns), for the checked Cholesky QR of TSQR panels.
+// Upper Gram of a narrow panel (nc <= 32 columns), for the checked Cholesky QR of TSQR panels.
 //
-// The general Gram's tiles pad 10 x 10 entries, of which 55 are wanted, to 16 x 16. Here a
-// lane holds a row of the panel and all the wanted sums (up to 11 columns) or those of
-// some of the columns (two warps share the rows beyond), so a row of 32 lanes takes
+// The general Gram's tiles pad 10 x 10 entries, of which 55 are wanted, to 16 x 16, and run
+// three of four 16 x 16 tiles for 32 columns, 768 products for 528. Here a lane holds a
+// row of the panel and all the wanted sums (up to 11 columns) or those of some of the
+// columns (2, 4 or 8 warps share the rows beyond), so a row of 32 lanes takes
 // nc (nc + 1) / 2 FP64 instructions and nothing is padded: 22 us at 10^5 x 10, 181 us at
-// 7 10^5 x 16 (150 us at the FP64 peak).
+// 7 10^5 x 16 (150 us at the FP64 peak), 416 us at 4 10^5 x 32 (335 us at the peak).
+// Up to 16 columns three CTAs share an SM and hide each other's loads. Beyond, the sums
+// fill the registers of one or two CTAs, so the rows come through a ring of stages in
+// shared memory, each warp copying its own columns: bcgsi2P2s at 400000 x 256, s = 32,
+// takes 22.3 ms with the general Gram, 20.4 ms with this one and loads straight into
+// registers, 20.9 ms with prefetches too (they spill), 19.5 ms with the ring.
 // The lanes' sums are added through shared memory once per CTA, the CTAs' by the sliced
 // reduction, all in a fixed order.
 #include "common.cuh"
@@ -13,20 +19,28 @@
 namespace bcgs {
 
 namespace {
-constexpr int PG_THREADS = 128;
-constexpr int PG_CTAS_PER_SM = 3;
-
-// Columns [0, pg_cut) go to the first warp of a pair, the rest to the second.
+// Warps that share a row group's sums, row groups of 32 a CTA takes at once, CTAs per SM.
 template <int NC>
-__host__ __device__ constexpr int pg_cut() {
-    return NC <= 11 ? NC : (NC * 7 + 5) / 10;   // about half of the sums
-}
+__host__ __device__ constexpr int pg_parts() { return NC <= 11 ? 1 : (NC <= 16 ? 2 : (NC <= 24 ? 4 : 8)); }
 template <int NC>
-__host__ __device__ constexpr int pg_slots() { return NC <= 11 ? 4 : 2; }   // row groups of 32 a CTA takes at once
+__host__ __device__ constexpr int pg_slots() { return NC <= 11 ? 4 : (NC <= 16 ? 2 : 1); }
+template <int NC>
+__host__ __device__ constexpr int pg_warps() { return pg_parts<NC>() * pg_slots<NC>(); }
+__host__ __device__ constexpr int pg_per_sm(int nc) { return nc <= 16 ? 3 : (nc <= 24 ? 2 : 1); }
 template <int NC>
 __host__ __device__ constexpr int pg_sums() { return NC * (NC + 1) / 2; }
 template <int NC>
 __host__ __device__ constexpr int pg_ld() { return 32 * pg_slots<NC>() + 1; }
+constexpr int PG_ST = 4;   // stages in shared memory of the forms whose registers leave no room for loads ahead
+template <int NC>
+__host__ __device__ constexpr bool pg_staged() { return pg_slots<NC>() == 1; }
+// Part q has columns [pg_cut(q), pg_cut(q + 1)): about as many sums as the others.
+template <int NC>
+__host__ __device__ constexpr int pg_cut(int q) {
+    int j = 0;
+    while (j < NC && j * (j + 1) / 2 * pg_parts<NC>() < q * pg_sums<NC>()) ++j;
+    return j;
+}
 
 // Columns [J0, J1) of the upper Gram over this warp's row groups, into red[sum][lane slot].
 template <int NC, int J0, int J1>
@@ -37,88 +51,131 @@ __device__ __forceinline__ void panel_sums(const double* __restrict__ V, i64 ld,
 #pragma unroll
     for (int k = 0; k < NA; ++k) acc[k] = 0.0;
     const i64 groups = (m + 31) / 32;
-    for (i64 g = g0; g < groups; g += step) {
-        const i64 r = g * 32 + (threadIdx.x & 31);
-#pragma unroll
-        for (int c = 0; c < J1; ++c) x[c] = c < nc && r < m ? V[r + (i64)c * ld] : 0.0;
+    auto add = [&] {
         int k = 0;
 #pragma unroll
         for (int j = J0; j < J1; ++j)
 #pragma unroll
             for (int i = 0; i <= j; ++i, ++k) acc[k] = fma(x[i], x[j], acc[k]);
+    };
+    if constexpr (pg_staged<NC>()) {
+        // red holds PG_ST stages of NC x 32 rows; this warp copies its own columns.
+        const int lane = threadIdx.x & 31;
+        auto copy = [&](i64 g, int st) {
+            const i64 r = g * 32 + lane;
+#pragma unroll
+            for (int c = J0; c < J1; ++c) {
+                const bool ok = c < nc && r < m;
+                cp_async8(red + (st * NC + c) * 32 + lane, ok ? V + r + (i64)c * ld : V, ok);
+            }
+            cp_async_commit();
+        };
+#pragma unroll
+        for (int st = 0; st < PG_ST - 1; ++st) copy(g0 + st * step, st);
+        int st = 0;
+        for (i64 g = g0; g < groups; g += step) {
+            cp_async_wait<PG_ST - 2>();
+            // The warps are here at different places of the code: a barrier by its number.
+            asm volatile("bar.sync 1, %0;" ::"n"(32 * pg_warps<NC>()) : "memory");
+            copy(g + (PG_ST - 1) * step, (st + PG_ST - 1) % PG_ST);
+#pragma unroll
+            for (int c = 0; c < J1; ++c) x[c] = red[(st * NC + c) * 32 + lane];
+            add();
+            st = (st + 1) % PG_ST;
+        }
+        cp_async_wait<0>();
+        asm volatile("bar.sync 1, %0;" ::"n"(32 * pg_warps<NC>()) : "memory");
+    } else {
+        for (i64 g = g0; g < groups; g += step) {
+            const i64 r = g * 32 + (threadIdx.x & 31);
+#pragma unroll
+            for (int c = 0; c < J1; ++c) x[c] = c < nc && r < m ? V[r + (i64)c * ld] : 0.0;
+            add();
+        }
     }
 #pragma unroll
     for (int k = 0; k < NA; ++k) red[(J0 * (J0 + 1) / 2 + k) * pg_ld<NC>() + col] = acc[k];
 }
 
+template <int NC, int Q>
+__device__ __forceinline__ void panel_part(int part, const double* __restrict__ V, i64 ld, i64 m, int nc, i64 g0,
+                                           i64 step, double* __restrict__ red, int col) {
+    if (part == Q) {
+        panel_sums<NC, pg_cut<NC>(Q), pg_cut<NC>(Q + 1)>(V, ld, m, nc, g0, step, red, col);
+        return;
+    }
+    if constexpr (Q + 1 < pg_parts<NC>()) panel_part<NC, Q + 1>(part, V, ld, m, nc, g0, step, red, col);
+}
+
 template <int NC>
-__global__ void __launch_bounds__(PG_THREADS)
+__global__ void __launch_bounds__(32 * pg_warps<NC>(), 1)
 panel_gram_kernel(const double* __restrict__ V, i64 ld, i64 m, int nc, double* __restrict__ part,
                   const int* __restrict__ gate) {
-    extern __shared__ double red[];   // sums x lane slots, then 4 x sums
+    extern __shared__ double red[];   // sums x lane slots, then warps x sums
     chain_enter();
     if (gate != nullptr && *gate == 0) return;
-    constexpr int SL = pg_slots<NC>(), NS = pg_sums<NC>(), LD = pg_ld<NC>(), CUT = pg_cut<NC>();
+    constexpr int SL = pg_slots<NC>(), NS = pg_sums<NC>(), LD = pg_ld<NC>(), NW = pg_warps<NC>();
+    constexpr int EACH = 32 * SL / NW;   // lane slots a warp adds
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int slot = warp % SL;
-    const i64 g0 = (i64)blockIdx.x * SL + slot, step = (i64)gridDim.x * SL;
-    if constexpr (CUT == NC) {
-        panel_sums<NC, 0, NC>(V, ld, m, nc, g0, step, red, slot * 32 + lane);
-    } else {
-        if (warp < SL) panel_sums<NC, 0, CUT>(V, ld, m, nc, g0, step, red, slot * 32 + lane);
-        else panel_sums<NC, CUT, NC>(V, ld, m, nc, g0, step, red, slot * 32 + lane);
-    }
+    // Warps w and w + 4 share an FP64 pipe: of eight parts, pair the ones that add up evenly.
+    const int mine = pg_parts<NC>() == 8 ? (0x37650124 >> (4 * warp)) & 7 : warp / SL;
+    panel_part<NC, 0>(mine, V, ld, m, nc, (i64)blockIdx.x * SL + slot, (i64)gridDim.x * SL, red, slot * 32 + lane);
     __syncthreads();
-    // Warp w adds the w-th quarter of the lane slots of every sum.
-    double* quarter = red + NS * LD;
+    double* sub = red + NS * LD;
     for (int o = lane; o < NS; o += 32) {
         double s = 0.0;
-#pragma unroll 8
-        for (int k = 0; k < 8 * SL; ++k) s += red[o * LD + warp * 8 * SL + k];
-        quarter[warp * NS + o] = s;
+#pragma unroll
+        for (int k = 0; k < EACH; ++k) s += red[o * LD + warp * EACH + k];
+        sub[warp * NS + o] = s;
     }
     __syncthreads();
-    for (int o = threadIdx.x; o < NS; o += PG_THREADS) {
+    for (int o = threadIdx.x; o < NS; o += 32 * NW) {
         int j = 0;
         while ((j + 1) * (j + 2) / 2 <= o) ++j;
         const int i = o - j * (j + 1) / 2;
-        if (j < nc)
-            part[(i64)blockIdx.x * nc * nc + i + (i64)j * nc] =
-                (quarter[o] + quarter[NS + o]) + (quarter[2 * NS + o] + quarter[3 * NS + o]);
+        double s = 0.0;
+#pragma unroll
+        for (int w = 0; w < NW; w += 4)
+            s += (sub[w * NS + o] + sub[(w + 1) * NS + o]) + (sub[(w + 2) * NS + o] + sub[(w + 3) * NS + o]);
+        if (j < nc) part[(i64)blockIdx.x * nc * nc + i + (i64)j * nc] = s;
     }
-}
-
-// At least four row groups per warp, at most PG_CTAS_PER_SM CTAs per SM.
-int panel_ctas(i64 m, int slots, int num_sms) {
-    const i64 want = ceil_div(ceil_div(m, 32), 4 * slots), most = (i64)PG_CTAS_PER_SM * num_sms;
-    return (int)(want < most ? want : most);
 }
 
 template <int NC>
 int run_panel(const double* V, i64 ld, i64 m, int nc, double* G, double* part, int num_sms, const int* gate,
               cudaStream_t st) {
-    const size_t smem = (size_t)(pg_sums<NC>() * (pg_ld<NC>() + 4)) * sizeof(double);
+    const size_t smem = (size_t)(pg_sums<NC>() * (pg_ld<NC>() + pg_warps<NC>())) * sizeof(double);
     int rc = smem_attr((const void*)panel_gram_kernel<NC>, (int)smem);
     if (rc) return rc;
-    const int ctas = panel_ctas(m, pg_slots<NC>(), num_sms);
-    launch_spread(panel_gram_kernel<NC>, (unsigned)ctas, PG_THREADS, smem, st, V, ld, m, nc, part, gate);
+    // At least four row groups per warp.
+    const i64 want = ceil_div(ceil_div(m, 32), 4 * pg_slots<NC>()), most = (i64)pg_per_sm(nc) * num_sms;
+    const int ctas = (int)(want < most ? want : most);
+    launch_spread(panel_gram_kernel<NC>, (unsigned)ctas, 32 * pg_warps<NC>(), smem, st, V, ld, m, nc, part, gate);
     g_launch_count += 1;
     rc = (int)cudaGetLastError();
     return rc ? rc : launch_gram_reduce_sliced(part, ctas, nc, nc, G, nc, false, st);
 }
 }  // namespace
 
-i64 panel_gram_part_doubles(int nc) { return (i64)PG_CTAS_PER_SM * kNumSMsDefault * nc * nc; }
+i64 panel_gram_part_doubles(int s) {
+    i64 most = 0;
+    for (int nc = 1; nc <= s && nc <= 32; ++nc) {
+        const i64 want = (i64)pg_per_sm(nc) * kNumSMsDefault * nc * nc;
+        most = want > most ? want : most;
+    }
+    return most;
+}
 
 int launch_panel_gram(const double* X, i64 ld, i64 m, int c0, int nc, double* G, double* part, int num_sms,
                       const int* gate, cudaStream_t st) {
     const double* V = X + (i64)c0 * ld;
     if (num_sms > kNumSMsDefault) num_sms = kNumSMsDefault;   // part's size
-    if (nc <= 8) return run_panel<8>(V, ld, m, nc, G, part, num_sms, gate, st);
-    if (nc <= 10) return run_panel<10>(V, ld, m, nc, G, part, num_sms, gate, st);
-    if (nc <= 12) return run_panel<12>(V, ld, m, nc, G, part, num_sms, gate, st);
-    if (nc <= 14) return run_panel<14>(V, ld, m, nc, G, part, num_sms, gate, st);
-    if (nc <= 16) return run_panel<16>(V, ld, m, nc, G, part, num_sms, gate, st);
+#define BCGS_PANEL(N) \
+    if (nc <= N) return run_panel<N>(V, ld, m, nc, G, part, num_sms, gate, st);
+    BCGS_PANEL(8) BCGS_PANEL(10) BCGS_PANEL(12) BCGS_PANEL(14) BCGS_PANEL(16) BCGS_PANEL(20) BCGS_PANEL(24) BCGS_PANEL(28)
+    BCGS_PANEL(32)
+#undef BCGS_PANEL
     return (int)cudaErrorInvalidValue;
 }
 

@@ -43,14 +43,6 @@ constexpr int GSEG = 2048;          // rows of one FMA chain: the chunks of a la
 
 __host__ __device__ inline int gram_width(int ta, int r) { return r * (GTHREADS / ta); }
 __host__ __device__ inline int gram_stage_doubles(int ta, int r) { return GR * ((ta + gram_width(ta, r)) | 1); }
-
-__device__ __forceinline__ void cp_async8(double* dst, const double* src, bool valid) {
-    const uint32_t d = (uint32_t)__cvta_generic_to_shared(dst);
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(d), "l"(src), "r"(valid ? 8 : 0) : "memory");
-}
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-template <int N>
-__device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
 }  // namespace
 
 // The tile at C rows ia0.., C columns jb0.., rows [r_begin, r_end) of X, written to

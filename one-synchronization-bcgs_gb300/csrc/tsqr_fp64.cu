@@ -549,7 +549,7 @@ static int tsqr_checked(double* X, i64 ld, i64 m, int c0, int nc, double* R, int
     double *G = ws, *R1 = ws + nn, *R2 = ws + 2 * nn;
     for (int pass = 0; pass < 2; ++pass) {
         const int* gate = pass ? done : nullptr;
-        int rc = nc <= 16 ? launch_panel_gram(X, ld, m, c0, nc, G, part, num_sms, gate, st)
+        int rc = nc <= 32 ? launch_panel_gram(X, ld, m, c0, nc, G, part, num_sms, gate, st)
                           : launch_gram_fp64(X, ld, m, c0, nc, c0, nc, G, nc, part, true, num_sms, st, gate, false);
         StepJob J;
         J.G = G; J.ldg = nc; J.ny = nc; J.T = pass ? R2 : R1;

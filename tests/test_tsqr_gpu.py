@@ -73,3 +73,12 @@ def test_tsqr_conditions(lib, s, kappa):
     V, _ = np.linalg.qr(rng.standard_normal((3000, s)))
     W, _ = np.linalg.qr(rng.standard_normal((s, s)))
     _check((V * np.logspace(0, -np.log10(kappa), s)) @ W)
+
+
+@pytest.mark.parametrize("s", [15, 21, 24, 25, 28, 29, 32])
+@pytest.mark.parametrize("m", [2999, 40001])
+def test_tsqr_checked_gram_widths(lib, m, s):
+    """Widths at the edges of the narrow Gram kernel's forms, with fewer row groups than CTAs and with
+    several to each."""
+    rng = np.random.default_rng(m + s)
+    _check(rng.standard_normal((m, s)) * np.logspace(0, -3, s))
