@@ -18,9 +18,7 @@
 // summation orders of the single-matrix driver: with the same Gram chunking
 // (orth_gb300_set_gram_chunk_rows) the results are bit-identical.
 //
-// Tuning: per block size s, the rows per Gram chunk are picked by timing each candidate
-// on a representative Gram stage of that class's matrices: 4096 ... 32768 rows, or
-// smaller chunks where the batch is too small to fill the GPU with those.
+// The rows per Gram chunk come from the shapes of the whole schedule (pick_rows).
 #include <algorithm>
 #include <cmath>
 #include <cstdio>
@@ -46,9 +44,8 @@ namespace {
 constexpr int kTR = 256;                // TSQR tile rows for nc <= 32
 constexpr int kMaxS = 16;
 constexpr int kClasses = 3;             // s <= 4, s <= 8, s <= 16
-constexpr int kRowsMin = 4096;          // smallest Gram chunk candidate of a batch that fills the GPU,
-constexpr int kRowsLeast = 256;         // and of any batch
-constexpr int kRowsCands = 4;           // candidates, each twice the one before
+constexpr int kRowsLeast = 256;         // rows per Gram chunk: powers of two from here
+constexpr int kRowsMost = 32768;        // to here
 
 int class_of(int s) { return s <= 4 ? 0 : (s <= 8 ? 1 : 2); }
 
@@ -58,7 +55,6 @@ struct Mat {
     double* X;
     double* R;
     int ldR;
-    int cls;
     // workspace
     double *G1, *G2, *Scol[2], *Sd[2], *Yd, *part, *tsqr;   // Scol, Sd: this step's and the next one's
     int* status;
@@ -96,8 +92,8 @@ i64 small_block_doubles(int n, int s) { return 2LL * (n + s) * 2 * s + 2LL * n *
 
 i64 tsqr_doubles(i64 m, int s) { return tsqr_workspace_doubles(m, s); }
 
-i64 part_doubles_of(i64 m, int n, int s, int rows_min) {
-    return ceil_div(m, rows_min) * (i64)(n + s) * (2 * s) + 64;
+i64 part_doubles_of(i64 m, int n, int s, int rows) {
+    return ceil_div(m, rows) * (i64)(n + s) * (2 * s) + 64;
 }
 
 }  // namespace
@@ -106,17 +102,13 @@ struct BatchPlan {
     int count = 0;
     std::vector<Mat> mats;
     int tb[kClasses] = {16, 16, 32};   // C columns of a Gram tile, for the report
-    int rows[kClasses] = {8192, 8192, 8192};
-    int rows_min = kRowsMin;
-    bool tuned = false;
+    int rows = kRowsMost;              // per Gram chunk
     // device memory: workspace (per-matrix blocks + status) and the job blob
     void* ws = nullptr;
     size_t ws_bytes = 0;
     void* jobs_dev = nullptr;
     size_t jobs_bytes = 0;
     std::vector<Stage> stages;
-    std::vector<std::vector<GramReq>> gram_reqs;   // per Gram stage, in stage order
-    std::vector<int> gram_stage_idx;
     cudaStream_t own_stream = nullptr;
     cudaGraph_t graph = nullptr;
     cudaGraphExec_t exec = nullptr;
@@ -154,7 +146,7 @@ size_t layout_workspace(BatchPlan& P, char* base) {
         M.Sd[0] = sb ? M.Scol[1] + (i64)n * s : nullptr;
         M.Sd[1] = sb ? M.Sd[0] + (i64)s * s : nullptr;
         M.Yd = sb ? M.Sd[1] + (i64)s * s : nullptr;
-        M.part = (double*)take((size_t)part_doubles_of(M.m, M.n, M.s, P.rows_min) * sizeof(double));
+        M.part = (double*)take((size_t)part_doubles_of(M.m, M.n, M.s, P.rows) * sizeof(double));
         M.tsqr = (double*)take((size_t)tsqr_doubles(M.m, M.s) * sizeof(double));
     }
     int* st = (int*)take((size_t)P.count * kStatusWords * sizeof(int));
@@ -199,8 +191,6 @@ GramJob make_gram_job(const Mat& M, const GramReq& q, int rows) {
 // Builds every stage of the schedule (jobs + prefix arrays in `blob`).
 void build_schedule(BatchPlan& P, Blob& blob) {
     P.stages.clear();
-    P.gram_reqs.clear();
-    P.gram_stage_idx.clear();
     const int B = P.count;
     std::vector<Mat>& mats = P.mats;
 
@@ -223,12 +213,14 @@ void build_schedule(BatchPlan& P, Blob& blob) {
         std::vector<int> counts;
         for (const GramReq& q : reqs) {
             const Mat& M = mats[q.mat];
-            GramJob J = make_gram_job(M, q, P.rows[M.cls]);
+            GramJob J = make_gram_job(M, q, P.rows);
             jobs.push_back(J);
-            counts.push_back(J.nchunks * J.tiles);
         }
-        P.gram_stage_idx.push_back((int)P.stages.size());
-        P.gram_reqs.push_back(reqs);
+        // The longest CTAs first: what starts last decides how evenly a stage ends.
+        std::stable_sort(jobs.begin(), jobs.end(), [](const GramJob& a, const GramJob& b) {
+            return a.r * a.rows_per_chunk > b.r * b.rows_per_chunk;
+        });
+        for (const GramJob& J : jobs) counts.push_back(J.nchunks * J.tiles);
         Stage S;
         S.kind = kStGram;
         S.njobs = (int)jobs.size();
@@ -497,63 +489,6 @@ int upload_schedule(BatchPlan& P) {
     return 0;
 }
 
-// Times the Gram of each class's matrices at their middle block step for every
-// candidate of the chunk rows and keeps the fastest.
-int autotune(BatchPlan& P, cudaStream_t st) {
-    cudaEvent_t e0, e1;
-    BCGS_CUDA_TRY(cudaEventCreate(&e0));
-    BCGS_CUDA_TRY(cudaEventCreate(&e1));
-    int rc = 0;
-    for (int c = 0; c < kClasses && !rc; ++c) {
-        std::vector<GramReq> reqs;
-        for (int b = 0; b < P.count && reqs.size() < 256; ++b) {
-            const Mat& M = P.mats[b];
-            if (M.cls != c) continue;
-            int na, b0, nb;
-            step_gram_shape(M, M.p > 1 ? std::max(1, (M.p - 1) / 2) : 0, na, b0, nb);
-            reqs.push_back({b, na, b0, nb, M.G1, na});
-        }
-        if (reqs.empty()) continue;
-        float best = 1e30f;
-        for (int k = 0; k < kRowsCands; ++k) {
-            const int rows = P.rows_min << k;
-            std::vector<GramJob> jobs;
-            std::vector<int> prefix(1, 0), prefix2(1, 0);
-            for (const GramReq& q : reqs) {
-                GramJob J = make_gram_job(P.mats[q.mat], q, rows);
-                P.tb[c] = J.r * (128 / J.ta);
-                jobs.push_back(J);
-                prefix.push_back(prefix.back() + J.nchunks * J.tiles);
-                prefix2.push_back(prefix2.back() + gram_reduce_ctas(J.na, J.nb));
-            }
-            Blob blob;
-            const size_t jo = blob.put(jobs), po = blob.put(prefix), p2 = blob.put(prefix2);
-            void* d = nullptr;
-            if ((rc = (int)cudaMalloc(&d, blob.bytes.size()))) break;
-            rc = (int)cudaMemcpy(d, blob.bytes.data(), blob.bytes.size(), cudaMemcpyHostToDevice);
-            float ms = 0.f;
-            for (int rep = 0; rep < 2 && !rc; ++rep) {
-                cudaEventRecord(e0, st);
-                rc = launch_gram_partial_batched((const GramJob*)((char*)d + jo), (const int*)((char*)d + po),
-                                                 (int)jobs.size(), prefix.back(), st);
-                if (!rc)
-                    rc = launch_gram_reduce_batched((const GramJob*)((char*)d + jo), (const int*)((char*)d + p2),
-                                                    (int)jobs.size(), prefix2.back(), st);
-                cudaEventRecord(e1, st);
-                if (!rc) rc = (int)cudaEventSynchronize(e1);
-                if (!rc) rc = (int)cudaEventElapsedTime(&ms, e0, e1);
-            }
-            cudaFree(d);
-            if (rc) break;
-            if (ms < best) { best = ms; P.rows[c] = rows; }
-        }
-    }
-    cudaEventDestroy(e0);
-    cudaEventDestroy(e1);
-    P.tuned = (rc == 0);
-    return rc;
-}
-
 void free_plan(BatchPlan* P) {
     if (!P) return;
     if (P->staged) split_staged_destroy(P->staged);
@@ -564,6 +499,50 @@ void free_plan(BatchPlan* P) {
     if (P->ws) cudaFree(P->ws);
     if (P->own_stream) cudaStreamDestroy(P->own_stream);
     delete P;
+}
+
+// Rows per Gram chunk, the same for the whole plan (its results depend on it): the
+// candidate with the least time over all Gram stages by this estimate. A CTA takes 64 r
+// clocks of its SM per row and about 1500 to start and finish; a stage takes the sum
+// over the SMs plus half a longest CTA for its uneven end, and no less than one alone at
+// 63 % of the FP64 pipe; then come the partials' traffic and the reduction's chain, 130
+// clocks a chunk. The late stages decide: they have only the matrices with many block
+// steps. 48 matrices of 2000 to 20000 rows, 60 to 256 columns: the Grams take 12.8 ms
+// with the chunks that are fastest at the middle steps (one choice per s), 9.8 ms with
+// this one, 256 (512 rows: 10.0, 1024: 11.2, 2048: 14.6, 8192: 27.3; the estimate has
+// them in this order).
+void pick_rows(BatchPlan& P) {
+    struct Shape { i64 m; int r; i64 tiles, entries; };
+    std::vector<std::vector<Shape>> stages;
+    for (const Mat& M : P.mats)
+        for (int i = 0; i < M.p; ++i) {
+            int na, b0, nb, ta, r;
+            step_gram_shape(M, i, na, b0, nb);
+            if (na <= 0 || nb <= 0) continue;
+            if ((int)stages.size() <= i) stages.resize(i + 1);
+            const i64 tiles = gram_batched_tile(na, b0, nb, &ta, &r);
+            stages[i].push_back({M.m, r, tiles, (i64)na * nb});
+            if (i == M.p / 2) P.tb[class_of(M.s)] = r * (128 / ta);
+        }
+    double best = -1.0;
+    for (int rows = kRowsMost; rows >= kRowsLeast; rows /= 2) {
+        double cost = 0.0;
+        for (const auto& stage : stages) {
+            double total = 0.0, longest = 0.0, bytes = 0.0;
+            i64 chain = 0;
+            for (const Shape& q : stage) {
+                const i64 nch = ceil_div(q.m, rows);
+                const double cta = 64.0 * q.r * (double)(ceil_div(ceil_div(q.m, nch), 32) * 32) + 1500.0;
+                total += cta * (double)(nch * q.tiles);
+                longest = std::max(longest, cta);
+                chain = std::max(chain, nch);
+                bytes += 16.0 * (double)(nch * q.entries);
+            }
+            cost += std::max(total / (0.97 * kNumSMsDefault) + 0.5 * longest, longest / 0.63);
+            cost += 130.0 * (double)chain + bytes / 3500.0;
+        }
+        if (best < 0.0 || cost < best) { best = cost; P.rows = rows; }
+    }
 }
 
 int fill_mats(BatchPlan& P, int count, const int* m, const int* n, const int* s, double* const* dX,
@@ -577,19 +556,8 @@ int fill_mats(BatchPlan& P, int count, const int* m, const int* n, const int* s,
         M.R = dR ? dR[b] : nullptr; M.ldR = ldR ? ldR[b] : n[b];
         if (M.s < 1 || M.s > kMaxS || M.n < 2 * M.s || M.m < M.n || M.ld < M.m || M.ldR < M.n) return 2;
         M.p = (M.n - M.s + M.s - 1) / M.s;
-        M.cls = class_of(M.s);
     }
-    // Chunks of 4096 rows and more unless their Gram tiles would leave SMs idle (fewer
-    // than 16 CTAs per SM at the matrices' middle block steps).
-    for (P.rows_min = kRowsMin; P.rows_min > kRowsLeast; P.rows_min /= 2) {
-        i64 ctas = 0;
-        for (const Mat& M : P.mats) {
-            int na, b0, nb, ta, r;
-            step_gram_shape(M, M.p > 1 ? std::max(1, (M.p - 1) / 2) : 0, na, b0, nb);
-            ctas += ceil_div(M.m, P.rows_min) * gram_batched_tile(na, b0, nb, &ta, &r);
-        }
-        if (ctas >= 16LL * kNumSMsDefault) break;
-    }
+    pick_rows(P);
     return 0;
 }
 
@@ -657,9 +625,6 @@ int orth_gb300_batch_create(orth_gb300_batch** out, int variant, int count, cons
     layout_workspace(*P, (char*)P->ws);
     if (cudaStreamCreateWithFlags(&P->own_stream, cudaStreamNonBlocking) != cudaSuccess) { free_plan(P); return 3; }
     if (!st) st = P->own_stream;
-    if (flags & ORTH_GB300_BATCH_TUNE) {
-        if (autotune(*P, st)) { free_plan(P); return 3; }
-    }
     if (upload_schedule(*P)) { free_plan(P); return 3; }
     // Capture the whole batched QR once; runs replay it.
     cudaStream_t cs = P->own_stream;
@@ -729,7 +694,7 @@ int orth_gb300_batch_info(const orth_gb300_batch* h, long long* launches_per_run
     if (P.staged && workspace_bytes) split_staged_info(P.staged, nullptr, workspace_bytes, nullptr, nullptr);
     if (graph_nodes) *graph_nodes = P.graph_nodes;
     if (tuned)
-        for (int c = 0; c < kClasses; ++c) { tuned[2 * c] = P.tb[c]; tuned[2 * c + 1] = P.rows[c]; }
+        for (int c = 0; c < kClasses; ++c) { tuned[2 * c] = P.tb[c]; tuned[2 * c + 1] = P.rows; }
     return 0;
 }
 
