@@ -508,7 +508,7 @@ def run_ours(args, rank, world, local_rank):
                 "frac": round(achieved / peak, 4),
                 "traffic": round(ratio * pc["traffic"] / calls) if ratio is not None else None,
                 "kernel": {"gram": "gram_tc_kernel<7> + gram_reduce",
-                           "update": "bbuild_fused + bdigit + update_tc_kernel<32,7> (fused Q_k/U_k+1 pass)"}[dom],
+                           "update": "bbuild + bdigit + update_tc_kernel<32,7> (fused Q_k/U_k+1 pass)"}[dom],
                 "peak_source": peak_src,
                 "launch_ms": round(launch_ms, 4),
                 "bytes_per_launch": round(pc["bytes"] / calls),

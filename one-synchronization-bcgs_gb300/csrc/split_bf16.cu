@@ -36,7 +36,8 @@
 // 16 KB slots, a B ring, and two TMEM accumulators so the epilogue of one window
 // overlaps the MMAs of the next. The update is persistent and takes row tiles from
 // a per-launch counter; the Gram's M-block CTAs of one row range run side by side
-// and share each B tile through L2 (B loaded evict_last, A evict_first). No load
+// and share each B tile through L2 (B loaded evict_last, A evict_first); in batches
+// the Gram is persistent over its items too. No load
 // is multicast. Every wait is bounded; a timeout sets an
 // error word and the kernel winds down.
 #include <algorithm>
