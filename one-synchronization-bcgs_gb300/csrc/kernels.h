@@ -91,17 +91,21 @@ int launch_step_batched(const StepJob* jobs, int njobs, int nmax, cudaStream_t s
 int launch_rblock(double* R, int ldR, int c0, int K, int ny, const double* A, int lda,
                   const double* B, int ldb, const double* Sd, const double* Yd, int mode, cudaStream_t st);
 
-// Upper Gram (nc x nc, ld nc) of X[:, c0:c0+nc], nc <= 32, through part (panel_gram_part_doubles
-// of the widest panel); gate as launch_gram_fp64.
-i64 panel_gram_part_doubles(int s);
+// Upper Gram (nc x nc, ld nc) of X[:, c0:c0+nc], nc <= 32, through part, which holds
+// panel_gram_part_doubles(m, s) for panels of up to s columns (the rows forced by
+// g_gram_chunk_rows play no part); gate as launch_gram_fp64.
+i64 panel_gram_part_doubles(i64 m, int s);
 int launch_panel_gram(const double* X, i64 ld, i64 m, int c0, int nc, double* G, double* part, int num_sms,
                       const int* gate, cudaStream_t st);
 
 // Explicit TSQR of X[:, c0:c0+nc] in place; R (nc x nc, ldR) upper with diag >= 0.
 int tsqr_tile_rows(int nc);
 i64 tsqr_workspace_doubles(i64 m, int nc);
-// part: gram_part_doubles_fp64(m, nc, nc) doubles. checked: panels of up to 16 columns may take
-// Cholesky QR too (not in BCGSI+P-1S, whose batched plans use the tree).
+// part: panel_gram_part_doubles(m, nc) doubles, or gram_part_doubles_fp64(m, nc, nc) for more
+// than 32 columns; only written before the tree runs, so it may lie in ws from
+// tsqr_check_doubles(nc) on. checked: panels of up to 16 columns may take Cholesky QR
+// too (not in BCGSI+P-1S, whose batched plans use the tree).
+inline i64 tsqr_check_doubles(int nc) { return 32 + 3LL * nc * nc; }   // the checked Cholesky's flag and blocks in ws
 int launch_tsqr(double* X, i64 ld, i64 m, int c0, int nc, double* R, int ldR, double* ws, double* part, int num_sms,
                 bool checked, cudaStream_t st);
 

@@ -72,7 +72,7 @@ int setup_device(DeviceSetup** out) {
 
 // Scratch layout (doubles), all offsets rounded to 32 doubles (256 bytes).
 struct Layout {
-    i64 status, G1, G2, Scol, Sd, Yd, part, tsqr, total;
+    i64 status, G1, G2, Scol, Sd, Yd, tsqr, part, panel, total;
 };
 
 i64 round32(i64 v) { return (v + 31) / 32 * 32; }
@@ -86,8 +86,15 @@ Layout layout_for(i64 m, int n, int s) {
     L.Scol = off;   off += round32((i64)n * s);
     L.Sd = off;     off += round32((i64)s * s);
     L.Yd = off;     off += round32((i64)s * s);
-    L.part = off;   off += round32(gram_part_doubles_fp64(m, n + s, 2 * s));
     L.tsqr = off;   off += round32(tsqr_workspace_doubles(m, s));
+    L.part = off;   off += round32(gram_part_doubles_fp64(m, n + s, 2 * s));
+    // The partials of block 1's narrow Gram (s <= 32) do not shrink with forced chunk rows
+    // as the other Grams' do. They lie over the TSQR tree's space, which is free until
+    // the check of the panel has failed, and on over the other partials, so that no
+    // shape needs more scratch for them than a few small ones with forced rows.
+    L.panel = L.tsqr + round32(tsqr_check_doubles(s));
+    if (s > 16 && s <= 32 && L.panel + panel_gram_part_doubles(m, s) > off)
+        off = L.panel + round32(panel_gram_part_doubles(m, s));
     L.total = off;
     return L;
 }
@@ -126,6 +133,7 @@ extern "C" int orth_gb300_bcgsi2P1s_dev_noalloc(int m, int n, int s, double* dX,
     double* Sd = base + L.Sd;
     double* Yd = base + L.Yd;
     double* part = base + L.part;
+    double* panel = s <= 32 ? base + L.panel : part;   // (not used up to 16 columns)
     double* tws = base + L.tsqr;
     const i64 M = m, ld = ldX;
 
@@ -157,7 +165,7 @@ extern "C" int orth_gb300_bcgsi2P1s_dev_noalloc(int m, int n, int s, double* dX,
     // BCGSI+P-1S, the same schedule as the allocating entry point
     // (reference SRC/orth.c:48-222).
     const int s0 = s, p = (n - s + s - 1) / s;
-    if (!err) err = launch_tsqr(dX, ld, M, 0, s0, dR, ldR, tws, part, d->num_sms, false, st);
+    if (!err) err = launch_tsqr(dX, ld, M, 0, s0, dR, ldR, tws, panel, d->num_sms, false, st);
     gram(2 * s, s0, s, W);
     run_step(factor(W, 2 * s, s0, s, Sd, 1));
     update(s0, s0, s, W, 2 * s, Sd, s);

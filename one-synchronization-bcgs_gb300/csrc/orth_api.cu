@@ -190,7 +190,7 @@ int init_ctx() {
 
 // Largest Gram-partial buffer any step or panel needs (doubles).
 i64 part_doubles(i64 m, int n, int s) {
-    return std::max(gram_part_doubles_fp64(m, n + s, 2 * s), panel_gram_part_doubles(s));
+    return std::max(gram_part_doubles_fp64(m, n + s, 2 * s), panel_gram_part_doubles(m, s));
 }
 
 // Small buffers carved from one allocation (doubles).

@@ -22,8 +22,9 @@ namespace {
 // Warps that share a row group's sums, row groups of 32 a CTA takes at once, CTAs per SM.
 template <int NC>
 __host__ __device__ constexpr int pg_parts() { return NC <= 11 ? 1 : (NC <= 16 ? 2 : (NC <= 24 ? 4 : 8)); }
+__host__ __device__ constexpr int pg_slots_of(int width) { return width <= 11 ? 4 : (width <= 16 ? 2 : 1); }
 template <int NC>
-__host__ __device__ constexpr int pg_slots() { return NC <= 11 ? 4 : (NC <= 16 ? 2 : 1); }
+__host__ __device__ constexpr int pg_slots() { return pg_slots_of(NC); }
 template <int NC>
 __host__ __device__ constexpr int pg_warps() { return pg_parts<NC>() * pg_slots<NC>(); }
 __host__ __device__ constexpr int pg_per_sm(int nc) { return nc <= 16 ? 3 : (nc <= 24 ? 2 : 1); }
@@ -142,15 +143,21 @@ panel_gram_kernel(const double* __restrict__ V, i64 ld, i64 m, int nc, double* _
     }
 }
 
+// CTAs for nc columns in code of the given width: at least four row groups per warp.
+int panel_ctas(i64 m, int nc, int width, int num_sms) {
+    const i64 want = ceil_div(ceil_div(m, 32), 4 * pg_slots_of(width)), most = (i64)pg_per_sm(nc) * num_sms;
+    return (int)(want < most ? want : most);
+}
+// Widths there is code for: 8, 10, 12, 14, 16, then every fourth.
+constexpr int pg_width(int nc) { return nc <= 8 ? 8 : (nc <= 16 ? (nc + 1) / 2 * 2 : (nc + 3) / 4 * 4); }
+
 template <int NC>
 int run_panel(const double* V, i64 ld, i64 m, int nc, double* G, double* part, int num_sms, const int* gate,
               cudaStream_t st) {
     const size_t smem = (size_t)(pg_sums<NC>() * (pg_ld<NC>() + pg_warps<NC>())) * sizeof(double);
     int rc = smem_attr((const void*)panel_gram_kernel<NC>, (int)smem);
     if (rc) return rc;
-    // At least four row groups per warp.
-    const i64 want = ceil_div(ceil_div(m, 32), 4 * pg_slots<NC>()), most = (i64)pg_per_sm(nc) * num_sms;
-    const int ctas = (int)(want < most ? want : most);
+    const int ctas = panel_ctas(m, nc, NC, num_sms);
     launch_spread(panel_gram_kernel<NC>, (unsigned)ctas, 32 * pg_warps<NC>(), smem, st, V, ld, m, nc, part, gate);
     g_launch_count += 1;
     rc = (int)cudaGetLastError();
@@ -158,10 +165,10 @@ int run_panel(const double* V, i64 ld, i64 m, int nc, double* G, double* part, i
 }
 }  // namespace
 
-i64 panel_gram_part_doubles(int s) {
+i64 panel_gram_part_doubles(i64 m, int s) {
     i64 most = 0;
     for (int nc = 1; nc <= s && nc <= 32; ++nc) {
-        const i64 want = (i64)pg_per_sm(nc) * kNumSMsDefault * nc * nc;
+        const i64 want = (i64)panel_ctas(m, nc, pg_width(nc), kNumSMsDefault) * nc * nc;
         most = want > most ? want : most;
     }
     return most;
@@ -171,12 +178,14 @@ int launch_panel_gram(const double* X, i64 ld, i64 m, int c0, int nc, double* G,
                       const int* gate, cudaStream_t st) {
     const double* V = X + (i64)c0 * ld;
     if (num_sms > kNumSMsDefault) num_sms = kNumSMsDefault;   // part's size
+    switch (pg_width(nc)) {
 #define BCGS_PANEL(N) \
-    if (nc <= N) return run_panel<N>(V, ld, m, nc, G, part, num_sms, gate, st);
-    BCGS_PANEL(8) BCGS_PANEL(10) BCGS_PANEL(12) BCGS_PANEL(14) BCGS_PANEL(16) BCGS_PANEL(20) BCGS_PANEL(24) BCGS_PANEL(28)
-    BCGS_PANEL(32)
+        case N: return run_panel<N>(V, ld, m, nc, G, part, num_sms, gate, st);
+        BCGS_PANEL(8) BCGS_PANEL(10) BCGS_PANEL(12) BCGS_PANEL(14) BCGS_PANEL(16) BCGS_PANEL(20) BCGS_PANEL(24)
+        BCGS_PANEL(28) BCGS_PANEL(32)
 #undef BCGS_PANEL
-    return (int)cudaErrorInvalidValue;
+        default: return (int)cudaErrorInvalidValue;
+    }
 }
 
 }  // namespace bcgs

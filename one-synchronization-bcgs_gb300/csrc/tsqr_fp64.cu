@@ -424,9 +424,9 @@ i64 tsqr_workspace_doubles(i64 m, int nc) {
         total += tiles * nc * nc;
         h = tiles * nc;
     }
-    total += 64 * 64;                                  // + the root tile's R
-    const i64 chol = 3LL * nc * nc;                    // or the checked Cholesky's three blocks
-    return 32 + (total > chol ? total : chol);         // + its flag
+    total += 64 * 64 + 32;                             // + the root tile's R and the checked Cholesky's flag
+    const i64 chol = tsqr_check_doubles(nc);           // or its flag and its three blocks
+    return total > chol ? total : chol;
 }
 
 // The tree from a given level on: level 0 here is (A0, rows0, ld0), factored in

@@ -108,3 +108,31 @@ def test_noalloc_rejects_oversized_shape(lib, capfd):
     assert "static workspace" in capfd.readouterr().err
     torch.cuda.synchronize()
     assert bool((dX == 7.0).all()) and bool((dR == -3.0).all())
+
+
+@pytest.mark.parametrize("m,n,s,rows", [(40000, 72, 24, 8192), (20000, 64, 32, 32768), (3000, 51, 17, 4096),
+                                        (9000, 80, 40, 4096)])
+def test_noalloc_forced_chunk_rows(lib, m, n, s, rows):
+    """Forced chunk rows shrink the Gram partials; block 1's narrow Gram, which they do
+    not touch, still has room for its own. Bit-identical to the allocating entry point."""
+    torch = pytest.importorskip("torch")
+    X = inputs.graded_host(m, n, 1e4, seed=m + s)
+    stream = torch.cuda.current_stream().cuda_stream
+    outs = []
+    lib.orth_gb300_set_gram_chunk_rows(rows)
+    try:
+        for noalloc in (False, True, True):
+            dX = _dev_copy(torch, X)
+            dR = torch.zeros((n, n), dtype=torch.float64, device="cuda")
+            if noalloc:
+                rc, st = orth.bcgsi2P1s_dev_noalloc(m, n, s, dX.data_ptr(), m, dR.data_ptr(), n, stream)
+            else:
+                rc, st = orth.run_dev("bcgsi2P1s", m, n, s, dX.data_ptr(), m, dR.data_ptr(), n, orth.FP64, stream)
+            assert rc == 0 and st["breakdown_step"] == 0 and st["cuda_error"] == 0
+            outs.append((dX.cpu().numpy(), np.triu(dR.cpu().numpy().T)))
+    finally:
+        lib.orth_gb300_set_gram_chunk_rows(0)
+    Q = outs[0][0].T
+    assert np.linalg.norm(Q.T @ Q - np.eye(n)) <= 1e-12
+    for Qn, Rn in outs[1:]:
+        assert np.array_equal(Qn, outs[0][0]) and np.array_equal(Rn, outs[0][1])
