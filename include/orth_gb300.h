@@ -153,11 +153,12 @@ int orth_gb300_run_sharded(int variant, long long m, int n, int s, double *dXsub
  * bcgsi2, :520-523 and :532-535, and in bcgsi2P2s, :612-614 and :649-652):
  *   ORTH_GB300_INTRA_TSQR     the hand-written TSQR tree (default, the reference's choice).
  *                             A panel of more than 16 columns (of 8 and more except
- *                             in bcgsi2P1s), none of them too close to those before
- *                             it (tested on its Gram's Cholesky pivots), is factored
- *                             by two rounds of Cholesky QR instead, to the same
- *                             contract: Q orthonormal to roundoff, no breakdown, no
- *                             counted reduction.
+ *                             in bcgsi2P1s) whose condition, its columns scaled to
+ *                             norm 1, is below about 3e4 (taken from the inverse of
+ *                             its Gram's Cholesky factor) is factored by two rounds
+ *                             of Cholesky QR instead, to the same contract: Q
+ *                             orthonormal to roundoff, no breakdown, no counted
+ *                             reduction.
  *   ORTH_GB300_INTRA_CHOLQR2  CholeskyQR2: twice G = V^T V (one deterministic
  *                             reduction each), T = chol(G), V = V T^{-1}; R = R2 R1.
  *                             Cheaper (two tall passes), but its Cholesky breaks down

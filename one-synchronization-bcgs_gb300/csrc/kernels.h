@@ -77,10 +77,11 @@ struct StepJob {
     int mode = -1, c0 = 0, ldR = 0, lda = 0;
     double* R = nullptr;
     const double *A = nullptr, *Sold = nullptr;
-    // If not null (K = 0): *ok = every pivot of T is at least ok_ratio times its diagonal
-    // entry of G, i.e. no column is closer than sqrt(ok_ratio) to those before it.
+    // If not null (K = 0, nz = 0): *ok = || D T^{-1} ||_F^2 <= ok_limit, D the square roots of
+    // G's diagonal: the squared condition of the columns behind G, each scaled to norm 1.
+    // T is only defined if it is.
     int* ok = nullptr;
-    double ok_ratio = 0.0;
+    double ok_limit = 0.0;
 };
 int launch_step(const StepJob& J, cudaStream_t st);
 // One job per matrix; nmax: the largest ny + nz, at most 32.

@@ -240,7 +240,7 @@ __device__ void step_body(const StepJob& J, int rank, double* sm) {
     // pivot go to slot r & 1 (the carried identity has 1 at c = r). A pivot that is
     // not a positive number of ordinary size ends the fast path (an integer test: a
     // comparison would be one more FP64 instruction).
-    const bool carry = J.Uinv != nullptr;
+    const bool carry = J.Uinv != nullptr || J.ok != nullptr;
     // (Loops over the columns are kept rolled: an FP64 instruction that is only
     // predicated off still takes its 64 clocks.)
     auto publish = [&](int r, double d, double x0) {
@@ -315,7 +315,6 @@ __device__ void step_body(const StepJob& J, int rank, double* sm) {
     if (fast) {
         // Row r of U is the eliminated row over the square root of its pivot; the
         // carried rows scale the same way and give U^{-T}.
-        bool close = false;
         for (int r = tid; r < n; r += ST_THREADS) {
             // v = 1 / sqrt(d), u = sqrt(d) = d v corrected once (half the cost of a
             // square root and a division).
@@ -323,11 +322,6 @@ __device__ void step_body(const StepJob& J, int rank, double* sm) {
             const double v = rsqrt(d), u = d * v;
             s_u[r] = fma(fma(-u, u, d), 0.5 * v, u);
             s_u[n + r] = v;
-            if (J.ok != nullptr) close |= !(d >= J.ok_ratio * __ldg(J.G + r + (i64)r * J.ldg));
-        }
-        if (J.ok != nullptr) {
-            const int any = __syncthreads_or(close);
-            if (tid == 0) *J.ok = !any;
         }
         __syncthreads();
         for (int r = warp; r < n; r += ST_WARPS) {
@@ -342,6 +336,25 @@ __device__ void step_body(const StepJob& J, int rank, double* sm) {
             }
         }
         __syncthreads();
+        if (J.ok != nullptr) {
+            // Row r of a's lower part is row r of U^{-T}: the sum of G_cc (U^{-T})_rc^2, in a
+            // fixed order. (A sum that is Inf or NaN is not within the limit.)
+            __shared__ double s_norm[ST_WARPS];
+            double p = 0.0;
+            for (int r = warp; r < n; r += ST_WARPS)
+                for (int c = lane; c <= r; c += 32) {
+                    const double x = c == r ? s_u[n + r] : a[r * ld + c];
+                    p = fma(x * x, __ldg(J.G + c + (i64)c * J.ldg), p);
+                }
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) p += __shfl_xor_sync(0xffffffffu, p, o);
+            if (lane == 0) s_norm[warp] = p;
+            __syncthreads();
+            if (tid == 0) {
+                for (int w = 1; w < ST_WARPS; ++w) p += s_norm[w];
+                *J.ok = p <= J.ok_limit;
+            }
+        }
     } else {
         // A pivot out of range: the same factorization by dot products. At a
         // breakdown (a pivot <= 0) the factor keeps the rows before it, and the rows
@@ -502,7 +515,8 @@ int launch_clustered(K kernel, unsigned grid, int ctas, size_t smem, bool chaine
 
 bool step_valid(const StepJob& J) {
     return J.ny >= 1 && J.ny <= SMAX && J.nz >= 0 && J.nz <= SMAX && J.K >= 0 && J.G != nullptr && J.T != nullptr &&
-           (J.nz == 0 || J.S != nullptr) && (!J.scaled || J.nz == 0 || J.Sd != nullptr);
+           (J.nz == 0 || J.S != nullptr) && (!J.scaled || J.nz == 0 || J.Sd != nullptr) &&
+           (J.ok == nullptr || (J.K == 0 && J.nz == 0));
 }
 
 }  // namespace

@@ -82,3 +82,38 @@ def test_tsqr_checked_gram_widths(lib, m, s):
     several to each."""
     rng = np.random.default_rng(m + s)
     _check(rng.standard_normal((m, s)) * np.logspace(0, -3, s))
+
+
+def _unit_upper(s, kind, a):
+    """Triangular factors whose diagonal says little about their condition: Kahan's
+    (unit columns, diagonal a^j) and I - a triu(ones, 1) (unit diagonal, inverse of
+    norm about (1 + a)^(s - 2))."""
+    if kind == "kahan":
+        T = np.eye(s) - np.sqrt(1.0 - a * a) * np.triu(np.ones((s, s)), 1)
+        return T * (a ** np.arange(s))[:, None]
+    return np.eye(s) - a * np.triu(np.ones((s, s)), 1)
+
+
+@pytest.mark.parametrize("kind,a", [("kahan", 0.9), ("kahan", 0.8), ("kahan", 0.7), ("kahan", 0.5), ("triu", 0.25),
+                                    ("triu", 0.5), ("triu", 1.0), ("triu", 2.0)])
+@pytest.mark.parametrize("s", [8, 12, 16, 20, 24, 32, 40, 48, 64])
+def test_tsqr_conditions_pivots_do_not_show(lib, s, kind, a):
+    """Panels whose Cholesky pivots stay large next to their diagonal while the condition grows
+    exponentially with the width: from harmless (8 columns) to numerically singular
+    (64), so both sides of the check that admits Cholesky QR are covered."""
+    for seed in range(3):
+        V, _ = np.linalg.qr(np.random.default_rng(100 * s + seed).standard_normal((4000, s)))
+        _check(V @ _unit_upper(s, kind, a))
+
+
+@pytest.mark.parametrize("s", [20, 32, 64])
+@pytest.mark.parametrize("variant", ["bcgsi2P1s", "bcgsi2P2s"])
+def test_first_block_pivots_do_not_show(lib, variant, s):
+    """Block 1 is orthogonalized once in every variant."""
+    rng = np.random.default_rng(s)
+    V, _ = np.linalg.qr(rng.standard_normal((4000, s)))
+    X = np.hstack([V @ _unit_upper(s, "triu", 1.0), rng.standard_normal((4000, s))])
+    Q, R, rc, st = orth.qr(variant, X, s)
+    assert rc == 0 and st["cuda_error"] == 0
+    Q1 = Q[:, :s]
+    assert np.linalg.norm(Q1.T @ Q1 - np.eye(s)) <= 40 * (s + 10) * U
