@@ -160,17 +160,20 @@ static GramTile gram_tile(int na, int nb, int upper) {
 }
 
 // blockIdx: chunk, live tile (no CTA for a skipped one: an SM that got one would be left
-// with less than its share while others take one more).
+// with less than its share while others take one more). A wide C has more than 65535
+// tiles, which go on in z.
 template <int R, int SEGR>
 __global__ void __launch_bounds__(GTHREADS)
 gram_fp64_partial(const double* __restrict__ X, i64 ld, i64 m, int a0, int na, int b0, int nb, int ta, int upper,
-                  i64 rows_per_chunk, double* __restrict__ part, const int* __restrict__ gate) {
+                  int live, i64 rows_per_chunk, double* __restrict__ part, const int* __restrict__ gate) {
     extern __shared__ double sm[];
     chain_enter();
     if (gate != nullptr && *gate == 0) return;
     const int chunk = blockIdx.x;
+    const int t = (int)(blockIdx.y + blockIdx.z * gridDim.y);
+    if (t >= live) return;
     int ia0, jb0;
-    gram_tile_of((int)blockIdx.y, upper, gram_width(ta, R), nb, ta, (na + ta - 1) / ta, ia0, jb0);
+    gram_tile_of(t, upper, gram_width(ta, R), nb, ta, (na + ta - 1) / ta, ia0, jb0);
     const i64 r_begin = (i64)chunk * rows_per_chunk;
     const i64 r_end = min(m, r_begin + rows_per_chunk);
     gram_partial_body<R, SEGR>(X, ld, a0, na, b0, nb, ta, r_begin, r_end, ia0, jb0, part + (i64)chunk * na * nb, sm);
@@ -179,13 +182,14 @@ gram_fp64_partial(const double* __restrict__ X, i64 ld, i64 m, int a0, int na, i
 template <int SEGR>
 static int launch_partial(const GramTile& t, int nchunks, const double* X, i64 ld, i64 m, int a0, int na, int b0,
                           int nb, int upper, i64 rows, double* part, const int* gate, cudaStream_t st) {
-    const dim3 grid((unsigned)nchunks, (unsigned)t.live);
+    const i64 layers = ceil_div(t.live, 65535);
+    const dim3 grid((unsigned)nchunks, (unsigned)ceil_div(t.live, layers), (unsigned)layers);
     const size_t smem = (size_t)GST * gram_stage_doubles(t.ta, t.r) * sizeof(double);
     switch (t.r) {
-#define BCGS_GP(RR)                                                                                              \
-    case RR:                                                                                                     \
-        launch_spread(gram_fp64_partial<RR, SEGR>, grid, GTHREADS, smem, st, X, ld, m, a0, na, b0, nb, t.ta, upper, rows, part,  \
-                                                            gate);                                            \
+#define BCGS_GP(RR)                                                                                               \
+    case RR:                                                                                                      \
+        launch_spread(gram_fp64_partial<RR, SEGR>, grid, GTHREADS, smem, st, X, ld, m, a0, na, b0, nb, t.ta, upper, \
+                      (int)t.live, rows, part, gate);                                                             \
         break;
         BCGS_GP(1) BCGS_GP(2) BCGS_GP(3) BCGS_GP(4) BCGS_GP(5) BCGS_GP(6) BCGS_GP(7) BCGS_GP(8)
 #undef BCGS_GP

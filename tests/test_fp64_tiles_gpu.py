@@ -61,3 +61,17 @@ def test_update_split_rule_edge(lib, m):
     E = X @ X.T - torch.eye(n, device="cuda", dtype=torch.float64)
     assert float(E.norm()) <= 1e-13
     assert float((X0 - torch.triu(R.T).T @ X).norm() / X0.norm()) <= 1e-14
+
+
+def test_gram_more_tiles_than_a_grid_dimension(lib):
+    """C of 8208 x 8208 has over 65535 tiles."""
+    torch = pytest.importorskip("torch")
+    m, n = 24, 8208
+    g = torch.Generator(device="cuda")
+    g.manual_seed(1)
+    X = torch.randn((n, m), generator=g, device="cuda", dtype=torch.float64)
+    C = torch.full((n, n), 7.0, device="cuda", dtype=torch.float64)
+    assert orth.gram_dev(m, n, 0, n, X.data_ptr(), m, C.data_ptr(), n, orth.FP64) == 0
+    torch.cuda.synchronize()
+    C -= X @ X.T
+    assert bool((C.abs() <= 2 * (m + 2) * U * (X.abs() @ X.abs().T)).all())
