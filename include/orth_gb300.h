@@ -323,6 +323,14 @@ int orth_gb300_poison_shared_memory(unsigned long long bits, void *stream);
  */
 int orth_gb300_timeout_probe(int code, void *stream, int out[2]);
 
+/*
+ * Diagnostic of the arithmetic: the reciprocal and the square root that the block
+ * step and the TSQR use in place of a division and sqrt, of n device numbers dx
+ * (positive, 2^-930 .. 2^930), into dRecip and dRoot, on `stream`. 0, 2 (invalid
+ * arguments) or 3.
+ */
+int orth_gb300_scalar_probe(long long n, const double *dx, double *dRecip, double *dRoot, void *stream);
+
 /* Status of the last run through the orth.h entry points on this thread. */
 void orth_gb300_last_status(orth_gb300_status *status);
 

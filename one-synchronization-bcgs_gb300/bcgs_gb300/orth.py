@@ -130,6 +130,8 @@ def load(path: str | None = None):
     lib.orth_gb300_poison_shared_memory.restype = ctypes.c_int
     lib.orth_gb300_timeout_probe.argtypes = [ctypes.c_int, ctypes.c_void_p, ctypes.POINTER(ctypes.c_int)]
     lib.orth_gb300_timeout_probe.restype = ctypes.c_int
+    lib.orth_gb300_scalar_probe.argtypes = [ctypes.c_longlong] + [ctypes.c_void_p] * 4
+    lib.orth_gb300_scalar_probe.restype = ctypes.c_int
     lib.orth_gb300_set_gram_chunk_rows.restype = None
     P_int, P_ll, P_vp = ctypes.POINTER(ctypes.c_int), ctypes.POINTER(ctypes.c_longlong), ctypes.POINTER(ctypes.c_void_p)
     lib.orth_gb300_batch_create.argtypes = [ctypes.POINTER(ctypes.c_void_p), ctypes.c_int, ctypes.c_int, P_int, P_int,
@@ -221,6 +223,12 @@ def timeout_probe(code: int, stream: int = 0):
     out = (ctypes.c_int * 2)()
     rc = int(load().orth_gb300_timeout_probe(code, ctypes.c_void_p(stream), out))
     return rc, out[0], out[1]
+
+
+def scalar_probe(n: int, x_ptr: int, recip_ptr: int, root_ptr: int, stream: int = 0) -> int:
+    """The kernels' 1/x and sqrt(x) of n device numbers (orth_gb300_scalar_probe)."""
+    return int(load().orth_gb300_scalar_probe(n, ctypes.c_void_p(x_ptr), ctypes.c_void_p(recip_ptr),
+                                              ctypes.c_void_p(root_ptr), ctypes.c_void_p(stream)))
 
 
 class HostBuffer:

@@ -9,6 +9,8 @@
 //    kernels' own bounded wait, on an mbarrier that nothing completes. The wait
 //    gives up after its time limit, records its code and returns, and the host
 //    reads the code; the context stays usable (tests/test_timeout_gpu.py).
+// 3. The kernels' reciprocal and square root on given numbers, for a comparison with
+//    CUDA's (tests/test_scalar_gpu.py).
 #include "../../include/orth_gb300.h"
 #include "common.cuh"
 #include "kernels.h"
@@ -39,7 +41,22 @@ __global__ void wait_timeout_probe_kernel(int code, int* out) {
     }
 }
 
+__global__ void scalar_probe_kernel(const double* x, long long n, double* r, double* u) {
+    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
+        r[i] = recip(x[i]);
+        u[i] = root(x[i], rsqrt(x[i]));
+    }
+}
+
 }  // namespace bcgs
+
+extern "C" int orth_gb300_scalar_probe(long long n, const double* dx, double* dRecip, double* dRoot, void* stream) {
+    using namespace bcgs;
+    if (n < 1 || !dx || !dRecip || !dRoot) return 2;
+    scalar_probe_kernel<<<kNumSMsDefault, 256, 0, (cudaStream_t)stream>>>(dx, n, dRecip, dRoot);
+    g_launch_count += 1;
+    return cudaGetLastError() == cudaSuccess ? 0 : 3;
+}
 
 extern "C" int orth_gb300_timeout_probe(int code, void* stream, int out[2]) {
     using namespace bcgs;

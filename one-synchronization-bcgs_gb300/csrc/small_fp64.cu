@@ -62,17 +62,6 @@ __device__ __forceinline__ void trap_rc(int e, int nr, int& r, int& c) {
     }
 }
 __host__ __device__ inline int trap_size(int nr, int n) { return nr * (nr + 1) / 2 + (n - nr) * nr; }
-
-// 1 / x for a normal x: the hardware's approximate reciprocal (rcp.approx.ftz.f64, 20
-// bits or more) corrected by r (1 + e + e^2), e = 1 - x r, which leaves a relative
-// error of e^3 and the roundings: three dependent operations on the elimination's
-// critical path. Only ever used as a multiplier of an elimination step.
-__device__ __forceinline__ double recip(double x) {
-    double r;
-    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(x));
-    const double e = fma(-x, r, 1.0);
-    return fma(r, fma(e, e, e), r);
-}
 }  // namespace
 
 // Shared memory of one CTA (doubles): the N x N matrix (also the staging tile of the
@@ -316,11 +305,8 @@ __device__ void step_body(const StepJob& J, int rank, double* sm) {
         // Row r of U is the eliminated row over the square root of its pivot; the
         // carried rows scale the same way and give U^{-T}.
         for (int r = tid; r < n; r += ST_THREADS) {
-            // v = 1 / sqrt(d), u = sqrt(d) = d v corrected once (half the cost of a
-            // square root and a division).
-            const double d = r < nr ? a[r * ld + r] : 1.0;
-            const double v = rsqrt(d), u = d * v;
-            s_u[r] = fma(fma(-u, u, d), 0.5 * v, u);
+            const double d = r < nr ? a[r * ld + r] : 1.0, v = rsqrt(d);
+            s_u[r] = root(d, v);
             s_u[n + r] = v;
         }
         __syncthreads();

@@ -160,23 +160,10 @@ __device__ __forceinline__ void make_reflector(double* a, double* tau, double* r
             p = below();
             q = fma(alpha, alpha, p);
         }
-        // 1 / sqrt(q), and sqrt(q) = q / sqrt(q) corrected once.
-        const double rs = rsqrt(q);
-        double nrm = q * rs;
-        nrm = fma(fma(-nrm, nrm, q), 0.5 * rs, nrm);
-        beta = -copysign(nrm, alpha);
+        beta = -copysign(root(q, rsqrt(q)), alpha);
         vc = alpha - beta;
         const double e = 0.5 * fma(vc, vc, p);   // t v^T v = 2 for the v that is stored
-        if (ordinary(e)) {
-            // 1 / e: the hardware's approximate reciprocal r (20 bits or more) times
-            // 1 + d + d^2, d = 1 - e r.
-            double r;
-            asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(e));
-            const double d = fma(-e, r, 1.0);
-            t = fma(r, fma(d, d, d), r);
-        } else {
-            t = 1.0 / e;
-        }
+        t = ordinary(e) ? recip(e) : 1.0 / e;
         if (__double_as_longlong(back) != __double_as_longlong(1.0)) beta *= back;
     }
 #pragma unroll
