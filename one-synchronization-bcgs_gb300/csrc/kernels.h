@@ -82,6 +82,7 @@ struct StepJob {
     // T is only defined if it is.
     int* ok = nullptr;
     double ok_limit = 0.0;
+    const int* gate = nullptr;   // if not null and *gate is 0, launch_step's kernel does nothing
 };
 int launch_step(const StepJob& J, cudaStream_t st);
 // One job per matrix; nmax: the largest ny + nz, at most 32.

@@ -341,12 +341,13 @@ __device__ void step_body(const StepJob& J, int rank, double* sm) {
                 *J.ok = p <= J.ok_limit;
             }
         }
+    } else if (J.ok != nullptr) {
+        if (tid == 0) *J.ok = 0;
     } else {
         // A pivot out of range: the same factorization by dot products. At a
         // breakdown (a pivot <= 0) the factor keeps the rows before it, and the rows
         // from it on hold the matrix that was to be factored, as dpotrf leaves
         // them; what follows goes on with that factor. Not a path for speed.
-        if (tid == 0 && J.ok != nullptr) *J.ok = 0;
         __syncthreads();
         for (int e = tid; e < E; e += ST_THREADS) {
             int r, c;
@@ -437,6 +438,7 @@ template <int C>
 __global__ void __launch_bounds__(ST_THREADS) step_kernel(const __grid_constant__ StepJob job) {
     extern __shared__ double sm[];
     chain_enter();
+    if (job.gate != nullptr && *job.gate == 0) return;   // (every CTA of the cluster reads the same)
     step_body<C>(job, C == 1 ? 0 : (int)blockIdx.x, sm);
 }
 

@@ -547,6 +547,7 @@ static int tsqr_checked(double* X, i64 ld, i64 m, int c0, int nc, double* R, int
         StepJob J;
         J.G = G; J.ldg = nc; J.ny = nc; J.T = pass ? R2 : R1;
         if (!pass) { J.ok = done; J.ok_limit = kCondLimit; }
+        J.gate = gate;
         if (!rc) rc = launch_step(J, st);
         if (!rc) rc = launch_update_fp64(X, ld, m, 0, 0, c0, nc, nullptr, 0, J.T, nc, true, st, done);
         if (rc) return rc;
