@@ -242,8 +242,8 @@ void orth_gb300_set_gram_chunk_rows(long long rows);
  * (n[b] x n[b], ldR[b]; upper block triangle written), block size s[b] <= 16,
  * n[b] >= 2 s[b], m[b] >= n[b]. Arrays are host arrays of count entries (ldX/ldR
  * may be NULL: tight). precision ORTH_GB300_FP64: variant ORTH_GB300_BCGSI2P1S,
- * s[b] <= 16. flags: ORTH_GB300_BATCH_TUNE asks for the Gram's chunk rows to suit the
- * batch; they always do (an estimate over the shapes of all its block steps).
+ * s[b] <= 16. flags: ORTH_GB300_BATCH_TUNE is accepted and has no effect (the Gram's
+ * chunk rows always come from an estimate over the shapes of all the block steps).
  * precision ORTH_GB300_SPLIT_BF16 / _FAST:
  *   - ORTH_GB300_BCGSI2P1S with every s[b] <= 16 (the default form): staged
  *     graphs. The matrices are taken in order into waves whose digit stores
@@ -280,9 +280,9 @@ int orth_gb300_batch_create(orth_gb300_batch **plan, int variant, int count, con
 int orth_gb300_batch_run(orth_gb300_batch *plan, void *stream);
 /* Per-matrix Cholesky breakdown (step, info; 0 if none) of the last run; waits for the device. */
 int orth_gb300_batch_status(orth_gb300_batch *plan, int *breakdown_step, int *breakdown_info, int *nbroken);
-/* Kernel launches per run, device bytes held, graph nodes, and the tuned
- * (panel width, chunk rows) for s <= 4, <= 8, <= 16 (tuned: 6 ints; the chunk rows are
- * the same for all). */
+/* Kernel launches per run, device bytes held, graph nodes, and for s <= 4, <= 8, <= 16
+ * (0, Gram chunk rows) of an FP64 plan (tuned: 6 ints; the chunk rows are the same for
+ * all; a zero stands for the panel width, which is chosen for each Gram). */
 int orth_gb300_batch_info(const orth_gb300_batch *plan, long long *launches_per_run, long long *workspace_bytes,
                           int *graph_nodes, int *tuned);
 void orth_gb300_batch_destroy(orth_gb300_batch *plan);

@@ -43,11 +43,8 @@ namespace {
 
 constexpr int kTR = 256;                // TSQR tile rows for nc <= 32
 constexpr int kMaxS = 16;
-constexpr int kClasses = 3;             // s <= 4, s <= 8, s <= 16
 constexpr int kRowsLeast = 256;         // rows per Gram chunk: powers of two from here
 constexpr int kRowsMost = 32768;        // to here
-
-int class_of(int s) { return s <= 4 ? 0 : (s <= 8 ? 1 : 2); }
 
 struct Mat {
     i64 m, ld;
@@ -101,7 +98,6 @@ i64 part_doubles_of(i64 m, int n, int s, int rows) {
 struct BatchPlan {
     int count = 0;
     std::vector<Mat> mats;
-    int tb[kClasses] = {16, 16, 32};   // C columns of a Gram tile, for the report
     int rows = kRowsMost;              // per Gram chunk
     // device memory: workspace (per-matrix blocks + status) and the job blob
     void* ws = nullptr;
@@ -522,7 +518,6 @@ void pick_rows(BatchPlan& P) {
             if ((int)stages.size() <= i) stages.resize(i + 1);
             const i64 tiles = gram_batched_tile(na, b0, nb, &ta, &r);
             stages[i].push_back({M.m, r, tiles, (i64)na * nb});
-            if (i == M.p / 2) P.tb[class_of(M.s)] = r * (128 / ta);
         }
     double best = -1.0;
     for (int rows = kRowsMost; rows >= kRowsLeast; rows /= 2) {
@@ -694,7 +689,7 @@ int orth_gb300_batch_info(const orth_gb300_batch* h, long long* launches_per_run
     if (P.staged && workspace_bytes) split_staged_info(P.staged, nullptr, workspace_bytes, nullptr, nullptr);
     if (graph_nodes) *graph_nodes = P.graph_nodes;
     if (tuned)
-        for (int c = 0; c < kClasses; ++c) { tuned[2 * c] = P.tb[c]; tuned[2 * c + 1] = P.rows; }
+        for (int c = 0; c < 3; ++c) { tuned[2 * c] = 0; tuned[2 * c + 1] = P.rows; }   // (s <= 4, <= 8, <= 16)
     return 0;
 }
 

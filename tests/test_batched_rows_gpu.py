@@ -49,3 +49,21 @@ def test_rows_and_bits(lib, name):
             orth.set_gram_chunk_rows(0)
         assert rc == 0
         assert torch.equal(Q, dX[b]) and torch.equal(R, dR[b])
+
+
+def test_report_and_tune_flag(lib):
+    """The report has no panel width (it differs from Gram to Gram), and the flag changes nothing."""
+    torch = pytest.importorskip("torch")
+    shapes = BATCHES["late steps of one matrix"]
+    X = [torch.zeros((n, m), dtype=torch.float64, device="cuda") for m, n, _ in shapes]
+    R = [torch.zeros((n, n), dtype=torch.float64, device="cuda") for _, n, _ in shapes]
+    infos = []
+    for tune in (False, True):
+        plan = orth.Batch([m for m, _, _ in shapes], [n for _, n, _ in shapes], [s for _, _, s in shapes],
+                          [x.data_ptr() for x in X], [r.data_ptr() for r in R], tune=tune,
+                          stream=torch.cuda.current_stream().cuda_stream)
+        assert plan.rc == 0
+        infos.append(plan.info())
+        plan.close()
+    assert infos[0] == infos[1]
+    assert all(v[0] == 0 for v in infos[0]["tuned"].values())
