@@ -451,7 +451,7 @@ int enqueue_all(BatchPlan& P, cudaStream_t st) {
                 break;
             }
             case kStSmall:
-                rc = launch_step_batched((const StepJob*)(base + S.job_off), S.njobs, 2 * kMaxS, st);
+                rc = launch_step_batched((const StepJob*)(base + S.job_off), S.njobs, st);
                 break;
             case kStUpd:
                 rc = launch_update_batched((const UpdJob*)(base + S.job_off), prefix, S.njobs, S.items, st);

@@ -85,8 +85,8 @@ struct StepJob {
     const int* gate = nullptr;   // if not null and *gate is 0, launch_step's kernel does nothing
 };
 int launch_step(const StepJob& J, cudaStream_t st);
-// One job per matrix; nmax: the largest ny + nz, at most 32.
-int launch_step_batched(const StepJob* jobs, int njobs, int nmax, cudaStream_t st);
+// One job per matrix, ny and nz at most 16 each.
+int launch_step_batched(const StepJob* jobs, int njobs, cudaStream_t st);
 
 // R[0:K, c0:c0+ny] = A + B Sd and R[c0:c0+ny, c0:] = Yd Sd (mode 0; Sd, Yd ny x ny,
 // upper, ld ny), or A + B and upper(Yd) (mode 1).

@@ -521,15 +521,19 @@ int launch_step(const StepJob& J, cudaStream_t st) {
     return launch_clustered(step_kernel<8>, 8, 8, step_smem_bytes(n, J.ny, 8), true, st, args);
 }
 
-// Batched: nmax = the largest ny + nz (<= 32). Enough CTAs per job to spread a small
-// batch over the SMs; one each once the jobs alone fill them.
-int launch_step_batched(const StepJob* jobs, int njobs, int nmax, cudaStream_t st) {
+// Batched: enough CTAs per job to spread a small batch over the SMs; one each once the
+// jobs alone fill them. Shared memory for the widest job a batch of blocks of up to 16
+// columns can have.
+int launch_step_batched(const StepJob* jobs, int njobs, cudaStream_t st) {
     if (njobs <= 0) return 0;
-    if (nmax < 1 || nmax > 32) return (int)cudaErrorInvalidValue;
+    constexpr int N = 32, NY = 16;
     void* args[1] = {(void*)&jobs};
-    if (njobs <= 64) return launch_clustered(step_batched<8>, (unsigned)njobs * 8, 8, step_smem_bytes(nmax, nmax / 2, 8), false, st, args);
-    if (njobs <= 512) return launch_clustered(step_batched<2>, (unsigned)njobs * 2, 2, step_smem_bytes(nmax, nmax / 2, 2), false, st, args);
-    return launch_clustered(step_batched<1>, (unsigned)njobs, 1, step_smem_bytes(nmax, nmax / 2, 1), false, st, args);
+    auto launch = [&](auto kernel, int ctas) {
+        return launch_clustered(kernel, (unsigned)(njobs * ctas), ctas, step_smem_bytes(N, NY, ctas), false, st, args);
+    };
+    if (njobs <= 64) return launch(step_batched<8>, 8);
+    if (njobs <= 512) return launch(step_batched<2>, 2);
+    return launch(step_batched<1>, 1);
 }
 
 int launch_rblock(double* R, int ldR, int c0, int K, int ny, const double* A, int lda, const double* B, int ldb,

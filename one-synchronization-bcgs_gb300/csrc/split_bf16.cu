@@ -2160,7 +2160,7 @@ int enqueue_wave(SplitStaged& S, SWave& W, cudaStream_t st) {
                                                        L.items, st);
                 break;
             case kSSmall:
-                rc = launch_step_batched(reinterpret_cast<const StepJob*>(jb + L.job_off), L.njobs, 32, st);
+                rc = launch_step_batched(reinterpret_cast<const StepJob*>(jb + L.job_off), L.njobs, st);
                 break;
             case kSBbuild:
                 bbuild_batched<<<items, BB_THREADS, 0, st>>>(reinterpret_cast<const BbuildJob*>(jb + L.job_off), pre, L.njobs);
