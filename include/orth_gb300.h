@@ -228,10 +228,11 @@ int orth_gb300_split_slice_dev(long long m, int n, const double *dX, long long l
 
 /*
  * Rows per chunk of the FP64 Gram's fixed-order reduction (0 = the default policy:
- * the most chunks whose 16-column strip CTAs all fit on the SMs in one wave, at
- * least 256 rows each). Results depend on the chunking only through the order
- * of the final sum; a batched plan with the same chunk rows reproduces the
- * single-matrix results bit for bit.
+ * as many chunks as lay the output tiles' CTAs on the SMs in whole rounds in the least
+ * estimated time, at least 64 rows each). Results depend on the chunking only through
+ * the order of the sums; a batched plan with the same chunk rows reproduces the
+ * single-matrix results bit for bit. The Gram by which the TSQR checks a panel of up to
+ * 32 columns keeps its own chunks.
  */
 void orth_gb300_set_gram_chunk_rows(long long rows);
 

@@ -32,8 +32,9 @@ __host__ __device__ inline i64 ceil_div(i64 a, i64 b) { return (a + b - 1) / b; 
 // SMs while this one runs (programmatic stream serialization). Each kernel so launched
 // starts with chain_enter: it waits until the grids before it in the stream have
 // completed and their writes are visible, and then lets its own successor be set up, so
-// that at most one grid waits at a time. Every kernel of this library that runs on the
-// caller's stream begins so, whichever way it is launched.
+// that at most one grid waits at a time. So begins every kernel that launch_chained or
+// launch_spread may launch; the others (batched, metrics, diagnostics) are launched plainly
+// and neither start early nor let their successors.
 #ifdef __CUDACC__
 __device__ __forceinline__ void chain_enter() {
     asm volatile("griddepcontrol.wait;" ::: "memory");

@@ -110,11 +110,6 @@ __device__ __forceinline__ void apply_own(double* a, int c, int nc, const double
     else if (c < nc) apply_cols<RPL, 1>(a, c, W, v, t, lane);
 }
 
-template <int W>
-__device__ __forceinline__ void tile_sync() {
-    if (W == 1) __syncwarp(); else __syncthreads();
-}
-
 // Whether d is a positive number of ordinary size, 2^-900 .. 2^900 (an integer test: a
 // comparison would be one more FP64 instruction).
 __device__ __forceinline__ bool ordinary(double d) {
@@ -208,9 +203,7 @@ __device__ __forceinline__ double load_reflector(const double* a, const double* 
 // Measured (before: one, four or 16 warps a tile with fixed groups of four columns,
 // unit-pivot reflectors with a division each, tau v published beside v): a level of one
 // tile of 256 x 10, whose chain of reflectors nothing hides, 124 -> 53 us; the leaves of
-// 10^5 x 10 133 -> 76 us, of 2^21 x 16 2.81 -> 2.70 ms, of 2^19 x 64 11.9 -> 11.3 ms, where
-// the FP64 pipe is active 86 %, 84 % and 76 % of the time at 16, 32 and 64 columns (4, 8 and
-// 16 warps); with half the warps 2.40 ms at 2^21 x 16.
+// 10^5 x 10 133 -> 76 us, of 2^21 x 16 2.81 -> 2.70 ms with 4 warps, 2.40 with 2.
 template <int NC, int W>
 __device__ void tsqr_tile_body(const double* A, i64 lda, i64 rows, int nc, double* Q, i64 ldq,
                                double* __restrict__ Rst, i64 ldr, i64 tile, double* smem) {
@@ -220,10 +213,10 @@ __device__ void tsqr_tile_body(const double* A, i64 lda, i64 rows, int nc, doubl
     double* tau = smem + TR * NC;
     double* rdiag = tau + NC;
     const int lane = threadIdx.x & 31;
-    const int warp = W == 1 ? 0 : (int)(threadIdx.x >> 5);
+    const int warp = (int)(threadIdx.x >> 5);
     const i64 row0 = tile * TR;
     const i64 h = min((i64)TR, rows - row0);
-    tile_sync<W>();
+    __syncthreads();
     for (int c = warp; c < nc; c += W)
 #pragma unroll
         for (int i = 0; i < RPL; ++i) {
@@ -238,7 +231,7 @@ __device__ void tsqr_tile_body(const double* A, i64 lda, i64 rows, int nc, doubl
         for (int i = 0; i < RPL; ++i) x[i] = a[lane + 32 * i];
         make_reflector<RPL>(a, tau, rdiag, 0, lane, x);
     }
-    tile_sync<W>();
+    __syncthreads();
 
     for (int j = 0; j + 1 < nc; ++j) {
         const double t = load_reflector<RPL>(a, tau, j, lane, v);
@@ -259,14 +252,14 @@ __device__ void tsqr_tile_body(const double* A, i64 lda, i64 rows, int nc, doubl
             c += W;
         }
         if (live) apply_own<RPL, W>(a, c, nc, v, t, lane);
-        tile_sync<W>();
+        __syncthreads();
     }
     // R to the stack (upper, lower zero).
     for (int e = threadIdx.x; e < nc * nc; e += 32 * W) {
         const int i = e % nc, c = e / nc;
         Rst[tile * nc + i + (i64)c * ldr] = i < c ? a[c * TR + i] : (i == c ? rdiag[c] : 0.0);
     }
-    tile_sync<W>();
+    __syncthreads();
     // Explicit Q in place (dorg2r): for j = nc-1 .. 0, apply H_j to columns j+1.. and set
     // column j to (I - t v v^T) e_j (its owner, after the barrier that ends every
     // warp's reading of reflector j).
@@ -274,7 +267,7 @@ __device__ void tsqr_tile_body(const double* A, i64 lda, i64 rows, int nc, doubl
         const double t = load_reflector<RPL>(a, tau, j, lane, v);
         if (__double_as_longlong(t) != 0LL)
             apply_own<RPL, W>(a, j + 1 + ((warp - (j + 1)) % W + W) % W, nc, v, t, lane);
-        tile_sync<W>();
+        __syncthreads();
         if (j % W == warp) {
             const double s = -t * __shfl_sync(0xffffffffu, j < 32 ? v[0] : v[1], j & 31);
 #pragma unroll

@@ -8,8 +8,8 @@
 // dgemm and dtrsm are one pass. Bound by the FP64 pipe: an instruction of one warp takes
 // its quarter of the SM for 64 clocks, so the time is K NC + NC^2 / 2 instructions per 32
 // rows, on the SM quarter that has the most of them. Hence
-//   * there is code for every width up to 16 and every fourth beyond (10 columns in 16
-//     accumulators cost 60 % more);
+//   * there is code for every width up to 16, every fourth to 32 and every eighth beyond (10
+//     columns in 16 accumulators cost 60 % more);
 //   * up to kSplitRows rows the warps of a CTA share 32 rows and split K four ways
 //     (SPLIT), because 32-row units of the whole K are too coarse for the 608 SM
 //     quarters: 10^5 rows are 5.1 units each, so some do 6.
