@@ -82,7 +82,7 @@ struct StepJob {
     // T is only defined if it is.
     int* ok = nullptr;
     double ok_limit = 0.0;
-    const int* gate = nullptr;   // if not null and *gate is 0, launch_step's kernel does nothing
+    const int* gate = nullptr;   // K = 0, nz = 0: if not null and *gate is 0, nothing is done
 };
 int launch_step(const StepJob& J, cudaStream_t st);
 // One job per matrix, ny and nz at most 16 each.

@@ -129,8 +129,9 @@ __device__ __forceinline__ double step_entry(const StepJob& J, int r, int c, int
            (((g[0] + g[1]) + (g[2] + g[3])) + ((g[4] + g[5]) + (g[6] + g[7])));
 }
 
-// One job by a cluster of C CTAs (rank = this CTA's), C | kGroups.
-template <int C>
+// One job by a cluster of C CTAs (rank = this CTA's), C | kGroups. PANEL: of a checked TSQR
+// panel (J.ok, J.gate), in code of its own so that the other steps carry none of it.
+template <int C, bool PANEL = false>
 __device__ void step_body(const StepJob& J, int rank, double* sm) {
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int ny = J.ny, nz = J.nz, n = ny + nz;
@@ -229,7 +230,7 @@ __device__ void step_body(const StepJob& J, int rank, double* sm) {
     // pivot go to slot r & 1 (the carried identity has 1 at c = r). A pivot that is
     // not a positive number of ordinary size ends the fast path (an integer test: a
     // comparison would be one more FP64 instruction).
-    const bool carry = J.Uinv != nullptr || J.ok != nullptr;
+    const bool carry = J.Uinv != nullptr || (PANEL && J.ok != nullptr);
     // (Loops over the columns are kept rolled: an FP64 instruction that is only
     // predicated off still takes its 64 clocks.)
     auto publish = [&](int r, double d, double x0) {
@@ -322,7 +323,7 @@ __device__ void step_body(const StepJob& J, int rank, double* sm) {
             }
         }
         __syncthreads();
-        if (J.ok != nullptr) {
+        if (PANEL && J.ok != nullptr) {
             // Row r of a's lower part is row r of U^{-T}: the sum of G_cc (U^{-T})_rc^2, in a
             // fixed order. (A sum that is Inf or NaN is not within the limit.)
             __shared__ double s_norm[ST_WARPS];
@@ -341,7 +342,7 @@ __device__ void step_body(const StepJob& J, int rank, double* sm) {
                 *J.ok = p <= J.ok_limit;
             }
         }
-    } else if (J.ok != nullptr) {
+    } else if (PANEL && J.ok != nullptr) {
         if (tid == 0) *J.ok = 0;
     } else {
         // A pivot out of range: the same factorization by dot products. At a
@@ -438,8 +439,14 @@ template <int C>
 __global__ void __launch_bounds__(ST_THREADS) step_kernel(const __grid_constant__ StepJob job) {
     extern __shared__ double sm[];
     chain_enter();
-    if (job.gate != nullptr && *job.gate == 0) return;   // (every CTA of the cluster reads the same)
     step_body<C>(job, C == 1 ? 0 : (int)blockIdx.x, sm);
+}
+
+__global__ void __launch_bounds__(ST_THREADS) step_panel_kernel(const __grid_constant__ StepJob job) {
+    extern __shared__ double sm[];
+    chain_enter();
+    if (job.gate != nullptr && *job.gate == 0) return;
+    step_body<1, true>(job, 0, sm);
 }
 
 // Batched form: CTAs [b C, (b + 1) C) run job b.
@@ -504,7 +511,7 @@ int launch_clustered(K kernel, unsigned grid, int ctas, size_t smem, bool chaine
 bool step_valid(const StepJob& J) {
     return J.ny >= 1 && J.ny <= SMAX && J.nz >= 0 && J.nz <= SMAX && J.K >= 0 && J.G != nullptr && J.T != nullptr &&
            (J.nz == 0 || J.S != nullptr) && (!J.scaled || J.nz == 0 || J.Sd != nullptr) &&
-           (J.ok == nullptr || (J.K == 0 && J.nz == 0));
+           ((J.ok == nullptr && J.gate == nullptr) || (J.K == 0 && J.nz == 0));
 }
 
 }  // namespace
@@ -516,6 +523,8 @@ int launch_step(const StepJob& J, cudaStream_t st) {
     if (!step_valid(J)) return (int)cudaErrorInvalidValue;
     const int n = J.ny + J.nz;
     void* args[1] = {const_cast<StepJob*>(&J)};
+    if (J.ok != nullptr || J.gate != nullptr)
+        return launch_clustered(step_panel_kernel, 1, 1, step_smem_bytes(n, J.ny, 1), true, st, args);
     if (J.K <= kTileRows && (i64)trap_size(n, n) * J.K <= 8192)
         return launch_clustered(step_kernel<1>, 1, 1, step_smem_bytes(n, J.ny, 1), true, st, args);
     return launch_clustered(step_kernel<8>, 8, 8, step_smem_bytes(n, J.ny, 8), true, st, args);
