@@ -114,7 +114,7 @@ __device__ __forceinline__ void r_diag(double* R, int ldR, int c0, int ny, const
 }
 
 // Entry e of the right-hand side: G[K + r, c] minus the groups' sums, group by group
-// in a fixed tree.
+// in a fixed tree. (Not for the entries of a breakdown: see the end of step_body.)
 template <int C>
 __device__ __forceinline__ double step_entry(const StepJob& J, int r, int c, int e, int E, double* gs) {
     double g[kGroups];
@@ -255,6 +255,7 @@ __device__ void step_body(const StepJob& J, int rank, double* sm) {
     const int slot = warp == 0 ? -1 : (warp == 4 ? 6 : (warp > 4 ? warp - 2 : warp - 1)) * 4 + (lane >> 3);
     const int l8 = lane & 7;
     bool fast = s_stop[0] == 0;
+    int stop = 0;   // the pivot that ended the fast path
     for (int j = 0; j < nr && fast; ++j) {
         const double* pr = a + j * ld;
         const double* t = s_t + (j & 1) * n;
@@ -299,7 +300,8 @@ __device__ void step_body(const StepJob& J, int rank, double* sm) {
         }
         __syncthreads();
         // Slot (j + 1) & 1 is next written after the barrier that ends step j + 1.
-        if (j + 1 < nr) fast = s_stop[(j + 1) & 1] == 0;
+        stop = j + 1;
+        if (stop < nr) fast = s_stop[stop & 1] == 0;
     }
 
     if (fast) {
@@ -349,11 +351,22 @@ __device__ void step_body(const StepJob& J, int rank, double* sm) {
         // breakdown (a pivot <= 0) the factor keeps the rows before it, and the rows
         // from it on hold the matrix that was to be factored, as dpotrf leaves
         // them; what follows goes on with that factor. Not a path for speed.
+        // The right-hand side is formed anew, each entry one chain that starts at G's:
+        // where a column is noise next to those before it, G minus a rounded sum is a
+        // small multiple of G's last bit, often 0, and dividing by that pivot would
+        // end in Inf and NaN; the chain keeps the products' lower bits. A pivot <= 0 of either
+        // form is reported: that of the rounded sums is the reference's (dgemm, then dpotrf).
+        int bad = a[stop * ld + stop] <= 0.0 ? stop + 1 : 0;   // 1-based pivot (thread 0's counts)
         __syncthreads();
         for (int e = tid; e < E; e += ST_THREADS) {
             int r, c;
             trap_rc(e, nr, r, c);
-            a[r * ld + c] = step_entry<C>(J, r, c, e, E, gs);
+            const double* x = J.G + (i64)r * J.ldg;
+            const double* y = J.G + (i64)c * J.ldg;
+            double v = __ldg(y + J.K + r);
+#pragma unroll 4
+            for (int l = 0; l < J.K; ++l) v = fma(-__ldg(x + l), __ldg(y + l), v);
+            a[r * ld + c] = v;
         }
         for (int e = tid; e < n * n; e += ST_THREADS) {
             const int r = e / n, c = e % n;
@@ -361,8 +374,8 @@ __device__ void step_body(const StepJob& J, int rank, double* sm) {
             if (r >= nr && c >= r) a[r * ld + c] = c == r ? 1.0 : 0.0;
         }
         __syncthreads();
-        // Upper Cholesky of rows and columns [o, o + k): false at a breakdown.
-        auto chol = [&](int o, int k, int step) {
+        // Upper Cholesky of rows and columns [o, o + k), up to a breakdown.
+        auto chol = [&](int o, int k) {
             for (int j = o; j < o + k; ++j) {
                 __syncthreads();
                 if (tid == 0) {
@@ -370,10 +383,7 @@ __device__ void step_body(const StepJob& J, int rank, double* sm) {
                     for (int i = o; i < j; ++i) d = fma(-a[i * ld + j], a[i * ld + j], d);
                     s_stop[0] = d <= 0.0;
                     a[j * ld + j] = d <= 0.0 ? d : sqrt(d);
-                    if (d <= 0.0 && J.status != nullptr && J.status[0] == 0) {
-                        J.status[0] = step;
-                        J.status[1] = j - o + 1;
-                    }
+                    if (d <= 0.0 && (bad == 0 || j < bad)) bad = j + 1;
                 }
                 __syncthreads();
                 if (s_stop[0] != 0) break;
@@ -385,7 +395,7 @@ __device__ void step_body(const StepJob& J, int rank, double* sm) {
             }
             __syncthreads();
         };
-        chol(0, ny, J.step);
+        chol(0, ny);
         // S_mid = T^{-T} (G_mid - Y^T Z), one column per thread.
         for (int c = ny + tid; c < n; c += ST_THREADS)
             for (int i = 0; i < ny; ++i) {
@@ -402,7 +412,11 @@ __device__ void step_body(const StepJob& J, int rank, double* sm) {
                 for (int l = 0; l < ny; ++l) v = fma(-a[l * ld + r], a[l * ld + c], v);
                 a[r * ld + c] = v;
             }
-            chol(ny, nz, J.step + 1);
+            chol(ny, nz);
+        }
+        if (tid == 0 && bad != 0 && J.status != nullptr && J.status[0] == 0) {
+            J.status[0] = J.step + (bad > ny ? 1 : 0);
+            J.status[1] = bad > ny ? bad - ny : bad;
         }
         for (int e = tid; e < n * n; e += ST_THREADS) {
             const int r = e / n, c = e % n;

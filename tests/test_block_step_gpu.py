@@ -59,3 +59,29 @@ def test_block_step_pivots_out_of_range(lib, variant, s, n, scale):
     tol = qr_tolerance(KAPPA)
     assert np.max(np.abs(Q1 - Q2)) <= tol
     assert np.max(np.abs(R1 - R2 / scale)) <= tol * np.max(np.abs(R1))
+
+
+@pytest.mark.parametrize("m,n,s", [(300, 64, 8), (4000, 128, 16), (1000, 48, 1), (3000, 96, 32)])
+@pytest.mark.parametrize("variant", ["bcgsi2P1s", "bcgspipi2"])
+@pytest.mark.parametrize("precision", ["fp64", "split7"])
+@pytest.mark.parametrize("kappa", [1e10, 1e12])
+def test_after_a_breakdown(lib, variant, precision, m, n, s, kappa):
+    """Beyond the Pythagorean Cholesky's range the status reports the breakdown, and Q stays
+    finite with columns of ordinary size: the pivots of columns that are noise are noise,
+    but not exact zeros, which would end in NaN. The second pass of each block (or the
+    lagged one) brings its columns back to norm 1 up to sqrt(s) where its Cholesky, too,
+    breaks down part way."""
+    prec = orth.FP64 if precision == "fp64" else orth.SPLIT_BF16
+    assert orth.set_host_precision(prec) == 0
+    norms = []
+    try:
+        for seed in range(9):
+            X = inputs.graded_host(m, n, kappa, seed=seed)
+            Q, R, rc, st = orth.qr(variant, X, s)
+            assert rc == 0 and st["cuda_error"] == 0
+            assert s == 1 or st["breakdown_step"] > 0
+            assert np.isfinite(Q).all() and np.isfinite(np.triu(R)).all()
+            norms.append(np.max(np.abs(np.linalg.norm(Q, axis=0) - 1.0)))
+    finally:
+        orth.set_host_precision(orth.FP64)
+    assert np.median(norms) <= np.sqrt(s)
