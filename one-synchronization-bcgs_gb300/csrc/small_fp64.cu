@@ -449,14 +449,18 @@ __device__ void step_body(const StepJob& J, int rank, double* sm) {
     if constexpr (C > 1) cg::this_cluster().sync();
 }
 
+// CTAs per SM given so that the registers come out as they are fastest. The cluster of eight
+// is left to the compiler (64 registers; with 112 bcgsi2P1s split at 2^19 x 512, s = 64,
+// 34.6 -> 34.7 ms); the others would be spilled to 64 or 80 (a batch of 96 in the split form
+// 10.59 -> 10.63 ms), except the batched form with many jobs, three of whose CTAs share an SM.
 template <int C>
-__global__ void __launch_bounds__(ST_THREADS) step_kernel(const __grid_constant__ StepJob job) {
+__global__ void __launch_bounds__(ST_THREADS, C == 8 ? 0 : 1) step_kernel(const __grid_constant__ StepJob job) {
     extern __shared__ double sm[];
     chain_enter();
     step_body<C>(job, C == 1 ? 0 : (int)blockIdx.x, sm);
 }
 
-__global__ void __launch_bounds__(ST_THREADS) step_panel_kernel(const __grid_constant__ StepJob job) {
+__global__ void __launch_bounds__(ST_THREADS, 1) step_panel_kernel(const __grid_constant__ StepJob job) {
     extern __shared__ double sm[];
     chain_enter();
     if (job.gate != nullptr && *job.gate == 0) return;
@@ -465,7 +469,7 @@ __global__ void __launch_bounds__(ST_THREADS) step_panel_kernel(const __grid_con
 
 // Batched form: CTAs [b C, (b + 1) C) run job b.
 template <int C>
-__global__ void __launch_bounds__(ST_THREADS) step_batched(const StepJob* __restrict__ jobs) {
+__global__ void __launch_bounds__(ST_THREADS, C == 1 ? 3 : 1) step_batched(const StepJob* __restrict__ jobs) {
     extern __shared__ double sm[];
     const StepJob J = jobs[blockIdx.x / C];
     step_body<C>(J, (int)(blockIdx.x % C), sm);
